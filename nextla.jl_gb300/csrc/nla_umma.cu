@@ -10,13 +10,13 @@
 // arithmetic on the FP64 bit pattern, so it issues no FP64 instruction.
 // A Float16 operand of the plain Float16 path is staged as one unscaled slice.
 //
-// The GEMM kernel (one 128 x 128 output tile per CTA, 6 warps):
+// The GEMM kernel (one 128 x 128 output tile per CTA, 11 warps):
 //   warp 0      TMA producer: per 64-wide K block, one 128 x 64 box per slice
 //               of each operand (128-byte swizzle) into a multi-stage ring;
 //   warp 1      allocates TMEM, and one elected lane issues tcgen05.mma for
 //               every slice pair (p, q) kept by the split, accumulating pairs
 //               of equal weight p + q in the same FP32 TMEM accumulator;
-//   warps 2-5   epilogue: tcgen05.ld of the accumulators, combination of the
+//   warps 2-9   epilogue: tcgen05.ld of the accumulators, combination of the
 //               weights in FP32, and the update of C (one FP64 operation per
 //               element for FP64 outputs; the power-of-two scale is applied
 //               to the exponent bits).
@@ -45,13 +45,14 @@ constexpr int BM = 128;
 constexpr int BN = 128;
 constexpr int BK = 64;                     // 64 16-bit elements = one 128-byte swizzle row
 constexpr int TILE_BYTES = BM * BK * 2;    // 16 KiB per slice tile (BN == BM)
-constexpr int GEMM_THREADS = 224;  // A producer, MMA, 4 epilogue warps, B producer
+constexpr int GEMM_THREADS = 352;  // A producer, MMA, 8 epilogue warps, B producer
 constexpr int MAX_PAIRS = 16;
 constexpr int MAX_ACC = 4;
 constexpr int SENTINEL_EXP = -2139062144;  // 0x80808080: "no element seen"
 constexpr int NONFINITE_EXP = 0x7fffffff;
 
 enum Epi { EPI_F64 = 0, EPI_F16 = 1 };
+constexpr int EPI_COLS = 16;  // columns of C per batch of epilogue loads
 
 struct GemmParams {
   int M, N;
@@ -76,12 +77,15 @@ struct GemmParams {
   int producers;  // TMA-issuing warps: 2 (A and B apart) or 1 (warp 0 loads both)
 };
 
+// The rare cases of scaled_double (subnormal or overflowing results), out of line.
+__device__ __noinline__ double scaled_double_slow(float v, int e) { return ldexp((double)v, e); }
+
 __device__ __forceinline__ double scaled_double(float v, int e) {
   const uint32_t fb = __float_as_uint(v);
   if ((fb << 1) == 0) return __longlong_as_double((unsigned long long)(fb >> 31) << 63);
   const int E = (int)((fb >> 23) & 0xFF);
   const int de = E - 127 + 1023 + e;
-  if (E == 0 || E == 255 || de <= 0 || de >= 2047) return ldexp((double)v, e);
+  if (E == 0 || E == 255 || de <= 0 || de >= 2047) return scaled_double_slow(v, e);
   const unsigned long long db = ((unsigned long long)(fb >> 31) << 63) | ((unsigned long long)de << 52) |
                                 ((unsigned long long)(fb & 0x7FFFFFu) << 29);
   return __longlong_as_double(db);
@@ -192,53 +196,78 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       umma::mbar_wait(umma::smem_u32(drain), 0, &s_abort, &g_device_error, 3, false);
     }
   } else {
-    // Epilogue warps 2..5 own TMEM lane quadrants (warp % 4).
+    // Epilogue warps 2..9: TMEM lane quadrant warp % 4, 64 of the tile's 128
+    // columns each.  The kernel's time at short K is the latency of this C
+    // update: a store to C may alias a later load as far as the compiler
+    // knows, so element-wise updates wait for memory once per column.  Here
+    // the loads of EPI_COLS columns are issued together, the first batch
+    // before the accumulators are ready and every next one before the
+    // stores of the batch in hand.
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int i = m0 + row;
+    const int cbase = ((warp - 2) >> 2) * (BN / 2);
+    using TC = typename std::conditional<EPI == EPI_F64, double, __half>::type;
+    TC* C = static_cast<TC*>(p.C) + i;
+    TC cv[EPI_COLS], nv[EPI_COLS];  // the batch in hand and the next one
+    int ej[EPI_COLS], ne[EPI_COLS];
+    auto fetch = [&](int c0, TC (&v)[EPI_COLS], int (&e)[EPI_COLS]) {
+#pragma unroll
+      for (int j = 0; j < EPI_COLS; ++j) {
+        const int col = n0 + cbase + c0 + j;
+        const bool in = i < p.M && col < p.N;
+        v[j] = in ? C[(int64_t)col * p.ldc] : TC(0.0f);
+        if (EPI == EPI_F64) e[j] = in && p.eb != nullptr ? __ldg(p.eb + col) : 0;
+      }
+    };
+    fetch(0, cv, ej);
+    int ei = 0;
+    bool row_nan = false;
+    if (EPI == EPI_F64 && p.ea != nullptr && i < p.M) {
+      ei = __ldg(p.ea + i);
+      row_nan = ei == NONFINITE_EXP;
+      ei = max(ei, -4000);
+    }
     // tcgen05.ld is warp-collective: the lanes act on one shared verdict.
     const bool ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(accf), 0, &s_abort, &g_device_error, 4));
     umma::fence_after_sync();
     if (ok) {
-      const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16);
-      int ei = 0;
-      bool row_nan = false;
-      if (EPI == EPI_F64 && p.ea != nullptr && i < p.M) {
-        ei = p.ea[i];
-        row_nan = ei == NONFINITE_EXP;
-        ei = max(ei, -4000);
-      }
-      for (int c0 = 0; c0 < BN; c0 += 16) {
-        float v[16];
-        uint32_t r[16];
+      const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cbase;
+#pragma unroll 1
+      for (int c0 = 0; c0 < BN / 2; c0 += EPI_COLS) {
+        float v[EPI_COLS];
+        uint32_t r[EPI_COLS];
         umma::tmem_ld16(tq + (uint32_t)c0, r);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
+        for (int j = 0; j < EPI_COLS; ++j) v[j] = __uint_as_float(r[j]);
         for (int a = 1; a < p.nacc; ++a) {
           umma::tmem_ld16(tq + (uint32_t)(a * BN + c0), r);
           const float w = p.acc_w[a];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = fmaf(__uint_as_float(r[j]), w, v[j]);
+          for (int j = 0; j < EPI_COLS; ++j) v[j] = fmaf(__uint_as_float(r[j]), w, v[j]);
         }
+        if (c0 + EPI_COLS < BN / 2) fetch(c0 + EPI_COLS, nv, ne);
         if (i < p.M) {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int col = n0 + c0 + j;
+          for (int j = 0; j < EPI_COLS; ++j) {
+            const int col = n0 + cbase + c0 + j;
             if (col >= p.N) continue;
-            if (EPI == EPI_F64) {
-              double* cp = static_cast<double*>(p.C) + i + (int64_t)col * p.ldc;
-              int ej = p.eb != nullptr ? p.eb[col] : 0;
-              if (row_nan || ej == NONFINITE_EXP) {
-                *cp = __longlong_as_double(0x7ff8000000000000ull);
-              } else {
-                const double d = scaled_double(v[j], ei + max(ej, -4000) + p.exp_bias);
-                *cp = fma(p.alpha, d, *cp);
-              }
+            TC* cp = C + (int64_t)col * p.ldc;
+            if constexpr (EPI == EPI_F64) {
+              const int e = ej[j];
+              double out = __longlong_as_double(0x7ff8000000000000ll);
+              if (!row_nan && e != NONFINITE_EXP)
+                out = fma(p.alpha, scaled_double(v[j], ei + max(e, -4000) + p.exp_bias), cv[j]);
+              *cp = out;
             } else {
-              __half* cp = static_cast<__half*>(p.C) + i + (int64_t)col * p.ldc;
-              *cp = __float2half_rn(fmaf((float)p.alpha, v[j], __half2float(*cp)));
+              *cp = __float2half_rn(fmaf((float)p.alpha, v[j], __half2float(cv[j])));
             }
           }
+        }
+#pragma unroll
+        for (int j = 0; j < EPI_COLS; ++j) {
+          cv[j] = nv[j];
+          ej[j] = ne[j];
         }
       }
     }
