@@ -3,39 +3,20 @@
 //             (src/trsm.jl:5-150);
 //   func 'M': the triangular multiply of LeftLowerTRMM! ... RightUpperTRMM!
 //             (src/trmm.jl:43-389).
-// The shared device code and the canonical-form mapping are in nla_leaf.cuh.
-//   multiply: each thread forms one output row as a dot product with
-//             increasing k (the reference's order, src/trmm.jl:90-94), reading
-//             A through staged slabs and B from shared memory, and writes it
-//             straight to global memory (B was fully staged first, so the
-//             in-place update has no hazard).
+// The canonical-form mapping and the column-per-thread Float64 solve are in
+// nla_leaf.cuh, the strip kernel that runs every other block in
+// nla_leaf_strip.cuh.
 #include <mutex>
 
 #include <cstdlib>
 
 #include "nla_leaf.cuh"
+#include "nla_leaf_strip.cuh"
 
 namespace nla {
 namespace {
 
 using namespace leafdev;
-
-template <typename T, int CW>
-__global__ void __launch_bounds__(LEAF_THREADS) leaf_solve_kernel(LeafArgs g) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t c0 = (int64_t)blockIdx.x * CW;
-  const int ncols = (int)(g.m - c0 < CW ? g.m - c0 : CW);
-  solve_block<T, CW>(g, c0, ncols, smem_raw, typename Elem<T>::compute(1));
-}
-
-// Wide blocks of right-hand sides, one per thread in the panel solves.
-template <typename T, int CW>
-__global__ void __launch_bounds__(LEAF_THREADS) leaf_solve_wide_kernel(LeafArgs g) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int64_t c0 = (int64_t)blockIdx.x * CW;
-  const int ncols = (int)(g.m - c0 < CW ? g.m - c0 : CW);
-  solve_block_wide<T, CW>(g, c0, ncols, smem_raw, typename Elem<T>::compute(1));
-}
 
 template <int HALVES, int CW>
 __global__ void __launch_bounds__(CW * HALVES, 1) leaf_solve_cols_kernel(LeafArgs g) {
@@ -45,117 +26,8 @@ __global__ void __launch_bounds__(CW * HALVES, 1) leaf_solve_cols_kernel(LeafArg
   solve_cols_f64<HALVES, CW>(g, c0, ncols, smem_raw, 1.0);
 }
 
-// Canonical lower-left multiply: X := L X for CW columns.
-template <typename T, int CW>
-__global__ void __launch_bounds__(LEAF_THREADS) leaf_mult_kernel(LeafArgs g) {
-  using Tc = typename Elem<T>::compute;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  Tc* X = reinterpret_cast<Tc*>(smem_raw);  // n x CW (original B)
-  Tc* slab = X + (size_t)g.n * CW;          // 128 x 33
-
-  const int64_t c0 = (int64_t)blockIdx.x * CW;
-  const int ncols = (int)(g.m - c0 < CW ? g.m - c0 : CW);
-  const int n = g.n;
-  T* Bp = static_cast<T*>(g.B);
-
-  load_block<T, Tc, CW>(g, X, c0, ncols);
-  __syncthreads();
-
-  constexpr int CT = CW / 4;
-  const int tr = threadIdx.x & 31, tc = threadIdx.x >> 5;
-  for (int r0 = 0; r0 < n; r0 += LEAF_THREADS) {
-    const int rows = min(LEAF_THREADS, n - r0);
-    const int kmax = min(n, r0 + rows);  // k <= r
-    Tc acc[4][CT];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < CT; ++c) acc[i][c] = Tc(0);
-    for (int k0 = 0; k0 < kmax; k0 += PANEL) {
-      const int kw = min(PANEL, kmax - k0);
-      const bool unit = g.unit != 0;
-      stage_slab<LEAF_THREADS, T>(g, slab, r0, rows, k0, kw, [unit](int i, int j) { return unit ? j < i : j <= i; });
-      __syncthreads();
-      tile_product<Tc, CW>(slab, X + (size_t)k0 * CW, kw, rows, acc);
-      __syncthreads();
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int r = tr + 32 * i;
-      if (r < rows) {
-#pragma unroll
-        for (int c = 0; c < CT; ++c)
-          if (tc * CT + c < ncols) {
-            // A unit diagonal contributes the row's own value of X.
-            const Tc v = g.unit ? acc[i][c] + X[(size_t)(r0 + r) * CW + tc * CT + c] : acc[i][c];
-            Elem<T>::store(Bp + b_off<T>(g, r0 + r, c0 + tc * CT + c), v);
-          }
-      }
-    }
-  }
-}
-
-template <typename T, int CW>
-size_t leaf_smem(char func, int n) {
-  using Tc = typename Elem<T>::compute;
-  size_t elems = (size_t)n * CW + (size_t)LEAF_THREADS * SLAB_PAD;
-  if (func == 'S') elems += (size_t)n + (size_t)PANEL * SLAB_PAD;
-  return elems * sizeof(Tc);
-}
-
-template <typename T, int CW>
-int leaf_smem_attr() {
-  static std::once_flag once;
-  static cudaError_t st = cudaSuccess;
-  std::call_once(once, [] {
-    st = cudaFuncSetAttribute(leaf_solve_kernel<T, CW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    if (st == cudaSuccess)
-      st = cudaFuncSetAttribute(leaf_mult_kernel<T, CW>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
-  return st == cudaSuccess ? NLA_OK : cuda_status(st, "cudaFuncSetAttribute(leaf kernels)");
-}
-
-template <typename T, int CW>
-int launch_leaf_t(char func, const LeafArgs& g, cudaStream_t s) {
-  const size_t smem = leaf_smem<T, CW>(func, g.n);
-  const int64_t grid = (g.m + CW - 1) / CW;
-  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf: too many right-hand sides");
-  if (smem > 200 * 1024) return fail(NLA_ERR_UNSUPPORTED, "leaf: shared memory plan too large");
-  NLA_TRY((leaf_smem_attr<T, CW>()));
-  // n^2 m flops per solve or multiply (the benchmark's convention); bytes:
-  // the triangle once plus B read and written.
-  TraceScope trace(func == 'S' ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, s, (double)g.n * g.n * (double)g.m,
-                   (double)sizeof(T) * ((double)g.n * (g.n + 1) / 2 + 2.0 * (double)g.n * g.m));
-  if (func == 'S')
-    leaf_solve_kernel<T, CW><<<(unsigned)grid, LEAF_THREADS, smem, s>>>(g);
-  else
-    leaf_mult_kernel<T, CW><<<(unsigned)grid, LEAF_THREADS, smem, s>>>(g);
-  NLA_CHECK_LAUNCH(func == 'S' ? "leaf_solve_kernel" : "leaf_mult_kernel");
-  return NLA_OK;
-}
-
-template <typename T, int CW>
-int launch_leaf_wide(const LeafArgs& g, cudaStream_t s) {
-  using Tc = typename Elem<T>::compute;
-  const size_t smem = leaf_solve_smem_elems(g.n, CW) * sizeof(Tc);
-  const int64_t grid = (g.m + CW - 1) / CW;
-  if (smem > 200 * 1024) return fail(NLA_ERR_UNSUPPORTED, "leaf: shared memory plan too large");
-  static std::once_flag once;
-  static cudaError_t st = cudaSuccess;
-  std::call_once(once, [] {
-    st = cudaFuncSetAttribute(leaf_solve_wide_kernel<T, CW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              200 * 1024);
-  });
-  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(leaf_solve_wide_kernel)");
-  TraceScope trace(NLA_K_LEAF_SOLVE, s, (double)g.n * g.n * (double)g.m,
-                   (double)sizeof(T) * ((double)g.n * (g.n + 1) / 2 + 2.0 * (double)g.n * g.m));
-  leaf_solve_wide_kernel<T, CW><<<(unsigned)grid, LEAF_THREADS, smem, s>>>(g);
-  NLA_CHECK_LAUNCH("leaf_solve_wide_kernel");
-  return NLA_OK;
-}
-
 // Threads per right-hand side of the Float64 column-per-thread leaf:
-// NLA_LEAF_COLS = 0 (use the panel-parallel kernels), 1 or 2 (default 2).
+// NLA_LEAF_COLS = 0 (use the strip kernel), 1 or 2 (default 2).
 int leaf_cols_mode() {
   static const int mode = [] {
     const char* v = getenv("NLA_LEAF_COLS");
@@ -208,33 +80,70 @@ int launch_leaf_cols2(const LeafArgs& g, cudaStream_t s) {
   }
 }
 
-// Wide solve blocks: the widest of 128/64/32 right-hand sides whose block
-// fits 128 KiB of shared memory and still gives two CTAs per SM; 0 when the
-// row-parallel kernel is the better choice (few right-hand sides).
-int wide_cols(int64_t n, int64_t m, size_t elem) {
-  if (m < 32) return 0;
-  const int64_t want = 2 * (int64_t)num_sms();
-  for (int cw : {128, 64, 32}) {
-    if ((size_t)n * cw * elem > 128 * 1024) continue;
-    if ((m + cw - 1) / cw >= want || cw == 32) return cw;
-  }
-  return 0;
+template <typename T, int PB, int NC, int WC, bool SOLVE>
+__global__ void __launch_bounds__(ST_THREADS) leaf_strip_kernel(const LeafArgs g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  strip_block<T, PB, NC, WC, SOLVE>(g, smem_raw);
 }
 
-template <typename T>
-int launch_solve_wide(const LeafArgs& g, int cw, cudaStream_t s) {
-  switch (cw) {
-    case 128: return launch_leaf_wide<T, 128>(g, s);
-    case 64: return launch_leaf_wide<T, 64>(g, s);
-    default: return launch_leaf_wide<T, 32>(g, s);
-  }
+constexpr size_t STRIP_SMEM_MAX = 200 * 1024;
+
+template <typename T, int PB, int NC, int WC, bool SOLVE>
+int launch_strip(const LeafArgs& g, cudaStream_t s) {
+  using Tc = typename Elem<T>::compute;
+  const size_t smem = strip_smem_elems<Tc>(g.n, PB, NC, WC) * sizeof(Tc);
+  constexpr int CW = 32 / PB * NC * WC;
+  const int64_t grid = (g.m + CW - 1) / CW;
+  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf: too many right-hand sides");
+  if (smem > STRIP_SMEM_MAX) return fail(NLA_ERR_UNSUPPORTED, "leaf: shared memory plan too large");
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  std::call_once(once, [] {
+    st = cudaFuncSetAttribute(leaf_strip_kernel<T, PB, NC, WC, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)STRIP_SMEM_MAX);
+  });
+  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(leaf_strip_kernel)");
+  // n^2 m flops per solve or multiply (the benchmark's convention); bytes:
+  // the triangle once plus B read and written.
+  TraceScope trace(SOLVE ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, s, (double)g.n * g.n * (double)g.m,
+                   (double)sizeof(T) * ((double)g.n * (g.n + 1) / 2 + 2.0 * (double)g.n * g.m));
+  leaf_strip_kernel<T, PB, NC, WC, SOLVE><<<(unsigned)grid, ST_THREADS, smem, s>>>(g);
+  NLA_CHECK_LAUNCH("leaf_strip_kernel");
+  return NLA_OK;
 }
 
-// Float64 register tiles wider than 32 columns do not fit the register file
-// without spilling, so Float64 uses 32-column blocks.
-template <>
-int launch_solve_wide<double>(const LeafArgs& g, int, cudaStream_t s) {
-  return launch_leaf_wide<double, 32>(g, s);
+// Right-hand sides per CTA: the width with the least ceil(CTAs / SMs) *
+// (width + c), where c is a strip's fixed time (the triangles' chains and
+// the staging of A) in columns' worth of its product: about one column in
+// Float64, whose product is bound by the DFMA pipe, and about 32 in Float32.
+// Float64 takes 16-row panels from 8 columns on (32-row triangles cost the
+// DFMA pipe more than the steps they save), Float32 always 32-row panels.
+// Measured against one warp-group CTA per 16 or 32 columns with 32-row
+// panels solved by one warp: Float64 96 x 24 97 -> 13 us, 256 x 256 560 ->
+// 42 us; Float32 256 x 8192 110 -> 47 us; Float16 256 x 4096 98 -> 41 us;
+// Float64 multiply 64 x 6144 115 -> 36 us.
+template <typename T, bool SOLVE>
+int launch_strips(const LeafArgs& g, cudaStream_t s) {
+  using Tc = typename Elem<T>::compute;
+  constexpr bool F64 = sizeof(Tc) == 8;
+  const int64_t sms = num_sms(), c = F64 ? 1 : 32;
+  int best = 0;
+  int64_t cost = 0;
+  for (int w : {64, 32, 16, 8, 4, 2}) {
+    if (F64 && w > 32) continue;
+    if (strip_smem_elems<Tc>(g.n, 32, w < 8 ? 1 : w / 8, w < 8 ? w : 8) * sizeof(Tc) > STRIP_SMEM_MAX && w > 2) continue;
+    const int64_t grid = (g.m + w - 1) / w, k = (grid + sms - 1) / sms * (w + c);
+    if (best == 0 || k < cost) best = w, cost = k;
+  }
+  switch (best) {
+    case 64:
+      if constexpr (!F64) return launch_strip<T, 32, 8, 8, SOLVE>(g, s);
+    case 32: return F64 ? launch_strip<T, 16, 2, 8, SOLVE>(g, s) : launch_strip<T, 32, 4, 8, SOLVE>(g, s);
+    case 16: return F64 ? launch_strip<T, 16, 1, 8, SOLVE>(g, s) : launch_strip<T, 32, 2, 8, SOLVE>(g, s);
+    case 8: return F64 ? launch_strip<T, 16, 1, 4, SOLVE>(g, s) : launch_strip<T, 32, 1, 8, SOLVE>(g, s);
+    case 4: return launch_strip<T, 32, 1, 4, SOLVE>(g, s);
+    default: return launch_strip<T, 32, 1, 2, SOLVE>(g, s);
+  }
 }
 
 }  // namespace
@@ -262,28 +171,23 @@ int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m
   }
   g.rev = uplo == 'U';
   if (func == 'S') {
-    // Float64 blocks of up to 128 rows with enough right-hand sides to fill
-    // the GPU: one right-hand side per thread, or two threads per right-hand
-    // side (NLA_LEAF_COLS=0 selects the panel-parallel kernels instead).
-    if (dtype == NLA_F64 && n <= COLS_MAX_N && m >= 8 * LEAF_THREADS && leaf_cols_mode() != 0)
+    // Float64 blocks of up to 128 rows where one wave of wide CTAs fits and
+    // strips of 32 columns would leave the last wave short: one right-hand
+    // side per thread, or two threads per right-hand side.  Measured at
+    // n = 64 (128) on 152 SMs, strips against columns: m = 8192 58 (174)
+    // against 70 (214) us, 14336 73 (235) against 78 (250), 16384 97 (315)
+    // against 83 (276), 20000 116 (383) against 174 (600).
+    // (NLA_LEAF_COLS=0 turns it off, NLA_LEAF_CW pins a width from m = 1024.)
+    const int64_t sms = num_sms();
+    const bool pinned = getenv("NLA_LEAF_CW") != nullptr && m >= 8 * LEAF_THREADS;
+    if (dtype == NLA_F64 && n <= COLS_MAX_N && ((m > 96 * sms && m <= 128 * sms) || pinned) && leaf_cols_mode() != 0)
       return leaf_cols_mode() == 1 ? launch_leaf_cols<1, LEAF_THREADS>(g, s) : launch_leaf_cols2(g, s);
-    const int cw = wide_cols(n, m, dtype == NLA_F64 ? 8 : 4);
-    if (cw) {
-      switch (dtype) {
-        case NLA_F64: return launch_solve_wide<double>(g, cw, s);
-        case NLA_F32: return launch_solve_wide<float>(g, cw, s);
-        case NLA_F16: return launch_solve_wide<__half>(g, cw, s);
-        default: break;
-      }
-    }
   }
+  const bool S = func == 'S';
   switch (dtype) {
-    case NLA_F64:
-      return n <= 512 ? launch_leaf_t<double, 16>(func, g, s) : launch_leaf_t<double, 8>(func, g, s);
-    case NLA_F32:
-      return n <= 512 ? launch_leaf_t<float, 32>(func, g, s) : launch_leaf_t<float, 16>(func, g, s);
-    case NLA_F16:
-      return n <= 512 ? launch_leaf_t<__half, 32>(func, g, s) : launch_leaf_t<__half, 16>(func, g, s);
+    case NLA_F64: return S ? launch_strips<double, true>(g, s) : launch_strips<double, false>(g, s);
+    case NLA_F32: return S ? launch_strips<float, true>(g, s) : launch_strips<float, false>(g, s);
+    case NLA_F16: return S ? launch_strips<__half, true>(g, s) : launch_strips<__half, false>(g, s);
     default: return fail(NLA_ERR_DTYPE, "diag block: unknown dtype");
   }
 }

@@ -1,5 +1,5 @@
-// Diagonal-block solve / multiply building blocks shared by the base-case
-// kernels (nla_leaf.cu) and the persistent batched solver (nla_batched.cu).
+// Diagonal-block solve / multiply building blocks of the base-case kernels
+// (nla_leaf.cu).
 //
 // All eight (func, side, uplo) forms map onto one canonical problem, a
 // LOWER triangle applied from the LEFT:
@@ -9,18 +9,11 @@
 //   (i -> n-1-i on rows and columns of A and on the rows of B).
 // Both are pure index maps, so no data is copied.
 //
-// One CTA of 128 threads (a warp-group) owns CW right-hand sides.  The CTA
-// stages its n x CW block of B in shared memory in the compute type and works
-// down the diagonal in 32-row panels: the panel's 32 x 32 triangle is solved
-// by one warp per group of columns, one row per lane, each solved value
-// broadcast to the lanes below with __shfl_sync; reciprocals of the diagonal
-// are formed once per CTA, not once per right-hand side; the rows below the
-// panel are then updated from a 128 x 32 slab of A staged through shared
-// memory with coalesced loads.  Float16 blocks are computed in Float32 and
-// rounded once when stored.
+// Here: the index maps and the Float64 solve with one right-hand side per
+// thread (many right-hand sides, blocks of at most 128 rows).  Everything
+// else runs on strips (nla_leaf_strip.cuh).  Float16 blocks are computed in
+// Float32 and rounded once when stored.
 #pragma once
-
-#include <type_traits>
 
 #include "nla_common.cuh"
 
@@ -29,7 +22,6 @@ namespace leafdev {
 
 constexpr int LEAF_THREADS = 128;
 constexpr int PANEL = 32;
-constexpr int SLAB_PAD = PANEL + 1;
 
 struct LeafArgs {
   const void* A;
@@ -54,298 +46,6 @@ template <typename T>
 __device__ __forceinline__ int64_t b_off(const LeafArgs& g, int i, int64_t c) {
   int mi = g.rev ? g.n - 1 - i : i;
   return mat_off(mi, c, g.ldb, g.tB);
-}
-
-// Stage Acan(r0 + t, k0 + kk), t < rows <= ROWS, kk < cols, into slab[t][kk] (zero
-// outside, and zero where keep(t, kk) is false).  Threads run along the index
-// that is contiguous in memory.
-template <int ROWS, typename T, typename Tc, typename Keep>
-__device__ __forceinline__ void stage_slab(const LeafArgs& g, Tc* slab, int r0, int rows, int k0, int cols,
-                                           Keep keep) {
-  const T* A = static_cast<const T*>(g.A);
-  for (int idx = threadIdx.x; idx < ROWS * PANEL; idx += LEAF_THREADS) {
-    int t, kk;
-    if (!g.tA) { t = idx % ROWS; kk = idx / ROWS; }
-    else { kk = idx % PANEL; t = idx / PANEL; }
-    Tc v = Tc(0);
-    if (t < rows && kk < cols && keep(r0 + t, k0 + kk)) v = Elem<T>::load(A + a_off<T>(g, r0 + t, k0 + kk));
-    slab[t * SLAB_PAD + kk] = v;
-  }
-}
-
-// With BATCH > 1 the loads are issued in batches of BATCH per thread before
-// any is used, so that a CTA that is alone on its SM keeps many requests in
-// flight; kernels with several CTAs per SM use BATCH = 1 (fewer registers).
-template <typename T, typename Tc, int CW, int BATCH = 1>
-__device__ __forceinline__ void load_block(const LeafArgs& g, Tc* X, int64_t c0, int ncols, Tc alpha = Tc(1)) {
-  const T* B = static_cast<const T*>(g.B);
-  const int total = g.n * CW;
-  for (int base = threadIdx.x; base < total; base += LEAF_THREADS * BATCH) {
-    Tc v[BATCH];
-#pragma unroll
-    for (int u = 0; u < BATCH; ++u) {
-      const int idx = base + u * LEAF_THREADS;
-      int i, c;
-      if (!g.tB) { i = idx % g.n; c = idx / g.n; }
-      else { c = idx % CW; i = idx / CW; }
-      v[u] = idx < total && c < ncols ? alpha * Elem<T>::load(B + b_off<T>(g, i, c0 + c)) : Tc(0);
-    }
-#pragma unroll
-    for (int u = 0; u < BATCH; ++u) {
-      const int idx = base + u * LEAF_THREADS;
-      int i, c;
-      if (!g.tB) { i = idx % g.n; c = idx / g.n; }
-      else { c = idx % CW; i = idx / CW; }
-      if (idx < total) X[i * CW + c] = v[u];
-    }
-  }
-}
-
-template <typename T, typename Tc, int CW>
-__device__ __forceinline__ void store_block(const LeafArgs& g, const Tc* X, int64_t c0, int ncols) {
-  T* B = static_cast<T*>(g.B);
-  const int total = g.n * CW;
-  for (int idx = threadIdx.x; idx < total; idx += LEAF_THREADS) {
-    int i, c;
-    if (!g.tB) { i = idx % g.n; c = idx / g.n; }
-    else { c = idx % CW; i = idx / CW; }
-    if (c < ncols) Elem<T>::store(B + b_off<T>(g, i, c0 + c), X[i * CW + c]);
-  }
-}
-
-// acc[i][c] += sum_kk slab[tr + 32 i][kk] * Xp[kk, tc * CW/4 + c] for
-// kk < pw: LEAF_THREADS threads as 32 row lanes (tr) x 4 column groups (tc,
-// one warp each, so the X reads are warp-wide broadcasts).  Each k step reads
-// 4 slab values and CW/4 values of X for 4 * CW/4 fused multiply-adds.  Row
-// slots past `rows` multiply zeros of the slab: skipping them (with
-// predicates or per-slot-count copies of the body) measured slower in the
-// persistent batched solver, whose CTAs see every chunk height.
-template <typename Tc, int CW>
-__device__ __forceinline__ void tile_product(const Tc* __restrict__ slab, const Tc* __restrict__ Xp, int pw,
-                                             int rows, Tc (&acc)[4][CW / 4]) {
-  (void)rows;
-  constexpr int CT = CW / 4;
-  const int tr = threadIdx.x & 31, tc = threadIdx.x >> 5;
-  for (int kk = 0; kk < pw; ++kk) {
-    Tc a[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = slab[(tr + 32 * i) * SLAB_PAD + kk];
-    Tc xv[CT];
-    const Tc* xr = Xp + kk * CW + tc * CT;
-#pragma unroll
-    for (int c = 0; c < CT; ++c) xv[c] = xr[c];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int c = 0; c < CT; ++c) acc[i][c] = fma(a[i], xv[c], acc[i][c]);
-  }
-}
-
-// Xo[r, :] -= sum_kk slab[r][kk] * Xp[kk, :] for r < rows, kk < pw.
-template <typename Tc, int CW>
-__device__ __forceinline__ void trailing_update(const Tc* __restrict__ slab, const Tc* __restrict__ Xp,
-                                                Tc* __restrict__ Xo, int rows, int pw) {
-  constexpr int CT = CW / 4;
-  const int tr = threadIdx.x & 31, tc = threadIdx.x >> 5;
-  Tc acc[4][CT];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int c = 0; c < CT; ++c) acc[i][c] = Tc(0);
-  tile_product<Tc, CW>(slab, Xp, pw, rows, acc);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int r = tr + 32 * i;
-    if (r < rows) {
-      Tc* xo = Xo + r * CW + tc * CT;
-#pragma unroll
-      for (int c = 0; c < CT; ++c) xo[c] -= acc[i][c];
-    }
-  }
-}
-
-// Canonical lower-left solve: X := L^{-1} (alpha X) for the CW columns
-// starting at c0 (ncols of them valid), run by one CTA of LEAF_THREADS.
-// smem holds leaf_solve_smem_elems(n, CW) compute-type elements.
-template <typename T, int CW>
-__device__ __forceinline__ void solve_block(const LeafArgs& g, int64_t c0, int ncols, unsigned char* smem_raw,
-                                            typename Elem<T>::compute alpha) {
-  using Tc = typename Elem<T>::compute;
-  Tc* X = reinterpret_cast<Tc*>(smem_raw);            // n x CW
-  Tc* inv_d = X + (size_t)g.n * CW;                   // n
-  Tc* slab = inv_d + g.n;                             // 128 x 33
-  Tc* diag = slab + LEAF_THREADS * SLAB_PAD;          // 32 x 33
-  const int n = g.n;
-  const T* A = static_cast<const T*>(g.A);
-
-  load_block<T, Tc, CW>(g, X, c0, ncols, alpha);
-  for (int i = threadIdx.x; i < n; i += LEAF_THREADS)
-    inv_d[i] = g.unit ? Tc(1) : Tc(1) / Elem<T>::load(A + a_off<T>(g, i, i));
-  __syncthreads();
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int CPW = CW / 4;  // columns per warp
-  for (int p0 = 0; p0 < n; p0 += PANEL) {
-    const int pw = min(PANEL, n - p0);
-    // Strictly-lower part of the panel's diagonal block.
-    stage_slab<PANEL, T>(g, diag, p0, pw, p0, pw, [](int i, int j) { return j < i; });
-    __syncthreads();
-
-    Tc x[CPW];
-#pragma unroll
-    for (int q = 0; q < CPW; ++q) x[q] = lane < pw ? X[(p0 + lane) * CW + warp + 4 * q] : Tc(0);
-    for (int i = 0; i < pw; ++i) {
-      const Tc lij = diag[lane * SLAB_PAD + i];
-      const Tc inv = inv_d[p0 + i];
-#pragma unroll
-      for (int q = 0; q < CPW; ++q) {
-        if (lane == i) x[q] *= inv;
-        const Tc xi = __shfl_sync(0xffffffffu, x[q], i);
-        if (lane > i) x[q] = fma(-lij, xi, x[q]);
-      }
-    }
-    if (lane < pw) {
-#pragma unroll
-      for (int q = 0; q < CPW; ++q) X[(p0 + lane) * CW + warp + 4 * q] = x[q];
-    }
-    __syncthreads();
-
-    // Rows below the panel: X[r, :] -= A[r, panel] * X[panel, :], as a
-    // register-tiled product: thread (tr, tc) owns rows r0 + tr + 32 i
-    // (i < 4) and the CW/4 columns of column group tc (its warp), so each
-    // k step reads 4 slab values and one broadcast vector of X for 4 * CW/4
-    // fused multiply-adds.
-    for (int r0 = p0 + pw; r0 < n; r0 += LEAF_THREADS) {
-      const int rows = min(LEAF_THREADS, n - r0);
-      stage_slab<LEAF_THREADS, T>(g, slab, r0, rows, p0, pw, [](int, int) { return true; });
-      __syncthreads();
-      trailing_update<Tc, CW>(slab, X + (size_t)p0 * CW, X + (size_t)r0 * CW, rows, pw);
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  store_block<T, Tc, CW>(g, X, c0, ncols);
-}
-
-// Xo[r, :] -= sum_kk slab[r][kk] * Xp[kk, :] for r < rows, kk < pw, for wide
-// column blocks: LEAF_THREADS threads as RG row groups x (LEAF_THREADS / RG)
-// column groups, each thread a 4-row x CT-column register tile (rows strided
-// by RG so that slab reads are conflict-free).  rows <= 4 * RG.
-template <typename Tc, int CW, int RG, int SLOTS>
-__device__ __forceinline__ void trailing_update_wide_n(const Tc* __restrict__ slab, const Tc* __restrict__ Xp,
-                                                       Tc* __restrict__ Xo, int rows, int pw) {
-  constexpr int CG = LEAF_THREADS / RG;
-  constexpr int CT = CW / CG;
-  const int tr = threadIdx.x % RG, tc = threadIdx.x / RG;
-  Tc acc[SLOTS][CT];
-#pragma unroll
-  for (int i = 0; i < SLOTS; ++i)
-#pragma unroll
-    for (int c = 0; c < CT; ++c) acc[i][c] = Tc(0);
-  for (int kk = 0; kk < pw; ++kk) {
-    Tc a[SLOTS];
-#pragma unroll
-    for (int i = 0; i < SLOTS; ++i) a[i] = slab[(tr + RG * i) * SLAB_PAD + kk];
-    const Tc* xr = Xp + kk * CW + tc * CT;
-#pragma unroll
-    for (int c = 0; c < CT; ++c) {
-      const Tc xv = xr[c];
-#pragma unroll
-      for (int i = 0; i < SLOTS; ++i) acc[i][c] = fma(a[i], xv, acc[i][c]);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < SLOTS; ++i) {
-    const int r = tr + RG * i;
-    if (r < rows) {
-      Tc* xo = Xo + r * CW + tc * CT;
-#pragma unroll
-      for (int c = 0; c < CT; ++c) xo[c] -= acc[i][c];
-    }
-  }
-}
-
-// Float64: row slots with RG * i >= rows hold no row of the chunk and are
-// skipped (the slot count is a compile-time constant of the body), which pays
-// on the 2-FMA-per-clock DFMA pipe.  Float32 keeps the single full-height
-// body, which measured faster there.
-template <typename Tc, int CW, int RG>
-__device__ __forceinline__ void trailing_update_wide(const Tc* __restrict__ slab, const Tc* __restrict__ Xp,
-                                                     Tc* __restrict__ Xo, int rows, int pw) {
-  if constexpr (!std::is_same<Tc, double>::value) {
-    trailing_update_wide_n<Tc, CW, RG, 4>(slab, Xp, Xo, rows, pw);
-    return;
-  }
-  switch ((rows + RG - 1) / RG) {
-    case 1: trailing_update_wide_n<Tc, CW, RG, 1>(slab, Xp, Xo, rows, pw); break;
-    case 2: trailing_update_wide_n<Tc, CW, RG, 2>(slab, Xp, Xo, rows, pw); break;
-    case 3: trailing_update_wide_n<Tc, CW, RG, 3>(slab, Xp, Xo, rows, pw); break;
-    default: trailing_update_wide_n<Tc, CW, RG, 4>(slab, Xp, Xo, rows, pw); break;
-  }
-}
-
-// Canonical lower-left solve for wide column blocks (CW in {16, 32, 64, 128}):
-// the same panels as solve_block, but each panel's 32 x 32 triangle is solved
-// with one right-hand side per thread (threads < CW), fully unrolled over the
-// panel's values in registers, so every lane does useful work and no value
-// has to cross lanes.
-template <typename T, int CW>
-__device__ __forceinline__ void solve_block_wide(const LeafArgs& g, int64_t c0, int ncols, unsigned char* smem_raw,
-                                                 typename Elem<T>::compute alpha) {
-  using Tc = typename Elem<T>::compute;
-  constexpr int RG = CW >= 128 ? 16 : 32;  // row groups of the trailing update
-  constexpr int CHUNK = 4 * RG;            // rows per trailing-update pass
-  Tc* X = reinterpret_cast<Tc*>(smem_raw);            // n x CW
-  Tc* inv_d = X + (size_t)g.n * CW;                   // n
-  Tc* slab = inv_d + g.n;                             // 128 x 33
-  Tc* diag = slab + LEAF_THREADS * SLAB_PAD;          // 32 x 33
-  const int n = g.n;
-  const T* A = static_cast<const T*>(g.A);
-
-  load_block<T, Tc, CW>(g, X, c0, ncols, alpha);
-  for (int i = threadIdx.x; i < n; i += LEAF_THREADS)
-    inv_d[i] = g.unit ? Tc(1) : Tc(1) / Elem<T>::load(A + a_off<T>(g, i, i));
-  __syncthreads();
-
-  const int t = threadIdx.x;
-  for (int p0 = 0; p0 < n; p0 += PANEL) {
-    const int pw = min(PANEL, n - p0);
-    stage_slab<PANEL, T>(g, diag, p0, pw, p0, pw, [](int i, int j) { return j < i; });
-    __syncthreads();
-    // The panel's serial chains run on CW threads.  In Float64 the warps
-    // that take them rotate with the panel and the CTA so that co-resident
-    // CTAs spread this FP64 work over all four SM sub-partitions.
-    const int rot = std::is_same<Tc, double>::value ? 32 * (int)((p0 / PANEL + blockIdx.x) % (LEAF_THREADS / 32)) : 0;
-    const int tt = (t - rot + LEAF_THREADS) % LEAF_THREADS;
-    if (tt < CW) {
-      // Right-looking: x_j is subtracted from every later row as soon as it
-      // is known.  Each row sees the same FMAs in the same order (j
-      // increasing) as a row-by-row dot product, so the bits are the same,
-      // and the dependent chain is one FMA and one multiply per row.
-      Tc y[PANEL];
-#pragma unroll
-      for (int r = 0; r < PANEL; ++r) y[r] = r < pw ? X[(p0 + r) * CW + tt] : Tc(0);
-#pragma unroll
-      for (int j = 0; j < PANEL; ++j) {
-        if (j < pw) {
-          const Tc xj = y[j] * inv_d[p0 + j];
-          X[(p0 + j) * CW + tt] = xj;
-#pragma unroll
-          for (int r = j + 1; r < PANEL; ++r) y[r] = fma(-diag[r * SLAB_PAD + j], xj, y[r]);
-        }
-      }
-    }
-    __syncthreads();
-    for (int r0 = p0 + pw; r0 < n; r0 += CHUNK) {
-      const int rows = min(CHUNK, n - r0);
-      stage_slab<CHUNK, T>(g, slab, r0, rows, p0, pw, [](int, int) { return true; });
-      __syncthreads();
-      trailing_update_wide<Tc, CW, RG>(slab, X + (size_t)p0 * CW, X + (size_t)r0 * CW, rows, pw);
-      __syncthreads();
-    }
-  }
-  __syncthreads();
-  store_block<T, Tc, CW>(g, X, c0, ncols);
 }
 
 // Float64 solve with one right-hand side per thread, for n <= COLS_MAX_N and
@@ -511,10 +211,6 @@ __device__ __forceinline__ void solve_cols_f64(const LeafArgs& g, int64_t c0, in
     else { cc = idx % CW; i = idx / CW; }
     if (cc < ncols) Bo[b_off<double>(g, i, c0 + cc)] = X[i * CW + cc];
   }
-}
-
-__host__ __device__ constexpr size_t leaf_solve_smem_elems(int n, int CW) {
-  return (size_t)n * CW + (size_t)n + (size_t)LEAF_THREADS * SLAB_PAD + (size_t)PANEL * SLAB_PAD;
 }
 
 }  // namespace leafdev
