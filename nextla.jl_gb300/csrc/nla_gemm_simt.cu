@@ -6,8 +6,8 @@
 // Float16 accumulates in Float32 (the tensor-core path for Float16 lives in
 // nla_umma.cu).
 //
-// Tiling: 256 threads as 16 x 16; each thread owns a (2V) x (2V) block made
-// of two V-wide strips in each direction, so shared-memory reads are V-wide
+// Tiling: 256 threads as 16 x 16; each thread owns 2V rows and RN columns
+// (RN = 2V or 1) made of V-wide strips, so shared-memory reads are V-wide
 // vectors and global stores of a column are 16V contiguous elements.
 // Tiles are double-buffered in shared memory with a register prefetch of the
 // next K slab.  Operand loads are layout-aware: threads run along whichever
@@ -27,14 +27,25 @@ template <> struct Vec<double, 2> {
   __device__ static void unpack(const double2& v, double* o) { o[0] = v.x; o[1] = v.y; }
 };
 
-template <typename T, int V, int BK>
+template <> struct Vec<float, 2> {
+  using type = float2;
+  __device__ static void unpack(const float2& v, float* o) { o[0] = v.x; o[1] = v.y; }
+};
+template <typename Tc> struct Vec<Tc, 1> {
+  using type = Tc;
+  __device__ static void unpack(const Tc& v, Tc* o) { o[0] = v; }
+};
+
+template <typename T, int V, int RN, int BK>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, int64_t K, double alpha,
                                                         const T* __restrict__ A, int64_t lda, int tA,
                                                         const T* __restrict__ B, int64_t ldb, int tB, T* C,
                                                         int64_t ldc) {
   using Tc = typename Elem<T>::compute;
-  constexpr int BM = 32 * V;  // = BN
-  constexpr int BN = 32 * V;
+  static_assert(RN == 2 * V || RN == 1, "columns per thread");
+  constexpr int BM = 32 * V;
+  constexpr int BN = 16 * RN;
+  constexpr int VN = RN == 1 ? 1 : V;
   constexpr int LA = BM * BK / 256;
   constexpr int LB = BK * BN / 256;
   __shared__ __align__(16) Tc As[2][BK][BM];
@@ -81,11 +92,11 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, in
     }
   };
 
-  Tc acc[2 * V][2 * V];
+  Tc acc[2 * V][RN];
 #pragma unroll
   for (int r = 0; r < 2 * V; ++r)
 #pragma unroll
-    for (int c = 0; c < 2 * V; ++c) acc[r][c] = Tc(0);
+    for (int c = 0; c < RN; ++c) acc[r][c] = Tc(0);
 
   const int64_t nk = (K + BK - 1) / BK;
   if (nk > 0) {
@@ -98,16 +109,18 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, in
     if (kt + 1 < nk) load_tiles((kt + 1) * BK);
 #pragma unroll
     for (int k = 0; k < BK; ++k) {
-      Tc a[2 * V], b[2 * V];
+      Tc a[2 * V], b[RN];
       using VT = typename Vec<Tc, V>::type;
+      using VTN = typename Vec<Tc, VN>::type;
       Vec<Tc, V>::unpack(*reinterpret_cast<const VT*>(&As[cur][k][V * tx]), a);
       Vec<Tc, V>::unpack(*reinterpret_cast<const VT*>(&As[cur][k][16 * V + V * tx]), a + V);
-      Vec<Tc, V>::unpack(*reinterpret_cast<const VT*>(&Bs[cur][k][V * ty]), b);
-      Vec<Tc, V>::unpack(*reinterpret_cast<const VT*>(&Bs[cur][k][16 * V + V * ty]), b + V);
+      Vec<Tc, VN>::unpack(*reinterpret_cast<const VTN*>(&Bs[cur][k][VN * ty]), b);
+      if constexpr (RN > 1)
+        Vec<Tc, VN>::unpack(*reinterpret_cast<const VTN*>(&Bs[cur][k][16 * V + V * ty]), b + V);
 #pragma unroll
       for (int r = 0; r < 2 * V; ++r)
 #pragma unroll
-        for (int c = 0; c < 2 * V; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+        for (int c = 0; c < RN; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
     }
     if (kt + 1 < nk) store_tiles(cur ^ 1);
     __syncthreads();
@@ -115,8 +128,8 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, in
 
   const Tc al = (Tc)alpha;
 #pragma unroll
-  for (int c = 0; c < 2 * V; ++c) {
-    int64_t j = col0 + (c < V ? V * ty + c : 16 * V + V * ty + (c - V));
+  for (int c = 0; c < RN; ++c) {
+    int64_t j = col0 + (c < V ? VN * ty + c : 16 * V + V * ty + (c - V));
     if (j >= M) continue;
 #pragma unroll
     for (int r = 0; r < 2 * V; ++r) {
@@ -128,19 +141,54 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, in
   }
 }
 
-template <typename T, int V, int BK>
+template <typename T, int V, int RN, int BK>
 int launch_simt(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
                 cudaStream_t s) {
-  constexpr int BM = 32 * V;
-  int64_t gx = (N + BM - 1) / BM, gy = (M + BM - 1) / BM;
+  constexpr int BM = 32 * V, BN = 16 * RN;
+  int64_t gx = (N + BM - 1) / BM, gy = (M + BN - 1) / BN;
   if (gx > 2147483647LL || gy > 65535) return fail(NLA_ERR_UNSUPPORTED, "gemm: matrix too large for one launch");
   TraceScope trace(NLA_K_GEMM_SIMT, s, 2.0 * (double)N * (double)M * (double)K,
                    (double)sizeof(T) * ((double)N * K + (double)K * M + 2.0 * (double)N * M));
-  gemm_simt_kernel<T, V, BK><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(
+  gemm_simt_kernel<T, V, RN, BK><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(
       N, M, K, alpha, static_cast<const T*>(A.p), A.ld, A.t, static_cast<const T*>(B.p), B.ld, B.t,
       static_cast<T*>(C.p), C.ld);
   NLA_CHECK_LAUNCH("gemm_simt_kernel");
   return NLA_OK;
+}
+
+// The time of a tiling in units of one output element's share of an SM's
+// FMAs: waves times (tile elements times the tile's cost per element plus a
+// fixed part per tile).
+double tiling_cost(int64_t N, int64_t M, int bm, int bn, double per_element, double fixed) {
+  const int64_t tiles = ((N + bm - 1) / bm) * ((M + bn - 1) / bn), sms = num_sms();
+  return (double)((tiles + sms - 1) / sms) * ((double)bm * bn * per_element + fixed);
+}
+
+// Float64: every tile keeps the DFMA pipe busy (2 per clock per SM), so the
+// tile that divides the output most evenly over the SMs wins.  Measured
+// against 64 x 64 alone (N x K x M): 256 x 256 x 256 270 -> 37 us (32 x 16),
+// 512 x 512 x 256 537 -> 139 (32 x 32), 256 x 256 x 8192 1038 -> 925.
+template <typename T>
+int launch_simt_f64(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
+                    cudaStream_t s) {
+  const double c64 = tiling_cost(N, M, 64, 64, 1.0, 64.0), c32 = tiling_cost(N, M, 32, 32, 1.0, 64.0),
+               c16 = tiling_cost(N, M, 32, 16, 1.0, 64.0);
+  if (c64 <= c32 && c64 <= c16) return launch_simt<T, 2, 4, 16>(N, M, K, alpha, A, B, C, s);
+  if (c32 <= c16 || M > 65535 * 16ll) return launch_simt<T, 1, 2, 32>(N, M, K, alpha, A, B, C, s);
+  return launch_simt<T, 1, 1, 32>(N, M, K, alpha, A, B, C, s);
+}
+
+// Float32 and Float16: smaller tiles read more shared memory per FMA.
+// Measured against 128 x 128 alone: 16 x 16 x 900 7.1 -> 3.3 us, 256 x 256 x
+// 256 44 -> 12 us (32 x 32), 476 x 1024 x 900 153 -> 57 us (64 x 64).
+template <typename T>
+int launch_simt_f32(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
+                    cudaStream_t s) {
+  const double c128 = tiling_cost(N, M, 128, 128, 1.0, 1024.0), c64 = tiling_cost(N, M, 64, 64, 1.4, 1024.0),
+               c32 = tiling_cost(N, M, 32, 32, 3.0, 1024.0);
+  if (c128 <= c64 && c128 <= c32) return launch_simt<T, 4, 8, 8>(N, M, K, alpha, A, B, C, s);
+  if (c64 <= c32 || M > 65535 * 32ll) return launch_simt<T, 2, 4, 16>(N, M, K, alpha, A, B, C, s);
+  return launch_simt<T, 1, 2, 32>(N, M, K, alpha, A, B, C, s);
 }
 
 }  // namespace
@@ -150,9 +198,9 @@ int launch_gemm_simt(int dtype, int64_t N, int64_t M, int64_t K, double alpha, c
   if (N <= 0 || M <= 0) return NLA_OK;
   if (C.t) return fail(NLA_ERR_UNSUPPORTED, "gemm: transposed output view");
   switch (dtype) {
-    case NLA_F64: return launch_simt<double, 2, 16>(N, M, K, alpha, A, B, C, s);
-    case NLA_F32: return launch_simt<float, 4, 8>(N, M, K, alpha, A, B, C, s);
-    case NLA_F16: return launch_simt<__half, 4, 8>(N, M, K, alpha, A, B, C, s);
+    case NLA_F64: return launch_simt_f64<double>(N, M, K, alpha, A, B, C, s);
+    case NLA_F32: return launch_simt_f32<float>(N, M, K, alpha, A, B, C, s);
+    case NLA_F16: return launch_simt_f32<__half>(N, M, K, alpha, A, B, C, s);
     default: return fail(NLA_ERR_DTYPE, "gemm: unknown dtype");
   }
 }
