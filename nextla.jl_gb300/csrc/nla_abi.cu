@@ -172,13 +172,36 @@ static bool umma_enabled() {
   return on;
 }
 
+// Float32 updates on the tensor cores (nla_umma_f32.cu) from about 1e8
+// products: staging and the kernel's prologue cost about 20 us, the CUDA-core
+// update runs at 15-40 TFLOP/s.  Measured (N x K x M, CUDA cores against
+// tensor cores, launches included): 512^3 34 / 31 us, 256 x 256 x 8192
+// 48 / 29, 1024 x 1024 x 8192 516 / 150, 4096 x 4096 x 8192 6889 / 1384.
+// Below K = 128 a chunk's truncated sums are no more accurate than the FMA
+// chain they replace.  Relative error against 64 bits at K = 128, 1024, 8192:
+// normal data 2.0e-7, 5.7e-7, 1.6e-6 before, 7.5e-8, 1.0e-7, 2.2e-7 now;
+// values spread over 2^+-12 1.5e-7, 4.0e-7, 1.1e-6 / 1.2e-7, 1.4e-7, 2.3e-7.
+static bool f32_umma_wanted(int64_t N, int64_t M, int64_t K) {
+  return umma_enabled() && N >= 64 && M >= 64 && K >= 128 && (double)N * (double)M * (double)K >= 1e8;
+}
+
+size_t update_scratch_bytes(int dtype, int64_t N, int64_t M, int64_t K) {
+  return dtype == NLA_F32 && f32_umma_wanted(N, M, K) ? f32_update_bytes(N, M, K) : 0;
+}
+
 // Float16 updates large enough to fill 128 x 128 tiles run on the tensor
-// cores (FP32 accumulation); everything else on CUDA cores.
+// cores (FP32 accumulation), Float32 ones as products of BF16 terms;
+// everything else on CUDA cores.
 int launch_gemm(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
-                cudaStream_t s) {
+                cudaStream_t s, void* ws, size_t ws_bytes) {
   if (is_complex(dtype)) return launch_gemm_complex(dtype, N, M, K, alpha, A, B, C, s);
   if (dtype == NLA_F16 && umma_enabled() && N >= 128 && M >= 128 && K >= 64)
     return launch_sliced_gemm(N, M, K, alpha, A, B, C, NLA_F16, NLA_F16, 1, false, nullptr, 0, s);
+  if (const size_t need = C.t ? 0 : update_scratch_bytes(dtype, N, M, K)) {
+    if (ws && ws_bytes >= need) return launch_gemm_f32_umma(N, M, K, alpha, A, B, C, ws, s);
+    const Scratch own(s, need);
+    if (own.p) return launch_gemm_f32_umma(N, M, K, alpha, A, B, C, own.p, s);
+  }
   return launch_gemm_simt(dtype, N, M, K, alpha, A, B, C, s);
 }
 
@@ -186,7 +209,7 @@ static int launch_update(const RecPlan& c, int64_t N, int64_t M, int64_t K, doub
                          const Mat& B, const Mat& C) {
   if (c.mode == GEMM_MIXED)
     return launch_sliced_gemm(N, M, K, alpha, A, B, C, NLA_F64, NLA_F64, c.S, c.bf16, nullptr, 0, c.s);
-  return launch_gemm(c.dtype, N, M, K, alpha, A, B, C, c.s);
+  return launch_gemm(c.dtype, N, M, K, alpha, A, B, C, c.s, c.ws, c.ws_bytes);
 }
 
 // ---------------------------------------------------------------------------
@@ -340,6 +363,11 @@ int trxm_impl(char side, char uplo, char trans, double alpha, char func, int dty
     return is_complex(dtype) ? launch_scale_complex(dtype, rows, cols, alpha, alpha_im, Bm, s)
                              : launch_scale(dtype, rows, cols, alpha, Bm, s);
   };
+  // Scratch for the largest update, the top split's.
+  const int64_t mid = split_point(n), big = mid > n - mid ? mid : n - mid;
+  const Scratch ws(s, n > c.threshold ? update_scratch_bytes(dtype, big, m, big) : 0);
+  c.ws = ws.p;
+  c.ws_bytes = ws.bytes;
   if (func == 'S') NLA_TRY(scale());  // src/rectrxm.jl:64
   NLA_TRY(recurse(c, Am, n, Bm));
   if (func == 'M') NLA_TRY(scale());  // src/rectrxm.jl:72

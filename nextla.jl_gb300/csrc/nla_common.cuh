@@ -114,9 +114,27 @@ struct TraceScope {
 // Kernel launchers (defined in the .cu files).
 // ---------------------------------------------------------------------------
 
-// out (N x M) += alpha * op(A) (N x K) * op(B) (K x M), plain dtype-preserving path.
+// Scratch of one call, ordered on its stream; null when there is none to be
+// had (stream capture, device memory exhausted).  Every allocation is the
+// caller's own, so calls on any streams and threads may overlap.
+void* scratch_alloc(cudaStream_t s, size_t bytes);
+void scratch_free(cudaStream_t s, void* p);
+struct Scratch {
+  cudaStream_t s;
+  void* p;
+  size_t bytes;
+  Scratch(cudaStream_t st, size_t n) : s(st), p(n ? scratch_alloc(st, n) : nullptr), bytes(p ? n : 0) {}
+  ~Scratch() { scratch_free(s, p); }
+  Scratch(const Scratch&) = delete;
+  Scratch& operator=(const Scratch&) = delete;
+};
+
+// out (N x M) += alpha * op(A) (N x K) * op(B) (K x M), plain dtype-preserving
+// path.  ws: scratch of update_scratch_bytes() that the calls of one
+// recursion share (null: the call takes its own).
 int launch_gemm(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
-                cudaStream_t s);
+                cudaStream_t s, void* ws = nullptr, size_t ws_bytes = 0);
+size_t update_scratch_bytes(int dtype, int64_t N, int64_t M, int64_t K);
 
 // Base case on a diagonal block: func 'S' (solve) or 'M' (multiply).
 int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A, const Mat& B,
@@ -141,6 +159,12 @@ int launch_scale_complex(int dtype, int64_t rows, int64_t cols, double alpha_re,
 int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
                        int in_dtype, int out_dtype, int S, bool bf16, void* ws, size_t ws_bytes, cudaStream_t s);
 size_t sliced_workspace_bytes(int64_t M, int64_t N, int64_t K, int S);
+
+// Float32 update on the tensor cores (nla_umma_f32.cu), scratch of
+// f32_update_bytes.
+int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
+                         void* ws, cudaStream_t s);
+size_t f32_update_bytes(int64_t M, int64_t N, int64_t K);
 
 // An operand staged for the tensor cores: S K-major 16-bit slices of a
 // rows x K view (padded to rows_pad x K_pad) and one exponent per row.
@@ -215,6 +239,8 @@ struct RecPlan {
   bool bf16;
   bool unit = false;  // unit diagonal
   const LeafInverses* inv = nullptr;  // leaves through their inverses (mixed exact solves)
+  void* ws = nullptr;  // scratch of the plain updates
+  size_t ws_bytes = 0;
 };
 int recurse(const RecPlan& c, const Mat& A, int64_t n, const Mat& B);
 // Mixed exact solves: whether the leaves go through inverses (a 7-slice solve

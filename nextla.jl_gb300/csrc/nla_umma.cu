@@ -1431,6 +1431,54 @@ int launch_exact_pairs(const ExactParams& p, const Staged& A, const Staged& B, c
 
 }  // namespace
 
+int staged_map(CUtensorMap* map, const void* base, uint64_t k_pad, uint64_t total_rows) {
+  return make_map(map, base, true, k_pad, total_rows);
+}
+
+// Scratch of the plain path: stream-ordered allocations from a pool of their
+// own, which keeps up to SCRATCH_KEEP bytes between calls (the default pool
+// would give everything back at each synchronisation).
+namespace {
+constexpr uint64_t SCRATCH_KEEP = 2ull << 30;
+constexpr int MAX_DEVICES = 64;
+std::mutex g_scratch_mu;
+cudaMemPool_t g_scratch_pool[MAX_DEVICES];
+
+cudaMemPool_t scratch_pool() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= MAX_DEVICES) return nullptr;
+  std::lock_guard<std::mutex> lk(g_scratch_mu);
+  if (!g_scratch_pool[dev]) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
+    uint64_t keep = SCRATCH_KEEP;
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    g_scratch_pool[dev] = pool;
+  }
+  return g_scratch_pool[dev];
+}
+}  // namespace
+
+void* scratch_alloc(cudaStream_t s, size_t bytes) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  void* p = nullptr;
+  cudaMemPool_t pool = nullptr;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+      !(pool = scratch_pool()) || cudaMallocFromPoolAsync(&p, bytes, pool, s) != cudaSuccess) {
+    cudaGetLastError();  // the caller runs without it
+    return nullptr;
+  }
+  return p;
+}
+
+void scratch_free(cudaStream_t s, void* p) {
+  if (p) cudaFreeAsync(p, s);
+}
+
 int workspace_get(cudaStream_t s, size_t bytes, void** out) {
   int dev = 0;
   cudaGetDevice(&dev);

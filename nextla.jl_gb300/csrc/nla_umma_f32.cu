@@ -1,0 +1,394 @@
+// Float32 off-diagonal update on the tensor cores (tcgen05):
+//   C (M x N) += alpha * op(A) (M x K) * op(B) (K x N)
+//
+// Each Float32 value is the sum of three BF16 values, x = h + m + l exactly
+// (24 bits of significand as 8 + 8 + 8, each rounded to nearest; the split
+// into BF16 terms is that of Henry, Tang and Heinecke, "Leveraging the
+// bfloat16 artificial intelligence datatype for higher-precision
+// computations", ARITH 2019).  Unlike the scaled integer slices of the
+// Float64 update, the terms carry their own exponents, so small elements of
+// a row keep their full precision.  Of the nine products the six of weight
+// up to 2^-16 are formed (h h; h m, m h; m m, h l, l h); the three left out
+// are below 2^-26 of |a||b| each, under the rounding of one Float32 FMA.
+//
+// Tensor-core accumulators do not round to nearest (their sums are biased
+// towards zero), so no sum stays in them for long: chunks of 64 values of K
+// are accumulated in TMEM (h h in one accumulator, the five smaller products
+// in another), and the drain warps add each chunk to Float32 registers with
+// ordinary rounded additions.  That leaves fewer roundings per element than
+// the FMA chain of the CUDA-core update, whose error grows with K.
+//
+// What bounds it: the TMA feed (96 KiB of tiles per 64 values of K for six
+// 128 x 128 x 64 products): 1190 TFLOP/s of executed products, 199 of the
+// update's, at 4096 x 4096 x 8192 (FFMA update: 39.9).  Warps: 0 loads A, 1 issues MMAs, 2 loads B,
+// 3-10 drain (two TMEM buffers of 256 columns) and update C.
+//
+// Rows of A and columns of B that hold Inf or NaN, or values so small or
+// large that low terms or sums would leave Float32's normal range, are
+// marked when they are staged; the outputs they touch are formed by the
+// drain warps from the original operands instead, with the FMA order of the
+// CUDA-core update.
+#include <cudaTypedefs.h>
+
+#include <mutex>
+
+#include "nla_common.cuh"
+#include "nla_umma.cuh"
+
+namespace nla {
+namespace {
+
+constexpr int BM = 128, BN = 128, BK = 64;
+constexpr int TILE_BYTES = BM * BK * 2;
+constexpr int SL = 3;
+constexpr int F32_THREADS = 352;
+constexpr int F32_STAGES = 2;
+constexpr int F32_STAGE_BYTES = 2 * SL * TILE_BYTES;
+constexpr int F32_CHUNK = 1;  // K blocks of 64 per drained chunk
+constexpr int F32_SMEM = F32_STAGES * F32_STAGE_BYTES + 1024 + 256;
+static_assert(F32_SMEM + 16 <= 232448, "shared memory above the per-block limit");
+
+// Row marks: 0 for a row of zeros, else the largest exponent field plus one
+// (1 .. 256, 256 for Inf and NaN), so that the row's largest value lies in
+// [2^(mark - 128), 2^(mark - 127)).  An output takes the careful path when its
+// row or column is not finite, when the low terms of either would be
+// subnormal, or when the products leave [2^-90, 2^106] (their low terms, or
+// sums of up to 2^20 of them, would leave the normal range).
+__device__ __forceinline__ bool careful(int ma, int mb) {
+  if (ma == 256 || mb == 256) return true;
+  if (ma == 0 || mb == 0) return false;
+  return ma < 28 || mb < 28 || ma + mb < 166 || ma + mb > 360;
+}
+
+struct F32Params {
+  int M, N, K;
+  int num_kb;
+  int tiles_m, tiles_n;
+  const float* A;  // element (i, k) at A[i * asi + k * ask]
+  int64_t asi, ask;
+  const float* B;  // element (k, j) at B[k * bsk + j * bsj]
+  int64_t bsk, bsj;
+  const int* mark_a;  // per 64-wide block of K and row: the block's mark at [kb * rows_pad + row]
+  const int* mark_b;
+  int rows_a, rows_b;  // padded
+  float* C;
+  int64_t ldc;
+  float alpha;
+  int* err;
+};
+
+// One element in the order of the CUDA-core update: FMAs with k increasing.
+__device__ __noinline__ float plain_dot(const F32Params& p, int i, int j) {
+  float s = 0.0f;
+  const float* a = p.A + (int64_t)i * p.asi;
+  const float* b = p.B + (int64_t)j * p.bsj;
+  for (int k = 0; k < p.K; ++k) s = fmaf(a[k * p.ask], b[k * p.bsk], s);
+  return s;
+}
+
+__global__ void __launch_bounds__(F32_THREADS, 1)
+    umma_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                    const __grid_constant__ F32Params p) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* fullA = reinterpret_cast<uint64_t*>(smem + F32_STAGES * F32_STAGE_BYTES);
+  uint64_t* fullB = fullA + F32_STAGES;
+  uint64_t* empty = fullB + F32_STAGES;
+  uint64_t* cfull = empty + F32_STAGES;
+  uint64_t* cempty = cfull + 2;
+  uint64_t* drain = cempty + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
+  __shared__ volatile int s_abort;
+  __shared__ int s_mark[2 * BM];  // marks of the tile's rows and columns
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // Output tiles are rasterised in groups of 8 tile rows for L2 reuse.
+  constexpr int group = 8;
+  const int per_group = group * p.tiles_n;
+  const int g = blockIdx.x / per_group;
+  const int first_m = g * group;
+  const int gsize = min(p.tiles_m - first_m, group);
+  const int local = blockIdx.x % per_group;
+  const int m0 = (first_m + local % gsize) * BM, n0 = (local / gsize) * BN;
+
+  if (threadIdx.x == 0) {
+    s_abort = 0;
+    for (int s = 0; s < F32_STAGES; ++s) {
+      umma::mbar_init(umma::smem_u32(&fullA[s]), 1);
+      umma::mbar_init(umma::smem_u32(&fullB[s]), 1);
+      umma::mbar_init(umma::smem_u32(&empty[s]), 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      umma::mbar_init(umma::smem_u32(&cfull[b]), 1);
+      umma::mbar_init(umma::smem_u32(&cempty[b]), 8);
+    }
+    umma::mbar_init(umma::smem_u32(drain), 1);
+    umma::fence_barrier_init();
+    umma::prefetch_tmap(&tmA);
+    umma::prefetch_tmap(&tmB);
+  }
+  if (warp == 1) umma::tmem_alloc(umma::smem_u32(tmem_slot), 512);
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0 || warp == 2) {
+    const bool is_a = warp == 0;
+    if (lane == 0) {
+      uint64_t* own = is_a ? fullA : fullB;
+      int kb = 0;
+      for (; kb < p.num_kb; ++kb) {
+        const int s = kb % F32_STAGES;
+        if (!umma::mbar_wait(umma::smem_u32(&empty[s]), ((uint32_t)(kb / F32_STAGES) & 1u) ^ 1u, &s_abort, p.err, 51))
+          break;
+        const uint32_t fb = umma::smem_u32(&own[s]);
+        uint8_t* st = smem + (size_t)s * F32_STAGE_BYTES + (is_a ? 0 : SL * TILE_BYTES);
+        umma::mbar_arrive_expect_tx(fb, SL * TILE_BYTES);
+        for (int sl = 0; sl < SL; ++sl)
+          umma::tma_load_2d(umma::smem_u32(st + sl * TILE_BYTES), is_a ? &tmA : &tmB, fb, kb * BK,
+                            (is_a ? m0 : n0) * SL + sl * BM);
+      }
+      umma::producer_quiesce(own, F32_STAGES, kb, &s_abort, p.err, 52);
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      const uint32_t id1 = umma::idesc_f16(BM, BN, true), id2 = umma::idesc_f16(BM, 2 * BN, true);
+      for (int kb = 0; kb < p.num_kb; ++kb) {
+        const int s = kb % F32_STAGES, ch = kb / F32_CHUNK, b = ch & 1;
+        const bool first = kb % F32_CHUNK == 0;
+        if ((first && !umma::mbar_wait(umma::smem_u32(&cempty[b]), ((uint32_t)(ch >> 1) & 1u) ^ 1u, &s_abort, p.err, 53)) ||
+            !umma::mbar_wait(umma::smem_u32(&fullA[s]), (uint32_t)(kb / F32_STAGES) & 1u, &s_abort, p.err, 54) ||
+            !umma::mbar_wait(umma::smem_u32(&fullB[s]), (uint32_t)(kb / F32_STAGES) & 1u, &s_abort, p.err, 54))
+          break;
+        umma::fence_after_sync();
+        const uint32_t a0 = umma::smem_u32(smem + (size_t)s * F32_STAGE_BYTES), b0 = a0 + SL * TILE_BYTES;
+        const uint32_t d0 = tmem + (uint32_t)(b * 2 * BN), d1 = d0 + (uint32_t)BN;
+        // A_h against (B_h, B_m), adjacent in shared memory: one MMA of
+        // N = 256 into both accumulators.
+#pragma unroll
+        for (int kk = 0; kk < BK / 16; ++kk)
+          umma::mma_f16(d0, umma::desc_kmajor_sw128(a0 + kk * 32), umma::desc_kmajor_sw128(b0 + kk * 32), id2,
+                        first && kk == 0 ? 0u : 1u);
+        constexpr int qa[4] = {1, 1, 0, 2}, qb[4] = {0, 1, 2, 0};  // m h, m m, h l, l h
+#pragma unroll
+        for (int pr = 0; pr < 4; ++pr)
+#pragma unroll
+          for (int kk = 0; kk < BK / 16; ++kk)
+            umma::mma_f16(d1, umma::desc_kmajor_sw128(a0 + qa[pr] * TILE_BYTES + kk * 32),
+                          umma::desc_kmajor_sw128(b0 + qb[pr] * TILE_BYTES + kk * 32), id1, 1u);
+        umma::mma_commit(umma::smem_u32(&empty[s]));
+        if (kb % F32_CHUNK == F32_CHUNK - 1 || kb == p.num_kb - 1) umma::mma_commit(umma::smem_u32(&cfull[b]));
+      }
+      umma::mma_commit(umma::smem_u32(drain));
+      umma::mbar_wait(umma::smem_u32(drain), 0, &s_abort, p.err, 55, false);
+    }
+  } else {
+    const int q = warp & 3;
+    const int h = (warp - 3) >> 2;  // column half: 0 (warps 3-6) or 1 (warps 7-10)
+    const int i = m0 + q * 32 + lane, c0 = n0 + h * 64;
+    {
+      // The marks of the tile's rows (threads 0-127) and columns (128-255).
+      const int t = (int)threadIdx.x - 96, r = t & (BM - 1);
+      const int* mk = t < BM ? p.mark_a + m0 + r : p.mark_b + n0 + r;
+      const int step = t < BM ? p.rows_a : p.rows_b;
+      int m = 0;
+#pragma unroll 4
+      for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, __ldg(mk + (int64_t)kb * step));
+      s_mark[t] = m;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    float acc[64];
+#pragma unroll
+    for (int j = 0; j < 64; ++j) acc[j] = 0.0f;
+    bool ok = true;
+    const int nch = (p.num_kb + F32_CHUNK - 1) / F32_CHUNK;
+    for (int ch = 0; ch < nch; ++ch) {
+      const int b = ch & 1;
+      ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&cfull[b]), (uint32_t)(ch >> 1) & 1u, &s_abort, p.err, 56));
+      if (!ok) break;
+      umma::fence_after_sync();
+      const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * BN + h * 64);
+#pragma unroll
+      for (int j0 = 0; j0 < 64; j0 += 16) {
+        uint32_t r0[16], r1[16];
+        umma::tmem_ld16(ta + (uint32_t)j0, r0);
+        umma::tmem_ld16(ta + (uint32_t)(BN + j0), r1);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j0 + j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
+      }
+      umma::fence_before_sync();
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(umma::smem_u32(&cempty[b]));
+    }
+    if (ok) {
+      const int ma = s_mark[q * 32 + lane];
+      const int* mb = s_mark + BM + h * 64;
+      float* C = p.C + i;
+      bool special = false;
+#pragma unroll
+      for (int j0 = 0; j0 < 64; j0 += 32) {
+        // All loads of C before the first store (a store may alias a later load).
+        float cv[32];
+        uint32_t skip = 0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          const int col = c0 + j0 + j;
+          const bool in = i < p.M && col < p.N;
+          cv[j] = in ? C[(int64_t)col * p.ldc] : 0.0f;
+          if (!in || careful(ma, mb[j0 + j])) skip |= 1u << j;
+          special |= in && (skip >> j & 1u);
+        }
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (!(skip >> j & 1u)) C[(int64_t)(c0 + j0 + j) * p.ldc] = fmaf(p.alpha, acc[j0 + j], cv[j]);
+      }
+      if (special)
+        for (int col = c0; col < min(c0 + 64, p.N); ++col)
+          if (i < p.M && careful(ma, mb[col - c0]))
+            C[(int64_t)col * p.ldc] = fmaf(p.alpha, plain_dot(p, i, col), C[(int64_t)col * p.ldc]);
+    }
+  }
+
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 1) {
+    __syncwarp();
+    umma::fence_after_sync();
+    umma::tmem_dealloc(tmem, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// Staging: the three BF16 terms of both operands in one launch, K-major,
+// rows padded to 128 and K to 64 with zeros; the terms of one 128-row tile
+// adjacent (row (t * 3 + term) * 128 + r for row t * 128 + r), and a mark per
+// row.  One 32 x 64 tile per CTA.
+// ---------------------------------------------------------------------------
+struct F32Job {
+  const float* X;  // element (row, k) at X[row * si + k * sk]
+  int64_t si, sk;
+  int rows, K;
+  __nv_bfloat16* out;
+  int64_t k_pad;
+  int* mark;   // the block of K's marks at mark[kb * rows_pad + row]
+  int blocks;  // 32-row blocks
+};
+
+// Rounded to BF16; values that would round to infinity stay finite (the next
+// term takes up the rest).
+__device__ __forceinline__ float bf16_near(float x) {
+  const float y = __bfloat162float(__float2bfloat16_rn(x));
+  return isinf(y) && !isinf(x) ? copysignf(__uint_as_float(0x7f7f0000u), x) : y;
+}
+
+__global__ void __launch_bounds__(256) stage_f32_kernel(const F32Job a, const F32Job b) {
+  __shared__ float tile[32][66];
+  const bool first = (int)blockIdx.x < a.blocks;
+  const F32Job j = first ? a : b;
+  const int i0 = (int)(first ? blockIdx.x : blockIdx.x - a.blocks) * 32, k0 = (int)blockIdx.y * 64;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  // Threads along the index that is contiguous in memory; loads all in flight.
+  const bool kfast = j.sk == 1;
+  float v[8];
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int idx = t + 256 * e;
+    const int i = kfast ? idx >> 6 : idx & 31, k = kfast ? idx & 63 : idx >> 5;
+    v[e] = i0 + i < j.rows && k0 + k < j.K ? __ldg(j.X + (i0 + i) * j.si + (k0 + k) * j.sk) : 0.0f;
+  }
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const int idx = t + 256 * e;
+    const int i = kfast ? idx >> 6 : idx & 31, k = kfast ? idx & 63 : idx >> 5;
+    tile[i][k] = v[e];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int pass = 0; pass < 4; ++pass) {
+    const int i = warp + 8 * pass, gi = i0 + i;
+    const float2 x = *reinterpret_cast<const float2*>(&tile[i][2 * lane]);
+    uint32_t* o = reinterpret_cast<uint32_t*>(j.out + ((int64_t)(gi >> 7) * SL * 128 + (gi & 127)) * j.k_pad + k0 + 2 * lane);
+    float r0 = x.x, r1 = x.y;
+#pragma unroll
+    for (int sl = 0; sl < SL; ++sl) {
+      const float h0 = bf16_near(r0), h1 = bf16_near(r1);
+      o[sl * (128 * j.k_pad / 2)] = (__float_as_uint(h0) >> 16) | (__float_as_uint(h1) & 0xffff0000u);
+      r0 -= h0;
+      r1 -= h1;
+    }
+    const uint32_t u0 = __float_as_uint(x.x) << 1, u1 = __float_as_uint(x.y) << 1;  // magnitude bits
+    const uint32_t um = max(u0, u1);
+    int mk = um ? (int)(um >> 24) + 1 : 0;
+    mk = __reduce_max_sync(0xffffffffu, mk);
+    if (lane == 0) j.mark[(int64_t)blockIdx.y * (j.blocks * 32) + gi] = mk;
+  }
+}
+
+int64_t pad_to(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
+size_t terms_bytes(int64_t rows, int64_t K) {
+  return (size_t)SL * (size_t)pad_to(rows, BM) * (size_t)pad_to(K, BK) * 2;  // a multiple of 1024
+}
+size_t marks_bytes(int64_t rows, int64_t K) { return (size_t)pad_to(rows, BM) * (size_t)(pad_to(K, BK) / BK) * sizeof(int); }
+
+}  // namespace
+
+size_t f32_update_bytes(int64_t M, int64_t N, int64_t K) {
+  return terms_bytes(M, K) + terms_bytes(N, K) + marks_bytes(M, K) + marks_bytes(N, K) + 1024;
+}
+
+int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
+                         void* ws, cudaStream_t s) {
+  const int64_t Mp = pad_to(M, BM), Np = pad_to(N, BN), Kp = pad_to(K, BK);
+  uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~uintptr_t(1023));
+  auto* ta = reinterpret_cast<__nv_bfloat16*>(base);
+  auto* tb = reinterpret_cast<__nv_bfloat16*>(base + terms_bytes(M, K));
+  int* marks = reinterpret_cast<int*>(base + terms_bytes(M, K) + terms_bytes(N, K));
+  int* err = device_error_word();
+  if (!err) return fail(NLA_ERR_UNSUPPORTED, "Float32 tensor-core update: no device error word");
+
+  F32Params p{};
+  p.M = (int)M;
+  p.N = (int)N;
+  p.K = (int)K;
+  p.num_kb = (int)(Kp / BK);
+  p.tiles_m = (int)(Mp / BM);
+  p.tiles_n = (int)(Np / BN);
+  p.A = static_cast<const float*>(A.p);
+  p.asi = A.t ? A.ld : 1;
+  p.ask = A.t ? 1 : A.ld;
+  p.B = static_cast<const float*>(B.p);
+  p.bsk = B.t ? B.ld : 1;
+  p.bsj = B.t ? 1 : B.ld;
+  p.mark_a = marks;
+  p.mark_b = marks + Mp * (Kp / BK);
+  p.rows_a = (int)Mp;
+  p.rows_b = (int)Np;
+  p.C = static_cast<float*>(C.p);
+  p.ldc = C.ld;
+  p.alpha = (float)alpha;
+  p.err = err;
+  {
+    TraceScope trace(NLA_K_SPLIT, s, 0.0, (double)(M + N) * (double)K * 4.0 + (double)(Mp + Np) * Kp * 2.0 * SL);
+    const F32Job ja{p.A, p.asi, p.ask, (int)M, (int)K, ta, Kp, marks, (int)(Mp / 32)};
+    const F32Job jb{p.B, p.bsj, p.bsk, (int)N, (int)K, tb, Kp, marks + Mp * (Kp / BK), (int)(Np / 32)};
+    stage_f32_kernel<<<dim3((unsigned)((Mp + Np) / 32), (unsigned)(Kp / 64)), 256, 0, s>>>(ja, jb);
+    NLA_CHECK_LAUNCH("stage_f32_kernel");
+  }
+  CUtensorMap mA, mB;
+  NLA_TRY(staged_map(&mA, ta, (uint64_t)Kp, (uint64_t)(SL * Mp)));
+  NLA_TRY(staged_map(&mB, tb, (uint64_t)Kp, (uint64_t)(SL * Np)));
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  std::call_once(once, [] {
+    st = cudaFuncSetAttribute(umma_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32_SMEM);
+  });
+  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(umma_f32_kernel)");
+  TraceScope trace(NLA_K_GEMM_UMMA, s, 6.0 * 2.0 * (double)M * (double)N * (double)K,
+                   (double)SL * 2.0 * (double)(Mp + Np) * Kp + 8.0 * (double)M * (double)N);
+  umma_f32_kernel<<<(unsigned)((int64_t)p.tiles_m * p.tiles_n), F32_THREADS, F32_SMEM, s>>>(mA, mB, p);
+  NLA_CHECK_LAUNCH("umma_f32_kernel");
+  return NLA_OK;
+}
+
+}  // namespace nla
