@@ -152,6 +152,8 @@ class NLAArgumentError(NLAError, ValueError):
 def load(path: str | None = None):
     """Load the library (built in-tree by build.py) and declare signatures."""
     global _lib
+    if _lib is not None:
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib

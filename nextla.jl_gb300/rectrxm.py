@@ -93,10 +93,11 @@ def _check_operands(A, B, side):
         raise ValueError("A and B must have the same element type (%s vs %s)" % (A.dtype, B.dtype))
     if A.device != B.device:
         raise ValueError("A and B must be on the same device")
-    n = A.shape[0]
-    if len(A.shape) != 2 or A.shape[1] != n:
+    sa, sb = A.shape, B.shape
+    n = sa[0]
+    if len(sa) != 2 or sa[1] != n:
         raise ValueError("A must be square, got %s" % (tuple(A.shape),))
-    if len(B.shape) != 2 or (side == "L" and B.shape[0] != n) or (side == "R" and B.shape[1] != n):
+    if len(sb) != 2 or (side == "L" and sb[0] != n) or (side == "R" and sb[1] != n):
         raise ValueError("B of shape %s does not conform with A of size %d for side %r" % (tuple(B.shape), n, side))
 
 
@@ -380,56 +381,71 @@ def unified_rectrxm_(side, uplo, transpose, alpha, func, A, B, *, native=False, 
     or forms B := alpha op(A) B ('M', 'L') / alpha B op(A) ('M', 'R'), in place
     in B, and returns B.  A is n x n; only its ``uplo`` triangle is read.
 
-    By default the recursion runs here, as the reference's Julia host code
-    does, with the reference's thresholds (256 for solves, 16 for multiplies,
-    src/rectrxm.jl:52,63) unless ``thresholds=(s, m)`` is given.  With
-    ``native=True`` the whole recursion runs inside the library (nla_trxm),
-    with its own tuned cut-offs unless ``thresholds`` is given.
+    The recursion runs inside the library, one call (nla_trxm_ex), with its
+    own tuned cut-offs unless ``thresholds=(s, m)`` is given (the reference's
+    are 256 for solves and 16 for multiplies, src/rectrxm.jl:52,63).  What
+    that call cannot express (conjugated or transposed views of a complex A
+    with 'C', a complex alpha with thresholds, thresholds outside 1..1024)
+    runs ``unified_rec`` here, as the reference's Julia host code does, with
+    the reference's thresholds; ``native=True`` refuses it instead.
     """
     _check_flags(side, uplo, transpose, func)
     _check_operands(A, B, side)
-    cplx = _is_complex(B)
     if B.is_conj():
         raise ValueError("B must not be a conjugate view (resolve it with B.resolve_conj())")
+    cplx = _is_complex(B)
     n = A.shape[0]
+    a, lda, ta = _mat(A)
     if native:
-        a, lda, ta = _mat(A)
-        b, ldb, tb = _mat(B)
-        if tb:
-            raise ValueError("B must be a column-major view")
         if ta & 2:
             raise ValueError("pass A without torch's conjugate bit and use transpose='C'")
-        tr, up = transpose, uplo
-        if ta:  # A is a transposed view of its parent: fold that into the flags
-            if cplx and transpose == "C":
-                raise ValueError("a transposed view of a complex A with transpose='C' is a conjugate without "
-                                 "transpose, which unified_rectrxm! cannot express; pass the parent")
-            tr = "N" if transpose in ("T", "C") else "T"
-            up = "U" if uplo == "L" else "L"
-        m = B.shape[1] if side == "L" else B.shape[0]
-        L = _lib.load()
-        if cplx and complex(alpha).imag != 0.0:
-            if thresholds is not None:
-                raise ValueError("thresholds are not supported with a complex alpha")
-            a_ = complex(alpha)
-            _lib.check(L.nla_trxm_complex(_lib.ch(side), _lib.ch(up), _lib.ch(tr), a_.real, a_.imag, _lib.ch(func),
+        if ta and cplx and transpose == "C":
+            raise ValueError("a transposed view of a complex A with transpose='C' is a conjugate without "
+                             "transpose, which unified_rectrxm! cannot express; pass the parent")
+        if cplx and complex(alpha).imag != 0.0 and thresholds is not None:
+            raise ValueError("thresholds are not supported with a complex alpha")
+    elif (ta & 2 or (ta and cplx and transpose == "C")
+          or (thresholds is not None and (not all(1 <= int(t) <= 1024 for t in thresholds)
+                                          or (cplx and complex(alpha).imag != 0.0)))):
+        return _host_driven(side, uplo, transpose, alpha, func, A, B, thresholds)
+    b, ldb, tb = _mat(B)
+    if tb:
+        raise ValueError("B must be a column-major view")
+    m = B.shape[1] if side == "L" else B.shape[0]
+    if ta:  # A is a transposed view of its parent: fold that into the flags
+        transpose = "T" if transpose == "N" else "N"
+        uplo = "U" if uplo == "L" else "L"
+    L = _lib.load()
+    if cplx:
+        al = complex(alpha)
+        if al.imag != 0.0:
+            _lib.check(L.nla_trxm_complex(_CH[side], _CH[uplo], _CH[transpose], al.real, al.imag, _CH[func],
                                           _dtype_code(B), n, m, a, lda, b, ldb, _stream(B)))
             return B
-        cs, cm = thresholds if thresholds is not None else (0, 0)
-        _lib.check(L.nla_trxm_ex(_lib.ch(side), _lib.ch(up), _lib.ch(tr), float(complex(alpha).real),
-                                 _lib.ch(func), _dtype_code(B), n, m, a, lda, b, ldb, int(cs), int(cm), _stream(B)))
-        return B
+        alpha = al.real
+    elif native:
+        alpha = complex(alpha).real
+    cs, cm = thresholds if thresholds is not None else (0, 0)
+    _lib.check(L.nla_trxm_ex(_CH[side], _CH[uplo], _CH[transpose], float(alpha), _CH[func], _dtype_code(B), n, m, a,
+                             lda, b, ldb, int(cs), int(cm), _stream(B)))
+    return B
 
+
+_CH = {c: c.encode() for c in "LRUNTCSM"}
+
+
+def _host_driven(side, uplo, transpose, alpha, func, A, B, thresholds):
+    """unified_rectrxm! with the recursion on the host (src/rectrxm.jl:43-76)."""
     threshold = 16 if thresholds is None else int(thresholds[1])
     if transpose in ("T", "C"):
         # Transpose(A), or Adjoint(A): for complex data the conjugate view,
         # which the base cases and updates read through torch's conjugate bit.
-        A = A.T.conj() if (cplx and transpose == "C") else A.T
+        A = A.T.conj() if (_is_complex(B) and transpose == "C") else A.T
         uplo = "U" if uplo == "L" else "L"
     if func == "S":
         threshold = 256 if thresholds is None else int(thresholds[0])
         scale_(B, alpha)
-    unified_rec(func, side, uplo, A, n, B, threshold)
+    unified_rec(func, side, uplo, A, A.shape[0], B, threshold)
     if func == "M":
         scale_(B, alpha)
     return B
