@@ -186,22 +186,25 @@ static bool f32_umma_wanted(int64_t N, int64_t M, int64_t K) {
 }
 
 size_t update_scratch_bytes(int dtype, int64_t N, int64_t M, int64_t K) {
-  return dtype == NLA_F32 && f32_umma_wanted(N, M, K) ? f32_update_bytes(N, M, K) : 0;
+  if (dtype == NLA_C32) N *= 2, K *= 2;  // real rows
+  return (dtype == NLA_F32 || dtype == NLA_C32) && f32_umma_wanted(N, M, K) ? f32_update_bytes(N, M, K) : 0;
 }
 
 // Float16 updates large enough to fill 128 x 128 tiles run on the tensor
-// cores (FP32 accumulation), Float32 ones as products of BF16 terms;
-// everything else on CUDA cores.
+// cores (FP32 accumulation), Float32 and ComplexF32 ones as products of BF16
+// terms; everything else on CUDA cores.
 int launch_gemm(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
                 cudaStream_t s, void* ws, size_t ws_bytes) {
-  if (is_complex(dtype)) return launch_gemm_complex(dtype, N, M, K, alpha, A, B, C, s);
   if (dtype == NLA_F16 && umma_enabled() && N >= 128 && M >= 128 && K >= 64)
     return launch_sliced_gemm(N, M, K, alpha, A, B, C, NLA_F16, NLA_F16, 1, false, nullptr, 0, s);
   if (const size_t need = C.t ? 0 : update_scratch_bytes(dtype, N, M, K)) {
-    if (ws && ws_bytes >= need) return launch_gemm_f32_umma(N, M, K, alpha, A, B, C, ws, s);
+    const bool cx = dtype == NLA_C32;
+    const int64_t rows = cx ? 2 * N : N, k = cx ? 2 * K : K;
+    if (ws && ws_bytes >= need) return launch_gemm_f32_umma(rows, M, k, alpha, A, B, C, ws, cx, s);
     const Scratch own(s, need);
-    if (own.p) return launch_gemm_f32_umma(N, M, K, alpha, A, B, C, own.p, s);
+    if (own.p) return launch_gemm_f32_umma(rows, M, k, alpha, A, B, C, own.p, cx, s);
   }
+  if (is_complex(dtype)) return launch_gemm_complex(dtype, N, M, K, alpha, A, B, C, s);
   return launch_gemm_simt(dtype, N, M, K, alpha, A, B, C, s);
 }
 
@@ -365,7 +368,9 @@ int trxm_impl(char side, char uplo, char trans, double alpha, char func, int dty
   };
   // Scratch for the largest update, the top split's.
   const int64_t mid = split_point(n), big = mid > n - mid ? mid : n - mid;
-  const Scratch ws(s, n > c.threshold ? update_scratch_bytes(dtype, big, m, big) : 0);
+  const Scratch ws(s, n <= c.threshold ? 0
+                      : side == 'L'  ? update_scratch_bytes(dtype, big, m, big)
+                                     : update_scratch_bytes(dtype, m, big, big));
   c.ws = ws.p;
   c.ws_bytes = ws.bytes;
   if (func == 'S') NLA_TRY(scale());  // src/rectrxm.jl:64

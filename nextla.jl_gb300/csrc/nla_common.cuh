@@ -148,6 +148,8 @@ int launch_scale(int dtype, int64_t rows, int64_t cols, double alpha, const Mat&
 bool is_complex(int dtype);
 int launch_leaf_complex(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A, const Mat& B,
                         cudaStream_t s, bool unit);
+int launch_leaf_strips_complex(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A,
+                               const Mat& B, cudaStream_t s, bool unit);
 int launch_gemm_complex(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B,
                         const Mat& C, cudaStream_t s);
 int launch_scale_complex(int dtype, int64_t rows, int64_t cols, double alpha_re, double alpha_im, const Mat& B,
@@ -160,10 +162,10 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
                        int in_dtype, int out_dtype, int S, bool bf16, void* ws, size_t ws_bytes, cudaStream_t s);
 size_t sliced_workspace_bytes(int64_t M, int64_t N, int64_t K, int S);
 
-// Float32 update on the tensor cores (nla_umma_f32.cu), scratch of
-// f32_update_bytes.
+// Float32 (or, with cplx, ComplexF32 in real rows) update on the tensor cores
+// (nla_umma_f32.cu), scratch of f32_update_bytes.
 int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
-                         void* ws, cudaStream_t s);
+                         void* ws, bool cplx, cudaStream_t s);
 size_t f32_update_bytes(int64_t M, int64_t N, int64_t K);
 
 // An operand staged for the tensor cores: S K-major 16-bit slices of a

@@ -6,145 +6,38 @@
 // (src/rectrxm.jl:101), though its base-case docstrings list complex ones
 // (src/trsm.jl:180-183).  These kernels run the same recursion on complex
 // data: trans 'T' reads A transposed, 'C' reads its conjugate transpose (the
-// Adjoint wrapper), and the arithmetic is ordinary complex arithmetic, every
-// product formed with fused multiply-adds of the real parts and every
-// quotient with Smith's algorithm (R. L. Smith, "Algorithm 116: Complex
-// division", CACM 5(8), 1962).
+// Adjoint wrapper), and the arithmetic is ordinary complex arithmetic
+// (nla_cplx.cuh).  Diagonal blocks run on the strip kernel of the real types
+// (nla_leaf_strip.cuh).
 //
 // Values are interleaved (re, im) pairs, column-major, as Julia and torch
-// store them.  All kernels work on the canonical lower-left problem of the
-// real diagonal-block kernels: side 'R' becomes side 'L' on transposed
-// views, uplo 'U' becomes lower by reversing the block's index order.
+// store them.
 #include <mutex>
 
 #include "nla_common.cuh"
+#include "nla_cplx.cuh"
 
 namespace nla {
 namespace cx {
-
-template <typename R>
-struct alignas(2 * sizeof(R)) cpx {
-  R re, im;
-};
-
-template <typename R> __device__ __forceinline__ cpx<R> mk(R a, R b) { return cpx<R>{a, b}; }
-template <typename R> __device__ __forceinline__ cpx<R> zero() { return cpx<R>{R(0), R(0)}; }
-template <typename R> __device__ __forceinline__ cpx<R> conj_if(cpx<R> a, bool c) { return c ? mk(a.re, -a.im) : a; }
-// c + a b
-template <typename R> __device__ __forceinline__ cpx<R> fma_c(cpx<R> a, cpx<R> b, cpx<R> c) {
-  return mk(fma(a.re, b.re, fma(-a.im, b.im, c.re)), fma(a.re, b.im, fma(a.im, b.re, c.im)));
-}
-// c - a b
-template <typename R> __device__ __forceinline__ cpx<R> fms_c(cpx<R> a, cpx<R> b, cpx<R> c) {
-  return mk(fma(-a.re, b.re, fma(a.im, b.im, c.re)), fma(-a.re, b.im, fma(-a.im, b.re, c.im)));
-}
-// a / b, Smith's algorithm.
-template <typename R> __device__ __forceinline__ cpx<R> div(cpx<R> a, cpx<R> b) {
-  if (fabs(b.re) >= fabs(b.im)) {
-    const R t = b.im / b.re, den = b.re + b.im * t;
-    return mk((a.re + a.im * t) / den, (a.im - a.re * t) / den);
-  }
-  const R t = b.re / b.im, den = b.im + b.re * t;
-  return mk((a.re * t + a.im) / den, (a.im * t - a.re) / den);
-}
-
-// Canonical-coordinate views (see the file comment): element (i, k) of the
-// canonical lower triangle and (i, c) of the right-hand sides.
-struct View {
-  const void* A;
-  int64_t lda;
-  int tA, conj, rev, unit;
-  void* B;
-  int64_t ldb;
-  int tB;
-  int n;
-  int64_t m;
-};
-
-template <typename R>
-__device__ __forceinline__ cpx<R> a_get(const View& v, int i, int k) {
-  const int r = v.rev ? v.n - 1 - i : i, c = v.rev ? v.n - 1 - k : k;
-  const cpx<R>* A = static_cast<const cpx<R>*>(v.A);
-  return conj_if(A[mat_off(r, c, v.lda, v.tA)], v.conj != 0);
-}
-template <typename R>
-__device__ __forceinline__ cpx<R>* b_ptr(const View& v, int i, int64_t col) {
-  const int r = v.rev ? v.n - 1 - i : i;
-  return static_cast<cpx<R>*>(v.B) + mat_off(r, col, v.ldb, v.tB);
-}
-
-constexpr int LEAF_COLS = 64;   // right-hand sides per CTA, one per thread
-constexpr int LEAF_PANEL = 32;  // rows of the triangle staged at a time
-
-// Diagonal-block solve X := L^{-1} X (func 'S') or multiply X := L X ('M')
-// for LEAF_COLS right-hand sides per CTA, one per thread.  The CTA's block of
-// X lives in shared memory (column per thread: conflict-free); the rows of L
-// are staged LEAF_PANEL at a time and read as broadcasts.
-// Solve: x_r = (b_r - sum_{k<r} l_rk x_k) / l_rr, rows in increasing order.
-// Multiply: x_r = sum_{k<=r} l_rk b_k with k increasing (the reference's
-// order, src/trmm.jl:90-94), rows from the last so that each b_k is still
-// the old value when read.
-template <typename R, bool SOLVE>
-__global__ void __launch_bounds__(LEAF_COLS) cplx_leaf_kernel(View v) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  cpx<R>* X = reinterpret_cast<cpx<R>*>(smem_raw);  // n x LEAF_COLS
-  cpx<R>* Lp = X + (size_t)v.n * LEAF_COLS;          // LEAF_PANEL x n
-  const int t = threadIdx.x, n = v.n;
-  const int64_t col = (int64_t)blockIdx.x * LEAF_COLS + t;
-  const bool live = col < v.m;
-  for (int r = 0; r < n; ++r) X[r * LEAF_COLS + t] = live ? *b_ptr<R>(v, r, col) : zero<R>();
-  const int npanels = (n + LEAF_PANEL - 1) / LEAF_PANEL;
-  for (int pi = 0; pi < npanels; ++pi) {
-    const int p = SOLVE ? pi : npanels - 1 - pi;
-    const int p0 = p * LEAF_PANEL, pw = min(LEAF_PANEL, n - p0);
-    __syncthreads();
-    // Rows p0 .. p0 + pw of L, columns 0 .. p0 + pw (k <= r; the diagonal
-    // is taken as 1 for a unit-diagonal view).
-    for (int idx = t; idx < pw * (p0 + pw); idx += LEAF_COLS) {
-      const int i = idx / (p0 + pw), k = idx % (p0 + pw);
-      const int r = p0 + i;
-      cpx<R> val = zero<R>();
-      if (k < r) val = a_get<R>(v, r, k);
-      else if (k == r) val = v.unit ? mk(R(1), R(0)) : a_get<R>(v, r, k);
-      Lp[i * n + k] = val;
-    }
-    __syncthreads();
-    for (int ii = 0; ii < pw; ++ii) {
-      const int i = SOLVE ? ii : pw - 1 - ii;
-      const int r = p0 + i;
-      const cpx<R>* l = Lp + i * n;
-      if (SOLVE) {
-        cpx<R> x = X[r * LEAF_COLS + t];
-        for (int k = 0; k < r; ++k) x = fms_c(l[k], X[k * LEAF_COLS + t], x);
-        X[r * LEAF_COLS + t] = div(x, l[r]);
-      } else {
-        cpx<R> x = zero<R>();
-        for (int k = 0; k <= r; ++k) x = fma_c(l[k], X[k * LEAF_COLS + t], x);
-        X[r * LEAF_COLS + t] = x;
-      }
-    }
-  }
-  if (live)
-    for (int r = 0; r < n; ++r) *b_ptr<R>(v, r, col) = X[r * LEAF_COLS + t];
-}
 
 // C (N x M) += alpha * op(A) (N x K) * op(B) (K x M), alpha real (+-1 in
 // the recursion).  64 x 64 tiles, 256 threads, each a 4 x 4 register tile;
 // K in chunks of 16 staged in shared memory; conjugation applied as the
 // operands are staged.
-constexpr int GT = 64, GK = 16;
-template <typename R>
+constexpr int GK = 16;
+template <typename R, int GT>
 __global__ void __launch_bounds__(256) cplx_gemm_kernel(int64_t N, int64_t M, int64_t K, R alpha, const cpx<R>* A,
                                                         int64_t lda, int tA, int cA, const cpx<R>* B, int64_t ldb,
                                                         int tB, int cB, cpx<R>* C, int64_t ldc) {
   __shared__ cpx<R> As[GK][GT + 1], Bs[GK][GT + 1];
   const int t = threadIdx.x, tr = t % 16, tc = t / 16;
   const int64_t i0 = (int64_t)blockIdx.x * GT, j0 = (int64_t)blockIdx.y * GT;
-  cpx<R> acc[4][4];
+  constexpr int RT = GT / 16;  // rows and columns per thread
+  cpx<R> acc[RT][RT];
 #pragma unroll
-  for (int a = 0; a < 4; ++a)
+  for (int a = 0; a < RT; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) acc[a][b] = zero<R>();
+    for (int b = 0; b < RT; ++b) acc[a][b] = zero<R>();
   for (int64_t k0 = 0; k0 < K; k0 += GK) {
     for (int idx = t; idx < GK * GT; idx += 256) {
       // op(A)(i, k): threads along i for a plain view, along k for a transposed one.
@@ -162,24 +55,24 @@ __global__ void __launch_bounds__(256) cplx_gemm_kernel(int64_t N, int64_t M, in
     __syncthreads();
 #pragma unroll 4
     for (int k = 0; k < GK; ++k) {
-      cpx<R> av[4], bv[4];
+      cpx<R> av[RT], bv[RT];
 #pragma unroll
-      for (int a = 0; a < 4; ++a) av[a] = As[k][tr + 16 * a];
+      for (int a = 0; a < RT; ++a) av[a] = As[k][tr + 16 * a];
 #pragma unroll
-      for (int b = 0; b < 4; ++b) bv[b] = Bs[k][tc + 16 * b];
+      for (int b = 0; b < RT; ++b) bv[b] = Bs[k][tc + 16 * b];
 #pragma unroll
-      for (int a = 0; a < 4; ++a)
+      for (int a = 0; a < RT; ++a)
 #pragma unroll
-        for (int b = 0; b < 4; ++b) acc[a][b] = fma_c(av[a], bv[b], acc[a][b]);
+        for (int b = 0; b < RT; ++b) acc[a][b] = fma_c(av[a], bv[b], acc[a][b]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int a = 0; a < 4; ++a) {
+  for (int a = 0; a < RT; ++a) {
     const int64_t i = i0 + tr + 16 * a;
     if (i >= N) continue;
 #pragma unroll
-    for (int b = 0; b < 4; ++b) {
+    for (int b = 0; b < RT; ++b) {
       const int64_t j = j0 + tc + 16 * b;
       if (j >= M) continue;
       cpx<R>* p = C + i + j * ldc;
@@ -205,30 +98,11 @@ __global__ void cplx_scale_kernel(int64_t rows, int64_t cols, double are, double
   }
 }
 
-template <typename R, bool SOLVE>
-int launch_leaf_r(const View& v, cudaStream_t s) {
-  const size_t smem = ((size_t)v.n * LEAF_COLS + (size_t)LEAF_PANEL * v.n) * sizeof(cpx<R>);
-  if (smem > 200 * 1024) return fail(NLA_ERR_UNSUPPORTED, "complex diag block: block too large");
-  const int64_t grid = (v.m + LEAF_COLS - 1) / LEAF_COLS;
-  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "complex diag block: too many right-hand sides");
-  static std::once_flag once;
-  static cudaError_t st = cudaSuccess;
-  std::call_once(once, [] {
-    st = cudaFuncSetAttribute(cplx_leaf_kernel<R, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-  });
-  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(cplx_leaf_kernel)");
-  TraceScope trace(SOLVE ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, s, 4.0 * (double)v.n * v.n * (double)v.m,
-                   (double)sizeof(cpx<R>) * ((double)v.n * (v.n + 1) / 2 + 2.0 * (double)v.n * v.m));
-  cplx_leaf_kernel<R, SOLVE><<<(unsigned)grid, LEAF_COLS, smem, s>>>(v);
-  NLA_CHECK_LAUNCH("cplx_leaf_kernel");
-  return NLA_OK;
-}
-
 }  // namespace cx
 
 bool is_complex(int dtype) { return dtype == NLA_C32 || dtype == NLA_C64; }
 
-constexpr int64_t CPLX_LEAF_MAX = 128;  // rows of a complex diagonal block held in shared memory
+constexpr int64_t CPLX_LEAF_MAX = 128;  // rows of a complex diagonal block
 
 int launch_leaf_complex(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A, const Mat& B,
                         cudaStream_t s, bool unit) {
@@ -242,45 +116,33 @@ int launch_leaf_complex(char func, char side, char uplo, int dtype, int64_t n, i
     c.unit = unit;
     return recurse(c, A, n, B);
   }
-  cx::View v;
-  v.A = A.p;
-  v.lda = A.ld;
-  v.tA = A.t;
-  v.conj = A.c;
-  v.B = B.p;
-  v.ldb = B.ld;
-  v.tB = 0;
-  v.unit = unit ? 1 : 0;
-  v.n = (int)n;
-  v.m = m;
-  if (side == 'R') {  // X op(A) = B  <=>  op(A)^T X^T = B^T (no conjugation added)
-    v.tA = !v.tA;
-    v.tB = 1;
-    uplo = uplo == 'L' ? 'U' : 'L';
-  }
-  v.rev = uplo == 'U';
-  if (dtype == NLA_C64)
-    return func == 'S' ? cx::launch_leaf_r<double, true>(v, s) : cx::launch_leaf_r<double, false>(v, s);
-  return func == 'S' ? cx::launch_leaf_r<float, true>(v, s) : cx::launch_leaf_r<float, false>(v, s);
+  return launch_leaf_strips_complex(func, side, uplo, dtype, n, m, A, B, s, unit);
 }
 
 int launch_gemm_complex(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, const Mat& B,
                         const Mat& C, cudaStream_t s) {
   if (N <= 0 || M <= 0) return NLA_OK;
   if (C.t) return fail(NLA_ERR_UNSUPPORTED, "gemm: transposed output view");
-  const int64_t gx = (N + cx::GT - 1) / cx::GT, gy = (M + cx::GT - 1) / cx::GT;
+  // Tiles as in the real update: 64 x 64, or 32 x 32 where that divides the
+  // output more evenly over the SMs (measured for ComplexF32 1000 x 128 x 128,
+  // 32 against 128 CTAs).
+  const int64_t sms = num_sms();
+  auto tiles = [&](int64_t t) { return ((N + t - 1) / t) * ((M + t - 1) / t); };
+  const int64_t w64 = (tiles(64) + sms - 1) / sms * (64 * 64), w32 = (tiles(32) + sms - 1) / sms * (32 * 32 * 3 / 2);
+  const int gt = w32 < w64 && M <= 65535 * 32ll ? 32 : 64;
+  const int64_t gx = (N + gt - 1) / gt, gy = (M + gt - 1) / gt;
   if (gx > 2147483647LL || gy > 65535) return fail(NLA_ERR_UNSUPPORTED, "gemm: matrix too large for one launch");
   const size_t es = dtype == NLA_C64 ? 16 : 8;
   TraceScope trace(NLA_K_GEMM_SIMT, s, 8.0 * (double)N * (double)M * (double)K,
                    (double)es * ((double)N * K + (double)K * M + 2.0 * (double)N * M));
-  if (dtype == NLA_C64)
-    cx::cplx_gemm_kernel<double><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(
-        N, M, K, alpha, static_cast<const cx::cpx<double>*>(A.p), A.ld, A.t, A.c,
-        static_cast<const cx::cpx<double>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<double>*>(C.p), C.ld);
-  else
-    cx::cplx_gemm_kernel<float><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(
-        N, M, K, (float)alpha, static_cast<const cx::cpx<float>*>(A.p), A.ld, A.t, A.c,
-        static_cast<const cx::cpx<float>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<float>*>(C.p), C.ld);
+  const dim3 grid((unsigned)gx, (unsigned)gy);
+  auto run = [&](auto kernel, auto one) {
+    using R = decltype(one);
+    kernel<<<grid, 256, 0, s>>>(N, M, K, (R)alpha, static_cast<const cx::cpx<R>*>(A.p), A.ld, A.t, A.c,
+                                static_cast<const cx::cpx<R>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<R>*>(C.p), C.ld);
+  };
+  if (dtype == NLA_C64) gt == 64 ? run(cx::cplx_gemm_kernel<double, 64>, 1.0) : run(cx::cplx_gemm_kernel<double, 32>, 1.0);
+  else gt == 64 ? run(cx::cplx_gemm_kernel<float, 64>, 1.0f) : run(cx::cplx_gemm_kernel<float, 32>, 1.0f);
   NLA_CHECK_LAUNCH("cplx_gemm_kernel");
   return NLA_OK;
 }

@@ -6,9 +6,9 @@
 // The canonical-form mapping and the column-per-thread Float64 solve are in
 // nla_leaf.cuh, the strip kernel that runs every other block in
 // nla_leaf_strip.cuh.
-#include <mutex>
-
 #include <cstdlib>
+#include <mutex>
+#include <type_traits>
 
 #include "nla_leaf.cuh"
 #include "nla_leaf_strip.cuh"
@@ -125,20 +125,24 @@ int launch_strip(const LeafArgs& g, cudaStream_t s) {
 template <typename T, bool SOLVE>
 int launch_strips(const LeafArgs& g, cudaStream_t s) {
   using Tc = typename Elem<T>::compute;
-  constexpr bool F64 = sizeof(Tc) == 8;
-  const int64_t sms = num_sms(), c = F64 ? 1 : 32;
+  constexpr bool CX = !std::is_floating_point<Tc>::value;
+  constexpr bool F64 = sizeof(Tc) == (CX ? 16 : 8);
+  constexpr int WIDEST = F64 ? (CX ? 16 : 32) : (CX ? 32 : 64);
+  const int64_t sms = num_sms(), c = F64 ? 1 : CX ? 8 : 32;
   int best = 0;
   int64_t cost = 0;
   for (int w : {64, 32, 16, 8, 4, 2}) {
-    if (F64 && w > 32) continue;
+    if (w > WIDEST) continue;
     if (strip_smem_elems<Tc>(g.n, 32, w < 8 ? 1 : w / 8, w < 8 ? w : 8) * sizeof(Tc) > STRIP_SMEM_MAX && w > 2) continue;
     const int64_t grid = (g.m + w - 1) / w, k = (grid + sms - 1) / sms * (w + c);
     if (best == 0 || k < cost) best = w, cost = k;
   }
   switch (best) {
     case 64:
-      if constexpr (!F64) return launch_strip<T, 32, 8, 8, SOLVE>(g, s);
-    case 32: return F64 ? launch_strip<T, 16, 2, 8, SOLVE>(g, s) : launch_strip<T, 32, 4, 8, SOLVE>(g, s);
+      if constexpr (WIDEST >= 64) return launch_strip<T, 32, 8, 8, SOLVE>(g, s);
+    case 32:
+      if constexpr (WIDEST >= 32)
+        return F64 ? launch_strip<T, 16, 2, 8, SOLVE>(g, s) : launch_strip<T, 32, 4, 8, SOLVE>(g, s);
     case 16: return F64 ? launch_strip<T, 16, 1, 8, SOLVE>(g, s) : launch_strip<T, 32, 2, 8, SOLVE>(g, s);
     case 8: return F64 ? launch_strip<T, 16, 1, 4, SOLVE>(g, s) : launch_strip<T, 32, 1, 8, SOLVE>(g, s);
     case 4: return launch_strip<T, 32, 1, 4, SOLVE>(g, s);
@@ -146,14 +150,9 @@ int launch_strips(const LeafArgs& g, cudaStream_t s) {
   }
 }
 
-}  // namespace
-
-int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A, const Mat& B,
-                cudaStream_t s, bool unit) {
-  if (is_complex(dtype)) return launch_leaf_complex(func, side, uplo, dtype, n, m, A, B, s, unit);
-  if (n <= 0 || m <= 0) return NLA_OK;
-  if (n > 1024) return fail(NLA_ERR_ARG, "diag block: n must be <= 1024");
-  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "diag block: transposed B view");
+// The canonical form of a diagonal block (side R as side L on transposed
+// views, uplo U as lower with the index order reversed).
+LeafArgs leaf_args(char side, char uplo, int64_t n, int64_t m, const Mat& A, const Mat& B, bool unit) {
   LeafArgs g;
   g.A = A.p;
   g.lda = A.ld;
@@ -162,6 +161,7 @@ int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m
   g.ldb = B.ld;
   g.tB = 0;
   g.unit = unit ? 1 : 0;
+  g.cj = A.c;
   g.n = (int)n;
   g.m = m;
   if (side == 'R') {  // X op(A) = B  <=>  op(A)^T X^T = B^T
@@ -170,6 +170,26 @@ int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m
     uplo = uplo == 'L' ? 'U' : 'L';
   }
   g.rev = uplo == 'U';
+  return g;
+}
+
+}  // namespace
+
+int launch_leaf_strips_complex(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A,
+                               const Mat& B, cudaStream_t s, bool unit) {
+  const LeafArgs g = leaf_args(side, uplo, n, m, A, B, unit);
+  if (dtype == NLA_C64)
+    return func == 'S' ? launch_strips<cx::cpx<double>, true>(g, s) : launch_strips<cx::cpx<double>, false>(g, s);
+  return func == 'S' ? launch_strips<cx::cpx<float>, true>(g, s) : launch_strips<cx::cpx<float>, false>(g, s);
+}
+
+int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m, const Mat& A, const Mat& B,
+                cudaStream_t s, bool unit) {
+  if (is_complex(dtype)) return launch_leaf_complex(func, side, uplo, dtype, n, m, A, B, s, unit);
+  if (n <= 0 || m <= 0) return NLA_OK;
+  if (n > 1024) return fail(NLA_ERR_ARG, "diag block: n must be <= 1024");
+  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "diag block: transposed B view");
+  const LeafArgs g = leaf_args(side, uplo, n, m, A, B, unit);
   if (func == 'S') {
     // Float64 blocks of up to 128 rows where one wave of wide CTAs fits and
     // strips of 32 columns would leave the last wave short: one right-hand

@@ -32,6 +32,7 @@ struct LeafArgs {
   int tB;
   int rev;
   int unit;  // unit diagonal: the diagonal of A is taken as 1 and not read
+  int cj;    // complex types: read the conjugates of A's elements
   int n;
   int64_t m;
 };

@@ -29,6 +29,7 @@
 // right-hand sides are read and written once.
 #pragma once
 
+#include "nla_cplx.cuh"
 #include "nla_leaf.cuh"
 
 namespace nla {
@@ -47,9 +48,55 @@ template <> struct StripTraits<float> {
   using Vec = float4;
   static constexpr int VK = 4;
 };
+template <> struct StripTraits<cx::cpx<float>> {
+  using Vec = float4;
+  static constexpr int VK = 2;
+};
+template <> struct StripTraits<cx::cpx<double>> {
+  using Vec = double2;
+  static constexpr int VK = 1;
+};
 constexpr int ST_KC = 128;  // columns of A per chunk
 __device__ __forceinline__ void st_unpack(const double2& v, double* o) { o[0] = v.x; o[1] = v.y; }
 __device__ __forceinline__ void st_unpack(const float4& v, float* o) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+
+__device__ __forceinline__ void st_unpack(const float4& v, cx::cpx<float>* o) {
+  o[0] = cx::mk(v.x, v.y);
+  o[1] = cx::mk(v.z, v.w);
+}
+__device__ __forceinline__ void st_unpack(const double2& v, cx::cpx<double>* o) { o[0] = cx::mk(v.x, v.y); }
+
+// The arithmetic of the strip, real and complex.
+template <typename Tc> struct StripMath {
+  __device__ static Tc zero() { return Tc(0); }
+  __device__ static Tc one() { return Tc(1); }
+  __device__ static Tc conj_if(Tc a, int) { return a; }
+  __device__ static Tc fma_(Tc a, Tc x, Tc c) { return fma(a, x, c); }
+  __device__ static Tc fms_(Tc a, Tc x, Tc c) { return fma(-a, x, c); }
+  __device__ static Tc shfl(Tc v, int src) { return __shfl_sync(0xffffffffu, v, src); }
+  __device__ static Tc inverse(Tc d) { return Tc(1) / d; }
+  // z / d with inv = 1 / d.
+  __device__ static Tc quotient(Tc z, Tc inv, Tc) { return z * inv; }
+};
+template <typename R> struct StripMath<cx::cpx<R>> {
+  using Tc = cx::cpx<R>;
+  __device__ static Tc zero() { return cx::zero<R>(); }
+  __device__ static Tc one() { return cx::mk(R(1), R(0)); }
+  __device__ static Tc conj_if(Tc a, int c) { return cx::conj_if(a, c != 0); }
+  __device__ static Tc fma_(Tc a, Tc x, Tc c) { return cx::fma_c(a, x, c); }
+  __device__ static Tc fms_(Tc a, Tc x, Tc c) { return cx::fms_c(a, x, c); }
+  __device__ static Tc shfl(Tc v, int src) {
+    return cx::mk(__shfl_sync(0xffffffffu, v.re, src), __shfl_sync(0xffffffffu, v.im, src));
+  }
+  __device__ static Tc inverse(Tc d) { return cx::div(one(), d); }
+  // The product with the reciprocal, corrected once by the remainder: as
+  // accurate as the quotient itself (a complex reciprocal carries several
+  // roundings), without a division in the triangle's chain.
+  __device__ static Tc quotient(Tc z, Tc inv, Tc d) {
+    const Tc q = cx::fma_c(z, inv, zero());
+    return cx::fma_c(cx::fms_c(q, d, z), inv, q);
+  }
+};
 
 // Column pitch of X: a multiple of the vector, at least n.
 template <typename Tc> __host__ __device__ constexpr int st_ldx(int n) {
@@ -63,7 +110,7 @@ template <typename Tc> __host__ __device__ constexpr size_t strip_smem_elems(int
   return (size_t)(32 / PB) * NC * WC * st_ldx<Tc>(n)              // X
          + (size_t)2 * PB * st_lda<Tc>()                          // A chunks
          + (size_t)2 * PB * (PB + 1)                              // panel triangles
-         + (size_t)((n + ST_ROWS - 1) / ST_ROWS * ST_ROWS)        // reciprocals of the diagonal
+         + (size_t)2 * ((n + ST_ROWS - 1) / ST_ROWS * ST_ROWS)    // the diagonal and its reciprocals
          + (WC < 8 ? (size_t)8 * NC * 32 : 0);                    // partial sums of the K groups
 }
 
@@ -73,6 +120,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   using Tc = typename Elem<T>::compute;
   using Tr = StripTraits<Tc>;
   using Vec = typename Tr::Vec;
+  using Mx = StripMath<Tc>;
   constexpr int KC = ST_KC, VK = Tr::VK, KG = 8 / WC, SUBS = 32 / PB, CW = SUBS * NC * WC;
   constexpr int DPER = PB * PB / ST_THREADS;    // triangle elements per thread
   constexpr int LDA = st_lda<Tc>();
@@ -82,7 +130,8 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   Tc* As = X + (size_t)CW * ldx;                    // 2 x PB x LDA
   Tc* Dg = As + 2 * PB * LDA;                    // 2 x PB x (PB + 1)
   Tc* inv = Dg + 2 * PB * (PB + 1);           // nr
-  Tc* part = inv + nr;                              // KG > 1: 8 warps x NC x 32
+  Tc* dia = inv + nr;                               // nr
+  Tc* part = dia + nr;                              // KG > 1: 8 warps x NC x 32
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int row = lane & (PB - 1), sub = lane / PB;
   const int wc = warp % WC, kg = warp / WC;
@@ -111,12 +160,12 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
     const T* p = A + (p0 + fi) * si + (k0 + fk) * sk;
     const int ni = n - p0 - fi, nk = kend - k0 - fk;  // slots inside: e ei < ni, e ek < nk
 #pragma unroll
-    for (int e = 0; e < PER; ++e) ra[e] = e * ei < ni && e * ek < nk ? Elem<T>::load(p + e * es) : Tc(0);
+    for (int e = 0; e < PER; ++e) ra[e] = e * ei < ni && e * ek < nk ? Mx::conj_if(Elem<T>::load(p + e * es), g.cj) : Mx::zero();
     if (diag) {
 #pragma unroll
       for (int e = 0; e < DPER; ++e) {
         const int i = g.tA ? di + e * de : di, k = g.tA ? dk : dk + e * de;
-        rd[e] = p0 + i < n && k < i ? Elem<T>::load(A + (p0 + i) * si + (p0 + k) * sk) : Tc(0);
+        rd[e] = p0 + i < n && k < i ? Mx::conj_if(Elem<T>::load(A + (p0 + i) * si + (p0 + k) * sk), g.cj) : Mx::zero();
       }
     }
   };
@@ -139,7 +188,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
           const int i = i0 + 32 * u;
-          v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c * bc) : Tc(0);
+          v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c * bc) : Mx::zero();
         }
 #pragma unroll
         for (int u = 0; u < BATCH; ++u)
@@ -153,7 +202,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
         const int i = i0 + RS * u;
-        v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c) : Tc(0);
+        v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c) : Mx::zero();
       }
 #pragma unroll
       for (int u = 0; u < BATCH; ++u)
@@ -161,8 +210,11 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
     }
   }
   if (SOLVE)
-    for (int i = t; i < nr; i += ST_THREADS)
-      inv[i] = g.unit || i >= n ? Tc(1) : Tc(1) / Elem<T>::load(A + i * (si + sk));
+    for (int i = t; i < nr; i += ST_THREADS) {
+      const Tc d = g.unit || i >= n ? Mx::one() : Mx::conj_if(Elem<T>::load(A + i * (si + sk)), g.cj);
+      dia[i] = d;
+      inv[i] = Mx::inverse(d);
+    }
   __syncthreads();
 
   Tc acc[NC];
@@ -170,7 +222,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   for (int p = 0; p < npan; ++p) {
     const int p0 = p * PB, kend = kend_of(p), nch = chunks_of(p);
 #pragma unroll
-    for (int q = 0; q < NC; ++q) acc[q] = Tc(0);
+    for (int q = 0; q < NC; ++q) acc[q] = Mx::zero();
     for (int ch = 0; ch < nch; ++ch, ++step) {
       const int k0 = ch * KC;
       Tc* Ab = As + (step & 1) * PB * LDA;
@@ -181,8 +233,8 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
         Tc v = ra[e];
         if (!SOLVE) {  // the panel's own triangle: zero above, one on a unit diagonal
           const int r = p0 + i, kk = k0 + k;
-          if (kk > r) v = Tc(0);
-          else if (kk == r && g.unit) v = r < n ? Tc(1) : Tc(0);
+          if (kk > r) v = Mx::zero();
+          else if (kk == r && g.unit) v = r < n ? Mx::one() : Mx::zero();
         }
         Ab[i * LDA + k] = v;
       }
@@ -212,7 +264,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
           Tc x[VK];
           st_unpack(*reinterpret_cast<const Vec*>(xr + (size_t)q * ldx + u * VK), x);
 #pragma unroll
-          for (int v = 0; v < VK; ++v) acc[q] = fma(a[v], x[v], acc[q]);
+          for (int v = 0; v < VK; ++v) acc[q] = Mx::fma_(a[v], x[v], acc[q]);
         }
       }
       if (last) {
@@ -234,12 +286,12 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 #pragma unroll
               for (int w = 1; w < KG; w *= 2)
 #pragma unroll
-                for (int h = 0; h + w < KG; h += 2 * w) s[h] += s[h + w];
+                for (int h = 0; h + w < KG; h += 2 * w) s[h] = s[h] + s[h + w];
               acc[q] = s[0];
             }
           }
           if constexpr (SOLVE) {
-            const Tc iv = inv[p0 + row];
+            const Tc iv = inv[p0 + row], dr = dia[p0 + row];
             Tc z[NC], d[PB - 1];
 #pragma unroll
             for (int j = 0; j < PB - 1; ++j) d[j] = Db[row * (PB + 1) + j];  // zero on and above the diagonal
@@ -249,11 +301,11 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
             for (int j = 0; j < PB - 1; ++j)
 #pragma unroll
               for (int q = 0; q < NC; ++q) {
-                const Tc xj = __shfl_sync(0xffffffffu, z[q] * iv, (lane & ~(PB - 1)) | j);
-                z[q] = row > j ? fma(-d[j], xj, z[q]) : z[q];
+                const Tc xj = Mx::shfl(Mx::quotient(z[q], iv, dr), (lane & ~(PB - 1)) | j);
+                if (row > j) z[q] = Mx::fms_(d[j], xj, z[q]);
               }
 #pragma unroll
-            for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = z[q] * iv;
+            for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = Mx::quotient(z[q], iv, dr);
             if constexpr (KG == 1) __syncwarp();
           } else {
 #pragma unroll

@@ -18,6 +18,10 @@
 // ordinary rounded additions.  That leaves fewer roundings per element than
 // the FMA chain of the CUDA-core update, whose error grows with K.
 //
+// ComplexF32 updates are the same product on real views: the complex C is
+// a real matrix of 2 M rows (re, im interleaved), op(B) one of 2 K rows, and
+// op(A) is staged as 2 M x 2 K, each a as the block (re, -im; im, re).
+//
 // What bounds it: the TMA feed (96 KiB of tiles per 64 values of K for six
 // 128 x 128 x 64 products): 1190 TFLOP/s of executed products, 199 of the
 // update's, at 4096 x 4096 x 8192 (FFMA update: 39.9).  Warps: 0 loads A, 1 issues MMAs, 2 loads B,
@@ -75,11 +79,23 @@ struct F32Params {
   int64_t ldc;
   float alpha;
   int* err;
+  int cplx;       // operands are complex (strides in complex elements), M and K count real rows
+  float ima, imb;  // -1 where the operand is conjugated, else 1
 };
 
 // One element in the order of the CUDA-core update: FMAs with k increasing.
 __device__ __noinline__ float plain_dot(const F32Params& p, int i, int j) {
   float s = 0.0f;
+  if (p.cplx) {
+    const float2* a = reinterpret_cast<const float2*>(p.A) + (int64_t)(i >> 1) * p.asi;
+    const float2* b = reinterpret_cast<const float2*>(p.B) + (int64_t)j * p.bsj;
+    for (int k = 0; k < p.K / 2; ++k) {
+      const float2 x = a[k * p.ask], y = b[k * p.bsk];
+      const float xi = p.ima * x.y, yi = p.imb * y.y;
+      s = (i & 1) ? fmaf(x.x, yi, fmaf(xi, y.x, s)) : fmaf(x.x, y.x, fmaf(-xi, yi, s));
+    }
+    return s;
+  }
   const float* a = p.A + (int64_t)i * p.asi;
   const float* b = p.B + (int64_t)j * p.bsj;
   for (int k = 0; k < p.K; ++k) s = fmaf(a[k * p.ask], b[k * p.bsk], s);
@@ -269,6 +285,8 @@ struct F32Job {
   const float* X;  // element (row, k) at X[row * si + k * sk]
   int64_t si, sk;
   int rows, K;
+  int cplx;  // 1: rows and K are pairs (re, im) of complex elements, as op(A); 2: only K, as op(B)
+  float im;  // sign of the imaginary parts
   __nv_bfloat16* out;
   int64_t k_pad;
   int* mark;   // the block of K's marks at mark[kb * rows_pad + row]
@@ -294,8 +312,16 @@ __global__ void __launch_bounds__(256) stage_f32_kernel(const F32Job a, const F3
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
     const int idx = t + 256 * e;
-    const int i = kfast ? idx >> 6 : idx & 31, k = kfast ? idx & 63 : idx >> 5;
-    v[e] = i0 + i < j.rows && k0 + k < j.K ? __ldg(j.X + (i0 + i) * j.si + (k0 + k) * j.sk) : 0.0f;
+    const int i = i0 + (kfast ? idx >> 6 : idx & 31), k = k0 + (kfast ? idx & 63 : idx >> 5);
+    const bool in = i < j.rows && k < j.K;
+    if (j.cplx == 0) {
+      v[e] = in ? __ldg(j.X + i * j.si + k * j.sk) : 0.0f;
+    } else {
+      const bool pair = j.cplx == 1;
+      const int part = pair ? (i ^ k) & 1 : k & 1;  // 0: real part, 1: imaginary
+      const float x = in ? __ldg(j.X + 2 * ((pair ? i >> 1 : i) * j.si + (k >> 1) * j.sk) + part) : 0.0f;
+      v[e] = part ? (pair && !(i & 1) ? -j.im : j.im) * x : x;
+    }
   }
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
@@ -337,8 +363,10 @@ size_t f32_update_bytes(int64_t M, int64_t N, int64_t K) {
   return terms_bytes(M, K) + terms_bytes(N, K) + marks_bytes(M, K) + marks_bytes(N, K) + 1024;
 }
 
+// cplx: ComplexF32 operands, with M and K counting their real rows (twice the
+// complex ones).
 int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
-                         void* ws, cudaStream_t s) {
+                         void* ws, bool cplx, cudaStream_t s) {
   const int64_t Mp = pad_to(M, BM), Np = pad_to(N, BN), Kp = pad_to(K, BK);
   uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(ws) + 1023) & ~uintptr_t(1023));
   auto* ta = reinterpret_cast<__nv_bfloat16*>(base);
@@ -365,13 +393,16 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.rows_a = (int)Mp;
   p.rows_b = (int)Np;
   p.C = static_cast<float*>(C.p);
-  p.ldc = C.ld;
+  p.ldc = cplx ? 2 * C.ld : C.ld;
   p.alpha = (float)alpha;
   p.err = err;
+  p.cplx = cplx ? 1 : 0;
+  p.ima = A.c ? -1.0f : 1.0f;
+  p.imb = B.c ? -1.0f : 1.0f;
   {
     TraceScope trace(NLA_K_SPLIT, s, 0.0, (double)(M + N) * (double)K * 4.0 + (double)(Mp + Np) * Kp * 2.0 * SL);
-    const F32Job ja{p.A, p.asi, p.ask, (int)M, (int)K, ta, Kp, marks, (int)(Mp / 32)};
-    const F32Job jb{p.B, p.bsj, p.bsk, (int)N, (int)K, tb, Kp, marks + Mp * (Kp / BK), (int)(Np / 32)};
+    const F32Job ja{p.A, p.asi, p.ask, (int)M, (int)K, p.cplx, p.ima, ta, Kp, marks, (int)(Mp / 32)};
+    const F32Job jb{p.B, p.bsj, p.bsk, (int)N, (int)K, 2 * p.cplx, p.imb, tb, Kp, marks + Mp * (Kp / BK), (int)(Np / 32)};
     stage_f32_kernel<<<dim3((unsigned)((Mp + Np) / 32), (unsigned)(Kp / 64)), 256, 0, s>>>(ja, jb);
     NLA_CHECK_LAUNCH("stage_f32_kernel");
   }

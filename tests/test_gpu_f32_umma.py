@@ -91,3 +91,64 @@ def test_f32_update_under_capture(pkg, cuda):
     graph.replay()
     torch.cuda.synchronize()
     assert np.linalg.norm(to_host(X) - to_host(Y)) < 1e-5 * np.linalg.norm(to_host(X))
+
+
+def _cdev(X, cuda, pad):
+    import torch
+
+    buf = torch.zeros((X.shape[1], X.shape[0] + pad), dtype=torch.complex64, device=cuda)
+    buf[:, : X.shape[0]] = torch.from_numpy(np.ascontiguousarray(X.T))
+    return buf.T[: X.shape[0]]
+
+
+@pytest.mark.parametrize("form", ["NN", "TN", "CN", "NC", "TT", "CC"])
+def test_c32_update(pkg, cuda, form):
+    """ComplexF32 on the same kernel (2 M x 2 K real operands): every
+    transposed and conjugated form, bound as above per real component with
+    sums of 2 K products."""
+    import torch
+
+    rng = np.random.default_rng(8)
+    for N, K, M in ((70, 130, 4000), (333, 129, 1000), (1001, 600, 130)):
+        A, B, C = ((rng.standard_normal(s) + 1j * rng.standard_normal(s)).astype(np.complex64)
+                   for s in ((N, K), (K, M), (N, M)))
+        op = {"N": lambda X: X, "T": lambda X: X.T, "C": lambda X: X.conj().T}
+        Ad, Bd, Cd = _cdev(op[form[0]](A), cuda, 1), _cdev(op[form[1]](B), cuda, 2), _cdev(C, cuda, 0)
+        view = {"N": lambda X: X, "T": lambda X: X.T, "C": lambda X: X.T.conj()}
+        pkg.matmul_(Cd, view[form[0]](Ad), view[form[1]](Bd), -1.0)
+        torch.cuda.synchronize()
+        got = Cd.cpu().numpy().astype(np.complex128)
+        A, B, C = (X.astype(np.complex128) for X in (A, B, C))
+        ref = C - A @ B
+        ar, ai, br, bi = np.abs(A.real), np.abs(A.imag), np.abs(B.real), np.abs(B.imag)
+        u = (12 + -(-2 * K // 64)) * 2.0 ** -24
+        assert (np.abs((got - ref).real) <= u * (np.abs(C.real) + ar @ br + ai @ bi)).all(), (form, N, K, M)
+        assert (np.abs((got - ref).imag) <= u * (np.abs(C.imag) + ar @ bi + ai @ br)).all(), (form, N, K, M)
+
+
+def test_c32_update_not_finite(pkg, cuda):
+    """An Inf or NaN component reaches exactly the outputs its products do."""
+    import torch
+
+    rng = np.random.default_rng(9)
+    N, K, M = 200, 200, 2000
+    A, B = ((rng.integers(-4, 5, s) + 1j * rng.integers(-4, 5, s)).astype(np.complex64) for s in ((N, K), (K, M)))
+    A[3, 4] = complex(np.inf, 1.0)
+    B[6, 77] = complex(2.0, np.nan)
+    Cd = _cdev(np.zeros((N, M), dtype=np.complex64), cuda, 0)
+    pkg.matmul_(Cd, _cdev(A, cuda, 0), _cdev(B, cuda, 0), 1.0)
+    torch.cuda.synchronize()
+    got = Cd.cpu().numpy()
+    with np.errstate(all="ignore"):
+        Ar, Ai, Br, Bi = (np.nan_to_num(X.astype(np.float64), nan=np.nan, posinf=np.inf) for X in
+                          (A.real, A.imag, B.real, B.imag))
+        re, im = Ar @ Br - Ai @ Bi, Ar @ Bi + Ai @ Br
+    keep = np.ones((N, M), dtype=bool)
+    keep[3, :] = False
+    keep[:, 77] = False
+    assert np.array_equal(got.real[keep], re[keep].astype(np.float32))
+    assert np.array_equal(got.imag[keep], im[keep].astype(np.float32))
+    rest = [j for j in range(M) if j != 77]
+    assert np.array_equal(np.isnan(got.real[3, rest]), np.isnan(re[3, rest]))
+    assert np.array_equal(np.isinf(got.real[3, rest]), np.isinf(re[3, rest]))
+    assert np.isnan(got.imag[:, 77]).all() and np.isnan(got.real[:, 77]).all()
