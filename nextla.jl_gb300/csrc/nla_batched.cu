@@ -584,30 +584,66 @@ struct MapArgs {
   int op;
 };
 
-// MAP_INIT: R = alpha B (Float64), X32 = (float) R, and (first group of each
-// system) A32 = (float) A over the n x n block; MAP_SET: B = (double) X32;
-// MAP_ADD: B += (double) X32.
+// MAP_INIT: R = alpha B (Float64), X32 = (float) R; MAP_SET: B = (double) X32;
+// MAP_ADD: B += (double) X32.  A warp per column, lanes along its rows, four
+// rows of loads in flight per lane.
+constexpr int MAP_UNROLL = 4;
 __global__ void __launch_bounds__(256) batched_map_kernel(MapArgs a) {
   const Group g = a.groups[blockIdx.x];
   const nla_batch_desc d = a.descs[g.sys];
-  const int n = (int)d.n;
-  const int total = n * g.ncols;
-  for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int64_t o = d.b_off + (int64_t)(idx % n) + (int64_t)(g.c0 + idx / n) * d.ldb;
-    if (a.op == MAP_INIT) {
-      const double r = a.alpha * a.B64[o];
-      a.R64[o] = r;
-      a.X32[o] = (float)r;
-    } else if (a.op == MAP_SET) {
-      a.B64[o] = (double)a.X32[o];
-    } else {
-      a.B64[o] += (double)a.X32[o];
+  const int n = (int)d.n, lane = threadIdx.x & 31;
+  for (int c = threadIdx.x >> 5; c < g.ncols; c += 8) {
+    const int64_t o = d.b_off + (int64_t)(g.c0 + c) * d.ldb;
+    for (int i0 = lane; i0 < n; i0 += 32 * MAP_UNROLL) {
+      double b[MAP_UNROLL];
+      float x[MAP_UNROLL];
+#pragma unroll
+      for (int u = 0; u < MAP_UNROLL; ++u) {
+        const int i = i0 + 32 * u;
+        b[u] = i < n && a.op != MAP_SET ? a.B64[o + i] : 0.0;
+        x[u] = i < n && a.op != MAP_INIT ? a.X32[o + i] : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < MAP_UNROLL; ++u) {
+        const int i = i0 + 32 * u;
+        if (i >= n) break;
+        if (a.op == MAP_INIT) {
+          const double r = a.alpha * b[u];
+          a.R64[o + i] = r;
+          a.X32[o + i] = (float)r;
+        } else if (a.op == MAP_SET) {
+          a.B64[o + i] = (double)x[u];
+        } else {
+          a.B64[o + i] = b[u] + (double)x[u];
+        }
+      }
     }
   }
-  if (a.op == MAP_INIT && g.c0 == 0) {
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-      const int64_t o = d.a_off + (int64_t)(idx % n) + (int64_t)(idx / n) * d.lda;
-      a.A32[o] = (float)a.A64[o];
+}
+
+// A32 = (float) A over the triangle the solves read (upper: stored above the
+// diagonal), one CTA per CAST_COLS columns of a system (the CTAs of its first
+// group), a warp per column.  Bound by DRAM; one CTA per system over the
+// whole block with a division per element took 2.9 ms for 2000 systems of
+// 16 to 1024 unknowns.
+constexpr int CAST_COLS = 64;
+__global__ void __launch_bounds__(256) batched_cast_kernel(MapArgs a, int upper) {
+  const Group g = a.groups[blockIdx.x];
+  if (g.c0 != 0) return;
+  const nla_batch_desc d = a.descs[g.sys];
+  const int n = (int)d.n, lane = threadIdx.x & 31;
+  const int c1 = min(n, ((int)blockIdx.y + 1) * CAST_COLS);
+  for (int c = (int)blockIdx.y * CAST_COLS + (threadIdx.x >> 5); c < c1; c += 8) {
+    const double* src = a.A64 + d.a_off + (int64_t)c * d.lda;
+    float* dst = a.A32 + d.a_off + (int64_t)c * d.lda;
+    const int r0 = upper ? 0 : c, r1 = upper ? c + 1 : n;
+    for (int i0 = r0 + lane; i0 < r1; i0 += 32 * MAP_UNROLL) {
+      double v[MAP_UNROLL];
+#pragma unroll
+      for (int u = 0; u < MAP_UNROLL; ++u) v[u] = i0 + 32 * u < r1 ? __ldg(src + i0 + 32 * u) : 0.0;
+#pragma unroll
+      for (int u = 0; u < MAP_UNROLL; ++u)
+        if (i0 + 32 * u < r1) dst[i0 + 32 * u] = (float)v[u];
     }
   }
 }
@@ -1665,6 +1701,10 @@ int nla_batch_solve_mixed_ex(nla_batch_plan p, double alpha, const void* A_pool,
   bat::MapArgs m{descs, groups, A64, p->a32, B64, p->r64, p->x32, alpha, bat::MAP_INIT};
   bat::batched_map_kernel<<<p->ngroups, 256, 0, s>>>(m);
   NLA_CHECK_LAUNCH("batched_map_kernel");
+  bat::batched_cast_kernel<<<dim3((unsigned)p->ngroups,
+                                  (unsigned)((p->n_max + bat::CAST_COLS - 1) / bat::CAST_COLS)),
+                             256, 0, s>>>(m, p->rev ^ p->tA);
+  NLA_CHECK_LAUNCH("batched_cast_kernel");
   auto solve32 = [&]() -> int {
     cudaError_t e = cudaMemsetAsync(p->p32->d_counters, 0, p->p32->counter_bytes, s);
     if (e != cudaSuccess) return cuda_status(e, "batch counter reset");
