@@ -204,6 +204,25 @@ struct ResidualTerm {
 int launch_exact_gemm(const Staged& A, const Staged& B, double alpha, const Mat& C, bool trans_out,
                       cudaStream_t s, const ResidualTerm* res = nullptr, long long* fixed_buf = nullptr);
 constexpr int EXACT_SLICES = 7;
+
+// The same exact product from 16 residues per element (nla_crt.cu).
+struct CrtStaged {
+  void* res;
+  int* e;
+  int64_t rows, rows_pad, K, K_pad;
+  int tri;  // as in Staged
+  bool row_operand;
+};
+bool crt_usable(int64_t M, int64_t N, int64_t K);
+size_t crt_staged_bytes(int64_t rows, int64_t K);
+size_t crt_planes_bytes(int64_t M, int64_t N);
+CrtStaged crt_layout(void* buf, int64_t rows, int64_t K, int tri, bool row_operand);
+int crt_stage(const Mat& X, const CrtStaged& sx, const Mat* Y, const CrtStaged* sy, cudaStream_t s);
+int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C, uint8_t* planes, cudaStream_t s,
+             const ResidualTerm* res = nullptr, bool d_col = false);
+int crt_set_wait_limit(uint64_t ns);
+bool crt_enabled();                                           // NLA_EXACT_KERNEL selects the slice kernels instead
+size_t crt_workspace_bytes(int64_t M, int64_t N, int64_t K);  // staged operands and planes of one update
 int workspace_get(cudaStream_t s, size_t bytes, void** out);
 int device_status(cudaStream_t s);
 int* device_error_word();  // device address of the error word nla_device_status reads (null on failure)

@@ -860,28 +860,71 @@ int leaf_pair_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   return NLA_OK;
 }
 
-// Stage the strict triangle of op(A) as the row operand of the residual
-// product: op(A) itself for side L, op(A)^T for side R.
-int stage_triangle(const Mat& Am, int64_t n, char side, char uplo, void* buf, Staged* out, cudaStream_t s) {
-  if (side == 'L') return stage_operand(Am, n, n, NLA_F64, EXACT_SLICES, true, uplo == 'L' ? 3 : 4, buf, out, s);
-  return stage_operand(transposed(Am), n, n, NLA_F64, EXACT_SLICES, true, uplo == 'L' ? 4 : 3, buf, out, s);
+// The exact residual product of a refinement: the strict triangle of op(A)
+// (op(A) itself for side L, op(A)^T for side R) staged once, X per sweep, as
+// residues (nla_crt.cu) or, where there is no memory for them, as slices.
+struct SplitResidual {
+  bool crt = false;
+  uint8_t* base = nullptr;  // op(A), then X, then the planes of the residues
+  Staged As{}, Xs{};
+  CrtStaged Ac{};
+};
+
+size_t split_residual_bytes(bool crt, char side, int64_t n, int64_t m) {
+  if (!crt) return staged_bytes(n, n, EXACT_SLICES) + staged_bytes(m, n, EXACT_SLICES) + 1024;
+  return crt_staged_bytes(n, n) + crt_staged_bytes(m, n) + (side == 'L' ? crt_planes_bytes(n, m) : crt_planes_bytes(m, n)) +
+         1024;
 }
 
-// R -= op(A) X (side L) or X op(A) (side R): exact slice products for the
-// strict triangle (As, staged by stage_triangle); the diagonal term and the
-// subtraction are folded into the exact kernel's epilogue (one rounding).
-int split_residual(const Mat& Am, const Staged& As, char side, int64_t n, int64_t m, const Mat& Xm, const Mat& Rm,
-                   void* xbuf, Staged* Xs, cudaStream_t s) {
-  // The epilogue subtracts the exact strict-triangle product and the FP64
-  // diagonal term from R (= alpha*B on entry) and rounds once.
-  const ResidualTerm term{static_cast<const double*>(Xm.p), Xm.ld, static_cast<const double*>(Am.p), Am.ld + 1};
-  if (side == 'L') {  // op(A) (n x n) times X (n x m): B-operand rows are X's columns
-    NLA_TRY(stage_operand(transposed(Xm), m, n, NLA_F64, EXACT_SLICES, true, 0, xbuf, Xs, s, false));
-    return launch_exact_gemm(As, *Xs, -1.0, Rm, false, s, &term);
+// The refinement buffers with `extra` bytes before the residual's, which
+// start at the next multiple of 1024.
+int split_residual_buffers(cudaStream_t s, size_t extra, char side, int64_t n, int64_t m, void** buf, SplitResidual* r) {
+  extra = (extra + 1023) & ~(size_t)1023;
+  r->crt = crt_enabled() && (side == 'L' ? crt_usable(n, m, n) : crt_usable(m, n, n));
+  int rc = refine_buffers(s, extra + split_residual_bytes(r->crt, side, n, m), buf);
+  if (rc != NLA_OK && r->crt) {
+    cudaGetLastError();
+    clear_error();
+    r->crt = false;
+    rc = refine_buffers(s, extra + split_residual_bytes(false, side, n, m), buf);
   }
-  // (X op(A))^T = op(A)^T X^T: B-operand rows are X's rows; written transposed
-  NLA_TRY(stage_operand(Xm, m, n, NLA_F64, EXACT_SLICES, true, 0, xbuf, Xs, s, false));
-  return launch_exact_gemm(As, *Xs, -1.0, Rm, true, s, &term);
+  r->base = static_cast<uint8_t*>(*buf) + extra;
+  return rc;
+}
+
+// Only op(A)'s strict triangle is staged (its rows then carry no diagonal,
+// whose size would coarsen the row scale); the diagonal term is FP64's.
+int stage_triangle(const Mat& Am, int64_t n, char side, char uplo, SplitResidual* r, cudaStream_t s) {
+  const bool lower_rows = (side == 'L') == (uplo == 'L');
+  const Mat X = side == 'L' ? Am : transposed(Am);
+  if (r->crt) {
+    r->Ac = crt_layout(r->base, n, n, lower_rows ? 3 : 4, true);
+    return crt_stage(X, r->Ac, nullptr, nullptr, s);
+  }
+  return stage_operand(X, n, n, NLA_F64, EXACT_SLICES, true, lower_rows ? 3 : 4, r->base, &r->As, s);
+}
+
+// R -= op(A) X (side L) or X op(A) (side R): exact products for the strict
+// triangle; the diagonal term and the subtraction are applied with one
+// rounding (R = alpha*B on entry).
+int split_residual(const Mat& Am, char side, int64_t n, int64_t m, const Mat& Xm, const Mat& Rm, SplitResidual* r,
+                   cudaStream_t s) {
+  const ResidualTerm term{static_cast<const double*>(Xm.p), Xm.ld, static_cast<const double*>(Am.p), Am.ld + 1};
+  // X as rows along K: its columns for side L, its rows for side R.
+  const Mat X = side == 'L' ? transposed(Xm) : Xm;
+  if (r->crt) {
+    uint8_t* xbuf = r->base + crt_staged_bytes(n, n);
+    uint8_t* planes = xbuf + crt_staged_bytes(m, n);
+    const CrtStaged Xc = crt_layout(xbuf, m, n, 0, false);
+    NLA_TRY(crt_stage(X, Xc, nullptr, nullptr, s));
+    // Side R: X op(A) = X (op(A)^T)^T, so the triangle is the column operand.
+    if (side == 'L') return crt_gemm(r->Ac, Xc, -1.0, Rm, planes, s, &term, false);
+    return crt_gemm(Xc, r->Ac, -1.0, Rm, planes, s, &term, true);
+  }
+  NLA_TRY(stage_operand(X, m, n, NLA_F64, EXACT_SLICES, true, 0, r->base + staged_bytes(n, n, EXACT_SLICES), &r->Xs, s,
+                        false));
+  // Side R: (X op(A))^T = op(A)^T X^T, written transposed.
+  return launch_exact_gemm(r->As, r->Xs, -1.0, Rm, side == 'R', s, &term);
 }
 
 int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m, const void* A, int64_t lda,
@@ -916,8 +959,14 @@ int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m
   const int64_t mid = split_point(n), rem = n - mid;
   const int64_t big = mid > rem ? mid : rem;
   void* ws = nullptr;
-  if (n > c->threshold) NLA_TRY(workspace_get(s, sliced_workspace_bytes(big, m, big, opts.split_terms), &ws));
-  return NLA_OK;
+  if (n <= c->threshold) return NLA_OK;
+  const int64_t rows_c = side == 'L' ? big : m, cols_c = side == 'L' ? m : big;
+  if (opts.split_terms == EXACT_SLICES && crt_enabled() && crt_usable(rows_c, cols_c, big) &&
+      workspace_get(s, crt_workspace_bytes(rows_c, cols_c, big), &ws) == NLA_OK)
+    return NLA_OK;
+  cudaGetLastError();
+  clear_error();
+  return workspace_get(s, sliced_workspace_bytes(big, m, big, opts.split_terms), &ws);
 }
 
 int trxm_mixed_impl(char side, char uplo, char trans, double alpha, char func, int64_t n, int64_t m,
@@ -956,14 +1005,14 @@ int trxm_mixed_impl(char side, char uplo, char trans, double alpha, char func, i
   // staged once (it does not change between sweeps) and X staged per sweep.
   const size_t elems = (size_t)rows * (size_t)cols;
   const bool split = opts.residual == NLA_RESIDUAL_SPLIT;
-  const size_t a_stage = split ? staged_bytes(n, n, EXACT_SLICES) : 0;
-  const size_t x_stage = split ? staged_bytes(m, n, EXACT_SLICES) : 0;
+  SplitResidual sr;
   void* buf = nullptr;
-  NLA_TRY(refine_buffers(s, 2 * elems * sizeof(double) + 2048 + a_stage + x_stage, &buf));
+  const size_t own = 2 * elems * sizeof(double) + 256;
+  if (split) NLA_TRY(split_residual_buffers(s, own, side, n, m, &buf, &sr));
+  else NLA_TRY(refine_buffers(s, own, &buf));
   double* B0 = static_cast<double*>(buf);
   double* R = B0 + elems;
   unsigned long long* amax = reinterpret_cast<unsigned long long*>(R + elems);
-  uint8_t* stage_base = reinterpret_cast<uint8_t*>(buf) + ((2 * elems * sizeof(double) + 256 + 1023) & ~(size_t)1023);
   const unsigned grid = grid_for((int64_t)elems);
   {
     TraceScope t(NLA_K_RESIDUAL, s, 0.0, 16.0 * (double)elems);
@@ -972,12 +1021,7 @@ int trxm_mixed_impl(char side, char uplo, char trans, double alpha, char func, i
   }
   NLA_TRY(recurse(mixed, Am, n, Bm));  // X0
 
-  // op(A) as the left operand (side L: op(A) X) or the right one (side R:
-  // X op(A), staged as op(A)^T); only its triangle is staged.
-  // The strict triangle is staged (its rows then carry no diagonal, whose
-  // size would coarsen the row scale); the diagonal term is applied in FP64.
-  Staged As{}, Xs{};
-  if (split) NLA_TRY(stage_triangle(Am, n, side, uplo, stage_base, &As, s));
+  if (split) NLA_TRY(stage_triangle(Am, n, side, uplo, &sr, s));
   RecPlan resid{'M', side, uplo, NLA_F64, m, 128, s, GEMM_PLAIN, 1, false};
   Mat Rm{R, rows, 0};
   for (int k = 0; k < opts.sweeps; ++k) {
@@ -987,7 +1031,7 @@ int trxm_mixed_impl(char side, char uplo, char trans, double alpha, char func, i
         copy_kernel<<<grid, 256, 0, s>>>(rows, cols, B0, rows, R, rows);
         NLA_CHECK_LAUNCH("copy_kernel");
       }
-      NLA_TRY(split_residual(Am, As, side, n, m, Bm, Rm, stage_base + a_stage, &Xs, s));
+      NLA_TRY(split_residual(Am, side, n, m, Bm, Rm, &sr, s));
     } else {
       {
         TraceScope t(NLA_K_RESIDUAL, s, 0.0, 16.0 * (double)elems);
@@ -1050,16 +1094,14 @@ int residual_impl(char side, char uplo, char trans, double alpha, int64_t n, int
     return NLA_OK;
   }
   if (mode == NLA_RESIDUAL_SPLIT) {
-    const size_t a_stage = staged_bytes(n, n, EXACT_SLICES), x_stage = staged_bytes(m, n, EXACT_SLICES);
+    SplitResidual sr;
     void* buf = nullptr;
-    NLA_TRY(refine_buffers(s, a_stage + x_stage + 1024, &buf));
-    uint8_t* base = static_cast<uint8_t*>(buf);
+    NLA_TRY(split_residual_buffers(s, 0, side, n, m, &buf, &sr));
     copy_kernel<<<grid, 256, 0, s>>>(rows, cols, B, ldb, R, ldr);
     NLA_CHECK_LAUNCH("copy_kernel");
     NLA_TRY(launch_scale(NLA_F64, rows, cols, alpha, Rm, s));
-    Staged As{}, Xs{};
-    NLA_TRY(stage_triangle(Am, n, side, uplo, base, &As, s));
-    return split_residual(Am, As, side, n, m, Xm, Rm, base + a_stage, &Xs, s);
+    NLA_TRY(stage_triangle(Am, n, side, uplo, &sr, s));
+    return split_residual(Am, side, n, m, Xm, Rm, &sr, s);
   }
   // FP64 pipe: R = op(A) X by the plain recursion, then R = alpha*B - R.
   void* buf = nullptr;

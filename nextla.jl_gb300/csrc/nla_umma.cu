@@ -1373,8 +1373,10 @@ int ensure_exact_smem() {
   return status == cudaSuccess ? NLA_OK : cuda_status(status, "cudaFuncSetAttribute(umma_exact_kernel)");
 }
 
-// Exact-kernel variant (NLA_EXACT_KERNEL, read once): "coupled" (pairs
-// sharing a B tile, the default) or "pairs" (pair by pair).
+// Slice-kernel variant (NLA_EXACT_KERNEL, read once): "coupled" (pairs
+// sharing a B tile) or "pairs" (pair by pair).  Unset, updates whose
+// workspace is the library's own run on residues (nla_crt.cu), and the
+// coupled kernel takes the others.
 bool exact_coupled() {
   static const bool on = [] {
     const char* e = getenv("NLA_EXACT_KERNEL");
@@ -1431,8 +1433,20 @@ int launch_exact_pairs(const ExactParams& p, const Staged& A, const Staged& B, c
 
 }  // namespace
 
-int staged_map(CUtensorMap* map, const void* base, uint64_t k_pad, uint64_t total_rows) {
-  return make_map(map, base, true, k_pad, total_rows);
+int staged_map(CUtensorMap* map, const void* base, uint64_t k_pad, uint64_t total_rows, uint32_t box_rows) {
+  return make_map(map, base, true, k_pad, total_rows, box_rows);
+}
+
+bool crt_enabled() {
+  static const bool on = [] {
+    const char* e = getenv("NLA_EXACT_KERNEL");
+    return !(e && (!strcmp(e, "pairs") || !strcmp(e, "coupled")));
+  }();
+  return on;
+}
+
+size_t crt_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  return crt_staged_bytes(M, K) + crt_staged_bytes(N, K) + crt_planes_bytes(M, N) + 1024;
 }
 
 // Scratch of the plain path: stream-ordered allocations from a pool of their
@@ -1655,8 +1669,21 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
     // Exact slice products (FP64-accurate update).
     if (!bf16) return fail(NLA_ERR_ARG, "exact updates use BF16 slices");
     if (out_dtype != NLA_F64) return fail(NLA_ERR_DTYPE, "exact updates produce Float64");
-    const size_t sa = staged_bytes(M, K, S), sb = staged_bytes(N, K, S), need = sa + sb + 1024;
     void* base = ws;
+    if (base == nullptr && crt_enabled() && crt_usable(M, N, K)) {
+      if (workspace_get(s, crt_workspace_bytes(M, N, K), &base) == NLA_OK) {
+        const CrtStaged a = crt_layout(base, M, K, 0, true);
+        const CrtStaged b = crt_layout(static_cast<uint8_t*>(base) + crt_staged_bytes(M, K), N, K, 0, false);
+        const Mat Bt = transposed(B);
+        NLA_TRY(crt_stage(A, a, &Bt, &b, s));
+        return crt_gemm(a, b, alpha, C,
+                        static_cast<uint8_t*>(base) + crt_staged_bytes(M, K) + crt_staged_bytes(N, K), s);
+      }
+      cudaGetLastError();  // too little memory for the residues: the slices take less
+      clear_error();
+      base = nullptr;
+    }
+    const size_t sa = staged_bytes(M, K, S), sb = staged_bytes(N, K, S), need = sa + sb + 1024;
     if (base == nullptr) {
       NLA_TRY(workspace_get(s, need + fixed_sums_bytes(M, N), &base));
       ws_bytes = need + fixed_sums_bytes(M, N);
@@ -1833,6 +1860,7 @@ int set_wait_limit(uint64_t ns) {
   const uint64_t v = ns == 0 ? umma::WAIT_LIMIT_NS : ns;
   const cudaError_t e = cudaMemcpyToSymbol(umma::g_wait_limit_ns, &v, sizeof(v));
   if (e != cudaSuccess) return cuda_status(e, "set wait limit");
+  NLA_TRY(crt_set_wait_limit(v));
   g_wait_limit_host.store(v);
   return NLA_OK;
 }

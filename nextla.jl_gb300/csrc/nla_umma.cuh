@@ -209,7 +209,7 @@ __host__ __device__ constexpr uint32_t idesc_f16(int M, int N, bool bf16) {
 
 }  // namespace umma
 
-// Tensor map of a staged BF16 operand: 128 x 64 boxes of a K-major array of
-// total_rows rows of k_pad values (nla_umma.cu).
-int staged_map(CUtensorMap* map, const void* base, uint64_t k_pad, uint64_t total_rows);
+// Tensor map of a staged BF16 operand: box_rows x 64 boxes of a K-major array
+// of total_rows rows of k_pad values (nla_umma.cu).
+int staged_map(CUtensorMap* map, const void* base, uint64_t k_pad, uint64_t total_rows, uint32_t box_rows = 128);
 }  // namespace nla
