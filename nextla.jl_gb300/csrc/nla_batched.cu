@@ -38,6 +38,7 @@
 #include <algorithm>
 #include <mutex>
 #include <queue>
+#include <type_traits>
 #include <vector>
 
 #include "nla_common.cuh"
@@ -389,73 +390,14 @@ __device__ bool run_update(const Args& a, const Node& nd, const Group& g, const 
   return true;
 }
 
-// ---------------------------------------------------------------------------
-// LEAF: solve the diagonal block rows r0 .. r0 + rows (at most 64) in place.
-// The block of A (lower, with the diagonal's reciprocals) and of X are staged
-// in shared memory; 16-row panels are solved one right-hand side per thread
-// (the panel's values in registers), and each panel's rows below it are then
-// updated with the register-tiled product.
-// ---------------------------------------------------------------------------
-template <typename T, int W>
-__device__ bool run_leaf(const Args& a, const Node& nd, const Group& g, const nla_batch_desc& d, void* smem,
-                         volatile int* s_ok) {
-  using Tc = typename Elem<T>::compute;
+// X := inv(L) X for a diagonal block staged in shared memory (L's strict
+// lower part, the reciprocals of its diagonal and X), in 16-row panels solved
+// one right-hand side per thread, the rows below each panel updated with the
+// register-tiled product.
+template <typename Tc, int W>
+__device__ __forceinline__ void solve_panels(const Tc* Ls, Tc* Xs, const Tc* inv, int rows, int ncols) {
   constexpr int LP = MAX_ROWS + LEAF_PAD, XP = W + 4, CT = W / 16;
-  Tc* Ls = static_cast<Tc*>(smem);    // [64][LP]: Ls[r][k], k < r, of the block
-  Tc* Xs = Ls + MAX_ROWS * LP;        // [64][XP]
-  Tc* inv = Xs + MAX_ROWS * XP;       // [64]
-  const T* A = static_cast<const T*>(a.A);
-  T* B = static_cast<T*>(a.B);
-  const int t = threadIdx.x, rows = nd.rows, ncols = g.ncols;
-  const bool first = nd.flags & FLAG_ALPHA;
-
-  // Stage the block of A (threads along the index contiguous in memory) and
-  // X; offsets are affine in the block's row and column (as in run_update).
-  // A's loads are issued before the dependency wait, X's (which other nodes
-  // write) after it, and every load before the first store, so that their
-  // latencies overlap instead of adding up.
-  const int64_t sgn = a.rev ? -1 : 1;
-  const int64_t dr = sgn * (a.tA ? d.lda : 1), dk = sgn * (a.tA ? 1 : d.lda);
-  const T* A0 = A + a_at(d, a.tA, a.rev, nd.r0, nd.r0);
-  constexpr int A_PER = MAX_ROWS * MAX_ROWS / NT, X_PER = MAX_ROWS * W / NT;
-  Tc va[A_PER];
-  T vx[X_PER];
-#pragma unroll
-  for (int u = 0; u < A_PER; ++u) {
-    const int idx = t + u * NT;
-    const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
-    va[u] = r < rows && k <= r ? to_c(A0[r * dr + k * dk]) : Tc(0);
-  }
-  if (!node_deps(a, nd, s_ok)) return false;
-  const T* X0 = B + b_at(d, a.rev, nd.r0, g.c0);
-  const int xr = t % MAX_ROWS;  // NT is a multiple of MAX_ROWS: each thread keeps one row of X
-#pragma unroll
-  for (int u = 0; u < X_PER; ++u) {
-    const int c = (t + u * NT) / MAX_ROWS;
-    vx[u] = xr < rows && c < ncols ? ldcg(X0 + xr * sgn + (int64_t)c * d.ldb) : T(0);
-  }
-#pragma unroll
-  for (int u = 0; u < A_PER; ++u) {
-    const int idx = t + u * NT;
-    const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
-    if (r < rows && k < r) Ls[r * LP + k] = va[u];
-    else if (r < rows && k == r) inv[r] = Tc(1) / va[u];
-  }
-  if (first) {  // node-uniform (see the update's epilogue)
-#pragma unroll
-    for (int u = 0; u < X_PER; ++u) {
-      const int c = (t + u * NT) / MAX_ROWS;
-      if (xr < rows) Xs[xr * XP + c] = scaled_node<T>(vx[u], a);
-    }
-  } else {
-#pragma unroll
-    for (int u = 0; u < X_PER; ++u) {
-      const int c = (t + u * NT) / MAX_ROWS;
-      if (xr < rows) Xs[xr * XP + c] = to_c(vx[u]);
-    }
-  }
-  __syncthreads();
-
+  const int t = threadIdx.x;
   const int tr = t % ROW_GROUPS, tc = t / ROW_GROUPS;
   for (int p0 = 0; p0 < rows; p0 += PANEL) {
     const int pw = min(PANEL, rows - p0);
@@ -511,6 +453,76 @@ __device__ bool run_leaf(const Args& a, const Node& nd, const Group& g, const nl
     }
     __syncthreads();
   }
+}
+
+// ---------------------------------------------------------------------------
+// LEAF: solve the diagonal block rows r0 .. r0 + rows (at most 64) in place.
+// The block of A (lower, with the diagonal's reciprocals) and of X are staged
+// in shared memory; 16-row panels are solved one right-hand side per thread
+// (the panel's values in registers), and each panel's rows below it are then
+// updated with the register-tiled product.
+// ---------------------------------------------------------------------------
+template <typename T, int W>
+__device__ bool run_leaf(const Args& a, const Node& nd, const Group& g, const nla_batch_desc& d, void* smem,
+                         volatile int* s_ok) {
+  using Tc = typename Elem<T>::compute;
+  constexpr int LP = MAX_ROWS + LEAF_PAD, XP = W + 4;
+  Tc* Ls = static_cast<Tc*>(smem);    // [64][LP]: Ls[r][k], k < r, of the block
+  Tc* Xs = Ls + MAX_ROWS * LP;        // [64][XP]
+  Tc* inv = Xs + MAX_ROWS * XP;       // [64]
+  const T* A = static_cast<const T*>(a.A);
+  T* B = static_cast<T*>(a.B);
+  const int t = threadIdx.x, rows = nd.rows, ncols = g.ncols;
+  const bool first = nd.flags & FLAG_ALPHA;
+
+  // Stage the block of A (threads along the index contiguous in memory) and
+  // X; offsets are affine in the block's row and column (as in run_update).
+  // A's loads are issued before the dependency wait, X's (which other nodes
+  // write) after it, and every load before the first store, so that their
+  // latencies overlap instead of adding up.
+  const int64_t sgn = a.rev ? -1 : 1;
+  const int64_t dr = sgn * (a.tA ? d.lda : 1), dk = sgn * (a.tA ? 1 : d.lda);
+  const T* A0 = A + a_at(d, a.tA, a.rev, nd.r0, nd.r0);
+  constexpr int A_PER = MAX_ROWS * MAX_ROWS / NT, X_PER = MAX_ROWS * W / NT;
+  Tc va[A_PER];
+  T vx[X_PER];
+#pragma unroll
+  for (int u = 0; u < A_PER; ++u) {
+    const int idx = t + u * NT;
+    const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
+    va[u] = r < rows && k <= r ? to_c(A0[r * dr + k * dk]) : Tc(0);
+  }
+  if (!node_deps(a, nd, s_ok)) return false;
+  const T* X0 = B + b_at(d, a.rev, nd.r0, g.c0);
+  const int xr = t % MAX_ROWS;  // NT is a multiple of MAX_ROWS: each thread keeps one row of X
+#pragma unroll
+  for (int u = 0; u < X_PER; ++u) {
+    const int c = (t + u * NT) / MAX_ROWS;
+    vx[u] = xr < rows && c < ncols ? ldcg(X0 + xr * sgn + (int64_t)c * d.ldb) : T(0);
+  }
+#pragma unroll
+  for (int u = 0; u < A_PER; ++u) {
+    const int idx = t + u * NT;
+    const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
+    if (r < rows && k < r) Ls[r * LP + k] = va[u];
+    else if (r < rows && k == r) inv[r] = Tc(1) / va[u];
+  }
+  if (first) {  // node-uniform (see the update's epilogue)
+#pragma unroll
+    for (int u = 0; u < X_PER; ++u) {
+      const int c = (t + u * NT) / MAX_ROWS;
+      if (xr < rows) Xs[xr * XP + c] = scaled_node<T>(vx[u], a);
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < X_PER; ++u) {
+      const int c = (t + u * NT) / MAX_ROWS;
+      if (xr < rows) Xs[xr * XP + c] = to_c(vx[u]);
+    }
+  }
+  __syncthreads();
+
+  solve_panels<Tc, W>(Ls, Xs, inv, rows, ncols);
   T* Xw = B + b_at(d, a.rev, nd.r0, g.c0);
   for (int idx = t; idx < MAX_ROWS * W; idx += NT) {
     const int r = idx % MAX_ROWS, c = idx / MAX_ROWS;
@@ -560,6 +572,210 @@ __global__ void __launch_bounds__(NT, 2) batched_node_kernel(Args a) {
     }
   }
 }
+
+// ---------------------------------------------------------------------------
+// Whole groups, one CTA each.  Where a batch has enough work that no single
+// group is longer than a CTA's share of it, nothing is gained by spreading a
+// group over CTAs, and its nodes' waits, descriptors, counters and the
+// traffic of the recursion's intermediate updates are pure cost.  A CTA then
+// takes a group (longest first, from the same kind of device counter) and
+// solves it block row by block row, left-looking: block rows of at most 64
+// rows, each X[r0 ..] = inv(L) (alpha B[r0 ..] - A[r0 .., 0 .. r0) X[0 .. r0))
+// with the product accumulated in registers over all of K, so that every
+// element of B is read and written once.
+// Bound by the products (3.4 of 6.1 ms for 10,000 Float32 systems of 16 to
+// 1024 unknowns, whose FMAs alone would take 1.5), the blocks' loads and the
+// triangles (1.4).  Against the node queue: 10,000 systems 7.00 -> 6.36 ms,
+// 3000 2.09 -> 1.88; at 1000 the longest group would exceed a CTA's share.
+// ---------------------------------------------------------------------------
+struct GroupItem {
+  int n, ncols, w, rb;  // order, right-hand sides, column template, rows per block
+  int64_t a_off, lda, b_off, ldb;  // b_off: of the group's first column
+};
+static_assert(sizeof(GroupItem) == 48, "group item layout");
+
+struct GroupArgs {
+  const GroupItem* items;
+  int count;
+  int* next;
+  const void* A;
+  void* B;
+  int tA, rev;
+  Args alpha;  // the scaling of B (scaled_node reads its alpha fields)
+};
+
+// Chunk buffers: three chunks of copies in flight (Float32), or one (Float64,
+// whose products take longer than a copy and whose buffers are twice as large).
+__host__ __device__ constexpr int group_stages(int esz) { return esz == 8 ? 2 : 4; }
+
+template <typename Tc, int W>
+__host__ __device__ constexpr size_t group_elems() {
+  constexpr int kc = kc_of(sizeof(Tc));
+  return group_stages(sizeof(Tc)) * update_elems(W, kc) + leaf_elems(W);
+}
+
+template <typename T>
+__device__ __forceinline__ void async_copy(uint32_t dst, const T* src, bool in) {
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "cp.async copies 4 or 8 bytes");
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(dst), "l"(src), "n"((int)sizeof(T)),
+               "r"(in ? (int)sizeof(T) : 0)
+               : "memory");
+}
+
+template <typename T, int W>
+__device__ void run_group(const GroupArgs& a, const GroupItem& it, void* smem) {
+  using Tc = typename Elem<T>::compute;
+  constexpr int KC = kc_of(sizeof(Tc)), CT = W / 16;
+  constexpr int AP = MAX_ROWS + 4, XP = W + 4, LP = MAX_ROWS + LEAF_PAD;
+  constexpr int A_PER = MAX_ROWS * KC / NT, X_PER = KC * W / NT;
+  constexpr int D_PER = MAX_ROWS * MAX_ROWS / NT, B_PER = MAX_ROWS * W / NT;
+  constexpr int ST = group_stages(sizeof(Tc));
+  Tc* As = static_cast<Tc*>(smem);      // [ST][KC][AP]
+  Tc* Xk = As + ST * KC * AP;           // [ST][KC][XP]
+  Tc* Ls = Xk + ST * KC * XP;           // [64][LP]
+  Tc* Xs = Ls + MAX_ROWS * LP;          // [64][XP]
+  Tc* inv = Xs + MAX_ROWS * XP;         // [64]
+  const int t = threadIdx.x, tr = t % ROW_GROUPS, tc = t / ROW_GROUPS;
+  const int n = it.n, ncols = it.ncols;
+  const bool warp_cols_live = (tc & ~1) * CT < ncols;
+  const int64_t sgn = a.rev ? -1 : 1;
+  const int64_t dr = sgn * (a.tA ? it.lda : 1), dk = sgn * (a.tA ? 1 : it.lda);
+  const T* A = static_cast<const T*>(a.A) + it.a_off + (a.rev ? (int64_t)(n - 1) * (it.lda + 1) : 0);
+  T* B = static_cast<T*>(a.B) + it.b_off + (a.rev ? n - 1 : 0);  // canonical row r at B[r sgn + c ldb]
+
+  // Staging slots of a chunk, as in run_update.
+  const int ar = a.tA ? t / KC : t % MAX_ROWS, ak = a.tA ? t % KC : t / MAX_ROWS;
+  const int ar_step = a.tA ? NT / KC : 0, ak_step = a.tA ? 0 : NT / MAX_ROWS;
+  const int64_t a_step = (int64_t)ar_step * dr + (int64_t)ak_step * dk;
+  const int xk = t % KC, xc = t / KC;
+  constexpr int XC_STEP = NT / KC;
+  const int64_t x_step = (int64_t)XC_STEP * it.ldb;
+  const T* X0 = B + sgn * xk + (int64_t)xc * it.ldb;
+  const int xr = t % MAX_ROWS, xcb = t / MAX_ROWS;  // slots of a block of B
+
+  for (int r0 = 0; r0 < n; r0 += it.rb) {
+    const int rows = min(it.rb, n - r0);
+    const T* Ar = A + (int64_t)r0 * dr;
+    // Asynchronous copies of a chunk into one of the buffers (zeros past
+    // the block's rows, the solved rows and the group's columns).
+    auto fetch = [&](int k0, int buf) {
+      const int kw = min(KC, r0 - k0);
+      const T* pA = Ar + ar * dr + (int64_t)(k0 + ak) * dk;
+      const T* pX = X0 + (int64_t)k0 * sgn;
+      const uint32_t sa = umma::smem_u32(As + (buf * KC + ak) * AP + ar);
+      const uint32_t sx = umma::smem_u32(Xk + (buf * KC + xk) * XP + xc);
+#pragma unroll
+      for (int u = 0; u < A_PER; ++u) {
+        const bool in = ar + u * ar_step < rows && ak + u * ak_step < kw;
+        async_copy<T>(sa + (uint32_t)(u * (ak_step * AP + ar_step) * (int)sizeof(T)), in ? pA + u * a_step : A, in);
+      }
+#pragma unroll
+      for (int u = 0; u < X_PER; ++u) {
+        const bool in = xk < kw && xc + u * XC_STEP < ncols;
+        async_copy<T>(sx + (uint32_t)(u * XC_STEP * (int)sizeof(T)), in ? pX + u * x_step : B, in);
+      }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    // The first chunk, the diagonal block and the block of B are all in
+    // flight together (the chunk buffers' last readers passed a barrier).
+    for (int st = 0; st < ST - 1; ++st) {
+      if (st * KC < r0) fetch(st * KC, st);
+      else asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    {
+      Tc va[D_PER];
+      T vb[B_PER];
+      const T* Ad = Ar + (int64_t)r0 * dk;
+#pragma unroll
+      for (int u = 0; u < D_PER; ++u) {
+        const int idx = t + u * NT;
+        const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
+        va[u] = r < rows && k <= r ? to_c(Ad[r * dr + k * dk]) : Tc(0);
+      }
+#pragma unroll
+      for (int u = 0; u < B_PER; ++u) {
+        const int c = xcb + u * (NT / MAX_ROWS);
+        vb[u] = xr < rows && c < ncols ? ldcg(B + (r0 + xr) * sgn + (int64_t)c * it.ldb) : T(0);
+      }
+      __syncthreads();  // the previous block (or group) no longer reads shared memory
+#pragma unroll
+      for (int u = 0; u < D_PER; ++u) {
+        const int idx = t + u * NT;
+        const int r = a.tA ? idx / MAX_ROWS : idx % MAX_ROWS, k = a.tA ? idx % MAX_ROWS : idx / MAX_ROWS;
+        if (r < rows && k < r) Ls[r * LP + k] = va[u];
+        else if (r < rows && k == r) inv[r] = Tc(1) / va[u];
+      }
+#pragma unroll
+      for (int u = 0; u < B_PER; ++u) Xs[xr * XP + xcb + u * (NT / MAX_ROWS)] = scaled_node<T>(vb[u], a.alpha);
+    }
+
+    if (r0 > 0) {
+      Tc acc[RT][CT];
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int c = 0; c < CT; ++c) acc[i][c] = Tc(0);
+      int buf = 0;
+      for (int k0 = 0; k0 < r0; k0 += KC, buf = buf + 1 == ST ? 0 : buf + 1) {
+        const Tc* Ab = As + buf * KC * AP;
+        const Tc* Xb = Xk + buf * KC * XP;
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();  // the chunk is in; the previous chunk's readers are past this
+        if (k0 + (ST - 1) * KC < r0) fetch(k0 + (ST - 1) * KC, buf == 0 ? ST - 1 : buf - 1);
+        else asm volatile("cp.async.commit_group;" ::: "memory");
+        const int kw = warp_cols_live ? min(KC, r0 - k0) : 0;
+#pragma unroll 4
+        for (int k = 0; k < kw; ++k) {
+          Tc av[RT], xv[CT];
+          lds_vec<RT>(Ab + k * AP + RT * tr, av);
+          lds_vec<CT>(Xb + k * XP + tc * CT, xv);
+#pragma unroll
+          for (int i = 0; i < RT; ++i)
+#pragma unroll
+            for (int c = 0; c < CT; ++c) acc[i][c] = fma(av[i], xv[c], acc[i][c]);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < RT; ++i)
+#pragma unroll
+        for (int c = 0; c < CT; ++c) Xs[(RT * tr + i) * XP + tc * CT + c] -= acc[i][c];
+    }
+    __syncthreads();
+    solve_panels<Tc, W>(Ls, Xs, inv, rows, ncols);
+#pragma unroll
+    for (int u = 0; u < B_PER; ++u) {
+      const int c = xcb + u * (NT / MAX_ROWS);
+      if (xr < rows && c < ncols)
+        Elem<T>::store(B + (r0 + xr) * sgn + (int64_t)c * it.ldb, Xs[xr * XP + c]);
+    }
+    __syncthreads();  // the block's X is in memory for the next block's chunks
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(NT, 2) batched_group_kernel(GroupArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ int s_idx;
+  for (;;) {
+    if (threadIdx.x == 0) s_idx = atomicAdd(a.next, 1);
+    __syncthreads();
+    const int idx = s_idx;
+    if (idx >= a.count) break;
+    const GroupItem it = a.items[idx];
+    switch (it.w) {
+      case 16: run_group<T, 16>(a, it, smem_raw); break;
+      case 32: run_group<T, 32>(a, it, smem_raw); break;
+      default: run_group<T, 64>(a, it, smem_raw); break;
+    }
+  }
+}
+
+// Shared memory of the group kernel for groups of width w_max.
+template <typename Tc>
+size_t group_smem_bytes(int w_max) {
+  return sizeof(Tc) * (w_max <= 16 ? group_elems<Tc, 16>() : w_max <= 32 ? group_elems<Tc, 32>() : group_elems<Tc, 64>());
+}
+constexpr int GROUP_W = 64;  // widest group: 128 columns would leave no registers for the staging (6.5 against 6.3 ms)
 
 size_t node_smem_bytes(int dtype, int w_max) {
   const int esz = dtype == NLA_F64 ? 8 : 4;
@@ -1077,6 +1293,8 @@ struct nla_batch_plan_s {
   std::vector<nla_batch_desc> h_descs;
   std::vector<nla::bat::Group> h_groups;
   int ngroups, nleaves, nnodes;
+  bool whole_groups;   // one CTA per group (batched_group_kernel); the queue then holds the groups
+  void* d_items;
   int n_max;
   int w_max;
   size_t smem;
@@ -1333,6 +1551,18 @@ int node_kernel_setup(size_t smem, int* per_sm) {
 }
 
 template <typename T>
+int group_kernel_setup(size_t smem, int* per_sm) {
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  std::call_once(once, [] {
+    st = cudaFuncSetAttribute(bat::batched_group_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 110 * 1024);
+  });
+  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(batched_group_kernel)");
+  const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, bat::batched_group_kernel<T>, bat::NT, smem);
+  return e == cudaSuccess ? NLA_OK : cuda_status(e, "batch: occupancy query");
+}
+
+template <typename T>
 int launch_nodes(nla_batch_plan p, double alpha, const void* A, void* B, cudaStream_t s) {
   int* c = p->d_counters;  // next, abort, solved[ngroups], applied[nleaves]
   bat::Args a{static_cast<const nla_batch_desc*>(p->d_descs), static_cast<const Group*>(p->d_groups),
@@ -1342,6 +1572,14 @@ int launch_nodes(nla_batch_plan p, double alpha, const void* A, void* B, cudaStr
   cudaError_t e = cudaGetSymbolAddress(&errp, bat::g_batch_error);
   if (e != cudaSuccess) return cuda_status(e, "batch error word");
   a.err = static_cast<int*>(errp);
+  if constexpr (!std::is_same<T, __half>::value) {
+    if (p->whole_groups) {
+      const bat::GroupArgs ga{static_cast<const bat::GroupItem*>(p->d_items), p->ngroups, c, A, B, p->tA, p->rev, a};
+      bat::batched_group_kernel<T><<<p->grid, bat::NT, p->smem, s>>>(ga);
+      NLA_CHECK_LAUNCH("batched_group_kernel");
+      return NLA_OK;
+    }
+  }
   bat::batched_node_kernel<T><<<p->grid, bat::NT, p->smem, s>>>(a);
   NLA_CHECK_LAUNCH("batched_node_kernel");
   return NLA_OK;
@@ -1395,24 +1633,19 @@ int plan_create(nla_batch_plan* out, int dtype, char uplo, char trans, int64_t c
   p->d_row_base = p->d_col_base = nullptr;
   p->d_row_exp = p->d_col_exp = nullptr;
   p->exec = nullptr;
-  p->d_descs = p->d_groups = p->d_nodes = nullptr;
+  p->d_descs = p->d_groups = p->d_nodes = p->d_items = nullptr;
+  p->whole_groups = false;
   p->d_counters = nullptr;
   p->cap_stream = nullptr;
 
   std::vector<Group> groups;
   std::vector<HostNode> nodes;
+  std::vector<bat::GroupItem> items;
   int leaves_total = 0;
-  for (int64_t i = 0; i < count; ++i) {
+  // Balanced blocks of right-hand sides of system i, each at most wcap wide,
+  // each run with the narrowest column template that holds it.
+  auto add_groups = [&](int64_t i, int wcap, auto&& each) {
     const nla_batch_desc& d = descs[i];
-    if (d.n == 0 || d.m == 0) continue;
-    p->a_elems = std::max<int64_t>(p->a_elems, d.a_off + (d.n - 1) * d.lda + d.n);
-    p->b_elems = std::max<int64_t>(p->b_elems, d.b_off + (d.m - 1) * d.ldb + d.n);
-    p->n_max = std::max<int>(p->n_max, (int)d.n);
-    p->flops += (double)d.n * d.n * d.m;
-    const int b = bucket_of(d.n);
-    const int wcap = dtype == NLA_F64 ? std::min(tun.cols[b], 64) : tun.cols[b];
-    // Balanced blocks of right-hand sides, each at most wcap wide, each run
-    // with the narrowest column template that holds it.
     const int64_t nblk = (d.m + wcap - 1) / wcap;
     for (int64_t k = 0; k < nblk; ++k) {
       const int64_t c0 = d.m * k / nblk, c1 = d.m * (k + 1) / nblk;
@@ -1424,58 +1657,124 @@ int plan_create(nla_batch_plan* out, int dtype, char uplo, char trans, int64_t c
       g.leaf_base = leaves_total;
       g.n = (int)d.n;
       p->w_max = std::max(p->w_max, g.w);
-      GroupBuilder gb;
-      gb.gi = (int)groups.size();
-      gb.cutoff = tun.cutoff[b];
-      gb.rev = p->rev != 0;
-      gb.nodes = &nodes;
-      gb.group_w = g.w;
-      gb.leaves(0, (int)d.n);
-      gb.chain.assign(gb.leaf_start.size(), 0);
-      gb.last_node.assign(gb.leaf_start.size(), -1);
-      gb.rec(0, (int)d.n);
-      leaves_total += (int)gb.leaf_start.size();
+      each(g);
       groups.push_back(g);
     }
+  };
+  for (int64_t i = 0; i < count; ++i) {
+    const nla_batch_desc& d = descs[i];
+    if (d.n == 0 || d.m == 0) continue;
+    p->a_elems = std::max<int64_t>(p->a_elems, d.a_off + (d.n - 1) * d.lda + d.n);
+    p->b_elems = std::max<int64_t>(p->b_elems, d.b_off + (d.m - 1) * d.ldb + d.n);
+    p->n_max = std::max<int>(p->n_max, (int)d.n);
+    p->flops += (double)d.n * d.n * d.m;
   }
-  if (groups.size() > (size_t)INT32_MAX / 2 || nodes.size() > (size_t)INT32_MAX / 2) {
-    delete p;
-    return fail(NLA_ERR_UNSUPPORTED, "batch too large");
+  int per_sm = 0, rc = NLA_OK;
+
+  // One CTA per group where the longest group is no longer than a CTA's share
+  // of all of them: its nodes need no queue order then.  Cost in microseconds
+  // of the group kernel, about 10 per block row and 2 to 5 per 64 x W product
+  // with 64 values of K.
+  if (dtype != NLA_F16) {
+    std::vector<double> cost;
+    double total = 0, longest = 0;
+    for (int64_t i = 0; i < count; ++i) {
+      const nla_batch_desc& d = descs[i];
+      if (d.n == 0 || d.m == 0) continue;
+      const int b = bucket_of(d.n), rb = tun.cutoff[b];
+      add_groups(i, std::min(tun.cols[b], bat::GROUP_W), [&](const Group& g) {
+        const double blocks = (double)((d.n + rb - 1) / rb);
+        const double c = 10.0 * blocks + blocks * (blocks - 1) / 2 * rb / 64.0 * (1.0 + 4.0 * g.w / 64.0);
+        items.push_back(bat::GroupItem{(int)d.n, g.ncols, g.w, rb, d.a_off, d.lda, d.b_off + g.c0 * d.ldb, d.ldb});
+        cost.push_back(c);
+        total += c;
+        longest = std::max(longest, c);
+      });
+    }
+    p->smem = dtype == NLA_F64 ? bat::group_smem_bytes<double>(p->w_max) : bat::group_smem_bytes<float>(p->w_max);
+    rc = dtype == NLA_F64 ? group_kernel_setup<double>(p->smem, &per_sm) : group_kernel_setup<float>(p->smem, &per_sm);
+    if (rc != NLA_OK) {
+      delete p;
+      return rc;
+    }
+    p->grid = std::max(1, std::min(std::max((int)groups.size(), 1), num_sms() * std::max(per_sm, 1)));
+    p->whole_groups = per_sm > 0 && groups.size() < (size_t)INT32_MAX / 2 && longest <= total / p->grid;
+    if (p->whole_groups) {  // longest first
+      std::vector<int> order(items.size());
+      for (size_t k = 0; k < order.size(); ++k) order[k] = (int)k;
+      std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+      std::vector<bat::GroupItem> sorted(items.size());
+      for (size_t k = 0; k < order.size(); ++k) sorted[k] = items[order[k]];
+      items.swap(sorted);
+      p->nnodes = (int)items.size();
+    } else {
+      groups.clear();
+      items.clear();
+      p->w_max = 16;
+    }
+  }
+  std::vector<Node> queue;
+  if (!p->whole_groups) {
+    for (int64_t i = 0; i < count; ++i) {
+      const nla_batch_desc& d = descs[i];
+      if (d.n == 0 || d.m == 0) continue;
+      const int b = bucket_of(d.n);
+      add_groups(i, dtype == NLA_F64 ? std::min(tun.cols[b], 64) : tun.cols[b], [&](const Group& g) {
+        GroupBuilder gb;
+        gb.gi = (int)groups.size();
+        gb.cutoff = tun.cutoff[b];
+        gb.rev = p->rev != 0;
+        gb.nodes = &nodes;
+        gb.group_w = g.w;
+        gb.leaves(0, (int)d.n);
+        gb.chain.assign(gb.leaf_start.size(), 0);
+        gb.last_node.assign(gb.leaf_start.size(), -1);
+        gb.rec(0, (int)d.n);
+        leaves_total += (int)gb.leaf_start.size();
+      });
+    }
+    if (groups.size() > (size_t)INT32_MAX / 2 || nodes.size() > (size_t)INT32_MAX / 2) {
+      delete p;
+      return fail(NLA_ERR_UNSUPPORTED, "batch too large");
+    }
+    p->nnodes = (int)nodes.size();
+    p->smem = bat::node_smem_bytes(dtype, p->w_max);
+    if (dtype == NLA_F64) rc = node_kernel_setup<double>(p->smem, &per_sm);
+    else if (dtype == NLA_F32) rc = node_kernel_setup<float>(p->smem, &per_sm);
+    else rc = node_kernel_setup<__half>(p->smem, &per_sm);
+    if (rc != NLA_OK) {
+      delete p;
+      return rc;
+    }
+    p->grid = std::max(1, std::min(std::max(p->nnodes, 1), num_sms() * std::max(per_sm, 1)));
+    const std::vector<int> order = schedule(nodes, p->grid);
+    queue.resize(nodes.size());
+    for (size_t k = 0; k < order.size(); ++k) queue[k] = nodes[order[k]].d;
   }
   p->h_groups = groups;
   p->ngroups = (int)groups.size();
   p->nleaves = leaves_total;
-  p->nnodes = (int)nodes.size();
-  p->smem = bat::node_smem_bytes(dtype, p->w_max);
-  int per_sm = 0, rc;
-  if (dtype == NLA_F64) rc = node_kernel_setup<double>(p->smem, &per_sm);
-  else if (dtype == NLA_F32) rc = node_kernel_setup<float>(p->smem, &per_sm);
-  else rc = node_kernel_setup<__half>(p->smem, &per_sm);
-  if (rc != NLA_OK) {
-    delete p;
-    return rc;
-  }
-  p->grid = std::max(1, std::min(std::max(p->nnodes, 1), num_sms() * std::max(per_sm, 1)));
-  const std::vector<int> order = schedule(nodes, p->grid);
-  std::vector<Node> queue(nodes.size());
-  for (size_t k = 0; k < order.size(); ++k) queue[k] = nodes[order[k]].d;
 
   p->counter_bytes = sizeof(int) * (size_t)(2 + p->ngroups + p->nleaves);
   cudaError_t e = cudaMalloc(&p->d_descs, sizeof(nla_batch_desc) * (size_t)std::max<int64_t>(count, 1));
   if (e == cudaSuccess) e = cudaMalloc(&p->d_groups, sizeof(Group) * (size_t)std::max(p->ngroups, 1));
-  if (e == cudaSuccess) e = cudaMalloc(&p->d_nodes, sizeof(Node) * (size_t)std::max(p->nnodes, 1));
+  if (e == cudaSuccess) e = cudaMalloc(&p->d_nodes, sizeof(Node) * std::max<size_t>(queue.size(), 1));
+  if (e == cudaSuccess) e = cudaMalloc(&p->d_items, sizeof(bat::GroupItem) * std::max<size_t>(items.size(), 1));
+  if (e == cudaSuccess && !items.empty())
+    e = cudaMemcpy(p->d_items, items.data(), sizeof(bat::GroupItem) * items.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMalloc(reinterpret_cast<void**>(&p->d_counters), p->counter_bytes);
   if (e == cudaSuccess && count > 0)
     e = cudaMemcpy(p->d_descs, descs, sizeof(nla_batch_desc) * (size_t)count, cudaMemcpyHostToDevice);
   if (e == cudaSuccess && p->ngroups > 0)
     e = cudaMemcpy(p->d_groups, groups.data(), sizeof(Group) * groups.size(), cudaMemcpyHostToDevice);
-  if (e == cudaSuccess && p->nnodes > 0)
+  if (e == cudaSuccess && !queue.empty())
     e = cudaMemcpy(p->d_nodes, queue.data(), sizeof(Node) * queue.size(), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->cap_stream, cudaStreamNonBlocking);
   if (e != cudaSuccess) {
     cudaFree(p->d_descs);
     cudaFree(p->d_groups);
     cudaFree(p->d_nodes);
+    cudaFree(p->d_items);
     cudaFree(p->d_counters);
     delete p;
     return cuda_status(e, "batch plan allocation");
@@ -1765,6 +2064,7 @@ int nla_batch_plan_destroy(nla_batch_plan p) {
   cudaFree(p->d_descs);
   cudaFree(p->d_groups);
   cudaFree(p->d_nodes);
+  cudaFree(p->d_items);
   cudaFree(p->d_counters);
   delete p;
   return NLA_OK;
