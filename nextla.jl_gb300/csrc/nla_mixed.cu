@@ -152,18 +152,22 @@ unsigned grid_for(int64_t total) {
   return (unsigned)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
-// FP64 diagonal blocks of the mixed recursion: 64 rows.  The FP64 leaf is
-// bound by GB300's FP64 pipe (2 FMA per clock per SM), so halving it from 128
-// moves half of its work onto the tensor cores as one more level of short
-// exact updates; with the fused staging, the short-K group table and the
-// finishing pass those cost less than the leaf time they save.
-int default_mixed_cutoff() {
+// Rows of the diagonal blocks of the mixed recursion.  Exact solves apply
+// 64-row blocks through their inverses on the tensor cores.  Elsewhere the
+// blocks run in FP64, bound by GB300's FP64 pipe (2 FMA per clock per SM), so
+// 64 rows move half of a 128-row block's work onto the tensor cores; with few
+// right-hand sides the short update between two 64-row blocks (staging,
+// product and their launches, about 30 us) costs more than that half, and
+// 128 rows are better.  Measured at 2048 right-hand sides (solve): 128 rows
+// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.
+int default_mixed_cutoff(int terms, char func, int64_t m) {
   const char* v = std::getenv("NLA_MIXED_CUTOFF");
   if (v && *v) {
     long x = std::atol(v);
     if (x > 0) return (int)(x > 1024 ? 1024 : x);
   }
-  return 64;
+  if (terms == EXACT_SLICES && func == 'S') return 64;
+  return m <= 24 * (int64_t)num_sms() ? 128 : 64;
 }
 
 }  // namespace
@@ -952,7 +956,7 @@ int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m
     uplo = uplo == 'L' ? 'U' : 'L';
   }
   *c = RecPlan{func, side, uplo, NLA_F64, m, opts.cutoff > 0 ? (opts.cutoff > 1024 ? 1024 : opts.cutoff)
-                                                             : default_mixed_cutoff(),
+                                                             : default_mixed_cutoff(opts.split_terms, func, m),
                s, GEMM_MIXED, opts.split_terms, opts.lowp == NLA_LOWP_BF16};
   if (n == 0 || m == 0) return NLA_OK;
   // Size the staging workspace once for the largest update (the top split).
