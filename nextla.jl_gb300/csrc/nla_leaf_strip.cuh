@@ -98,6 +98,10 @@ template <typename R> struct StripMath<cx::cpx<R>> {
   }
 };
 
+template <typename T> __device__ __forceinline__ T raw_zero() { return T(0.0f); }
+template <> __device__ __forceinline__ cx::cpx<float> raw_zero() { return cx::zero<float>(); }
+template <> __device__ __forceinline__ cx::cpx<double> raw_zero() { return cx::zero<double>(); }
+
 // Column pitch of X: a multiple of the vector, at least n.
 template <typename Tc> __host__ __device__ constexpr int st_ldx(int n) {
   constexpr int VK = StripTraits<Tc>::VK;
@@ -148,8 +152,8 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   // A chunk of the panel's rows, K columns k0 ..: slot e of a thread is
   // element (fi + e ei, fk + e ek), threads along the index that is
   // contiguous in memory.
-  Tc ra[PER];
-  Tc rd[DPER];
+  T ra[PER];  // as stored: converted when they go to shared memory, so that the loads stay together
+  T rd[DPER];
   const int fi = g.tA ? t / KC : t & (PB - 1), fk = g.tA ? t & (KC - 1) : t / PB;
   const int ei = g.tA ? ST_THREADS / KC : 0, ek = g.tA ? 0 : ST_THREADS / PB;
   const int64_t es = g.tA ? ei * si : ek * sk;
@@ -160,12 +164,12 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
     const T* p = A + (p0 + fi) * si + (k0 + fk) * sk;
     const int ni = n - p0 - fi, nk = kend - k0 - fk;  // slots inside: e ei < ni, e ek < nk
 #pragma unroll
-    for (int e = 0; e < PER; ++e) ra[e] = e * ei < ni && e * ek < nk ? Mx::conj_if(Elem<T>::load(p + e * es), g.cj) : Mx::zero();
+    for (int e = 0; e < PER; ++e) ra[e] = e * ei < ni && e * ek < nk ? p[e * es] : raw_zero<T>();
     if (diag) {
 #pragma unroll
       for (int e = 0; e < DPER; ++e) {
         const int i = g.tA ? di + e * de : di, k = g.tA ? dk : dk + e * de;
-        rd[e] = p0 + i < n && k < i ? Mx::conj_if(Elem<T>::load(A + (p0 + i) * si + (p0 + k) * sk), g.cj) : Mx::zero();
+        rd[e] = p0 + i < n && k < i ? A[(p0 + i) * si + (p0 + k) * sk] : raw_zero<T>();
       }
     }
   };
@@ -184,29 +188,29 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   if (!g.tB) {
     for (int c = warp; c < CW; c += 8)
       for (int i0 = lane; i0 < nr; i0 += 32 * BATCH) {
-        Tc v[BATCH];
+        T v[BATCH];
 #pragma unroll
         for (int u = 0; u < BATCH; ++u) {
           const int i = i0 + 32 * u;
-          v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c * bc) : Mx::zero();
+          v[u] = i < n && c < ncols ? B[i * bi + c * bc] : raw_zero<T>();
         }
 #pragma unroll
         for (int u = 0; u < BATCH; ++u)
-          if (i0 + 32 * u < nr) X[(size_t)c * ldx + i0 + 32 * u] = v[u];
+          if (i0 + 32 * u < nr) X[(size_t)c * ldx + i0 + 32 * u] = Elem<T>::load(&v[u]);
       }
   } else {
     constexpr int RS = ST_THREADS / CW;  // rows per pass
     const int c = t % CW;
     for (int i0 = t / CW; i0 < nr; i0 += RS * BATCH) {
-      Tc v[BATCH];
+      T v[BATCH];
 #pragma unroll
       for (int u = 0; u < BATCH; ++u) {
         const int i = i0 + RS * u;
-        v[u] = i < n && c < ncols ? Elem<T>::load(B + i * bi + c) : Mx::zero();
+        v[u] = i < n && c < ncols ? B[i * bi + c] : raw_zero<T>();
       }
 #pragma unroll
       for (int u = 0; u < BATCH; ++u)
-        if (i0 + RS * u < nr) X[(size_t)c * ldx + i0 + RS * u] = v[u];
+        if (i0 + RS * u < nr) X[(size_t)c * ldx + i0 + RS * u] = Elem<T>::load(&v[u]);
     }
   }
   if (SOLVE)
@@ -230,7 +234,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 #pragma unroll
       for (int e = 0; e < PER; ++e) {
         const int i = fi + e * ei, k = fk + e * ek;
-        Tc v = ra[e];
+        Tc v = Mx::conj_if(Elem<T>::load(&ra[e]), g.cj);
         if (!SOLVE) {  // the panel's own triangle: zero above, one on a unit diagonal
           const int r = p0 + i, kk = k0 + k;
           if (kk > r) v = Mx::zero();
@@ -243,7 +247,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 #pragma unroll
         for (int e = 0; e < DPER; ++e) {
           const int i2 = g.tA ? di + e * de : di, k2 = g.tA ? dk : dk + e * de;
-          Db[i2 * (PB + 1) + k2] = rd[e];
+          Db[i2 * (PB + 1) + k2] = Mx::conj_if(Elem<T>::load(&rd[e]), g.cj);
         }
       }
       __syncthreads();
