@@ -236,3 +236,29 @@ def test_exact_finish_pass_matches_epilogue(pkg, cuda, monkeypatch):
             out.append(C)
         assert torch.isnan(out[0][1]).all() and torch.isnan(out[0][:, 4]).all()
         assert torch.equal(out[0].nan_to_num(7.0), out[1].nan_to_num(7.0)), (N, R, M, t1)
+
+
+@pytest.mark.parametrize("pad,off", [(0, 0), (8, 0), (1, 0), (0, 8), (0, 4)])
+def test_f16_operands_read_in_place(pkg, oracle, cuda, pad, off):
+    """Float16 updates whose operands lie K-contiguous on 16-byte boundaries
+    are read where they are (pitch a multiple of 8, base aligned), others are
+    staged: both give the Float32-accumulated product, one rounding (2^-11)
+    per element, with remainders in every dimension."""
+    import torch
+
+    rng = np.random.default_rng(pad + off)
+    for N, K, M in ((136, 72, 200), (300, 100, 129), (129, 1000, 260)):
+        A, B, C = (rng.uniform(-1, 1, s).astype(np.float16) for s in ((N, K), (K, M), (N, M)))
+        ld = -(-K // 8) * 8 + pad
+        buf_a = torch.zeros(off + N * ld, dtype=torch.float16, device=cuda)
+        buf_b = torch.zeros(off + M * ld, dtype=torch.float16, device=cuda)
+        At = buf_a[off:].view(N, ld)[:, :K]  # row-major: the transposed view of a column-major parent
+        Bd = buf_b[off:].view(M, ld)[:, :K].T
+        At.copy_(torch.from_numpy(A))
+        Bd.copy_(torch.from_numpy(B))
+        Cd = torch.from_numpy(np.ascontiguousarray(C.T)).to(cuda).T
+        pkg.matmul_(Cd, At, Bd, -1.0)
+        torch.cuda.synchronize()
+        ref = C.astype(np.float64) - A.astype(np.float64) @ B.astype(np.float64)
+        got = Cd.cpu().numpy().astype(np.float64)
+        assert (np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) * 1.01 + K * 2.0 ** -23).all(), (N, K, M)
