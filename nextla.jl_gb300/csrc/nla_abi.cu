@@ -116,6 +116,7 @@ int num_sms() {
 // ---------------------------------------------------------------------------
 template <typename T, typename Tm>
 __global__ void scale_kernel(int64_t rows, int64_t cols, Tm alpha, T* B, int64_t ldb, int tB) {
+  chain_begin();
   const int64_t total = rows * cols;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
@@ -150,8 +151,7 @@ int launch_scale(int dtype, int64_t rows, int64_t cols, double alpha, const Mat&
       break;
     case NLA_F16:
       if (f32_exact)
-        scale_kernel<__half, float><<<(unsigned)blocks, 256, 0, s>>>(rows, cols, (float)alpha, (__half*)B.p, B.ld,
-                                                                      B.t);
+        scale_kernel<__half, float><<<(unsigned)blocks, 256, 0, s>>>(rows, cols, (float)alpha, (__half*)B.p, B.ld, B.t);
       else
         scale_kernel<__half, double><<<(unsigned)blocks, 256, 0, s>>>(rows, cols, alpha, (__half*)B.p, B.ld, B.t);
       break;

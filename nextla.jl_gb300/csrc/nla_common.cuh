@@ -67,6 +67,41 @@ inline Mat transposed(const Mat& v) {
   return r;
 }
 
+// Chained launches (programmatic dependent launch).  The recursions are
+// chains of short kernels on one stream, each launch of which costs about 2
+// us between the end of one kernel and the start of the next.  A chained
+// kernel is set up on the SMs while its predecessor still runs and waits in
+// chain_begin(), before it touches memory, until that one has completed with
+// its writes visible; it then lets its own successor be set up.  So at most
+// two kernels of a chain are in flight and every access keeps its order.
+// (Tensor memory too is taken only after the wait: the predecessor may hold
+// all of it.)  Chained are the tensor-core kernels, which take an SM each, and
+// the staging and finishing passes around them.  Kernels of few CTAs that
+// share SMs (the strips, the CUDA-core updates) are not: set up early, their
+// CTAs gather on the SMs that the predecessor leaves free (1024 x 256 Float64
+// solve 445 -> 628 us).  They still let a chained successor be set up.
+// Measured: Float16 8192 x 4096 2.37 -> 2.26 ms, LU solve of 3001 1163 -> 1083
+// us, 3-term solve 11.76 -> 11.53 ms, Float32 8192^2 5.58 -> 5.48 ms.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... Params, typename... Args>
+void launch_chained(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);  // errors: NLA_CHECK_LAUNCH
+}
+
 // Element conversions between storage and compute types.
 template <typename T> struct Elem;
 template <> struct Elem<double> {

@@ -29,6 +29,7 @@ template <typename R, int GT>
 __global__ void __launch_bounds__(256) cplx_gemm_kernel(int64_t N, int64_t M, int64_t K, R alpha, const cpx<R>* A,
                                                         int64_t lda, int tA, int cA, const cpx<R>* B, int64_t ldb,
                                                         int tB, int cB, cpx<R>* C, int64_t ldc) {
+  chain_begin();
   __shared__ cpx<R> As[GK][GT + 1], Bs[GK][GT + 1];
   const int t = threadIdx.x, tr = t % 16, tc = t / 16;
   const int64_t i0 = (int64_t)blockIdx.x * GT, j0 = (int64_t)blockIdx.y * GT;
@@ -138,8 +139,7 @@ int launch_gemm_complex(int dtype, int64_t N, int64_t M, int64_t K, double alpha
   const dim3 grid((unsigned)gx, (unsigned)gy);
   auto run = [&](auto kernel, auto one) {
     using R = decltype(one);
-    kernel<<<grid, 256, 0, s>>>(N, M, K, (R)alpha, static_cast<const cx::cpx<R>*>(A.p), A.ld, A.t, A.c,
-                                static_cast<const cx::cpx<R>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<R>*>(C.p), C.ld);
+    kernel<<<grid, 256, 0, s>>>(N, M, K, (R)alpha, static_cast<const cx::cpx<R>*>(A.p), A.ld, A.t, A.c, static_cast<const cx::cpx<R>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<R>*>(C.p), C.ld);
   };
   if (dtype == NLA_C64) gt == 64 ? run(cx::cplx_gemm_kernel<double, 64>, 1.0) : run(cx::cplx_gemm_kernel<double, 32>, 1.0);
   else gt == 64 ? run(cx::cplx_gemm_kernel<float, 64>, 1.0f) : run(cx::cplx_gemm_kernel<float, 32>, 1.0f);

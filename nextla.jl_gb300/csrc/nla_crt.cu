@@ -255,6 +255,7 @@ __device__ __forceinline__ void split_tile(const Job& j, const double (*tile)[65
 // Row exponents of both operands, one 32 x 64 tile per CTA (e preset to
 // SENTINEL_EXP).
 __global__ void __launch_bounds__(256) crt_exp_kernel(const Job a, const Job b, int blocks_a) {
+  chain_begin();
   __shared__ int sred[8][32];
   const bool first = (int)blockIdx.x < blocks_a;
   const Job j = first ? a : b;
@@ -274,6 +275,7 @@ __global__ void __launch_bounds__(256) crt_exp_kernel(const Job a, const Job b, 
 }
 
 __global__ void __launch_bounds__(256) crt_split_kernel(const Job a, const Job b, int blocks_a) {
+  chain_begin();
   __shared__ double tile[32][65];
   __shared__ int sexp[32];
   const bool first = (int)blockIdx.x < blocks_a;
@@ -291,6 +293,7 @@ __global__ void __launch_bounds__(256) crt_split_kernel(const Job a, const Job b
 // Short K: exponents and residues of 32 rows by one CTA (the second pass over
 // its rows reads L2), so one launch stages both operands.
 __global__ void __launch_bounds__(256) crt_stage_kernel(const Job a, const Job b, int blocks_a) {
+  chain_begin();
   __shared__ double tile[2][32][65];
   __shared__ int sred[8][32];
   __shared__ int sexp[32];
@@ -384,6 +387,7 @@ __device__ __forceinline__ uint4 signed_bytes(const float (&z)[16]) {
 
 __global__ void __launch_bounds__(THREADS, 1)
     crt_gemm_kernel(const __grid_constant__ CUtensorMap tmU, const __grid_constant__ CUtensorMap tmV, const GemmArgs p) {
+  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* fullU = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
@@ -646,6 +650,7 @@ constexpr int FIN_PITCH = 36;    // four rows of 32 lanes, staggered over the ba
 // bytes of every plane as one word, forms their integers, and the results
 // pass through shared memory so that C is read and written along its rows.
 __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) {
+  chain_begin();
   __shared__ double buf[8][4 * FIN_PITCH];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = blockIdx.x * 128;
@@ -799,16 +804,16 @@ int crt_stage(const Mat& X, const CrtStaged& sx, const Mat* Y, const CrtStaged* 
   if (Y) elems += (double)sy->rows * (double)sy->K;
   TraceScope trace(NLA_K_SPLIT, s, 0.0, elems * (16.0 + 2.0 * L));
   if (kmax <= 256) {
-    crt_stage_kernel<<<(unsigned)(ba + bb), 256, 0, s>>>(a, b, ba);
+    launch_chained(crt_stage_kernel, (unsigned)(ba + bb), 256, 0, s, a, b, ba);
     NLA_CHECK_LAUNCH("crt_stage_kernel");
     return NLA_OK;
   }
   cudaMemsetAsync(sx.e, 0x80, (size_t)sx.rows_pad * sizeof(int), s);
   if (Y) cudaMemsetAsync(sy->e, 0x80, (size_t)sy->rows_pad * sizeof(int), s);
   const dim3 grid((unsigned)(ba + bb), (unsigned)(kmax / 64));
-  crt_exp_kernel<<<grid, 256, 0, s>>>(a, b, ba);
+  launch_chained(crt_exp_kernel, grid, 256, 0, s, a, b, ba);
   NLA_CHECK_LAUNCH("crt_exp_kernel");
-  crt_split_kernel<<<grid, 256, 0, s>>>(a, b, ba);
+  launch_chained(crt_split_kernel, grid, 256, 0, s, a, b, ba);
   NLA_CHECK_LAUNCH("crt_split_kernel");
   trace_kernels(1);
   return NLA_OK;
@@ -853,7 +858,7 @@ int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C,
   TraceScope trace(NLA_K_GEMM_UMMA, s, 2.0 * (double)g.M * g.N * (double)g.K * L * tri_frac,
                    2.0 * L * (double)(A.rows_pad + B.rows_pad) * A.K_pad + (2.0 * L + 16.0) * (double)g.M * g.N);
   const int sms = num_sms();
-  crt_gemm_kernel<<<(unsigned)(g.items < sms ? g.items : sms), THREADS, SMEM, s>>>(mU, mV, g);
+  launch_chained(crt_gemm_kernel, (unsigned)(g.items < sms ? g.items : sms), THREADS, SMEM, s, mU, mV, g);
   NLA_CHECK_LAUNCH("crt_gemm_kernel");
   FinishArgs f{};
   f.planes = planes;
@@ -875,7 +880,7 @@ int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C,
     f.d_col = d_col ? 1 : 0;
   }
   const dim3 grid((unsigned)(A.rows_pad / 128), (unsigned)((g.N + 8 * FIN_COLS - 1) / (8 * FIN_COLS)));
-  crt_finish_kernel<<<grid, 256, 0, s>>>(f);
+  launch_chained(crt_finish_kernel, grid, 256, 0, s, f);
   NLA_CHECK_LAUNCH("crt_finish_kernel");
   trace_kernels(1);
   return NLA_OK;

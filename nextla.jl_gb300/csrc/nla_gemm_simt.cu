@@ -41,6 +41,7 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(int64_t N, int64_t M, in
                                                         const T* __restrict__ A, int64_t lda, int tA,
                                                         const T* __restrict__ B, int64_t ldb, int tB, T* C,
                                                         int64_t ldc) {
+  chain_begin();
   using Tc = typename Elem<T>::compute;
   static_assert(RN == 2 * V || RN == 1, "columns per thread");
   constexpr int BM = 32 * V;
@@ -149,9 +150,7 @@ int launch_simt(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, con
   if (gx > 2147483647LL || gy > 65535) return fail(NLA_ERR_UNSUPPORTED, "gemm: matrix too large for one launch");
   TraceScope trace(NLA_K_GEMM_SIMT, s, 2.0 * (double)N * (double)M * (double)K,
                    (double)sizeof(T) * ((double)N * K + (double)K * M + 2.0 * (double)N * M));
-  gemm_simt_kernel<T, V, RN, BK><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(
-      N, M, K, alpha, static_cast<const T*>(A.p), A.ld, A.t, static_cast<const T*>(B.p), B.ld, B.t,
-      static_cast<T*>(C.p), C.ld);
+  gemm_simt_kernel<T, V, RN, BK><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, s>>>(N, M, K, alpha, static_cast<const T*>(A.p), A.ld, A.t, static_cast<const T*>(B.p), B.ld, B.t, static_cast<T*>(C.p), C.ld);
   NLA_CHECK_LAUNCH("gemm_simt_kernel");
   return NLA_OK;
 }

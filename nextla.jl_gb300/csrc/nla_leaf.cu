@@ -82,6 +82,7 @@ int launch_leaf_cols2(const LeafArgs& g, cudaStream_t s) {
 
 template <typename T, int PB, int NC, int WC, bool SOLVE>
 __global__ void __launch_bounds__(ST_THREADS) leaf_strip_kernel(const LeafArgs g) {
+  chain_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   strip_block<T, PB, NC, WC, SOLVE>(g, smem_raw);
 }

@@ -434,6 +434,7 @@ struct LeafProdArgs {
 };
 
 __global__ void __launch_bounds__(LP_THREADS, 1) leaf_product_kernel(const LeafProdArgs a) {
+  chain_begin();
   extern __shared__ uint8_t lp_smem_raw[];
   const LpShared s = lp_shared(lp_smem_raw);
   __shared__ volatile int s_abort;
@@ -568,6 +569,7 @@ __device__ __forceinline__ void lp_tile_store(const double* tile, double* X, int
 
 template <bool SIDE_R>
 __global__ void __launch_bounds__(LP_THREADS, 1) leaf_pair_kernel(const LeafPairArgs a) {
+  chain_begin();
   extern __shared__ uint8_t lp_smem_raw[];
   const LpShared s = lp_shared(lp_smem_raw);
   __shared__ volatile int s_abort;
@@ -803,7 +805,7 @@ int leaf_inverse_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) 
   const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
   if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf product: too many right-hand sides");
   TraceScope trace(NLA_K_LEAF_SOLVE, c.s, 2.0 * (double)n * n * (double)c.m, 16.0 * (double)n * (double)c.m);
-  leaf_product_kernel<<<(unsigned)grid, LP_THREADS, LP_SMEM, c.s>>>(g);
+  launch_chained(leaf_product_kernel, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
   NLA_CHECK_LAUNCH("leaf_product_kernel");
   return NLA_OK;
 }
@@ -858,8 +860,8 @@ int leaf_pair_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf pair: too many right-hand sides");
   TraceScope trace(NLA_K_LEAF_SOLVE, c.s, 2.0 * (double)(nf * nf + ns * ns + nf * ns) * (double)c.m,
                    8.0 * (double)(2 * n + ns) * (double)c.m);
-  if (R) leaf_pair_kernel<true><<<(unsigned)grid, LP_THREADS, LP_SMEM, c.s>>>(g);
-  else leaf_pair_kernel<false><<<(unsigned)grid, LP_THREADS, LP_SMEM, c.s>>>(g);
+  if (R) launch_chained(leaf_pair_kernel<true>, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
+  else launch_chained(leaf_pair_kernel<false>, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
   NLA_CHECK_LAUNCH("leaf_pair_kernel");
   return NLA_OK;
 }

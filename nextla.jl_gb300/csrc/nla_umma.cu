@@ -95,6 +95,7 @@ template <int EPI>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
     umma_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                      const GemmParams p) {
+  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + (size_t)p.stages * p.stage_bytes);
@@ -999,6 +1000,7 @@ __device__ __forceinline__ bool in_tri(int tri, int64_t i, int64_t k) {
 template <typename T>
 __global__ void __launch_bounds__(256) row_exp_kernel(const T* __restrict__ X, int64_t ld, int t, int64_t rows,
                                                       int64_t cols, int tri, int* __restrict__ e) {
+  chain_begin();
   __shared__ int se[64];
   if (threadIdx.x < 64) se[threadIdx.x] = SENTINEL_EXP;
   __syncthreads();
@@ -1184,6 +1186,7 @@ __global__ void __launch_bounds__(256) split_kernel(const T* __restrict__ X, int
                                                     int64_t cols, int tri, const int* __restrict__ e,
                                                     Sl* __restrict__ out, int64_t rows_pad, int64_t cols_pad,
                                                     float* __restrict__ nrm) {
+  chain_begin();
   __shared__ double tile[32][65];
   const int64_t i0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 64;
   (void)rows_pad;
@@ -1224,6 +1227,7 @@ struct StageJob {
 // stream operations of two separately staged operands.
 template <typename Sl, int NS>
 __global__ void __launch_bounds__(256, 4) stage_pair_kernel(const StageJob a, const StageJob b) {
+  chain_begin();
   __shared__ double tile[2][32][65];
   __shared__ int sred[8][32];
   __shared__ int sexp[32];
@@ -1575,7 +1579,7 @@ int stage_operand(const Mat& X, int64_t rows, int64_t K, int in_dtype, int S, bo
                    (double)rows * (double)K * (double)dtype_size(in_dtype) * (copy ? 1 : 2) + (double)S * Rp * Kp * 2);
   const dim3 gs((unsigned)(Rp / 32), (unsigned)(Kp / 64));
   if (copy) {
-    split_kernel<__half, __half, 0><<<gs, 256, 0, s>>>((const __half*)X.p, X.ld, X.t, rows, K, tri, nullptr,
+    launch_chained(split_kernel<__half, __half, 0>, gs, 256, 0, s, (const __half*)X.p, X.ld, X.t, rows, K, tri, nullptr,
                                                        (__half*)out->slices, Rp, Kp, nullptr);
     NLA_CHECK_LAUNCH("split_kernel");
     return NLA_OK;
@@ -1592,18 +1596,18 @@ int stage_operand(const Mat& X, int64_t rows, int64_t K, int in_dtype, int S, bo
   if (bf16) {
     auto* o = static_cast<__nv_bfloat16*>(out->slices);
     switch (S) {
-      case 1: split_kernel<double, __nv_bfloat16, 1><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
-      case 2: split_kernel<double, __nv_bfloat16, 2><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
-      case 3: split_kernel<double, __nv_bfloat16, 3><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
-      case EXACT_SLICES: split_kernel<double, __nv_bfloat16, EXACT_SLICES><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 1: launch_chained(split_kernel<double, __nv_bfloat16, 1>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 2: launch_chained(split_kernel<double, __nv_bfloat16, 2>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 3: launch_chained(split_kernel<double, __nv_bfloat16, 3>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case EXACT_SLICES: launch_chained(split_kernel<double, __nv_bfloat16, EXACT_SLICES>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
       default: return fail(NLA_ERR_ARG, "BF16 slices: 1, 2, 3 or 7 terms");
     }
   } else {
     auto* o = static_cast<__half*>(out->slices);
     switch (S) {
-      case 1: split_kernel<double, __half, 1><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
-      case 2: split_kernel<double, __half, 2><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
-      case 3: split_kernel<double, __half, 3><<<gs, 256, 0, s>>>(xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 1: launch_chained(split_kernel<double, __half, 1>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 2: launch_chained(split_kernel<double, __half, 2>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
+      case 3: launch_chained(split_kernel<double, __half, 3>, gs, 256, 0, s, xp, X.ld, X.t, rows, K, tri, out->e, o, Rp, Kp, out->nrm); break;
       default: return fail(NLA_ERR_ARG, "FP16 slices: 1, 2 or 3 terms");
     }
   }
@@ -1807,10 +1811,10 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
   if (smem > GEMM_DYN_SMEM) return fail(NLA_ERR_UNSUPPORTED, "tensor-core update: shared memory plan too large");
   if (out_dtype == NLA_F64) {
     NLA_TRY(ensure_gemm_smem<EPI_F64>());
-    umma_gemm_kernel<EPI_F64><<<(unsigned)grid, GEMM_THREADS, smem, s>>>(mA, mB, p);
+    launch_chained(umma_gemm_kernel<EPI_F64>, (unsigned)grid, GEMM_THREADS, smem, s, mA, mB, p);
   } else if (out_dtype == NLA_F16) {
     NLA_TRY(ensure_gemm_smem<EPI_F16>());
-    umma_gemm_kernel<EPI_F16><<<(unsigned)grid, GEMM_THREADS, smem, s>>>(mA, mB, p);
+    launch_chained(umma_gemm_kernel<EPI_F16>, (unsigned)grid, GEMM_THREADS, smem, s, mA, mB, p);
   } else {
     return fail(NLA_ERR_DTYPE, "tensor-core update: unsupported output type");
   }

@@ -105,6 +105,7 @@ __device__ __noinline__ float plain_dot(const F32Params& p, int i, int j) {
 __global__ void __launch_bounds__(F32_THREADS, 1)
     umma_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ F32Params p) {
+  chain_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* fullA = reinterpret_cast<uint64_t*>(smem + F32_STAGES * F32_STAGE_BYTES);
@@ -301,6 +302,7 @@ __device__ __forceinline__ float bf16_near(float x) {
 }
 
 __global__ void __launch_bounds__(256) stage_f32_kernel(const F32Job a, const F32Job b) {
+  chain_begin();
   __shared__ float tile[32][66];
   const bool first = (int)blockIdx.x < a.blocks;
   const F32Job j = first ? a : b;
@@ -403,7 +405,7 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
     TraceScope trace(NLA_K_SPLIT, s, 0.0, (double)(M + N) * (double)K * 4.0 + (double)(Mp + Np) * Kp * 2.0 * SL);
     const F32Job ja{p.A, p.asi, p.ask, (int)M, (int)K, p.cplx, p.ima, ta, Kp, marks, (int)(Mp / 32)};
     const F32Job jb{p.B, p.bsj, p.bsk, (int)N, (int)K, 2 * p.cplx, p.imb, tb, Kp, marks + Mp * (Kp / BK), (int)(Np / 32)};
-    stage_f32_kernel<<<dim3((unsigned)((Mp + Np) / 32), (unsigned)(Kp / 64)), 256, 0, s>>>(ja, jb);
+    launch_chained(stage_f32_kernel, dim3((unsigned)((Mp + Np) / 32), (unsigned)(Kp / 64)), 256, 0, s, ja, jb);
     NLA_CHECK_LAUNCH("stage_f32_kernel");
   }
   CUtensorMap mA, mB;
@@ -417,7 +419,7 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
   if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(umma_f32_kernel)");
   TraceScope trace(NLA_K_GEMM_UMMA, s, 6.0 * 2.0 * (double)M * (double)N * (double)K,
                    (double)SL * 2.0 * (double)(Mp + Np) * Kp + 8.0 * (double)M * (double)N);
-  umma_f32_kernel<<<(unsigned)((int64_t)p.tiles_m * p.tiles_n), F32_THREADS, F32_SMEM, s>>>(mA, mB, p);
+  launch_chained(umma_f32_kernel, (unsigned)((int64_t)p.tiles_m * p.tiles_n), F32_THREADS, F32_SMEM, s, mA, mB, p);
   NLA_CHECK_LAUNCH("umma_f32_kernel");
   return NLA_OK;
 }
