@@ -37,10 +37,11 @@ namespace {
 constexpr int L = 16;
 constexpr int BU = 128, BV = 256, BK = 64;
 constexpr int U_BYTES = BU * BK * 2, V_BYTES = BV * BK * 2;
-constexpr int STAGES = 4, STAGE_BYTES = U_BYTES + V_BYTES;
+constexpr int RING_BYTES = 4 * (U_BYTES + V_BYTES);  // four stages, or six of 128 + 128 rows
+constexpr int MAX_STAGES = RING_BYTES / (2 * U_BYTES);
 constexpr int DRAIN_WARPS = 16, THREADS = (3 + DRAIN_WARPS) * 32;
 constexpr int CHUNK = 16;  // K blocks of 64 per exact FP32 sum: 1024 x 2^14 = 2^24
-constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
+constexpr int SMEM = RING_BYTES + 1024 + 256;
 static_assert(SMEM + 64 <= 232448, "shared memory above the per-block limit");
 constexpr int SENTINEL_EXP = -2139062144;  // 0x80808080: "no element seen"
 constexpr int NONFINITE_EXP = 0x7fffffff;
@@ -56,8 +57,7 @@ constexpr int GROUPS = (L + 2) / 3;
 
 struct Tables {
   float p[L], inv_p[L];      // modulus and its reciprocal
-  uint32_t t0[2][L], t1[2][L];  // bytes 2^(8 i) f mod p, i = 0..3 and 4..7
-  uint32_t off[2][L];           // -2^55 f mod p; f = 1, or (P / p)^-1 for C's row operand
+  float k[2][L][4];  // 2^(14 i) f mod p, balanced; f = 1, or (P / p)^-1 for C's row operand
   uint32_t in[L];            // P_g / p
   uint32_t m[GROUPS][4];     // P / P_g, 32-bit limbs
   uint32_t q[GROUPS];        // round(2^54 / P_g)
@@ -84,13 +84,10 @@ constexpr Tables make_tables() {
     T.inv_p[l] = 1.0f / (float)p;
     for (int o = 0; o < 2; ++o) {
       uint32_t f = o ? w : 1;
-      for (int i = 0; i < 8; ++i) {
-        (i < 4 ? T.t0[o][l] : T.t1[o][l]) |= f << (8 * (i & 3));
-        f = f * 256 % p;
+      for (int i = 0; i < 4; ++i) {
+        T.k[o][l][i] = f > p / 2 ? (float)f - (float)p : (float)f;
+        f = f * (16384u % p) % p;
       }
-      f = o ? w : 1;
-      for (int i = 0; i < 55; ++i) f = f * 2 % p;
-      T.off[o][l] = (p - f) % p;
     }
   }
   for (int g = 0; g < GROUPS; ++g) {
@@ -171,14 +168,22 @@ __device__ __forceinline__ long long fixed_of(double x, int ex, int bits) {
 }
 
 // One 32 x 64 tile (rows i0.., K k0..): eight loads per thread, all in
-// flight, along the index that is contiguous in memory.
+// flight, along the index that is contiguous in memory (slot e at row
+// i + e di, K k + e dk of the thread's first).
 __device__ __forceinline__ void load_tile(const Job& j, int64_t i0, int64_t k0, double (&v)[8]) {
   const bool kfast = j.sk == 1;
+  const int t = threadIdx.x, ti = kfast ? t >> 6 : t & 31, tk = kfast ? t & 63 : t >> 5;
+  const int di = kfast ? 4 : 0, dk = kfast ? 0 : 8;
+  const double* p = j.X + (i0 + ti) * j.si + (k0 + tk) * j.sk;
+  const int64_t step = kfast ? 4 * j.si : 8 * j.sk;
+  const int ni = (int)min((int64_t)64, j.rows - i0) - ti, nk = (int)min((int64_t)64, j.K - k0) - tk;
+  if (j.tri == 0) {
 #pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    const int idx = threadIdx.x + 256 * e;
-    const int64_t i = i0 + (kfast ? idx >> 6 : idx & 31), k = k0 + (kfast ? idx & 63 : idx >> 5);
-    v[e] = i < j.rows && k < j.K && in_tri(j.tri, i, k) ? j.X[i * j.si + k * j.sk] : 0.0;
+    for (int e = 0; e < 8; ++e) v[e] = e * di < ni && e * dk < nk ? p[e * step] : 0.0;
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      v[e] = e * di < ni && e * dk < nk && in_tri(j.tri, i0 + ti + e * di, k0 + tk + e * dk) ? p[e * step] : 0.0;
   }
 }
 
@@ -216,11 +221,21 @@ __device__ __forceinline__ int row_max_of(const Job& j, int (*sred)[32], int r) 
   return x;
 }
 
-// The residues of the tile.  y + 2^55 is taken byte by byte: sum_i byte_i
-// (2^(8 i) mod p) + (-2^55 mod p) < 2^20 by two dot products, and its
-// balanced residue in float arithmetic.  C's row operand carries the factor
-// (P / p)^-1 of the reconstruction in the same constants.  Two adjacent K values per lane, one
+// The residues of the tile.  y is cut into 14-bit pieces (the top one
+// signed), whose products with 2^(14 i) mod p and their sum stay below 2^23:
+// exact in Float32, on the FMA pipe rather than the integer one (four dot
+// products of bytes, the form before, took 276 instructions per element and
+// 1.4 times as long).  C's row operand carries the factor (P / p)^-1 of the
+// reconstruction in the same constants.  Two adjacent K values per lane, one
 // 32-bit store per modulus.
+__device__ __forceinline__ void pieces14(long long y, float (&c)[4]) {
+  const uint32_t lo = (uint32_t)y, hi = (uint32_t)((unsigned long long)y >> 32);
+  c[0] = __uint_as_float(0x4B000000u | (lo & 0x3FFFu)) - 8388608.0f;
+  c[1] = __uint_as_float(0x4B000000u | ((lo >> 14) & 0x3FFFu)) - 8388608.0f;
+  c[2] = __uint_as_float(0x4B000000u | (__funnelshift_r(lo, hi, 28) & 0x3FFFu)) - 8388608.0f;
+  c[3] = __int_as_float(0x4B400000 + ((int)hi >> 10)) - MAGIC;
+}
+
 template <int F>
 __device__ __forceinline__ void split_tile_f(const Job& j, const double (*tile)[65], const int* ex_rows, int64_t i0,
                                              int64_t k0) {
@@ -230,18 +245,19 @@ __device__ __forceinline__ void split_tile_f(const Job& j, const double (*tile)[
   for (int pass = 0; pass < 4; ++pass) {
     const int i = warp + 8 * pass;
     const int ex = ex_rows[i];
-    const long long y0 = fixed_of(tile[i][2 * lane], ex, j.bits) + (1ll << 55);
-    const long long y1 = fixed_of(tile[i][2 * lane + 1], ex, j.bits) + (1ll << 55);
-    const uint32_t l0 = (uint32_t)y0, h0 = (uint32_t)(y0 >> 32), l1 = (uint32_t)y1, h1 = (uint32_t)(y1 >> 32);
+    float c0[4], c1[4];
+    pieces14(fixed_of(tile[i][2 * lane], ex, j.bits), c0);
+    pieces14(fixed_of(tile[i][2 * lane + 1], ex, j.bits), c1);
     uint32_t* o = reinterpret_cast<uint32_t*>(j.out) + ((i0 + i) * j.K_pad + k0) / 2 + lane;
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      const uint32_t t0 = c_t.t0[F][l], t1 = c_t.t1[F][l], off = c_t.off[F][l];
-      const uint32_t s0 = __dp4a(l0, t0, __dp4a(h0, t1, off)), s1 = __dp4a(l1, t0, __dp4a(h1, t1, off));
-      const float r0 = mod_balanced(__uint_as_float(0x4B000000u | s0) - 8388608.0f, c_t.p[l], c_t.inv_p[l]);
-      const float r1 = mod_balanced(__uint_as_float(0x4B000000u | s1) - 8388608.0f, c_t.p[l], c_t.inv_p[l]);
+      const float* k = c_t.k[F][l];
+      const float s0 = fmaf(c0[3], k[3], fmaf(c0[2], k[2], fmaf(c0[1], k[1], c0[0] * k[0])));
+      const float s1 = fmaf(c1[3], k[3], fmaf(c1[2], k[2], fmaf(c1[1], k[1], c1[0] * k[0])));
+      const float r0 = mod_balanced(s0, c_t.p[l], c_t.inv_p[l]), r1 = mod_balanced(s1, c_t.p[l], c_t.inv_p[l]);
       // An integer of at most 8 bits: its BF16 pattern is the float's upper half.
-      o[l * plane] = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+      *o = __byte_perm(__float_as_uint(r0), __float_as_uint(r1), 0x7632);
+      o += plane;
     }
   }
 }
@@ -335,6 +351,7 @@ struct GemmArgs {
   int M, N, K;          // rows and columns of C
   int tiles_u, tiles_v, items;
   int bv;               // rows of C per tile: 256, or 128 when C has no more
+  int stages, stage_bytes;
   int rows_u, rows_v;   // padded: modulus l's plane starts at row l * rows
   int tri_u, tri_v;
   uint8_t* planes;      // byte (i, j) of modulus l at l * plane + i + j * ldp
@@ -390,10 +407,10 @@ __global__ void __launch_bounds__(THREADS, 1)
   chain_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* fullU = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);
-  uint64_t* fullV = fullU + STAGES;
-  uint64_t* empty = fullV + STAGES;
-  uint64_t* cfull = empty + STAGES;
+  uint64_t* fullU = reinterpret_cast<uint64_t*>(smem + RING_BYTES);
+  uint64_t* fullV = fullU + MAX_STAGES;
+  uint64_t* empty = fullV + MAX_STAGES;
+  uint64_t* cfull = empty + MAX_STAGES;
   uint64_t* cempty = cfull + 2;
   uint64_t* drain = cempty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
@@ -402,7 +419,7 @@ __global__ void __launch_bounds__(THREADS, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     s_abort = 0;
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < MAX_STAGES; ++s) {
       umma::mbar_init(umma::smem_u32(&fullU[s]), 1);
       umma::mbar_init(umma::smem_u32(&fullV[s]), 1);
       umma::mbar_init(umma::smem_u32(&empty[s]), 1);
@@ -428,28 +445,30 @@ __global__ void __launch_bounds__(THREADS, 1)
     if (lane == 0) {
       uint64_t* own = is_u ? fullU : fullV;
       const uint32_t bytes = (uint32_t)(is_u ? U_BYTES : p.bv * BK * 2);
-      int n = 0;
+      int n = 0, s = 0;
+      uint32_t par = 1;  // of the empty barriers: the first round passes
       for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x) {
         const Item it = item_at(p, w);
         const int y = it.l * (is_u ? p.rows_u : p.rows_v) + (is_u ? it.u0 : it.v0);
         for (int kb = it.kb0; kb < it.kb1; ++kb, ++n) {
-          const int s = n % STAGES;
-          if (!umma::mbar_wait(umma::smem_u32(&empty[s]), ((uint32_t)(n / STAGES) & 1u) ^ 1u, &s_abort, p.err, 61)) {
+          if (!umma::mbar_wait(umma::smem_u32(&empty[s]), par, &s_abort, p.err, 61)) {
             ok = false;
             break;
           }
           const uint32_t fb = umma::smem_u32(&own[s]);
           umma::mbar_arrive_expect_tx(fb, bytes);
-          umma::tma_load_2d(umma::smem_u32(smem + s * STAGE_BYTES + (is_u ? 0 : U_BYTES)), is_u ? &tmU : &tmV, fb,
+          umma::tma_load_2d(umma::smem_u32(smem + s * p.stage_bytes + (is_u ? 0 : U_BYTES)), is_u ? &tmU : &tmV, fb,
                             kb * BK, y);
+          if (++s == p.stages) s = 0, par ^= 1;
         }
       }
-      umma::producer_quiesce(own, STAGES, n, &s_abort, p.err, 62);
+      umma::producer_quiesce(own, p.stages, n, &s_abort, p.err, 62);
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t idesc = umma::idesc_f16(BU, p.bv, true);
-      int n = 0, ch = 0;
+      int s = 0, ch = 0;
+      uint32_t par = 0;
       for (int w = blockIdx.x; w < p.items && ok; w += gridDim.x) {
         const Item it = item_at(p, w);
         for (int c0 = it.kb0; c0 < it.kb1 && ok; c0 += CHUNK, ++ch) {
@@ -460,21 +479,20 @@ __global__ void __launch_bounds__(THREADS, 1)
           }
           umma::fence_after_sync();
           const uint32_t d = tmem + (uint32_t)(b * BV);
-          for (int kb = c0; kb < min(c0 + CHUNK, it.kb1); ++kb, ++n) {
-            const int s = n % STAGES;
-            const uint32_t par = (uint32_t)(n / STAGES) & 1u;
+          for (int kb = c0; kb < min(c0 + CHUNK, it.kb1); ++kb) {
             if (!umma::mbar_wait(umma::smem_u32(&fullU[s]), par, &s_abort, p.err, 64) ||
                 !umma::mbar_wait(umma::smem_u32(&fullV[s]), par, &s_abort, p.err, 64)) {
               ok = false;
               break;
             }
             umma::fence_after_sync();
-            const uint32_t a0 = umma::smem_u32(smem + s * STAGE_BYTES), b0 = a0 + U_BYTES;
+            const uint32_t a0 = umma::smem_u32(smem + s * p.stage_bytes), b0 = a0 + U_BYTES;
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk)
               umma::mma_f16(d, umma::desc_kmajor_sw128(a0 + kk * 32), umma::desc_kmajor_sw128(b0 + kk * 32), idesc,
                             (kb > c0 || kk > 0) ? 1u : 0u);
             umma::mma_commit(umma::smem_u32(&empty[s]));
+            if (++s == p.stages) s = 0, par ^= 1;
           }
           if (ok) umma::mma_commit(umma::smem_u32(&cfull[b]));
         }
@@ -831,6 +849,8 @@ int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C,
   g.N = (int)B.rows;
   g.K = (int)A.K;
   g.bv = A.rows_pad > 128 ? BV : 128;
+  g.stage_bytes = U_BYTES + g.bv * BK * 2;
+  g.stages = RING_BYTES / g.stage_bytes;
   g.tiles_u = (int)(B.rows_pad / BU);
   g.tiles_v = (int)((A.rows_pad + g.bv - 1) / g.bv);
   g.items = L * g.tiles_u * g.tiles_v;
