@@ -62,10 +62,14 @@ struct Tables {
   uint32_t m[GROUPS][4];     // P / P_g, 32-bit limbs
   uint32_t q[GROUPS];        // round(2^54 / P_g)
   uint32_t P[4];
-  // The planes hold z + 128 after a sign flip: 128 times the sums of the
-  // constants above, to be taken off.
+  // Starting values of the sums.  The planes hold z + 128 after a sign flip,
+  // so 128 times the sums of the constants above are taken off.  q0 makes
+  // the quotient's sum positive (QB too many, plus a half to round), and
+  // m0 takes QB P off for adding (QB - quotient) P; every limb starts
+  // 2^62 higher, which its successor takes back, so that all stay positive.
   unsigned long long m0[4], q0;
 };
+constexpr unsigned QB = 64;
 
 // Pairwise coprime, and small enough that a balanced residue that is off by
 // one from rounding (p / 2 + 1) is still a signed byte.
@@ -105,6 +109,9 @@ constexpr Tables make_tables() {
       T.q0 += g + 1 < GROUPS ? 128ull * T.in[l] * T.q[g] : (128ull * T.in[l] * T.q[g]) << 23;
     }
   }
+  for (int i = 0; i < 4; ++i)
+    T.m0[i] = 0 - T.m0[i] - (unsigned long long)QB * T.P[i] + (1ull << 62) - (i > 0 ? 1ull << 30 : 0);
+  T.q0 = ((unsigned long long)QB << 54) + (1ull << 53) - T.q0;
   return T;
 }
 __constant__ const Tables c_t = make_tables();
@@ -656,6 +663,33 @@ __device__ __forceinline__ double to_f64(unsigned long long m, int e, bool neg) 
   return __longlong_as_double((long long)(bits | (neg ? 1ull << 63 : 0ull)));
 }
 
+// The general case of round_wide, out of line.
+__device__ __noinline__ double round_wide_slow(unsigned long long hi, unsigned long long lo, bool neg, int e) {
+  const Wide x{hi, lo, neg};
+  int k;
+  const unsigned long long m = leading53(x, k);
+  return to_f64(m, k + e, neg);
+}
+
+// (-1)^(sign != 0) (u3 : u2 : u1 : u0) 2^e to nearest even, in 32-bit steps.
+__device__ __forceinline__ double round_wide(uint32_t u3, uint32_t u2, uint32_t u1, uint32_t u0, uint32_t sign, int e) {
+  // The three limbs from the leading one on, and whether any bit follows.
+  const bool top = u3 != 0;
+  const uint32_t a = top ? u3 : u2, b = top ? u2 : u1, c = top ? u1 : u0;
+  const uint32_t rest = top ? u0 : 0u;
+  const int lz = __clz((int)a);
+  const uint32_t n2 = __funnelshift_l(b, a, lz), n1 = __funnelshift_l(c, b, lz), n0 = c << lz;
+  const int biased = 1023 + (top ? 127 : 95) - lz + e;
+  if (a == 0 || biased <= 0 || biased >= 2046)
+    return round_wide_slow(((unsigned long long)u3 << 32) | u2, ((unsigned long long)u1 << 32) | u0, sign != 0, e);
+  const uint32_t ml = __funnelshift_r(n1, n2, 11);  // mantissa: n2 : n1 without its last 11 bits
+  const uint32_t up = ((n1 & 0x7FFu) + 0x3FFu + ((ml & 1u) | (uint32_t)((n0 | rest) != 0))) >> 11;
+  // The leading bit adds one to the exponent field, as does a carry.
+  const unsigned long long bits =
+      (((unsigned long long)(((uint32_t)(biased - 1) << 20) + (n2 >> 11)) << 32) | ml) + up;
+  return __longlong_as_double((long long)(bits | ((unsigned long long)(sign & 0x80000000u) << 32)));
+}
+
 __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e) {
   s = a + b;
   const double bp = s - a;
@@ -673,9 +707,12 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int i0 = blockIdx.x * 128;
   const int ib = i0 + 4 * lane;
-  int ei[4];
+  int er[4];  // row exponents with the bias (at least -4200: far below any sum that matters)
 #pragma unroll
-  for (int r = 0; r < 4; ++r) ei[r] = ib + r < p.M ? __ldg(p.ea + ib + r) : 0;
+  for (int r = 0; r < 4; ++r) {
+    er[r] = ib + r < p.M ? __ldg(p.ea + ib + r) : 0;
+    if (er[r] != NONFINITE_EXP) er[r] = max(er[r], -4000) + p.e_bias;
+  }
 #pragma unroll 1
   for (int cc = 0; cc < FIN_COLS; ++cc) {
     const int64_t col = ((int64_t)blockIdx.y * 8 + warp) * FIN_COLS + cc;
@@ -690,12 +727,14 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
       const int i = i0 + lane + 32 * r;
       cv[r] = i < p.M ? p.C[i + col * p.ldc] : 0.0;
     }
-    const int ej = __ldg(p.eb + col);
+    int ejc = __ldg(p.eb + col);
+    if (ejc != NONFINITE_EXP) ejc = max(ejc, -4000);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       // x = sum_l y_l (P / p_l) - round(sum_l y_l / p_l) P, |x| < 0.45 P.
-      unsigned long long a0 = 0 - c_t.m0[0], a1 = 0 - c_t.m0[1], a2 = 0 - c_t.m0[2], a3 = 0 - c_t.m0[3];
-      unsigned long long qs = (1ull << 53) - c_t.q0;
+      // The leading limb needs only its value modulo 2^32.
+      unsigned long long a0 = c_t.m0[0], a1 = c_t.m0[1], a2 = c_t.m0[2], qs = c_t.q0;
+      uint32_t a3 = (uint32_t)c_t.m0[3];
 #pragma unroll
       for (int g = 0; g < GROUPS; ++g) {
         uint32_t sg = 0;
@@ -706,26 +745,40 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
         a0 += (unsigned long long)sg * c_t.m[g][0];
         a1 += (unsigned long long)sg * c_t.m[g][1];
         a2 += (unsigned long long)sg * c_t.m[g][2];
-        a3 += (unsigned long long)sg * c_t.m[g][3];
+        a3 += sg * c_t.m[g][3];
       }
-      const long long q = (long long)qs >> 54;
-      long long s0 = (long long)(a0 - (unsigned long long)(q * (long long)c_t.P[0]));
-      long long s1 = (long long)(a1 - (unsigned long long)(q * (long long)c_t.P[1])) + (s0 >> 32);
-      long long s2 = (long long)(a2 - (unsigned long long)(q * (long long)c_t.P[2])) + (s1 >> 32);
-      long long s3 = (long long)(a3 - (unsigned long long)(q * (long long)c_t.P[3])) + (s2 >> 32);
-      Wide x;
-      x.lo = (unsigned long long)(uint32_t)s0 | ((unsigned long long)(uint32_t)s1 << 32);
-      x.hi = (unsigned long long)(uint32_t)s2 | ((unsigned long long)s3 << 32);
-      x.neg = (long long)x.hi < 0;
-      if (x.neg) {
-        x.lo = 0ull - x.lo;
-        x.hi = ~x.hi + (x.lo == 0 ? 1ull : 0ull);
+      const uint32_t nq = 2 * QB - (uint32_t)(qs >> 54);  // 2 QB - (quotient + QB)
+      a0 += (unsigned long long)nq * c_t.P[0];
+      a1 += (unsigned long long)nq * c_t.P[1] + (a0 >> 32);
+      a2 += (unsigned long long)nq * c_t.P[2] + (a1 >> 32);
+      a3 += nq * c_t.P[3] + (uint32_t)(a2 >> 32);
+      uint32_t u0 = (uint32_t)a0, u1 = (uint32_t)a1, u2 = (uint32_t)a2, u3 = a3;
+      const uint32_t sign = (uint32_t)((int)u3 >> 31);
+      {
+        // |x|
+        const unsigned long long lo = (((unsigned long long)(u1 ^ sign) << 32) | (u0 ^ sign)) + (sign & 1u);
+        const unsigned long long hi =
+            (((unsigned long long)(u3 ^ sign) << 32) | (u2 ^ sign)) + ((sign & 1u) && lo == 0 ? 1ull : 0ull);
+        u0 = (uint32_t)lo;
+        u1 = (uint32_t)(lo >> 32);
+        u2 = (uint32_t)hi;
+        u3 = (uint32_t)(hi >> 32);
       }
-      const bool bad = ei[r] == NONFINITE_EXP || ej == NONFINITE_EXP;
-      const int e = max(ei[r], -4000) + max(ej, -4000) + p.e_bias;
-      int k;
-      const unsigned long long m = leading53(x, k);
-      double v = to_f64(m, k + e, x.neg);
+      const int e = er[r] + ejc;
+      const bool bad = er[r] == NONFINITE_EXP || ejc == NONFINITE_EXP;
+      double v;
+      Wide x{};
+      unsigned long long m = 0;
+      int k = 0;
+      if (p.res_x == nullptr) {
+        v = round_wide(u3, u2, u1, u0, sign, e);
+      } else {
+        x.hi = ((unsigned long long)u3 << 32) | u2;
+        x.lo = ((unsigned long long)u1 << 32) | u0;
+        x.neg = sign != 0;
+        m = leading53(x, k);
+        v = to_f64(m, k + e, x.neg);
+      }
       if (bad) v = __longlong_as_double(0x7ff8000000000000ll);
       if (p.res_x != nullptr && ib + r < p.M) {
         // The rest of the exact product below its leading 53 bits.
