@@ -159,14 +159,17 @@ unsigned grid_for(int64_t total) {
 // right-hand sides the short update between two 64-row blocks (staging,
 // product and their launches, about 30 us) costs more than that half, and
 // 128 rows are better.  Measured at 2048 right-hand sides (solve): 128 rows
-// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.
+// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.  An exact solve
+// of few right-hand sides takes them too: a pair of inverse blocks costs 49
+// us however few there are (and their inversion once), the 128-row block 32
+// us at 1024 and less below.
 int default_mixed_cutoff(int terms, char func, int64_t m) {
   const char* v = std::getenv("NLA_MIXED_CUTOFF");
   if (v && *v) {
     long x = std::atol(v);
     if (x > 0) return (int)(x > 1024 ? 1024 : x);
   }
-  if (terms == EXACT_SLICES && func == 'S') return 64;
+  if (terms == EXACT_SLICES && func == 'S') return m <= 8 * (int64_t)num_sms() ? 128 : 64;
   return m <= 24 * (int64_t)num_sms() ? 128 : 64;
 }
 
@@ -201,47 +204,60 @@ struct LeafInvArgs {
 
 // One CTA per leaf.  The block is read in canonical lower orientation (an
 // upper block with its indices reversed), the inverse formed column by
-// column by right-looking substitution (four threads per column, in one
-// warp, rows split by residue mod 4), and written back in the block's own
-// orientation.
-constexpr int INV_SMEM = (2 * LEAF_INV_N * (LEAF_INV_N + 1) + LEAF_INV_N) * (int)sizeof(double);
+// column by right-looking substitution, and written back in the block's own
+// orientation.  Four threads per column keep it in registers (rows rg + 4 u),
+// so a step is one product, one shuffle and the FMAs of the rows below;
+// warps begin at the first row of their columns.  Bound by the FP64 pipe
+// (about 1800 warp instructions of 16 clocks) and the 64-step chain: with the
+// columns in shared memory it took 53 us.
+constexpr int INV_SMEM = (LEAF_INV_N * (LEAF_INV_N + 1) + LEAF_INV_N) * (int)sizeof(double);
 
 __global__ void __launch_bounds__(256) leaf_inverse_kernel(const __grid_constant__ LeafInvArgs g) {
   extern __shared__ double inv_smem[];
   auto T = reinterpret_cast<double (*)[LEAF_INV_N + 1]>(inv_smem);
-  auto S = reinterpret_cast<double (*)[LEAF_INV_N + 1]>(inv_smem + LEAF_INV_N * (LEAF_INV_N + 1));
-  double* dinv = inv_smem + 2 * LEAF_INV_N * (LEAF_INV_N + 1);
+  double* dinv = inv_smem + LEAF_INV_N * (LEAF_INV_N + 1);
   const int b = blockIdx.x, t = threadIdx.x, n = g.nl[b];
   const double* Ab = g.A + (int64_t)g.k[b] * (g.lda + 1);
-  for (int idx = t; idx < n * n; idx += blockDim.x) {
-    const int i = idx % n, j = idx / n;
+#pragma unroll 4
+  for (int idx = t; idx < LEAF_INV_N * LEAF_INV_N; idx += 256) {
+    const int i = idx % LEAF_INV_N, j = idx / LEAF_INV_N;
     double v = 0.0;
-    if (j <= i) {
+    if (j <= i && i < n) {
       const int ri = g.upper ? n - 1 - i : i, rj = g.upper ? n - 1 - j : j;
       v = g.tA ? Ab[rj + (int64_t)ri * g.lda] : Ab[ri + (int64_t)rj * g.lda];
     }
     T[i][j] = v;
-    S[i][j] = i == j ? 1.0 : 0.0;
   }
   __syncthreads();
-  if (t < n) dinv[t] = g.unit ? 1.0 : 1.0 / T[t][t];
+  if (t < LEAF_INV_N) dinv[t] = g.unit || t >= n ? 1.0 : 1.0 / T[t][t];
   __syncthreads();
-  const int j = t >> 2, rg = t & 3;
-  for (int i = 0; i < n; ++i) {
-    double x = 0.0;
-    if (j < n && i >= j) x = S[i][j] * dinv[i];
-    __syncwarp();
-    if (j < n && i >= j) {
-      if (rg == (i & 3)) S[i][j] = x;
-      for (int r = i + 1 + ((rg - i - 1) & 3); r < n; r += 4) S[r][j] -= T[r][i] * x;
+  const int j = t >> 2, rg = t & 3, base = (t & 31) & ~3;  // the column's four lanes
+  const int j0 = (t >> 5) * 8;                             // the warp's first column
+  double y[LEAF_INV_N / 4];
+#pragma unroll
+  for (int u = 0; u < LEAF_INV_N / 4; ++u) y[u] = rg + 4 * u == j ? 1.0 : 0.0;
+#pragma unroll
+  for (int u = 0; u < LEAF_INV_N / 4; ++u) {
+    if (4 * u + 3 < j0 || 4 * u >= n) continue;  // uniform over the warp: its columns are zero above j0
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int i = 4 * u + q;
+      if (rg == q) y[u] *= dinv[i];
+      const double x = __shfl_sync(0xffffffffu, y[u], base + q);
+      if (rg > q) y[u] -= T[i - q + rg][i] * x;
+#pragma unroll
+      for (int v = u + 1; v < LEAF_INV_N / 4; ++v) y[v] -= T[rg + 4 * v][i] * x;
     }
-    __syncwarp();
   }
-  __syncthreads();
   double* W = g.W + (int64_t)(g.first_slot + b) * LEAF_INV_N * LEAF_INV_N;
+  // Through shared memory, so that the writes run along the columns.
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < LEAF_INV_N / 4; ++u) T[rg + 4 * u][j] = y[u];
+  __syncthreads();
   for (int idx = t; idx < n * n; idx += blockDim.x) {
     const int i = idx % n, jj = idx / n;
-    const double v = jj <= i ? S[i][jj] : 0.0;
+    const double v = jj <= i ? T[i][jj] : 0.0;
     const int ri = g.upper ? n - 1 - i : i, rj = g.upper ? n - 1 - jj : jj;
     W[ri + (int64_t)rj * LEAF_INV_N] = v;
   }
