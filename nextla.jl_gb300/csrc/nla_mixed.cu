@@ -159,17 +159,18 @@ unsigned grid_for(int64_t total) {
 // right-hand sides the short update between two 64-row blocks (staging,
 // product and their launches, about 30 us) costs more than that half, and
 // 128 rows are better.  Measured at 2048 right-hand sides (solve): 128 rows
-// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.  An exact solve
-// of few right-hand sides takes them too: a pair of inverse blocks costs 49
-// us however few there are (and their inversion once), the 128-row block 32
-// us at 1024 and less below.
-int default_mixed_cutoff(int terms, char func, int64_t m) {
+// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.  A small
+// exact solve takes them too: a 128-row block costs about 28 us against 20 for
+// a pair of inverse blocks, but those need their inversion first (25 us once).
+// Measured (n x m, 64 / 128 rows): 200 x 100 96 / 63 us, 512 x 128 182 / 164,
+// 1000 x 300 377 / 467.
+int default_mixed_cutoff(int terms, char func, int64_t n, int64_t m) {
   const char* v = std::getenv("NLA_MIXED_CUTOFF");
   if (v && *v) {
     long x = std::atol(v);
     if (x > 0) return (int)(x > 1024 ? 1024 : x);
   }
-  if (terms == EXACT_SLICES && func == 'S') return m <= 8 * (int64_t)num_sms() ? 128 : 64;
+  if (terms == EXACT_SLICES && func == 'S') return n <= 512 && m <= 2 * (int64_t)num_sms() ? 128 : 64;
   return m <= 24 * (int64_t)num_sms() ? 128 : 64;
 }
 
@@ -696,6 +697,205 @@ __global__ void __launch_bounds__(LP_THREADS, 1) leaf_pair_kernel(const LeafPair
   }
 }
 
+// The same node for few right-hand sides: 32 per CTA instead of 128.  The
+// wide kernel is bound by the integer work of its CTA's 128 columns (split,
+// sums, rounding: about 9 of 16 us per product), so with few of them most
+// SMs idle while 12 CTAs work through 1500 right-hand sides.  Here W's slices
+// are the MMA's M operand and the right-hand sides its N operand (D = W X);
+// W's 64 rows are stored twice, so that all four TMEM lane quarters hold the
+// results and every warp drains four columns.  The products, their scales and
+// roundings are those of the wide kernel: the results are the same bits.
+constexpr int LN_COLS = 32;
+constexpr int LN_W_BYTES = split7::SLICES * 128 * 128;       // 7 slices of 2 x 64 rows
+constexpr int LN_X_BYTES = split7::SLICES * LN_COLS * 128;   // 7 slices of 32 rows
+constexpr int LN_TP = LEAF_INV_N + 1;                        // pitch of the tiles of right-hand sides
+constexpr int LN_TILE = LN_COLS * LN_TP;                     // doubles
+constexpr int LN_SMEM = LN_W_BYTES + LN_X_BYTES + 2 * LN_TILE * 8 + (8 * LN_COLS + 8 * LEAF_INV_N) * 4 + 1024 + 512;
+constexpr int LN_TMEM = 256;                                 // 7 accumulators of 32 columns
+
+template <bool SIDE_R>
+__global__ void __launch_bounds__(LP_THREADS, 1) leaf_pair_narrow_kernel(const LeafPairArgs a) {
+  using namespace split7;
+  chain_begin();
+  extern __shared__ uint8_t lp_smem_raw[];
+  uint8_t* sW = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(lp_smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* sX = sW + LN_W_BYTES;
+  double* tile = reinterpret_cast<double*>(sX + LN_X_BYTES);  // column j of the right-hand sides at tile + j LN_TP
+  double* tile_s = tile + LN_TILE;                            // X_s
+  int* xpart = reinterpret_cast<int*>(tile_s + LN_TILE);      // [8][32]
+  int* wpart = xpart + 8 * LN_COLS;                           // [8][64]
+  __shared__ int ex_s[LN_COLS], ew_s[LEAF_INV_N];
+  __shared__ uint64_t bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int s_abort;
+
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int64_t j0 = (int64_t)blockIdx.x * LN_COLS;
+  const int ncols = (int)min((int64_t)LN_COLS, a.m - j0);
+  auto wat = [&](int i, int k) -> int { return SIDE_R ? k + i * LEAF_INV_N : i + k * LEAF_INV_N; };
+  if (t == 0) {
+    s_abort = 0;
+    umma::mbar_init(umma::smem_u32(&bar), 1);
+    umma::fence_barrier_init();
+  }
+  if (warp == 0) umma::tmem_alloc(umma::smem_u32(&tmem_slot), LN_TMEM);
+
+  // Blocks of right-hand sides to and from the tiles, along the index that is
+  // contiguous in memory.
+  auto fetch = [&](double* dst, const double* X, int nk) {
+#pragma unroll
+    for (int e = 0; e < LN_COLS * LEAF_INV_N / LP_THREADS; ++e) {
+      const int idx = t + LP_THREADS * e;
+      const int j = SIDE_R ? idx & 31 : idx >> 6, k = SIDE_R ? idx >> 5 : idx & 63;
+      const bool in = j < ncols && k < nk;
+      const double* src = in ? X + (SIDE_R ? j0 + j + k * a.ldx : k + (j0 + j) * a.ldx) : X;
+      asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(umma::smem_u32(dst + j * LN_TP + k)), "l"(src),
+                   "r"(in ? 8 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto put = [&](double* X, int nk) {
+#pragma unroll
+    for (int e = 0; e < LN_COLS * LEAF_INV_N / LP_THREADS; ++e) {
+      const int idx = t + LP_THREADS * e;
+      const int j = SIDE_R ? idx & 31 : idx >> 6, k = SIDE_R ? idx >> 5 : idx & 63;
+      if (j < ncols && k < nk) X[SIDE_R ? j0 + j + k * a.ldx : k + (j0 + j) * a.ldx] = tile[j * LN_TP + k];
+    }
+  };
+  fetch(tile, a.Xf, a.nf);
+  fetch(tile_s, a.Xs, a.ns);
+
+  // This thread's 8 values of the W operand (row wi, k = 8 wp ..), of the
+  // right-hand sides (threads below 256: column xj, k = 8 xp ..), and its
+  // results: row ri of columns rc .. rc + 3.
+  const int wi = t & 63, wp = t >> 6, xj = t & 31, xp = t >> 5;
+  const int ri = (warp & 1) * 32 + lane, rc = ((warp >> 2) * 2 + ((warp >> 1) & 1)) * 4;
+  double vw[8];
+#pragma unroll
+  for (int u = 0; u < 8; ++u) {
+    const int k = wp * 8 + u;
+    vw[u] = wi < a.nf && k < a.nf ? a.Wf[wat(wi, k)] : 0.0;
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  umma::fence_before_sync();
+  __syncthreads();
+  umma::fence_after_sync();
+  const uint32_t tmem = tmem_slot;
+
+  // Steps as in leaf_pair_kernel.
+#pragma unroll 1
+  for (int st = 0; st < 3; ++st) {
+    double vx[8];
+    int bw = 0, bx = 0;
+#pragma unroll
+    for (int u = 0; u < 8; ++u) bw = max(bw, exp_field(vw[u]));
+    wpart[wp * LEAF_INV_N + wi] = bw;
+    if (t < 256) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        vx[u] = tile[xj * LN_TP + xp * 8 + u];
+        bx = max(bx, exp_field(vx[u]));
+      }
+      xpart[xp * LN_COLS + xj] = bx;
+    }
+    __syncthreads();
+    if (t < LN_COLS + LEAF_INV_N) {
+      const int* part = t < LN_COLS ? xpart + t : wpart + t - LN_COLS;
+      const int step = t < LN_COLS ? LN_COLS : LEAF_INV_N;
+      int m8 = 0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) m8 = max(m8, part[q * step]);
+      (t < LN_COLS ? ex_s[t] : ew_s[t - LN_COLS]) = scale_exp(m8);
+    }
+    __syncthreads();
+    {
+      long long y[8];
+      const int ew = ew_s[wi];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) y[u] = fixed56(vw[u], ew);
+      store_chunks(sW, 128 * 128, wi, wp, y, wi + 64);
+      if (t < 256) {
+        const int ex = ex_s[xj];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) y[u] = fixed56(vx[u], ex);
+        store_chunks(sX, LN_COLS * 128, xj, xp, y);
+      }
+    }
+    // The tensor cores read shared memory through the async proxy.
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    umma::fence_before_sync();
+    __syncthreads();
+    umma::fence_after_sync();
+    if (t == 0) {
+      // Slice p of W against slices 0 .. 6 - p of the right-hand sides,
+      // stacked in shared memory, into the adjacent accumulators p + q.
+      const uint32_t w0 = umma::smem_u32(sW), x0 = umma::smem_u32(sX);
+#pragma unroll 1
+      for (int p = 0; p < SLICES; ++p) {
+        const uint32_t idesc = umma::idesc_f16(128, LN_COLS * (SLICES - p), true);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma::mma_f16(tmem + (uint32_t)(p * LN_COLS), umma::desc_kmajor_sw128(w0 + p * 128 * 128 + kk * 32),
+                        umma::desc_kmajor_sw128(x0 + kk * 32), idesc, (p > 0 || kk > 0) ? 1u : 0u);
+      }
+      umma::mma_commit(umma::smem_u32(&bar));
+    }
+    // The next product's W operand, in flight during the MMAs.
+    if (st < 2) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int k = wp * 8 + u;
+        if (st == 0) vw[u] = wi < a.ns && k < a.nf ? a.G[wi * a.gsi + k * a.gsk] : 0.0;
+        else vw[u] = wi < a.ns && k < a.ns ? a.Ws[wat(wi, k)] : 0.0;
+      }
+    }
+    __syncwarp();
+    bool ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&bar), (uint32_t)(st & 1), &s_abort, a.err, 45));
+    umma::fence_after_sync();
+    ok = __syncthreads_and(ok ? 1 : 0) != 0;
+    if (!ok) {
+      // Let the MMAs finish (with the default limit) before TMEM is released.
+      if (t == 0) umma::mbar_wait(umma::smem_u32(&bar), (uint32_t)(st & 1), &s_abort, a.err, 46, false);
+      break;
+    }
+    // Sums as in lp_drain, for 4 columns.
+    long long tot[4] = {0, 0, 0, 0};
+    {
+      uint32_t rr[SLICES][4];
+      const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)rc;
+      umma::tmem_ld7x4(ta, (uint32_t)LN_COLS, rr);
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int w = 4; w < SLICES; ++w) tot[c] += (long long)__float2int_rn(__uint_as_float(rr[w][c])) << (48 - 8 * w);
+        tot[c] = (tot[c] + (1ll << 5)) >> 6;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) tot[c] += (long long)__float2int_rn(__uint_as_float(rr[w][c])) << (42 - 8 * w);
+      }
+    }
+    const int nout = st == 0 ? a.nf : a.ns;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      double v = 0.0;
+      if (ri < nout) {
+        v = lp_value(tot[c], ex_s[rc + c], ew_s[ri]);
+        if (st == 1) v = tile_s[(rc + c) * LN_TP + ri] - v;
+      }
+      tile[(rc + c) * LN_TP + ri] = v;
+    }
+    umma::fence_before_sync();
+    __syncthreads();
+    if (st != 1) put(st == 0 ? a.Xf : a.Xs, nout);
+  }
+  umma::fence_before_sync();
+  __syncthreads();
+  if (warp == 0) {
+    umma::fence_after_sync();
+    umma::tmem_dealloc(tmem, LN_TMEM);
+  }
+}
+
 std::mutex g_inv_mu;
 std::unordered_map<uint64_t, Buf> g_inv_bufs;
 
@@ -798,11 +998,11 @@ int leaf_slot(const LeafInverses& L, int64_t k, int64_t* slot) {
 
 // The shared-memory opt-in of one leaf product kernel, once per process
 // (one flag per kernel: the template argument is the kernel itself).
-template <auto Kernel>
+template <auto Kernel, int BYTES = LP_SMEM>
 int allow_smem(const char* name) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
-  std::call_once(once, [] { attr = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LP_SMEM); });
+  std::call_once(once, [] { attr = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, BYTES); });
   return attr == cudaSuccess ? NLA_OK : cuda_status(attr, name);
 }
 
@@ -848,8 +1048,15 @@ int leaf_pair_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   int64_t slot_f = 0, slot_s = 0;
   NLA_TRY(leaf_slot(L, k0 + of, &slot_f));
   NLA_TRY(leaf_slot(L, k0 + os, &slot_s));
-  NLA_TRY(R ? allow_smem<leaf_pair_kernel<true>>("cudaFuncSetAttribute(leaf_pair_kernel)")
-            : allow_smem<leaf_pair_kernel<false>>("cudaFuncSetAttribute(leaf_pair_kernel)"));
+  // 32 right-hand sides per CTA while that is one wave (1500 right-hand
+  // sides: 21 against 49 us); beyond, the wide kernel's tiles are full.
+  const bool narrow = c.m <= (int64_t)LN_COLS * num_sms();
+  if (narrow)
+    NLA_TRY(R ? (allow_smem<leaf_pair_narrow_kernel<true>, LN_SMEM>("cudaFuncSetAttribute(leaf_pair_narrow_kernel)"))
+              : (allow_smem<leaf_pair_narrow_kernel<false>, LN_SMEM>("cudaFuncSetAttribute(leaf_pair_narrow_kernel)")));
+  else
+    NLA_TRY(R ? allow_smem<leaf_pair_kernel<true>>("cudaFuncSetAttribute(leaf_pair_kernel)")
+              : allow_smem<leaf_pair_kernel<false>>("cudaFuncSetAttribute(leaf_pair_kernel)"));
   LeafPairArgs g{};
   g.Wf = L.w + slot_f * LEAF_INV_N * LEAF_INV_N;
   g.Ws = L.w + slot_s * LEAF_INV_N * LEAF_INV_N;
@@ -872,11 +1079,13 @@ int leaf_pair_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   g.nf = (int)nf;
   g.ns = (int)ns;
   g.err = L.err;
-  const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
+  const int64_t per = narrow ? LN_COLS : LP_COLS, grid = (c.m + per - 1) / per;
   if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf pair: too many right-hand sides");
   TraceScope trace(NLA_K_LEAF_SOLVE, c.s, 2.0 * (double)(nf * nf + ns * ns + nf * ns) * (double)c.m,
                    8.0 * (double)(2 * n + ns) * (double)c.m);
-  if (R) launch_chained(leaf_pair_kernel<true>, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
+  if (narrow)
+    launch_chained(R ? leaf_pair_narrow_kernel<true> : leaf_pair_narrow_kernel<false>, (unsigned)grid, LP_THREADS, LN_SMEM, c.s, g);
+  else if (R) launch_chained(leaf_pair_kernel<true>, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
   else launch_chained(leaf_pair_kernel<false>, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
   NLA_CHECK_LAUNCH("leaf_pair_kernel");
   return NLA_OK;
@@ -974,7 +1183,7 @@ int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m
     uplo = uplo == 'L' ? 'U' : 'L';
   }
   *c = RecPlan{func, side, uplo, NLA_F64, m, opts.cutoff > 0 ? (opts.cutoff > 1024 ? 1024 : opts.cutoff)
-                                                             : default_mixed_cutoff(opts.split_terms, func, m),
+                                                             : default_mixed_cutoff(opts.split_terms, func, n, m),
                s, GEMM_MIXED, opts.split_terms, opts.lowp == NLA_LOWP_BF16};
   if (n == 0 || m == 0) return NLA_OK;
   // Size the staging workspace once for the largest update (the top split).

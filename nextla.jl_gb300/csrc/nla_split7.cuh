@@ -51,7 +51,9 @@ __device__ __forceinline__ uint32_t digit_f32(uint32_t w, uint32_t sel) {
 // bytes of y + 0x0080808080808080 minus 128 (the top digit: bits 48 and up),
 // so no carries need propagating; an integer |d| <= 256 is exact in BF16,
 // which is the upper half of its FP32 pattern.
-__device__ __forceinline__ void store_chunks(uint8_t* base, int slice_bytes, int row, int j, const long long (&y)[8]) {
+// With row2 >= 0 the chunks are stored at that row as well.
+__device__ __forceinline__ void store_chunks(uint8_t* base, int slice_bytes, int row, int j, const long long (&y)[8],
+                                             int row2 = -1) {
   uint32_t lo[8], hi[8];
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
@@ -75,6 +77,7 @@ __device__ __forceinline__ void store_chunks(uint8_t* base, int slice_bytes, int
     q.z = __byte_perm(f[4], f[5], 0x7632);
     q.w = __byte_perm(f[6], f[7], 0x7632);
     *reinterpret_cast<uint4*>(base + p * slice_bytes + off) = q;
+    if (row2 >= 0) *reinterpret_cast<uint4*>(base + p * slice_bytes + row2 * 128 + ((j ^ (row2 & 7)) << 4)) = q;
   }
 }
 

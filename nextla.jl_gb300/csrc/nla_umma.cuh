@@ -168,6 +168,25 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t* r) {
       : "memory");
 }
 
+// 7 groups of 4 columns, `pitch` columns apart, with one wait.  The wait
+// takes the registers as operands, so that no use of them moves above it.
+__device__ __forceinline__ void tmem_ld7x4(uint32_t taddr, uint32_t pitch, uint32_t (&r)[7][4]) {
+#pragma unroll
+  for (int w = 0; w < 7; ++w)
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];\n"
+                 : "=r"(r[w][0]), "=r"(r[w][1]), "=r"(r[w][2]), "=r"(r[w][3])
+                 : "r"(taddr + (uint32_t)w * pitch)
+                 : "memory");
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(r[0][0]), "+r"(r[0][1]), "+r"(r[0][2]), "+r"(r[0][3]), "+r"(r[1][0]), "+r"(r[1][1]),
+                 "+r"(r[1][2]), "+r"(r[1][3]), "+r"(r[2][0]), "+r"(r[2][1]), "+r"(r[2][2]), "+r"(r[2][3]),
+                 "+r"(r[3][0]), "+r"(r[3][1]), "+r"(r[3][2]), "+r"(r[3][3]), "+r"(r[4][0]), "+r"(r[4][1]),
+                 "+r"(r[4][2]), "+r"(r[4][3]), "+r"(r[5][0]), "+r"(r[5][1]), "+r"(r[5][2]), "+r"(r[5][3]),
+                 "+r"(r[6][0]), "+r"(r[6][1]), "+r"(r[6][2]), "+r"(r[6][3])
+               :
+               : "memory");
+}
+
 // 32 consecutive 32-bit TMEM columns of this thread's lane, one wait.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t* r) {
   asm volatile(

@@ -183,3 +183,23 @@ def test_leaf_pairs_match_separate_leaves(pkg, oracle, workloads, cuda, monkeypa
         good = out["0"][:, ~touched] if side == "L" else out["0"][~touched, :]
         good1 = out["1"][:, ~touched] if side == "L" else out["1"][~touched, :]
         assert oracle.rel_err(good1, good) < 1e-14, side
+
+
+@pytest.mark.parametrize("side,uplo,trans", [("L", "L", "N"), ("L", "U", "T"), ("R", "U", "N"), ("R", "L", "T")])
+def test_narrow_leaf_pairs_match_wide(pkg, workloads, cuda, side, uplo, trans):
+    """Pairs of leaves on 32 right-hand sides per CTA (up to one wave of them)
+    and on 128 per CTA give the same bits: a solve of few right-hand sides
+    equals the same columns of a wide one.  cutoff=64 keeps the inverse leaves
+    that the library would not choose for so few."""
+    import torch
+
+    n, m = 200, 5000
+    A, B = workloads.problem(n, m, side, uplo, seed=77)
+    Ad = to_dev(A, np.float64, cuda)
+    wide = to_dev(B, np.float64, cuda)
+    pkg.unified_rectrxm_mixed_(side, uplo, trans, 0.5, "S", Ad, wide, split_terms=7, sweeps=0, cutoff=64)
+    for c0, k in ((0, 1), (31, 33), (64, 100), (4000, 1000)):
+        part = to_dev(B[:, c0:c0 + k] if side == "L" else B[c0:c0 + k, :], np.float64, cuda)
+        pkg.unified_rectrxm_mixed_(side, uplo, trans, 0.5, "S", Ad, part, split_terms=7, sweeps=0, cutoff=64)
+        torch.cuda.synchronize()
+        assert torch.equal(part, wide[:, c0:c0 + k] if side == "L" else wide[c0:c0 + k, :]), (c0, k)
