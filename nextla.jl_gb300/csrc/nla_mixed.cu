@@ -441,7 +441,10 @@ __device__ __forceinline__ double lp_value(long long tot, int ex, int ew) {
 }
 
 struct LeafProdArgs {
-  const double* W;  // column-major, leading dimension LEAF_INV_N
+  const double* W;   // W(i, k) at W[i * wsi + k * wsk]
+  int64_t wsi, wsk;
+  int tri;           // W's stored part: 0 all of it, 1 k <= i, 2 k >= i (the rest counts as zero)
+  int unit;          // ones on the diagonal, which is not read
   double* X;
   int64_t ldx;
   int64_t m;
@@ -458,10 +461,8 @@ __global__ void __launch_bounds__(LP_THREADS, 1) leaf_product_kernel(const LeafP
 
   const int t = threadIdx.x, warp = t >> 5, n = a.n;
   const int64_t j0 = (int64_t)blockIdx.x * LP_COLS;
-  // Element (k, j) of the right-hand sides (k < n, j < m) and (i, k) of the
-  // W operand (W itself for side L, W^T for side R).
+  // Element (k, j) of the right-hand sides (k < n, j < m).
   auto xat = [&](int k, int64_t j) -> int64_t { return a.side_r ? j + (int64_t)k * a.ldx : k + j * a.ldx; };
-  auto wat = [&](int i, int k) -> int { return a.side_r ? k + i * LEAF_INV_N : i + k * LEAF_INV_N; };
 
   if (t == 0) {
     s_abort = 0;
@@ -482,7 +483,9 @@ __global__ void __launch_bounds__(LP_THREADS, 1) leaf_product_kernel(const LeafP
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int k = wp * 8 + u;
-    vw[u] = wi < n && k < n ? a.W[wat(wi, k)] : 0.0;
+    const bool diag = a.unit && k == wi;
+    const bool in = wi < n && k < n && !diag && (a.tri == 0 || (a.tri == 1 ? k <= wi : k >= wi));
+    vw[u] = in ? a.W[wi * a.wsi + k * a.wsk] : diag && k < n ? 1.0 : 0.0;
   }
   lp_stage(s, vx, vw);
   const uint32_t tmem = *s.tmem_slot;
@@ -1008,22 +1011,47 @@ int allow_smem(const char* name) {
 
 }  // namespace
 
+static int launch_leaf_product(const RecPlan& c, int64_t n, const Mat& B, const double* W, int64_t wsi, int64_t wsk,
+                               int tri, bool unit, int* err) {
+  NLA_TRY(allow_smem<leaf_product_kernel>("cudaFuncSetAttribute(leaf_product_kernel)"));
+  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "leaf product: transposed B view");
+  const LeafProdArgs g{W, wsi, wsk, tri, unit ? 1 : 0, static_cast<double*>(B.p), B.ld, c.m, (int)n, c.side == 'R' ? 1 : 0, err};
+  const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
+  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf product: too many right-hand sides");
+  TraceScope trace(c.func == 'S' ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, c.s, 2.0 * (double)n * n * (double)c.m,
+                   16.0 * (double)n * (double)c.m);
+  launch_chained(leaf_product_kernel, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
+  NLA_CHECK_LAUNCH("leaf_product_kernel");
+  return NLA_OK;
+}
+
 int leaf_inverse_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   if (n <= 0 || c.m <= 0) return NLA_OK;
   const LeafInverses& L = *c.inv;
   int64_t slot = 0;
   NLA_TRY(leaf_slot(L, (static_cast<const double*>(A.p) - L.a_base) / (L.lda + 1), &slot));
   // X := inv(T) X  (side L)  or  X inv(T)  (side R), one kernel.
-  NLA_TRY(allow_smem<leaf_product_kernel>("cudaFuncSetAttribute(leaf_product_kernel)"));
-  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "leaf product: transposed B view");
-  LeafProdArgs g{L.w + slot * LEAF_INV_N * LEAF_INV_N, static_cast<double*>(B.p), B.ld, c.m, (int)n,
-                 c.side == 'R' ? 1 : 0, L.err};
-  const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
-  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf product: too many right-hand sides");
-  TraceScope trace(NLA_K_LEAF_SOLVE, c.s, 2.0 * (double)n * n * (double)c.m, 16.0 * (double)n * (double)c.m);
-  launch_chained(leaf_product_kernel, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
-  NLA_CHECK_LAUNCH("leaf_product_kernel");
-  return NLA_OK;
+  const bool R = c.side == 'R';  // X inv(T): the operand is inv(T)^T
+  return launch_leaf_product(c, n, B, L.w + slot * LEAF_INV_N * LEAF_INV_N, R ? LEAF_INV_N : 1, R ? 1 : LEAF_INV_N, 0,
+                             0, L.err);
+}
+
+// The multiply's leaf in a mixed recursion, B := T B or B T for a triangle of
+// at most 64 rows: the exact product, rounded once per element.  On the FP64
+// pipe it took 38 us at 6144 right-hand sides.
+bool leaf_product_wanted(const RecPlan& c) {
+  return c.mode == GEMM_MIXED && c.func == 'M' && c.dtype == NLA_F64 && c.threshold <= LEAF_INV_N;
+}
+
+int leaf_product_multiply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
+  if (n <= 0 || c.m <= 0) return NLA_OK;
+  int* err = device_error_word();
+  if (!err) return fail(NLA_ERR_UNSUPPORTED, "leaf product: no device error word");
+  const bool R = c.side == 'R';
+  const int64_t si = A.t ? A.ld : 1, sk = A.t ? 1 : A.ld;  // T(i, k) at i si + k sk
+  const bool lower = (c.uplo == 'L') != R;                 // of the operand: T, or T^T for side R
+  return launch_leaf_product(c, n, B, static_cast<const double*>(A.p), R ? sk : si, R ? si : sk, lower ? 1 : 2, c.unit,
+                             err);
 }
 
 bool leaf_pair_wanted(const RecPlan& c, int64_t n) {

@@ -203,3 +203,25 @@ def test_narrow_leaf_pairs_match_wide(pkg, workloads, cuda, side, uplo, trans):
         pkg.unified_rectrxm_mixed_(side, uplo, trans, 0.5, "S", Ad, part, split_terms=7, sweeps=0, cutoff=64)
         torch.cuda.synchronize()
         assert torch.equal(part, wide[:, c0:c0 + k] if side == "L" else wide[c0:c0 + k, :]), (c0, k)
+
+
+@pytest.mark.parametrize("diag", ["N", "U"])
+def test_mixed_multiply_leaf_products(pkg, oracle, workloads, cuda, diag):
+    """The diagonal blocks of a mixed multiply as exact products (wide
+    right-hand sides; cutoff by the library) against BLAS: exact updates, so
+    only FP64 roundings remain (1e-14), every side, uplo and transpose; the
+    other triangle and a unit diagonal hold NaN and are never used."""
+    import torch
+
+    for (n, m), side, uplo, trans in itertools.product([(50, 4000), (200, 3700)], "LR", "LU", "NT"):
+        A, B = workloads.problem(n, m, side, uplo, seed=n)
+        An = A.copy()
+        An[np.triu_indices(n, 1) if uplo == "L" else np.tril_indices(n, -1)] = np.nan
+        if diag == "U":
+            An[np.diag_indices(n)] = np.nan
+            A[np.diag_indices(n)] = 1.0
+        Bd = to_dev(B, np.float64, cuda)
+        pkg.trmm(side, uplo, trans, diag, to_dev(An, np.float64, cuda), Bd, -0.5, mixed=True)
+        torch.cuda.synchronize()
+        ref = oracle.blas_rectrxm(side, uplo, trans, -0.5, "M", A, B)
+        assert oracle.rel_err(to_host(Bd), ref) < 1e-14, (n, side, uplo, trans, diag)
