@@ -80,19 +80,19 @@ int launch_leaf_cols2(const LeafArgs& g, cudaStream_t s) {
   }
 }
 
-template <typename T, int PB, int NC, int WC, bool SOLVE>
-__global__ void __launch_bounds__(ST_THREADS) leaf_strip_kernel(const LeafArgs g) {
+template <typename T, int PB, int NC, int WC, bool SOLVE, int NW = 8>
+__global__ void __launch_bounds__(32 * NW) leaf_strip_kernel(const LeafArgs g) {
   chain_begin();
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  strip_block<T, PB, NC, WC, SOLVE>(g, smem_raw);
+  strip_block<T, PB, NC, WC, NW, SOLVE>(g, smem_raw);
 }
 
 constexpr size_t STRIP_SMEM_MAX = 200 * 1024;
 
-template <typename T, int PB, int NC, int WC, bool SOLVE>
+template <typename T, int PB, int NC, int WC, bool SOLVE, int NW = 8>
 int launch_strip(const LeafArgs& g, cudaStream_t s) {
   using Tc = typename Elem<T>::compute;
-  const size_t smem = strip_smem_elems<Tc>(g.n, PB, NC, WC) * sizeof(Tc);
+  const size_t smem = strip_smem_elems<Tc>(g.n, PB, NC, WC, NW) * sizeof(Tc);
   constexpr int CW = 32 / PB * NC * WC;
   const int64_t grid = (g.m + CW - 1) / CW;
   if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf: too many right-hand sides");
@@ -100,7 +100,7 @@ int launch_strip(const LeafArgs& g, cudaStream_t s) {
   static std::once_flag once;
   static cudaError_t st = cudaSuccess;
   std::call_once(once, [] {
-    st = cudaFuncSetAttribute(leaf_strip_kernel<T, PB, NC, WC, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    st = cudaFuncSetAttribute(leaf_strip_kernel<T, PB, NC, WC, SOLVE, NW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)STRIP_SMEM_MAX);
   });
   if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(leaf_strip_kernel)");
@@ -108,7 +108,7 @@ int launch_strip(const LeafArgs& g, cudaStream_t s) {
   // the triangle once plus B read and written.
   TraceScope trace(SOLVE ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, s, (double)g.n * g.n * (double)g.m,
                    (double)sizeof(T) * ((double)g.n * (g.n + 1) / 2 + 2.0 * (double)g.n * g.m));
-  leaf_strip_kernel<T, PB, NC, WC, SOLVE><<<(unsigned)grid, ST_THREADS, smem, s>>>(g);
+  leaf_strip_kernel<T, PB, NC, WC, SOLVE, NW><<<(unsigned)grid, 32 * NW, smem, s>>>(g);
   NLA_CHECK_LAUNCH("leaf_strip_kernel");
   return NLA_OK;
 }
@@ -121,7 +121,7 @@ int launch_strip(const LeafArgs& g, cudaStream_t s) {
 // DFMA pipe more than the steps they save), Float32 always 32-row panels.
 // Measured against one warp-group CTA per 16 or 32 columns with 32-row
 // panels solved by one warp: Float64 96 x 24 97 -> 13 us, 256 x 256 560 ->
-// 42 us; Float32 256 x 8192 110 -> 47 us; Float16 256 x 4096 98 -> 41 us;
+// 42 us; Float32 256 x 8192 110 -> 44 us; Float16 256 x 4096 98 -> 32 us;
 // Float64 multiply 64 x 6144 115 -> 36 us.
 template <typename T, bool SOLVE>
 int launch_strips(const LeafArgs& g, cudaStream_t s) {
@@ -130,20 +130,27 @@ int launch_strips(const LeafArgs& g, cudaStream_t s) {
   constexpr bool F64 = sizeof(Tc) == (CX ? 16 : 8);
   constexpr int WIDEST = F64 ? (CX ? 16 : 32) : (CX ? 32 : 64);
   const int64_t sms = num_sms(), c = F64 ? 1 : CX ? 8 : 32;
+  // Warps on 32 and 64 columns.  Float32 products wait for shared memory with
+  // two warps per scheduler; a second K group gives it four (and costs one
+  // sum through shared memory per panel): solve 256 x 8192 47.9 -> 44.4 us,
+  // multiply 128 x 8192 16.3 -> 14.3 us, 64 x 6144 8.4 -> 7.3 us.  On 8 and
+  // 16 columns, where the triangles' chains bound, it gave nothing (25.2 us
+  // at 256 x 1000 either way).
+  constexpr int NWW = CX || F64 ? 8 : 16;
   int best = 0;
   int64_t cost = 0;
   for (int w : {64, 32, 16, 8, 4, 2}) {
     if (w > WIDEST) continue;
-    if (strip_smem_elems<Tc>(g.n, 32, w < 8 ? 1 : w / 8, w < 8 ? w : 8) * sizeof(Tc) > STRIP_SMEM_MAX && w > 2) continue;
+    if (strip_smem_elems<Tc>(g.n, 32, w < 8 ? 1 : w / 8, w < 8 ? w : 8, w < 32 ? 8 : NWW) * sizeof(Tc) > STRIP_SMEM_MAX && w > 2) continue;
     const int64_t grid = (g.m + w - 1) / w, k = (grid + sms - 1) / sms * (w + c);
     if (best == 0 || k < cost) best = w, cost = k;
   }
   switch (best) {
     case 64:
-      if constexpr (WIDEST >= 64) return launch_strip<T, 32, 8, 8, SOLVE>(g, s);
+      if constexpr (WIDEST >= 64) return launch_strip<T, 32, 8, 8, SOLVE, NWW>(g, s);
     case 32:
       if constexpr (WIDEST >= 32)
-        return F64 ? launch_strip<T, 16, 2, 8, SOLVE>(g, s) : launch_strip<T, 32, 4, 8, SOLVE>(g, s);
+        return F64 ? launch_strip<T, 16, 2, 8, SOLVE>(g, s) : launch_strip<T, 32, 4, 8, SOLVE, NWW>(g, s);
     case 16: return F64 ? launch_strip<T, 16, 1, 8, SOLVE>(g, s) : launch_strip<T, 32, 2, 8, SOLVE>(g, s);
     case 8: return F64 ? launch_strip<T, 16, 1, 4, SOLVE>(g, s) : launch_strip<T, 32, 1, 8, SOLVE>(g, s);
     case 4: return launch_strip<T, 32, 1, 4, SOLVE>(g, s);

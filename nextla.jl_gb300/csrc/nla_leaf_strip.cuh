@@ -1,5 +1,5 @@
 // Diagonal-block solve / multiply on strips of right-hand sides: one CTA of
-// eight warps takes CW right-hand sides through the whole n x n block
+// NW (8 or 16) warps takes CW right-hand sides through the whole n x n block
 // (canonical lower-left form, nla_leaf.cuh).
 //
 // What bounds it.  Float64: the DFMA pipe (2 per clock per SM, one warp
@@ -35,7 +35,6 @@
 namespace nla {
 namespace leafdev {
 
-constexpr int ST_THREADS = 256;
 constexpr int ST_ROWS = 32;  // the strip's rows are padded to a multiple of this
 
 template <typename Tc> struct StripTraits;
@@ -109,24 +108,26 @@ template <typename Tc> __host__ __device__ constexpr int st_ldx(int n) {
 }
 template <typename Tc> __host__ __device__ constexpr int st_lda() { return ST_KC + StripTraits<Tc>::VK; }
 
-// PB rows per panel, WC warps across the columns with 32 / PB NC columns each.
-template <typename Tc> __host__ __device__ constexpr size_t strip_smem_elems(int n, int PB, int NC, int WC) {
+// PB rows per panel, NW warps, WC of them across the columns with 32 / PB NC
+// columns each.
+template <typename Tc> __host__ __device__ constexpr size_t strip_smem_elems(int n, int PB, int NC, int WC, int NW) {
   return (size_t)(32 / PB) * NC * WC * st_ldx<Tc>(n)              // X
          + (size_t)2 * PB * st_lda<Tc>()                          // A chunks
          + (size_t)2 * PB * (PB + 1)                              // panel triangles
          + (size_t)2 * ((n + ST_ROWS - 1) / ST_ROWS * ST_ROWS)    // the diagonal and its reciprocals
-         + (WC < 8 ? (size_t)8 * NC * 32 : 0);                    // partial sums of the K groups
+         + (WC < NW ? (size_t)NW * NC * 32 : 0);                  // partial sums of the K groups
 }
 
-// CW = (32 / PB) NC WC columns per CTA: WC warps across them, KG = 8 / WC across K.
-template <typename T, int PB, int NC, int WC, bool SOLVE>
+// CW = (32 / PB) NC WC columns per CTA: WC warps across them, KG = NW / WC across K.
+template <typename T, int PB, int NC, int WC, int NW, bool SOLVE>
 __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* smem_raw) {
   using Tc = typename Elem<T>::compute;
   using Tr = StripTraits<Tc>;
   using Vec = typename Tr::Vec;
   using Mx = StripMath<Tc>;
-  constexpr int KC = ST_KC, VK = Tr::VK, KG = 8 / WC, SUBS = 32 / PB, CW = SUBS * NC * WC;
-  constexpr int DPER = PB * PB / ST_THREADS;    // triangle elements per thread
+  constexpr int ST_THREADS = 32 * NW;
+  constexpr int KC = ST_KC, VK = Tr::VK, KG = NW / WC, SUBS = 32 / PB, CW = SUBS * NC * WC;
+  constexpr int DPER = (PB * PB + ST_THREADS - 1) / ST_THREADS;  // triangle elements per thread
   constexpr int LDA = st_lda<Tc>();
   constexpr int PER = PB * KC / ST_THREADS;  // chunk elements per thread
   const int n = g.n, ldx = st_ldx<Tc>(n), nr = (n + ST_ROWS - 1) / ST_ROWS * ST_ROWS;
@@ -135,7 +136,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   Tc* Dg = As + 2 * PB * LDA;                    // 2 x PB x (PB + 1)
   Tc* inv = Dg + 2 * PB * (PB + 1);           // nr
   Tc* dia = inv + nr;                               // nr
-  Tc* part = dia + nr;                              // KG > 1: 8 warps x NC x 32
+  Tc* part = dia + nr;                              // KG > 1: NW warps x NC x 32
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int row = lane & (PB - 1), sub = lane / PB;
   const int wc = warp % WC, kg = warp / WC;
@@ -182,11 +183,11 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 
   fetch(0, 0, kend_of(0), SOLVE && chunks_of(0) == 1);
   // The strip of B, several loads in flight per thread; zeros past the block.
-  // Along the rows a warp takes columns warp, warp + 8, ...; along the
+  // Along the rows a warp takes columns warp, warp + NW, ...; along the
   // columns consecutive threads take consecutive columns.
   constexpr int BATCH = 8;
   if (!g.tB) {
-    for (int c = warp; c < CW; c += 8)
+    for (int c = warp; c < CW; c += NW)
       for (int i0 = lane; i0 < nr; i0 += 32 * BATCH) {
         T v[BATCH];
 #pragma unroll
@@ -323,7 +324,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
   if (SOLVE) {
     __syncthreads();
     if (!g.tB) {
-      for (int c = warp; c < ncols; c += 8)
+      for (int c = warp; c < ncols; c += NW)
         for (int i = lane; i < n; i += 32) Elem<T>::store(B + i * bi + c * bc, X[(size_t)c * ldx + i]);
     } else if (t % CW < ncols) {
       for (int i = t / CW; i < n; i += ST_THREADS / CW)

@@ -38,3 +38,24 @@ def test_strip_edges(pkg, oracle, workloads, cuda, dtype, func):
         torch.cuda.synchronize()
         ref = oracle.blas_rectrxm(side, uplo, "N", 1.0, func, A.astype(np.float64), B.astype(np.float64))
         assert oracle.rel_err(to_host(Bd), ref) < TOL[dtype], (n, m, side, uplo, ta)
+
+
+# Strips of 32 and 64 columns (16 warps in Float32 and Float16), whole and
+# with a remainder, both orientations of B and of A; same tolerances.
+@pytest.mark.parametrize("dtype", [np.float32, np.float16])
+@pytest.mark.parametrize("n,m", [(33, 2500), (256, 2433), (130, 5001), (257, 9728)])
+@pytest.mark.parametrize("func", ["S", "M"])
+def test_strip_wide(pkg, oracle, workloads, cuda, dtype, func, n, m):
+    import torch
+
+    rt = pkg.rectrxm
+    for side, uplo, ta in [("L", "L", False), ("L", "U", True), ("R", "L", True), ("R", "U", False)]:
+        A, B = workloads.problem(n, m, side, uplo, seed=n + m)
+        A, B = A.astype(dtype), B.astype(dtype)
+        stored = A.T if ta else A
+        Ad = to_dev(stored, dtype, cuda, ld=n + 3)
+        Bd = to_dev(B, dtype, cuda, ld=B.shape[0] + 1)
+        rt._diag_block(func, side, uplo, Ad.T if ta else Ad, Bd)
+        torch.cuda.synchronize()
+        ref = oracle.blas_rectrxm(side, uplo, "N", 1.0, func, A.astype(np.float64), B.astype(np.float64))
+        assert oracle.rel_err(to_host(Bd), ref) < TOL[dtype], (side, uplo, ta)
