@@ -58,7 +58,7 @@ struct GemmParams {
   int M, N;
   int num_kb;
   int tiles_m, tiles_n;
-  int a_rows, b_rows;  // padded rows of the operands (multiples of 128)
+  int bn;              // columns of C per tile: 128, 64 or 32
   int sa, sb;          // slices of A and B loaded per stage
   int stages;
   int stage_bytes;
@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
   const int local = blockIdx.x % per_group;
   const int tm = first_m + local % gsize;
   const int tn = local / gsize;
-  const int m0 = tm * BM, n0 = tn * BN;
+  const int m0 = tm * BM, n0 = tn * p.bn;
+  const int b_bytes = p.bn * BK * 2;  // one slice tile of B
 
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -155,13 +156,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         if (!umma::mbar_wait(umma::smem_u32(&empty[s]), (round & 1u) ^ 1u, &s_abort, &g_device_error, 1)) break;
         const uint32_t fb = umma::smem_u32(&own[s]);
         uint8_t* st = smem + (size_t)s * p.stage_bytes;
-        umma::mbar_arrive_expect_tx(fb, (uint32_t)(((both ? p.sa + p.sb : is_a ? p.sa : p.sb)) * TILE_BYTES));
+        umma::mbar_arrive_expect_tx(fb, (uint32_t)((is_a ? p.sa * TILE_BYTES : 0) + (!is_a || both ? p.sb * b_bytes : 0)));
         if (is_a)
           for (int sl = 0; sl < p.sa; ++sl)
             umma::tma_load_2d(umma::smem_u32(st + sl * TILE_BYTES), &tmA, fb, kb * BK, m0 * p.sa + sl * BM);
         if (!is_a || both)
           for (int sl = 0; sl < p.sb; ++sl)
-            umma::tma_load_2d(umma::smem_u32(st + (p.sa + sl) * TILE_BYTES), &tmB, fb, kb * BK, n0 * p.sb + sl * BN);
+            umma::tma_load_2d(umma::smem_u32(st + p.sa * TILE_BYTES + sl * b_bytes), &tmB, fb, kb * BK,
+                              (n0 / BN * p.sb + sl) * BN + n0 % BN);
       }
       umma::producer_quiesce(own, p.stages, kb, &s_abort, &g_device_error, 5);
     }
@@ -180,8 +182,8 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const uint32_t st = umma::smem_u32(smem + (size_t)s * p.stage_bytes);
         for (int pr = 0; pr < p.npairs; ++pr) {
           const uint32_t a0 = st + p.pair_a[pr] * TILE_BYTES;
-          const uint32_t b0 = st + (p.sa + p.pair_b[pr]) * TILE_BYTES;
-          const uint32_t d = tmem + (uint32_t)(p.pair_acc[pr] * BN);
+          const uint32_t b0 = st + p.sa * TILE_BYTES + p.pair_b[pr] * b_bytes;
+          const uint32_t d = tmem + (uint32_t)(p.pair_acc[pr] * p.bn);
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk) {
             const uint32_t acc = (kb > 0 || kk > 0 || !p.pair_first[pr]) ? 1u : 0u;
@@ -197,7 +199,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
       umma::mbar_wait(umma::smem_u32(drain), 0, &s_abort, &g_device_error, 3, false);
     }
   } else {
-    // Epilogue warps 2..9: TMEM lane quadrant warp % 4, 64 of the tile's 128
+    // Epilogue warps 2..9: TMEM lane quadrant warp % 4, half of the tile's
     // columns each.  The kernel's time at short K is the latency of this C
     // update: a store to C may alias a later load as far as the compiler
     // knows, so element-wise updates wait for memory once per column.  Here
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     const int q = warp & 3;
     const int row = q * 32 + lane;
     const int i = m0 + row;
-    const int cbase = ((warp - 2) >> 2) * (BN / 2);
+    const int cbase = ((warp - 2) >> 2) * (p.bn / 2);
     using TC = typename std::conditional<EPI == EPI_F64, double, __half>::type;
     TC* C = static_cast<TC*>(p.C) + i;
     TC cv[EPI_COLS], nv[EPI_COLS];  // the batch in hand and the next one
@@ -235,19 +237,19 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
     if (ok) {
       const uint32_t tq = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)cbase;
 #pragma unroll 1
-      for (int c0 = 0; c0 < BN / 2; c0 += EPI_COLS) {
+      for (int c0 = 0; c0 < p.bn / 2; c0 += EPI_COLS) {
         float v[EPI_COLS];
         uint32_t r[EPI_COLS];
         umma::tmem_ld16(tq + (uint32_t)c0, r);
 #pragma unroll
         for (int j = 0; j < EPI_COLS; ++j) v[j] = __uint_as_float(r[j]);
         for (int a = 1; a < p.nacc; ++a) {
-          umma::tmem_ld16(tq + (uint32_t)(a * BN + c0), r);
+          umma::tmem_ld16(tq + (uint32_t)(a * p.bn + c0), r);
           const float w = p.acc_w[a];
 #pragma unroll
           for (int j = 0; j < EPI_COLS; ++j) v[j] = fmaf(__uint_as_float(r[j]), w, v[j]);
         }
-        if (c0 + EPI_COLS < BN / 2) fetch(c0 + EPI_COLS, nv, ne);
+        if (c0 + EPI_COLS < p.bn / 2) fetch(c0 + EPI_COLS, nv, ne);
         if (i < p.M) {
 #pragma unroll
           for (int j = 0; j < EPI_COLS; ++j) {
@@ -1339,14 +1341,14 @@ int make_map(CUtensorMap* map, const void* base, bool bf16, uint64_t cols_pad, u
 // zeros past K and past the rows).  Such an operand needs no staging: X of a
 // left-side solve is staged again at every level otherwise (0.66 of 3.3 ms
 // for 8192 x 4096).
-int direct_map(CUtensorMap* map, const Mat& X, int64_t rows, int64_t K, bool* ok) {
+int direct_map(CUtensorMap* map, const Mat& X, int64_t rows, int64_t K, int box_rows, bool* ok) {
   *ok = X.t && (reinterpret_cast<uintptr_t>(X.p) & 15) == 0 && X.ld % 8 == 0 && X.ld * 2 < (1ll << 40);
   if (!*ok) return NLA_OK;
   auto fn = encode_fn();
   if (!fn) return fail(NLA_ERR_UNSUPPORTED, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t dims[2] = {(cuuint64_t)K, (cuuint64_t)rows};
   cuuint64_t strides[1] = {(cuuint64_t)X.ld * 2};
-  cuuint32_t box[2] = {BK, BM}, estr[2] = {1, 1};
+  cuuint32_t box[2] = {BK, (cuuint32_t)box_rows}, estr[2] = {1, 1};
   const CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, X.p, dims, strides, box, estr,
                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1377,6 +1379,21 @@ int gemm_producers() {
     return v && v[0] == '1' && v[1] == 0 ? 1 : 2;
   }();
   return n;
+}
+
+// Columns of C per tile.  At short K a tile's time is its C update (about
+// 4 FP64-rate operations per element and their loads, per SM), so while all
+// tiles fit one wave, half the columns on twice the SMs is faster: the 93
+// updates of a refined solve of 4096 x 2048 (16 to 128 tiles of 128 columns)
+// 3.21 -> 2.42 ms, the 95 of a multiply of 6144 x 6144 3.41 -> 2.85 ms,
+// Float16 8192 x 4096 2241 -> 2197 us per solve.  Beyond one wave the wider
+// tile reads its operands fewer times; a rule by waves times (width + 48)
+// instead was no better (multiply 6294 against 6266 us in all).
+int gemm_tile_cols(int64_t M, int64_t N) {
+  const int64_t tm = (M + BM - 1) / BM, sms = num_sms();
+  int bn = BN;
+  while (bn > 32 && tm * ((N + bn / 2 - 1) / (bn / 2)) <= sms) bn /= 2;
+  return bn;
 }
 
 template <int EPI>
@@ -1741,12 +1758,13 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
   } else if (ws_bytes < need) {
     return fail(NLA_ERR_WORKSPACE, "workspace too small for the tensor-core update");
   }
+  const int bn = gemm_tile_cols(M, N);
   Staged As, Bs;
   CUtensorMap mA, mB;
   bool directA = false, directB = false;  // Float16 operands that TMA can read where they are
   if (copy) {
-    NLA_TRY(direct_map(&mA, A, M, K, &directA));
-    NLA_TRY(direct_map(&mB, transposed(B), N, K, &directB));
+    NLA_TRY(direct_map(&mA, A, M, K, BM, &directA));
+    NLA_TRY(direct_map(&mB, transposed(B), N, K, bn, &directB));
   }
   // N x K view: row j is column j of op(B)
   if (!copy && K <= FUSED_STAGE_MAX_K && stage_fused_enabled()) {
@@ -1761,20 +1779,19 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
 
   const bool use_bf16 = copy ? false : As.bf16;
   if (!directA) NLA_TRY(make_map(&mA, As.slices, use_bf16, (uint64_t)Kp, (uint64_t)(S * Mp)));
-  if (!directB) NLA_TRY(make_map(&mB, Bs.slices, use_bf16, (uint64_t)Kp, (uint64_t)(S * Np)));
+  if (!directB) NLA_TRY(make_map(&mB, Bs.slices, use_bf16, (uint64_t)Kp, (uint64_t)(S * Np), (uint32_t)bn));
 
   GemmParams p{};
   p.M = (int)M;
   p.N = (int)N;
   p.num_kb = (int)(Kp / BK);
   p.tiles_m = (int)(Mp / BM);
-  p.tiles_n = (int)(Np / BN);
-  p.a_rows = (int)Mp;
-  p.b_rows = (int)Np;
+  p.tiles_n = (int)((N + bn - 1) / bn);
+  p.bn = bn;
   p.sa = S;
   p.sb = S;
   p.producers = gemm_producers();
-  p.stage_bytes = 2 * S * TILE_BYTES;
+  p.stage_bytes = S * (TILE_BYTES + bn * BK * 2);
   p.stages = (GEMM_DYN_SMEM - 1024 - 256) / p.stage_bytes;
   if (p.stages > 6) p.stages = 6;
   // Slice pairs (a, b) with a + b <= S - 1 (0-based), grouped by weight.
@@ -1792,9 +1809,9 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
     }
   }
   uint32_t cols = 32;
-  while (cols < (uint32_t)(p.nacc * BN)) cols <<= 1;
+  while (cols < (uint32_t)(p.nacc * bn)) cols <<= 1;
   p.tmem_cols = cols;
-  p.idesc = umma::idesc_f16(BM, BN, use_bf16);
+  p.idesc = umma::idesc_f16(BM, bn, use_bf16);
   p.C = C.p;
   p.ldc = C.ld;
   p.alpha = alpha;

@@ -262,3 +262,46 @@ def test_f16_operands_read_in_place(pkg, oracle, cuda, pad, off):
         ref = C.astype(np.float64) - A.astype(np.float64) @ B.astype(np.float64)
         got = Cd.cpu().numpy().astype(np.float64)
         assert (np.abs(got - ref) <= 2.0 ** -11 * np.abs(ref) * 1.01 + K * 2.0 ** -23).all(), (N, K, M)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (100, 33), (128, 31), (129, 2400), (128, 4097), (128, 4865), (200, 4900),
+                                   (300, 6500)])
+@pytest.mark.parametrize("terms", [2, 3])
+def test_update_tile_widths(pkg, cuda, shape, terms):
+    """Tiles of 32, 64 and 128 columns (chosen by how many fill the GPU), with
+    remainders in every dimension.  Products and sums of these integers are
+    exact in Float32 (300 * 60^2 < 2^24), so the result must be bit-exact, and
+    the rows and columns around the view of C stay as they were."""
+    import torch
+
+    g = torch.Generator(device=cuda).manual_seed(shape[0] + shape[1])
+    N, M = shape
+    for R, t2 in ((64, False), (70, True), (300, False)):
+        A = _col_major(torch.randint(-60, 61, (N, R), device=cuda, generator=g).double())
+        B = torch.randint(-60, 61, (R, M), device=cuda, generator=g).double()
+        opB = B if t2 else _col_major(B)
+        parent = _col_major(torch.full((N + 5, M + 3), 7.0, device=cuda, dtype=torch.float64))
+        C = parent[2:N + 2, 1:M + 1]
+        ref = 7.0 - A @ B
+        pkg.matmul_mixed_(C, A, opB, -1.0, lowp="bf16", split_terms=terms)
+        pkg.device_status(C)
+        assert torch.equal(C, ref), (shape, terms, R, t2)
+        C.fill_(7.0)
+        assert bool((parent == 7.0).all()), (shape, terms, R, t2)
+
+
+@pytest.mark.parametrize("shape", [(100, 33), (129, 2400), (128, 4865), (200, 4900)])
+def test_f16_update_tile_widths(pkg, cuda, shape):
+    """The same widths in Float16: integer results below 2048 are exact."""
+    import torch
+
+    g = torch.Generator(device=cuda).manual_seed(shape[0])
+    N, M = shape
+    for R, t1, t2 in ((64, False, False), (72, True, False), (130, True, True)):
+        A = torch.randint(-3, 4, (N, R), device=cuda, generator=g).half()
+        B = torch.randint(-3, 4, (R, M), device=cuda, generator=g).half()
+        C = _col_major(torch.ones(N, M, device=cuda).half())
+        ref = (1.0 - A.double() @ B.double()).half()
+        pkg.GEMM_SUB_(C, A if t1 else _col_major(A), B if t2 else _col_major(B))
+        pkg.device_status(C)
+        assert torch.equal(C, ref), (shape, R, t1, t2)
