@@ -13,10 +13,11 @@ n^2 m flop count of a triangular solve.
 Variants:
   plain   the dtype-preserving Float64 path (DFMA GEMM updates, FP64 leaves).
   mixed   the mixed-precision form (default): every GEMM update on the BF16
-          tensor cores.  With --terms 7 (default) each FP64 operand is split
-          into 7 BF16 slices and the 28 significant slice pairs accumulate
-          exactly (FP32 chunks drained into int64), so the updates are as
-          accurate as FP64 and no refinement sweep is needed (--sweeps 0).
+          tensor cores.  With --terms 7 (default) the updates are exact
+          products of the operands rounded to 56 bits, formed modulo 16
+          coprime moduli (one BF16 product each, FP32 sums that are exact
+          integers), so they are as accurate as FP64 and no refinement sweep
+          is needed (--sweeps 0).
           --terms 1-3 with --sweeps >= 1 is the cheaper split plus
           FP64-residual iterative refinement.
 
@@ -170,7 +171,7 @@ PLAIN_STEPS = 3  # timed solves of the plain FP64 comparison
 E2E_STEPS = 15   # synchronised end-to-end steps (host buffers to host result)
 
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per launch of the
-# exact tensor-core kernel, averaged over the 127 updates of one default
+# residue product kernel, averaged over the 127 updates of one default
 # solve at n = m = 16384 (the 128 updates between sibling leaves run inside
 # the leaf pair kernel).  ncu cannot run inside the timed bench, so this is
 # the figure of one ncu capture of the same workload, with the commit and
@@ -753,13 +754,12 @@ def run_config3(args):
 def run_kernel_case(args):
     """Single launches of one kernel on an s x s case (s = --case-size),
     sized so that operands exceed L2 but the device holds a few GB at most:
-      exact  one exact slice-product update, C (s x s) -= A (s x s) B (s x s),
-             7 BF16 slices per operand (--case-shape M,N,K for C (M x N) -=
-             A (M x K) B (K x N));
-      fast   the same with 3 BF16 slices (FP32 accumulation);
+      exact  one exact update, C (s x s) -= A (s x s) B (s x s), on the tensor
+             cores (--case-shape M,N,K for C (M x N) -= A (M x K) B (K x N));
+      fast   the same from 3 BF16 slices per operand (FP32 accumulation);
       leaf   one FP64 diagonal-block solve of order 128 with 8 s right-hand
              sides (--case-shape n,m for order n with m right-hand sides);
-      pair   one exact mixed solve (L/L/N, 7 BF16 slices, 0 sweeps) of order
+      pair   one exact mixed solve (L/L/N, 7 terms, 0 sweeps) of order
              s with 4 s right-hand sides, whose 128-row nodes each run one
              leaf_pair_kernel launch (s / 128 per solve);
       dfma   one FP64 update on CUDA cores, s x s x s."""
@@ -1038,12 +1038,13 @@ def main():
         name, (launches, kms, kflops, kbytes) = dom
         achieved = kflops / (kms / 1e3) / 1e12
         share = kms / sum(v[1] for v in trace.values())
-        # The committed DRAM capture covers the exact 7-slice updates of the
+        # The committed DRAM capture covers the exact updates of the
         # 16384 x 16384 solve only.
         exact_headline = (args.variant == "mixed" and args.terms == 7 and args.n == 16384 and args.m == 16384)
         if name == "gemm_umma":
             peak = float(pk.get("bf16_tflops_sustained", pk.get("bf16_tflops")))
-            roofline = {"kernel": "umma_gemm/umma_exact (tcgen05 BF16 slice products)", "bound": "tensor",
+            roofline = {"kernel": ("crt_gemm + crt_finish (tcgen05 BF16 products of residues)" if args.terms == 7
+                                   else "umma_gemm (tcgen05 BF16/FP16 slice products)"), "bound": "tensor",
                         "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                         "traffic": TRAFFIC_BYTES_PER_LAUNCH if exact_headline else None,
                         "traffic_source": TRAFFIC_SOURCE if exact_headline else None,
