@@ -176,10 +176,10 @@ E2E_STEPS = 15   # synchronised end-to-end steps (host buffers to host result)
 # the leaf pair kernel).  ncu cannot run inside the timed bench, so this is
 # the figure of one ncu capture of the same workload, with the commit and
 # command it was taken on (TRAFFIC_SOURCE).
-TRAFFIC_BYTES_PER_LAUNCH = 421.6e6
-TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:umma_exact "
+TRAFFIC_BYTES_PER_LAUNCH = 659.4e6
+TRAFFIC_SOURCE = ("ncu --metrics dram__bytes_read.sum,dram__bytes_write.sum --clock-control none -k regex:crt_gemm "
                   "-s 127 -c 127 python bench.py --steps 1 --warmup 1 --no-plain --no-cpu-baseline (the timed "
-                  "solve's 127 updates), at commit 125abf4")
+                  "solve's 127 updates), at commit 400fc1e")
 
 
 def make_inputs(n, m, seed=0):

@@ -187,7 +187,7 @@ NLA_API int nla_host_free(void* p);
                                 the FP64 pipe, rounded once (for measuring errors) */
 typedef struct {
   int lowp;          /* NLA_LOWP_BF16 or NLA_LOWP_F16 */
-  int split_terms;   /* 1, 2 or 3 slices per operand; 7 = exact BF16 slice products (FP64-accurate updates) */
+  int split_terms;   /* 1, 2 or 3 slices per operand; 7 = exact BF16 products (FP64-accurate updates) */
   int sweeps;        /* refinement sweeps for solves, 0..8 */
   int residual;      /* how the residual product is formed */
   int64_t cutoff;    /* FP64 diagonal block size; <= 0 selects the default */

@@ -10,7 +10,8 @@
 // arithmetic on the FP64 bit pattern, so it issues no FP64 instruction.
 // A Float16 operand of the plain Float16 path is staged as one unscaled slice.
 //
-// The GEMM kernel (one 128 x 128 output tile per CTA, 11 warps):
+// The GEMM kernel (one output tile of 128 rows and 128, 64 or 32 columns per
+// CTA, 11 warps):
 //   warp 0      TMA producer: per 64-wide K block, one 128 x 64 box per slice
 //               of each operand (128-byte swizzle) into a multi-stage ring;
 //   warp 1      allocates TMEM, and one elected lane issues tcgen05.mma for

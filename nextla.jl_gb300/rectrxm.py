@@ -320,7 +320,7 @@ def trsm(side, uplo, transa, diag, A, B, alpha=1.0, *, mixed=False):
     ignoring transa and diag (so it is limited to n <= 1024 and op(A) = A);
     here the call runs the whole recursion (nla_trxm_diag), honours transa
     and applies diag 'U' (unit diagonal, never read).  With ``mixed=True``
-    (Float64 only) the updates run on the tensor cores with exact 7-slice
+    (Float64 only) the updates run on the tensor cores with exact
     products (nla_trxm_mixed_diag)."""
     return _trxm_diag("S", side, uplo, transa, diag, A, B, alpha, mixed)
 
@@ -617,7 +617,7 @@ def unified_rectrxm_mixed_host_(side, uplo, transpose, alpha, func, A, B, *, X=N
                                 synchronize=True):
     """The mixed-precision unified_rectrxm! on Float64 host tensors (see
     ``unified_rectrxm_host_`` for the buffers and ``unified_rectrxm_mixed_``
-    for the options; here the defaults are the exact 7-slice updates without
+    for the options; here the defaults are the exact updates without
     refinement)."""
     import ctypes
 
