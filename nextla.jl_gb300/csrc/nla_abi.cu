@@ -172,17 +172,17 @@ static bool umma_enabled() {
   return on;
 }
 
-// Float32 updates on the tensor cores (nla_umma_f32.cu) from about 1e8
-// products: staging and the kernel's prologue cost about 20 us, the CUDA-core
-// update runs at 15-40 TFLOP/s.  Measured (N x K x M, CUDA cores against
-// tensor cores, launches included): 512^3 34 / 31 us, 256 x 256 x 8192
-// 48 / 29, 1024 x 1024 x 8192 516 / 150, 4096 x 4096 x 8192 6889 / 1384.
+// Float32 updates on the tensor cores (nla_umma_f32.cu) from about 3e7
+// products: staging and the kernel's prologue cost about 15 us, the CUDA-core
+// update runs at 5-40 TFLOP/s.  Measured (N x K x M, CUDA cores against
+// tensor cores, launches included): 256^3 13.4 / about 14 us, 256 x 256 x 900
+// 19.0 / 15.4, 512^3 34 / 17, 256 x 256 x 8192 48 / 25, 1024 x 1024 x 8192 516 / 150, 4096 x 4096 x 8192 6889 / 1384.
 // Below K = 128 a chunk's truncated sums are no more accurate than the FMA
 // chain they replace.  Relative error against 64 bits at K = 128, 1024, 8192:
 // normal data 2.0e-7, 5.7e-7, 1.6e-6 before, 7.5e-8, 1.0e-7, 2.2e-7 now;
 // values spread over 2^+-12 1.5e-7, 4.0e-7, 1.1e-6 / 1.2e-7, 1.4e-7, 2.3e-7.
 static bool f32_umma_wanted(int64_t N, int64_t M, int64_t K) {
-  return umma_enabled() && N >= 64 && M >= 64 && K >= 128 && (double)N * (double)M * (double)K >= 1e8;
+  return umma_enabled() && N >= 64 && M >= 64 && K >= 128 && (double)N * (double)M * (double)K >= 3e7;
 }
 
 size_t update_scratch_bytes(int dtype, int64_t N, int64_t M, int64_t K) {

@@ -1,5 +1,6 @@
 // Float32 off-diagonal update on the tensor cores (tcgen05):
 //   C (M x N) += alpha * op(A) (M x K) * op(B) (K x N)
+// in tiles of 128 rows and 128, 64 or 32 columns.
 //
 // Each Float32 value is the sum of three BF16 values, x = h + m + l exactly
 // (24 bits of significand as 8 + 8 + 8, each rounded to nearest; the split
@@ -22,8 +23,10 @@
 // a real matrix of 2 M rows (re, im interleaved), op(B) one of 2 K rows, and
 // op(A) is staged as 2 M x 2 K, each a as the block (re, -im; im, re).
 //
-// What bounds it: the TMA feed (96 KiB of tiles per 64 values of K for six
-// 128 x 128 x 64 products): 1190 TFLOP/s of executed products, 199 of the
+// What bounds it: shared memory (per 64 values of K and 128 x 128 outputs the
+// six products read 176 KiB of operands from it, and TMA writes 96 KiB;
+// stages of 32 values of K were slower, fewer drains hardly faster):
+// 1190 TFLOP/s of executed products, 199 of the
 // update's, at 4096 x 4096 x 8192 (FFMA update: 39.9).  Warps: 0 loads A, 1 issues MMAs, 2 loads B,
 // 3-10 drain (two TMEM buffers of 256 columns) and update C.
 //
@@ -46,11 +49,12 @@ constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int TILE_BYTES = BM * BK * 2;
 constexpr int SL = 3;
 constexpr int F32_THREADS = 352;
-constexpr int F32_STAGES = 2;
-constexpr int F32_STAGE_BYTES = 2 * SL * TILE_BYTES;
 constexpr int F32_CHUNK = 1;  // K blocks of 64 per drained chunk
-constexpr int F32_SMEM = F32_STAGES * F32_STAGE_BYTES + 1024 + 256;
-static_assert(F32_SMEM + 16 <= 232448, "shared memory above the per-block limit");
+// Tiles of 128 rows and TN (128, 64 or 32) columns: two or three stages.
+constexpr int f32_stages(int TN) { return TN == 128 ? 2 : 3; }
+constexpr int f32_stage_bytes(int TN) { return SL * (BM + TN) * BK * 2; }
+constexpr int f32_smem(int TN) { return f32_stages(TN) * f32_stage_bytes(TN) + 1024 + 256; }
+static_assert(f32_smem(128) + 1056 <= 232448 && f32_smem(64) + 1056 <= 232448, "shared memory above the per-block limit");
 
 // Row marks: 0 for a row of zeros, else the largest exponent field plus one
 // (1 .. 256, 256 for Inf and NaN), so that the row's largest value lies in
@@ -102,9 +106,14 @@ __device__ __noinline__ float plain_dot(const F32Params& p, int i, int j) {
   return s;
 }
 
+template <int TN>
 __global__ void __launch_bounds__(F32_THREADS, 1)
     umma_f32_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     const __grid_constant__ F32Params p) {
+  constexpr int F32_STAGES = f32_stages(TN), F32_STAGE_BYTES = f32_stage_bytes(TN);
+  constexpr int B_BYTES = TN * BK * 2;  // one term's tile of B
+  constexpr int HALF = TN / 2;          // columns per drain warp
+  constexpr int CB = HALF < 32 ? HALF : 32;  // columns of C per batch of loads
   chain_begin();
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -126,7 +135,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
   const int first_m = g * group;
   const int gsize = min(p.tiles_m - first_m, group);
   const int local = blockIdx.x % per_group;
-  const int m0 = (first_m + local % gsize) * BM, n0 = (local / gsize) * BN;
+  const int m0 = (first_m + local % gsize) * BM, n0 = (local / gsize) * TN;
 
   if (threadIdx.x == 0) {
     s_abort = 0;
@@ -161,16 +170,16 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
           break;
         const uint32_t fb = umma::smem_u32(&own[s]);
         uint8_t* st = smem + (size_t)s * F32_STAGE_BYTES + (is_a ? 0 : SL * TILE_BYTES);
-        umma::mbar_arrive_expect_tx(fb, SL * TILE_BYTES);
+        const int bytes = is_a ? TILE_BYTES : B_BYTES, row0 = is_a ? m0 * SL : n0 / BN * BN * SL + n0 % BN;
+        umma::mbar_arrive_expect_tx(fb, (uint32_t)(SL * bytes));
         for (int sl = 0; sl < SL; ++sl)
-          umma::tma_load_2d(umma::smem_u32(st + sl * TILE_BYTES), is_a ? &tmA : &tmB, fb, kb * BK,
-                            (is_a ? m0 : n0) * SL + sl * BM);
+          umma::tma_load_2d(umma::smem_u32(st + sl * bytes), is_a ? &tmA : &tmB, fb, kb * BK, row0 + sl * BM);
       }
       umma::producer_quiesce(own, F32_STAGES, kb, &s_abort, p.err, 52);
     }
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t id1 = umma::idesc_f16(BM, BN, true), id2 = umma::idesc_f16(BM, 2 * BN, true);
+      const uint32_t id1 = umma::idesc_f16(BM, TN, true), id2 = umma::idesc_f16(BM, 2 * TN, true);
       for (int kb = 0; kb < p.num_kb; ++kb) {
         const int s = kb % F32_STAGES, ch = kb / F32_CHUNK, b = ch & 1;
         const bool first = kb % F32_CHUNK == 0;
@@ -180,9 +189,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
           break;
         umma::fence_after_sync();
         const uint32_t a0 = umma::smem_u32(smem + (size_t)s * F32_STAGE_BYTES), b0 = a0 + SL * TILE_BYTES;
-        const uint32_t d0 = tmem + (uint32_t)(b * 2 * BN), d1 = d0 + (uint32_t)BN;
+        const uint32_t d0 = tmem + (uint32_t)(b * 2 * TN), d1 = d0 + (uint32_t)TN;
         // A_h against (B_h, B_m), adjacent in shared memory: one MMA of
-        // N = 256 into both accumulators.
+        // N = 2 TN into both accumulators.
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk)
           umma::mma_f16(d0, umma::desc_kmajor_sw128(a0 + kk * 32), umma::desc_kmajor_sw128(b0 + kk * 32), id2,
@@ -193,7 +202,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 #pragma unroll
           for (int kk = 0; kk < BK / 16; ++kk)
             umma::mma_f16(d1, umma::desc_kmajor_sw128(a0 + qa[pr] * TILE_BYTES + kk * 32),
-                          umma::desc_kmajor_sw128(b0 + qb[pr] * TILE_BYTES + kk * 32), id1, 1u);
+                          umma::desc_kmajor_sw128(b0 + qb[pr] * B_BYTES + kk * 32), id1, 1u);
         umma::mma_commit(umma::smem_u32(&empty[s]));
         if (kb % F32_CHUNK == F32_CHUNK - 1 || kb == p.num_kb - 1) umma::mma_commit(umma::smem_u32(&cfull[b]));
       }
@@ -203,7 +212,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
   } else {
     const int q = warp & 3;
     const int h = (warp - 3) >> 2;  // column half: 0 (warps 3-6) or 1 (warps 7-10)
-    const int i = m0 + q * 32 + lane, c0 = n0 + h * 64;
+    const int i = m0 + q * 32 + lane, c0 = n0 + h * HALF;
     {
       // The marks of the tile's rows (threads 0-127) and columns (128-255).
       const int t = (int)threadIdx.x - 96, r = t & (BM - 1);
@@ -211,13 +220,13 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
       const int step = t < BM ? p.rows_a : p.rows_b;
       int m = 0;
 #pragma unroll 4
-      for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, __ldg(mk + (int64_t)kb * step));
+      for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, t < BM + TN ? __ldg(mk + (int64_t)kb * step) : 0);
       s_mark[t] = m;
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
-    float acc[64];
+    float acc[HALF];
 #pragma unroll
-    for (int j = 0; j < 64; ++j) acc[j] = 0.0f;
+    for (int j = 0; j < HALF; ++j) acc[j] = 0.0f;
     bool ok = true;
     const int nch = (p.num_kb + F32_CHUNK - 1) / F32_CHUNK;
     for (int ch = 0; ch < nch; ++ch) {
@@ -225,12 +234,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
       ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&cfull[b]), (uint32_t)(ch >> 1) & 1u, &s_abort, p.err, 56));
       if (!ok) break;
       umma::fence_after_sync();
-      const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * BN + h * 64);
+      const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * TN + h * HALF);
 #pragma unroll
-      for (int j0 = 0; j0 < 64; j0 += 16) {
+      for (int j0 = 0; j0 < HALF; j0 += 16) {
         uint32_t r0[16], r1[16];
         umma::tmem_ld16(ta + (uint32_t)j0, r0);
-        umma::tmem_ld16(ta + (uint32_t)(BN + j0), r1);
+        umma::tmem_ld16(ta + (uint32_t)(TN + j0), r1);
 #pragma unroll
         for (int j = 0; j < 16; ++j) acc[j0 + j] += __uint_as_float(r0[j]) + __uint_as_float(r1[j]);
       }
@@ -240,16 +249,16 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
     }
     if (ok) {
       const int ma = s_mark[q * 32 + lane];
-      const int* mb = s_mark + BM + h * 64;
+      const int* mb = s_mark + BM + h * HALF;
       float* C = p.C + i;
       bool special = false;
 #pragma unroll
-      for (int j0 = 0; j0 < 64; j0 += 32) {
+      for (int j0 = 0; j0 < HALF; j0 += CB) {
         // All loads of C before the first store (a store may alias a later load).
-        float cv[32];
+        float cv[CB];
         uint32_t skip = 0;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+        for (int j = 0; j < CB; ++j) {
           const int col = c0 + j0 + j;
           const bool in = i < p.M && col < p.N;
           cv[j] = in ? C[(int64_t)col * p.ldc] : 0.0f;
@@ -257,11 +266,11 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
           special |= in && (skip >> j & 1u);
         }
 #pragma unroll
-        for (int j = 0; j < 32; ++j)
+        for (int j = 0; j < CB; ++j)
           if (!(skip >> j & 1u)) C[(int64_t)(c0 + j0 + j) * p.ldc] = fmaf(p.alpha, acc[j0 + j], cv[j]);
       }
       if (special)
-        for (int col = c0; col < min(c0 + 64, p.N); ++col)
+        for (int col = c0; col < min(c0 + HALF, p.N); ++col)
           if (i < p.M && careful(ma, mb[col - c0]))
             C[(int64_t)col * p.ldc] = fmaf(p.alpha, plain_dot(p, i, col), C[(int64_t)col * p.ldc]);
     }
@@ -359,6 +368,18 @@ size_t terms_bytes(int64_t rows, int64_t K) {
 }
 size_t marks_bytes(int64_t rows, int64_t K) { return (size_t)pad_to(rows, BM) * (size_t)(pad_to(K, BK) / BK) * sizeof(int); }
 
+// Columns of C per tile: the narrowest whose tiles still are one wave, since
+// with few tiles a launch's time is one tile's loads, products and C update.
+// Measured (rows x K x columns, 128 columns against the rule, with staging):
+// 512^3 24.4 -> 17.7 us, 476 x 1024 x 900 38.3 -> 27.6, 1024^3 38.6 -> 30.6;
+// the same bits.  Beyond one wave wide tiles read their operands fewer times.
+int f32_tile_cols(int64_t M, int64_t N) {
+  const int64_t tm = (M + BM - 1) / BM;
+  int tn = BN;
+  while (tn > 32 && tm * ((N + tn / 2 - 1) / (tn / 2)) <= num_sms()) tn /= 2;
+  return tn;
+}
+
 }  // namespace
 
 size_t f32_update_bytes(int64_t M, int64_t N, int64_t K) {
@@ -383,7 +404,8 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
   p.K = (int)K;
   p.num_kb = (int)(Kp / BK);
   p.tiles_m = (int)(Mp / BM);
-  p.tiles_n = (int)(Np / BN);
+  const int tn = f32_tile_cols(M, N);
+  p.tiles_n = (int)((N + tn - 1) / tn);
   p.A = static_cast<const float*>(A.p);
   p.asi = A.t ? A.ld : 1;
   p.ask = A.t ? 1 : A.ld;
@@ -410,16 +432,21 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
   }
   CUtensorMap mA, mB;
   NLA_TRY(staged_map(&mA, ta, (uint64_t)Kp, (uint64_t)(SL * Mp)));
-  NLA_TRY(staged_map(&mB, tb, (uint64_t)Kp, (uint64_t)(SL * Np)));
+  NLA_TRY(staged_map(&mB, tb, (uint64_t)Kp, (uint64_t)(SL * Np), (uint32_t)tn));
   static std::once_flag once;
   static cudaError_t st = cudaSuccess;
   std::call_once(once, [] {
-    st = cudaFuncSetAttribute(umma_f32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, F32_SMEM);
+    st = cudaFuncSetAttribute(umma_f32_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem(128));
+    if (st == cudaSuccess)
+      st = cudaFuncSetAttribute(umma_f32_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem(64));
+    if (st == cudaSuccess)
+      st = cudaFuncSetAttribute(umma_f32_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, f32_smem(32));
   });
   if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(umma_f32_kernel)");
   TraceScope trace(NLA_K_GEMM_UMMA, s, 6.0 * 2.0 * (double)M * (double)N * (double)K,
                    (double)SL * 2.0 * (double)(Mp + Np) * Kp + 8.0 * (double)M * (double)N);
-  launch_chained(umma_f32_kernel, (unsigned)((int64_t)p.tiles_m * p.tiles_n), F32_THREADS, F32_SMEM, s, mA, mB, p);
+  launch_chained(tn == 128 ? umma_f32_kernel<128> : tn == 64 ? umma_f32_kernel<64> : umma_f32_kernel<32>, (unsigned)((int64_t)p.tiles_m * p.tiles_n),
+                 F32_THREADS, f32_smem(tn), s, mA, mB, p);
   NLA_CHECK_LAUNCH("umma_f32_kernel");
   return NLA_OK;
 }

@@ -152,3 +152,26 @@ def test_c32_update_not_finite(pkg, cuda):
     assert np.array_equal(np.isnan(got.real[3, rest]), np.isnan(re[3, rest]))
     assert np.array_equal(np.isinf(got.real[3, rest]), np.isinf(re[3, rest]))
     assert np.isnan(got.imag[:, 77]).all() and np.isnan(got.real[:, 77]).all()
+
+
+@pytest.mark.parametrize("shape", [(64, 300, 2000), (100, 200, 1601), (129, 140, 2400), (128, 256, 4900),
+                                   (257, 130, 3100), (257, 128, 6500)])
+@pytest.mark.parametrize("special", [False, True])
+def test_f32_update_tile_widths(pkg, cuda, shape, special):
+    """Tiles of 32, 64 and 128 columns (chosen by how many fill the GPU), from
+    the smallest sizes that take this path, with remainders; the tolerance of
+    this file, and with Inf and NaN the plain product's pattern of them."""
+    N, K, M = shape
+    rng = np.random.default_rng(N + M)
+    A, B, C = (rng.standard_normal(s).astype(np.float32) for s in ((N, K), (K, M), (N, M)))
+    if special:
+        A[3, 5], A[N - 1, K - 1], B[1, M - 1], B[K - 1, 40] = np.inf, np.nan, -np.inf, np.nan
+    for ta, tb in ((0, 0), (1, 1)):
+        got = _update(pkg, cuda, A, B, C, ta, tb, -1.0)
+        with np.errstate(all="ignore"):
+            A8, B8, C8 = (X.astype(np.float64) for X in (A, B, C))
+            ref = C8 - A8 @ B8
+            bound = (12 + -(-K // 64)) * 2.0 ** -24 * (np.abs(C8) + np.abs(A8) @ np.abs(B8))
+        ok = np.isfinite(ref)
+        assert np.array_equal(np.isnan(got), np.isnan(ref)) and np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+        assert (np.abs(got - ref)[ok] <= bound[ok]).all(), (shape, ta, tb)
