@@ -214,12 +214,11 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
         if (i0 + RS * u < nr) X[(size_t)c * ldx + i0 + RS * u] = Elem<T>::load(&v[u]);
     }
   }
-  if (SOLVE)
-    for (int i = t; i < nr; i += ST_THREADS) {
-      const Tc d = g.unit || i >= n ? Mx::one() : Mx::conj_if(Elem<T>::load(A + i * (si + sk)), g.cj);
-      dia[i] = d;
-      inv[i] = Mx::inverse(d);
-    }
+  for (int i = t; i < nr; i += ST_THREADS) {
+    const Tc d = g.unit || i >= n ? Mx::one() : Mx::conj_if(Elem<T>::load(A + i * (si + sk)), g.cj);
+    dia[i] = d;
+    if (SOLVE) inv[i] = Mx::inverse(d);
+  }
   __syncthreads();
 
   Tc acc[NC];
@@ -236,11 +235,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
       for (int e = 0; e < PER; ++e) {
         const int i = fi + e * ei, k = fk + e * ek;
         Tc v = Mx::conj_if(Elem<T>::load(&ra[e]), g.cj);
-        if (!SOLVE) {  // the panel's own triangle: zero above, one on a unit diagonal
-          const int r = p0 + i, kk = k0 + k;
-          if (kk > r) v = Mx::zero();
-          else if (kk == r && g.unit) v = r < n ? Mx::one() : Mx::zero();
-        }
+        if (!SOLVE && k0 + k >= p0 + i) v = Mx::zero();  // strictly below the diagonal
         Ab[i * LDA + k] = v;
       }
       const bool last = ch + 1 == nch;
@@ -268,6 +263,11 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
         for (int q = 0; q < NC; ++q) {
           Tc x[VK];
           st_unpack(*reinterpret_cast<const Vec*>(xr + (size_t)q * ldx + u * VK), x);
+          if (!SOLVE && k0 + (u + 1) * VK > p0) {  // the panel's own rows: no Inf or NaN from above the diagonal
+#pragma unroll
+            for (int v = 0; v < VK; ++v)
+              if (k0 + u * VK + v >= p0 + row) x[v] = Mx::zero();
+          }
 #pragma unroll
           for (int v = 0; v < VK; ++v) acc[q] = Mx::fma_(a[v], x[v], acc[q]);
         }
@@ -314,8 +314,12 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
             if constexpr (KG == 1) __syncwarp();
           } else {
 #pragma unroll
-            for (int q = 0; q < NC; ++q)
-              if (p0 + row < n && col0 + q < ncols) Elem<T>::store(B + (p0 + row) * bi + (col0 + q) * bc, acc[q]);
+            for (int q = 0; q < NC; ++q) {
+              // The diagonal's product last, on the whole sum: usually the
+              // largest term, so the row is rounded at its size once.
+              const Tc y = Mx::fma_(dia[p0 + row], X[(size_t)(col0 + q) * ldx + p0 + row], acc[q]);
+              if (p0 + row < n && col0 + q < ncols) Elem<T>::store(B + (p0 + row) * bi + (col0 + q) * bc, y);
+            }
           }
         }
       }

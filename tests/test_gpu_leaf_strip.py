@@ -59,3 +59,39 @@ def test_strip_wide(pkg, oracle, workloads, cuda, dtype, func, n, m):
         torch.cuda.synchronize()
         ref = oracle.blas_rectrxm(side, uplo, "N", 1.0, func, A.astype(np.float64), B.astype(np.float64))
         assert oracle.rel_err(to_host(Bd), ref) < TOL[dtype], (side, uplo, ta)
+
+
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+@pytest.mark.parametrize("n,m", [(17, 3), (40, 24), (96, 300), (128, 2500)])
+def test_strip_multiply_rows(pkg, workloads, cuda, dtype, n, m):
+    """A row of a multiply takes nothing from the rows past it (Inf and NaN
+    there do not reach it), and its largest term, the diagonal's, is rounded
+    once.  Bound per element: at most n + 4 roundings of the off-diagonal sums
+    plus one of the result, u (n + 4) S_off + 1.01 u |y| (u the unit roundoff,
+    S_off = sum of |a x| left of the diagonal)."""
+    import torch
+
+    rng = np.random.default_rng(n)
+    A = np.tril(rng.standard_normal((n, n)) / np.sqrt(n), -1) + np.diag(2 + np.abs(rng.standard_normal(n)))
+    B = rng.uniform(-1, 1, (n, m))
+    A, B = A.astype(dtype), B.astype(dtype)
+    u = np.finfo(dtype).eps / 2
+    for bad in (None, n // 2, n - 1):
+        Bb = B.copy()
+        if bad is not None:
+            Bb[bad, 0], Bb[bad, m - 1] = np.inf, np.nan
+        Ad, Bd = to_dev(A, dtype, cuda, ld=n + 1), to_dev(Bb, dtype, cuda, ld=n + 2)
+        pkg.rectrxm._diag_block("M", "L", "L", Ad, Bd)
+        torch.cuda.synchronize()
+        got = to_host(Bd).astype(np.longdouble)
+        with np.errstate(all="ignore"):
+            A8, B8 = A.astype(np.longdouble), B.astype(np.longdouble)
+            ref = A8 @ B8
+            off = np.abs(np.tril(A8, -1)) @ np.abs(B8)
+        rows = slice(0, n if bad is None else bad)
+        err = np.abs(got - ref)[rows]
+        assert (err <= (u * (n + 4) * off + u * 1.01 * np.abs(ref))[rows]).all(), (n, m, bad)
+        if bad is not None:
+            assert not np.isfinite(got[bad:, [0, m - 1]]).any()
+            keep = slice(1, m - 1)
+            assert np.isfinite(got[:, keep]).all()
