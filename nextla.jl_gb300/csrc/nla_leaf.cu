@@ -133,7 +133,8 @@ int launch_strips(const LeafArgs& g, cudaStream_t s) {
   // Warps on 32 and 64 columns.  Float32 products wait for shared memory with
   // two warps per scheduler; a second K group gives it four (and costs one
   // sum through shared memory per panel): solve 256 x 8192 47.9 -> 44.4 us,
-  // multiply 128 x 8192 16.3 -> 14.3 us, 64 x 6144 8.4 -> 7.3 us.  On 8 and
+  // multiply 128 x 8192 16.3 -> 14.3 us (15.2 since multiplies stop at
+  // the diagonal), 64 x 6144 8.4 -> 7.3 us.  On 8 and
   // 16 columns, where the triangles' chains bound, it gave nothing (25.2 us
   // at 256 x 1000 either way).
   constexpr int NWW = CX || F64 ? 8 : 16;

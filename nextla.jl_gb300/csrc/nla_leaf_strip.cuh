@@ -255,23 +255,29 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
       const int units = kw > 0 ? (kw + VK - 1) / VK : 0;  // A is staged as zeros past kend, X holds zeros past n
       const Tc* ar = Ab + row * LDA;
       const Tc* xr = X + (size_t)col0 * ldx + k0;
-#pragma unroll 4
-      for (int u = kg; u < units; u += KG) {
+      // Multiplies: units of the panel's own rows (from `own` on) take X only
+      // left of the diagonal, so that no Inf or NaN from past it is used.
+      const int own = SOLVE ? units : min(units, max(0, (p0 - k0) / VK));
+      auto unit = [&](int u, bool mask) {
         Tc a[VK];
         st_unpack(*reinterpret_cast<const Vec*>(ar + u * VK), a);
 #pragma unroll
         for (int q = 0; q < NC; ++q) {
           Tc x[VK];
           st_unpack(*reinterpret_cast<const Vec*>(xr + (size_t)q * ldx + u * VK), x);
-          if (!SOLVE && k0 + (u + 1) * VK > p0) {  // the panel's own rows: no Inf or NaN from above the diagonal
 #pragma unroll
-            for (int v = 0; v < VK; ++v)
-              if (k0 + u * VK + v >= p0 + row) x[v] = Mx::zero();
+          for (int v = 0; v < VK; ++v) {
+            if (mask && k0 + u * VK + v >= p0 + row) x[v] = Mx::zero();
+            acc[q] = Mx::fma_(a[v], x[v], acc[q]);
           }
-#pragma unroll
-          for (int v = 0; v < VK; ++v) acc[q] = Mx::fma_(a[v], x[v], acc[q]);
         }
-      }
+      };
+      int u = kg;
+#pragma unroll 4
+      for (; u < own; u += KG) unit(u, false);
+      if (!SOLVE)
+#pragma unroll 2
+        for (; u < units; u += KG) unit(u, true);
       if (last) {
         if constexpr (KG > 1) {
           if (kg > 0) {
