@@ -74,6 +74,9 @@ inline Mat transposed(const Mat& v) {
 // chain_begin(), before it touches memory, until that one has completed with
 // its writes visible; it then lets its own successor be set up.  So at most
 // two kernels of a chain are in flight and every access keeps its order.
+// Chained kernels load with ordinary loads only: the non-coherent path (__ldg,
+// const __restrict__) is defined for data that nothing writes while the kernel
+// is resident, and the predecessor still writes then.
 // (Tensor memory too is taken only after the wait: the predecessor may hold
 // all of it.)  Chained are the tensor-core kernels, which take an SM each, and
 // the staging and finishing passes around them.  Kernels of few CTAs that

@@ -710,7 +710,7 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
   int er[4];  // row exponents with the bias (at least -4200: far below any sum that matters)
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    er[r] = ib + r < p.M ? __ldg(p.ea + ib + r) : 0;
+    er[r] = ib + r < p.M ? p.ea[ib + r] : 0;
     if (er[r] != NONFINITE_EXP) er[r] = max(er[r], -4000) + p.e_bias;
   }
 #pragma unroll 1
@@ -720,14 +720,14 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
     uint32_t w[L];
 #pragma unroll
     for (int l = 0; l < L; ++l)
-      w[l] = __ldg(reinterpret_cast<const uint32_t*>(p.planes + l * p.plane + ib + col * p.ldp)) ^ 0x80808080u;
+      w[l] = *reinterpret_cast<const uint32_t*>(p.planes + l * p.plane + ib + col * p.ldp) ^ 0x80808080u;
     double cv[4];
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
       const int i = i0 + lane + 32 * r;
       cv[r] = i < p.M ? p.C[i + col * p.ldc] : 0.0;
     }
-    int ejc = __ldg(p.eb + col);
+    int ejc = p.eb[col];
     if (ejc != NONFINITE_EXP) ejc = max(ejc, -4000);
 #pragma unroll
     for (int r = 0; r < 4; ++r) {

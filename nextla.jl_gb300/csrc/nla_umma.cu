@@ -221,14 +221,14 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
         const int col = n0 + cbase + c0 + j;
         const bool in = i < p.M && col < p.N;
         v[j] = in ? C[(int64_t)col * p.ldc] : TC(0.0f);
-        if (EPI == EPI_F64) e[j] = in && p.eb != nullptr ? __ldg(p.eb + col) : 0;
+        if (EPI == EPI_F64) e[j] = in && p.eb != nullptr ? p.eb[col] : 0;
       }
     };
     fetch(0, cv, ej);
     int ei = 0;
     bool row_nan = false;
     if (EPI == EPI_F64 && p.ea != nullptr && i < p.M) {
-      ei = __ldg(p.ea + i);
+      ei = p.ea[i];
       row_nan = ei == NONFINITE_EXP;
       ei = max(ei, -4000);
     }
@@ -1001,7 +1001,7 @@ __device__ __forceinline__ bool in_tri(int tri, int64_t i, int64_t k) {
 // row and reduces it with one warp-wide max, so no shared-memory atomics
 // collide.
 template <typename T>
-__global__ void __launch_bounds__(256) row_exp_kernel(const T* __restrict__ X, int64_t ld, int t, int64_t rows,
+__global__ void __launch_bounds__(256) row_exp_kernel(const T* X, int64_t ld, int t, int64_t rows,
                                                       int64_t cols, int tri, int* __restrict__ e) {
   chain_begin();
   __shared__ int se[64];
@@ -1090,7 +1090,7 @@ __device__ __forceinline__ long long fixed_of(double x, int ex) {
 // by memory-level parallelism, not by their integer work).  Zeros outside
 // the view and outside the staged triangle.
 template <typename T>
-__device__ __forceinline__ void load_tile(const T* __restrict__ X, int64_t ld, int t, int64_t rows, int64_t cols,
+__device__ __forceinline__ void load_tile(const T* X, int64_t ld, int t, int64_t rows, int64_t cols,
                                           int tri, int64_t i0, int64_t k0, double (&v)[8]) {
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -1185,8 +1185,8 @@ __device__ __forceinline__ void split_tile(const double (*tile)[65], int64_t i0,
 // products along that row (in units of the row's scale 2^e) for a partner
 // whose elements are below 1/2.
 template <typename T, typename Sl, int NS>
-__global__ void __launch_bounds__(256) split_kernel(const T* __restrict__ X, int64_t ld, int t, int64_t rows,
-                                                    int64_t cols, int tri, const int* __restrict__ e,
+__global__ void __launch_bounds__(256) split_kernel(const T* X, int64_t ld, int t, int64_t rows,
+                                                    int64_t cols, int tri, const int* e,
                                                     Sl* __restrict__ out, int64_t rows_pad, int64_t cols_pad,
                                                     float* __restrict__ nrm) {
   chain_begin();

@@ -220,7 +220,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
       const int step = t < BM ? p.rows_a : p.rows_b;
       int m = 0;
 #pragma unroll 4
-      for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, t < BM + TN ? __ldg(mk + (int64_t)kb * step) : 0);
+      for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, t < BM + TN ? mk[(int64_t)kb * step] : 0);
       s_mark[t] = m;
       asm volatile("bar.sync 1, 256;" ::: "memory");
     }
@@ -326,11 +326,11 @@ __global__ void __launch_bounds__(256) stage_f32_kernel(const F32Job a, const F3
     const int i = i0 + (kfast ? idx >> 6 : idx & 31), k = k0 + (kfast ? idx & 63 : idx >> 5);
     const bool in = i < j.rows && k < j.K;
     if (j.cplx == 0) {
-      v[e] = in ? __ldg(j.X + i * j.si + k * j.sk) : 0.0f;
+      v[e] = in ? j.X[i * j.si + k * j.sk] : 0.0f;
     } else {
       const bool pair = j.cplx == 1;
       const int part = pair ? (i ^ k) & 1 : k & 1;  // 0: real part, 1: imaginary
-      const float x = in ? __ldg(j.X + 2 * ((pair ? i >> 1 : i) * j.si + (k >> 1) * j.sk) + part) : 0.0f;
+      const float x = in ? j.X[2 * ((pair ? i >> 1 : i) * j.si + (k >> 1) * j.sk) + part] : 0.0f;
       v[e] = part ? (pair && !(i & 1) ? -j.im : j.im) * x : x;
     }
   }
