@@ -298,7 +298,6 @@ int recurse(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   if (c.inv && leaf_pair_wanted(c, n)) return leaf_pair_apply(c, A, n, B);
   if (n <= c.threshold) {
     if (c.inv) return leaf_inverse_apply(c, A, n, B);
-    if (leaf_product_wanted(c)) return leaf_product_multiply(c, A, n, B);
     return launch_leaf(c.func, c.side, c.uplo, c.dtype, n, c.m, A, B, c.s, c.unit);
   }
   const int64_t mid = split_point(n), rem = n - mid;

@@ -308,9 +308,6 @@ int recurse(const RecPlan& c, const Mat& A, int64_t n, const Mat& B);
 bool leaf_inverses_wanted(const RecPlan& c);
 int leaf_inverses_upfront(const RecPlan& c, const Mat& A, int64_t n, LeafInverses* out);
 int leaf_inverse_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B);
-// The same kernel as the leaf of a mixed multiply, on the triangle itself.
-bool leaf_product_wanted(const RecPlan& c);
-int leaf_product_multiply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B);
 // A recursion node whose two halves are both leaves, solved with the update
 // between them in one launch (nla_mixed.cu).
 bool leaf_pair_wanted(const RecPlan& c, int64_t n);

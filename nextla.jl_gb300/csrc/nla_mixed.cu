@@ -159,11 +159,14 @@ unsigned grid_for(int64_t total) {
 // right-hand sides the short update between two 64-row blocks (staging,
 // product and their launches, about 30 us) costs more than that half, and
 // 128 rows are better.  Measured at 2048 right-hand sides (solve): 128 rows
-// 44 us against 2 x 20 + 28; at 6144 (multiply) about equal.  A small
+// 44 us against 2 x 20 + 28.  Multiplies (3 terms, 64 / 128 rows): 4096 x
+// 2048 2.75 / 2.68 ms, 6144 x 6144 8.28 / 9.54 ms.  A small
 // exact solve takes them too: a 128-row block costs about 28 us against 20 for
 // a pair of inverse blocks, but those need their inversion first (25 us once).
 // Measured (n x m, 64 / 128 rows): 200 x 100 96 / 63 us, 512 x 128 182 / 164,
-// 1000 x 300 377 / 467.
+// 1000 x 300 377 / 467.  A multiply's blocks stay in FP64 at either size: the
+// product on inverse blocks scales a column of right-hand sides by its largest
+// element in the block, and rows of a triangle do not read all of it.
 int default_mixed_cutoff(int terms, char func, int64_t n, int64_t m) {
   const char* v = std::getenv("NLA_MIXED_CUTOFF");
   if (v && *v) {
@@ -441,10 +444,7 @@ __device__ __forceinline__ double lp_value(long long tot, int ex, int ew) {
 }
 
 struct LeafProdArgs {
-  const double* W;   // W(i, k) at W[i * wsi + k * wsk]
-  int64_t wsi, wsk;
-  int tri;           // W's stored part: 0 all of it, 1 k <= i, 2 k >= i (the rest counts as zero)
-  int unit;          // ones on the diagonal, which is not read
+  const double* W;  // column-major, leading dimension LEAF_INV_N
   double* X;
   int64_t ldx;
   int64_t m;
@@ -461,8 +461,10 @@ __global__ void __launch_bounds__(LP_THREADS, 1) leaf_product_kernel(const LeafP
 
   const int t = threadIdx.x, warp = t >> 5, n = a.n;
   const int64_t j0 = (int64_t)blockIdx.x * LP_COLS;
-  // Element (k, j) of the right-hand sides (k < n, j < m).
+  // Element (k, j) of the right-hand sides (k < n, j < m) and (i, k) of the
+  // W operand (W itself for side L, W^T for side R).
   auto xat = [&](int k, int64_t j) -> int64_t { return a.side_r ? j + (int64_t)k * a.ldx : k + j * a.ldx; };
+  auto wat = [&](int i, int k) -> int { return a.side_r ? k + i * LEAF_INV_N : i + k * LEAF_INV_N; };
 
   if (t == 0) {
     s_abort = 0;
@@ -483,9 +485,7 @@ __global__ void __launch_bounds__(LP_THREADS, 1) leaf_product_kernel(const LeafP
 #pragma unroll
   for (int u = 0; u < 8; ++u) {
     const int k = wp * 8 + u;
-    const bool diag = a.unit && k == wi;
-    const bool in = wi < n && k < n && !diag && (a.tri == 0 || (a.tri == 1 ? k <= wi : k >= wi));
-    vw[u] = in ? a.W[wi * a.wsi + k * a.wsk] : diag && k < n ? 1.0 : 0.0;
+    vw[u] = wi < n && k < n ? a.W[wat(wi, k)] : 0.0;
   }
   lp_stage(s, vx, vw);
   const uint32_t tmem = *s.tmem_slot;
@@ -1011,47 +1011,22 @@ int allow_smem(const char* name) {
 
 }  // namespace
 
-static int launch_leaf_product(const RecPlan& c, int64_t n, const Mat& B, const double* W, int64_t wsi, int64_t wsk,
-                               int tri, bool unit, int* err) {
-  NLA_TRY(allow_smem<leaf_product_kernel>("cudaFuncSetAttribute(leaf_product_kernel)"));
-  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "leaf product: transposed B view");
-  const LeafProdArgs g{W, wsi, wsk, tri, unit ? 1 : 0, static_cast<double*>(B.p), B.ld, c.m, (int)n, c.side == 'R' ? 1 : 0, err};
-  const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
-  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf product: too many right-hand sides");
-  TraceScope trace(c.func == 'S' ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, c.s, 2.0 * (double)n * n * (double)c.m,
-                   16.0 * (double)n * (double)c.m);
-  launch_chained(leaf_product_kernel, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
-  NLA_CHECK_LAUNCH("leaf_product_kernel");
-  return NLA_OK;
-}
-
 int leaf_inverse_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
   if (n <= 0 || c.m <= 0) return NLA_OK;
   const LeafInverses& L = *c.inv;
   int64_t slot = 0;
   NLA_TRY(leaf_slot(L, (static_cast<const double*>(A.p) - L.a_base) / (L.lda + 1), &slot));
   // X := inv(T) X  (side L)  or  X inv(T)  (side R), one kernel.
-  const bool R = c.side == 'R';  // X inv(T): the operand is inv(T)^T
-  return launch_leaf_product(c, n, B, L.w + slot * LEAF_INV_N * LEAF_INV_N, R ? LEAF_INV_N : 1, R ? 1 : LEAF_INV_N, 0,
-                             0, L.err);
-}
-
-// The multiply's leaf in a mixed recursion, B := T B or B T for a triangle of
-// at most 64 rows: the exact product, rounded once per element.  On the FP64
-// pipe it took 38 us at 6144 right-hand sides.
-bool leaf_product_wanted(const RecPlan& c) {
-  return c.mode == GEMM_MIXED && c.func == 'M' && c.dtype == NLA_F64 && c.threshold <= LEAF_INV_N;
-}
-
-int leaf_product_multiply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
-  if (n <= 0 || c.m <= 0) return NLA_OK;
-  int* err = device_error_word();
-  if (!err) return fail(NLA_ERR_UNSUPPORTED, "leaf product: no device error word");
-  const bool R = c.side == 'R';
-  const int64_t si = A.t ? A.ld : 1, sk = A.t ? 1 : A.ld;  // T(i, k) at i si + k sk
-  const bool lower = (c.uplo == 'L') != R;                 // of the operand: T, or T^T for side R
-  return launch_leaf_product(c, n, B, static_cast<const double*>(A.p), R ? sk : si, R ? si : sk, lower ? 1 : 2, c.unit,
-                             err);
+  NLA_TRY(allow_smem<leaf_product_kernel>("cudaFuncSetAttribute(leaf_product_kernel)"));
+  if (B.t) return fail(NLA_ERR_UNSUPPORTED, "leaf product: transposed B view");
+  LeafProdArgs g{L.w + slot * LEAF_INV_N * LEAF_INV_N, static_cast<double*>(B.p), B.ld, c.m, (int)n,
+                 c.side == 'R' ? 1 : 0, L.err};
+  const int64_t grid = (c.m + LP_COLS - 1) / LP_COLS;
+  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf product: too many right-hand sides");
+  TraceScope trace(NLA_K_LEAF_SOLVE, c.s, 2.0 * (double)n * n * (double)c.m, 16.0 * (double)n * (double)c.m);
+  launch_chained(leaf_product_kernel, (unsigned)grid, LP_THREADS, LP_SMEM, c.s, g);
+  NLA_CHECK_LAUNCH("leaf_product_kernel");
+  return NLA_OK;
 }
 
 bool leaf_pair_wanted(const RecPlan& c, int64_t n) {
