@@ -29,6 +29,8 @@
 // right-hand sides are read and written once.
 #pragma once
 
+#include <type_traits>
+
 #include "nla_cplx.cuh"
 #include "nla_leaf.cuh"
 
@@ -90,11 +92,15 @@ template <typename R> struct StripMath<cx::cpx<R>> {
   __device__ static Tc inverse(Tc d) { return cx::div(one(), d); }
   // The product with the reciprocal, corrected once by the remainder: as
   // accurate as the quotient itself (a complex reciprocal carries several
-  // roundings), without a division in the triangle's chain.
+  // roundings), without a division in the triangle's chain.  Where the
+  // reciprocal or the quotient overflows it is not finite; strip_block then
+  // solves the panel again by divisions.
   __device__ static Tc quotient(Tc z, Tc inv, Tc d) {
     const Tc q = cx::fma_c(z, inv, zero());
     return cx::fma_c(cx::fms_c(q, d, z), inv, q);
   }
+  __device__ static bool finite(Tc a) { return isfinite(a.re) && isfinite(a.im); }
+  __device__ __noinline__ static Tc divided(Tc z, Tc d) { return cx::div(z, d); }
 };
 
 template <typename T> __device__ __forceinline__ T raw_zero() { return T(0.0f); }
@@ -316,7 +322,33 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
                 if (row > j) z[q] = Mx::fms_(d[j], xj, z[q]);
               }
 #pragma unroll
-            for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = Mx::quotient(z[q], iv, dr);
+            for (int q = 0; q < NC; ++q) z[q] = Mx::quotient(z[q], iv, dr);
+            if constexpr (!std::is_floating_point<Tc>::value) {
+              // The chain's time is in its steps, so the test for results that
+              // are not finite (a pivot without a finite reciprocal, a quotient
+              // that overflows) comes once per panel; the divisions then give
+              // what is finite, and infinities where there is none.
+              bool again = false;
+#pragma unroll
+              for (int q = 0; q < NC; ++q) again |= !Mx::finite(z[q]);
+              if (__any_sync(0xffffffffu, again)) {
+#pragma unroll
+                for (int q = 0; q < NC; ++q) z[q] = X[(size_t)(col0 + q) * ldx + p0 + row] - acc[q];
+#pragma unroll 1
+                for (int j = 0; j < PB - 1; ++j) {
+                  const Tc dj = Db[row * (PB + 1) + j];
+#pragma unroll
+                  for (int q = 0; q < NC; ++q) {
+                    const Tc xj = Mx::shfl(Mx::divided(z[q], dr), (lane & ~(PB - 1)) | j);
+                    if (row > j) z[q] = Mx::fms_(dj, xj, z[q]);
+                  }
+                }
+#pragma unroll
+                for (int q = 0; q < NC; ++q) z[q] = Mx::divided(z[q], dr);
+              }
+            }
+#pragma unroll
+            for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = z[q];
             if constexpr (KG == 1) __syncwarp();
           } else {
 #pragma unroll
