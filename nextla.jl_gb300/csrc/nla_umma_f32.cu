@@ -8,7 +8,7 @@
 // bfloat16 artificial intelligence datatype for higher-precision
 // computations", ARITH 2019).  Unlike the scaled integer slices of the
 // Float64 update, the terms carry their own exponents, so small elements of
-// a row keep their full precision.  Of the nine products the six of weight
+// a row keep their full precision (down to 2^-100, see careful()).  Of the nine products the six of weight
 // up to 2^-16 are formed (h h; h m, m h; m m, h l, l h); the three left out
 // are below 2^-26 of |a||b| each, under the rounding of one Float32 FMA.
 //
@@ -32,9 +32,9 @@
 //
 // Rows of A and columns of B that hold Inf or NaN, or values so small or
 // large that low terms or sums would leave Float32's normal range, are
-// marked when they are staged; the outputs they touch are formed by the
-// drain warps from the original operands instead, with the FMA order of the
-// CUDA-core update.
+// marked when they are staged; a tile with outputs that they touch forms
+// those outputs from the original operands by a tiled loop of FMAs after its
+// products (plain_tile), or instead of them when that is all of its outputs.
 #include <cudaTypedefs.h>
 
 #include <mutex>
@@ -58,14 +58,16 @@ static_assert(f32_smem(128) + 1056 <= 232448 && f32_smem(64) + 1056 <= 232448, "
 
 // Row marks: 0 for a row of zeros, else the largest exponent field plus one
 // (1 .. 256, 256 for Inf and NaN), so that the row's largest value lies in
-// [2^(mark - 128), 2^(mark - 127)).  An output takes the careful path when its
-// row or column is not finite, when the low terms of either would be
-// subnormal, or when the products leave [2^-90, 2^106] (their low terms, or
-// sums of up to 2^20 of them, would leave the normal range).
+// [2^(mark - 128), 2^(mark - 127)); MARK_TINY more when the row holds a
+// nonzero value below 2^-100, whose low terms would be subnormal.  An output
+// is left to the plain product when its row or column is not finite or has
+// such a value, or when the largest products leave [2^-90, 2^106] (their low
+// terms, or sums of up to 2^20 of them, would leave the normal range).
+constexpr int MARK_LOW = 28, MARK_TINY = 512;  // the mark of 2^-100
 __device__ __forceinline__ bool careful(int ma, int mb) {
-  if (ma == 256 || mb == 256) return true;
+  if (ma >= 256 || mb >= 256) return true;
   if (ma == 0 || mb == 0) return false;
-  return ma < 28 || mb < 28 || ma + mb < 166 || ma + mb > 360;
+  return ma + mb < 166 || ma + mb > 360;
 }
 
 struct F32Params {
@@ -87,23 +89,101 @@ struct F32Params {
   float ima, imb;  // -1 where the operand is conjugated, else 1
 };
 
-// One element in the order of the CUDA-core update: FMAs with k increasing.
-__device__ __noinline__ float plain_dot(const F32Params& p, int i, int j) {
-  float s = 0.0f;
-  if (p.cplx) {
-    const float2* a = reinterpret_cast<const float2*>(p.A) + (int64_t)(i >> 1) * p.asi;
-    const float2* b = reinterpret_cast<const float2*>(p.B) + (int64_t)j * p.bsj;
-    for (int k = 0; k < p.K / 2; ++k) {
-      const float2 x = a[k * p.ask], y = b[k * p.bsk];
-      const float xi = p.ima * x.y, yi = p.imb * y.y;
-      s = (i & 1) ? fmaf(x.x, yi, fmaf(xi, y.x, s)) : fmaf(x.x, y.x, fmaf(-xi, yi, s));
+// The careful outputs of a tile by FMAs with k increasing (the order of the
+// CUDA-core update), the whole tile formed by the 256 threads of the drain
+// warps: 8 x TN / 16 outputs each, K slabs of 8 double-buffered in the ring's
+// shared memory with the next slab in registers.  Bound by the FMA pipe with
+// two warps per scheduler.  Measured at 2048^3, where the tensor cores take
+// 136 us and the CUDA-core update 531: one row of A that is not finite 381 us,
+// every output outside the range 688 us.  (One serial sum per output, 64 of
+// them in the lane of such a row, took 4670 and 8420 us.)  At 4096 x 4096 x
+// 8192: 1.41 ms, 6.92, 1.61 and 8.37 ms.
+constexpr int PK = 8;
+template <int TN>
+__device__ __noinline__ void plain_tile(const F32Params& p, float* smem, const int* mark, int m0, int n0) {
+  constexpr int CPT = TN / 16, CV = CPT < 4 ? CPT : 4;  // columns per thread, adjacent ones
+  constexpr int LDA = BM + 4, LDB = TN + 4, LA = BM * PK / 256, LB = TN * PK / 256;
+  float* As = smem;                 // [2][PK][LDA]
+  float* Bs = smem + 2 * PK * LDA;  // [2][PK][LDB]
+  const int t = (int)threadIdx.x - 96, tx = t & 15, ty = t >> 4;
+  // Slot e of a slab is element (ai + e ai_step, ak + e ak_step) of op(A), likewise
+  // (bk + .., bj + ..) of op(B), threads along the index that is
+  // contiguous in memory.  In the real view of complex operands (re, -im; im,
+  // re) and (re; im) those steps are even, so a thread stays on one part.
+  const bool ka = p.ask == 1, kb = p.bsk == 1, cx = p.cplx != 0;
+  const int ai = ka ? t / PK : t % BM, ak = ka ? t % PK : t / BM;
+  const int bj = kb ? t / PK : t % TN, bk = kb ? t % PK : t / TN;
+  const int ai_step = ka ? 256 / PK : 0, ak_step = ka ? 0 : 256 / BM;
+  const int bj_step = kb ? 256 / PK : 0, bk_step = kb ? 0 : 256 / TN;
+  const int64_t sa = ai_step * p.asi + ak_step * p.ask, sb = (cx ? 2 : 1) * bj_step * p.bsj + bk_step * p.bsk;
+  const int i0 = m0 + ai, j0 = n0 + bj;
+  const float* pa = p.A + (cx ? 2 * ((i0 >> 1) * p.asi + (ak >> 1) * p.ask) + ((i0 ^ ak) & 1) : i0 * p.asi + ak * p.ask);
+  const float* pb = p.B + (cx ? 2 * ((bk >> 1) * p.bsk + j0 * p.bsj) + (bk & 1) : bk * p.bsk + j0 * p.bsj);
+  const float fa = cx && ((i0 ^ ak) & 1) ? (i0 & 1 ? p.ima : -p.ima) : 1.0f, fb = cx && (bk & 1) ? p.imb : 1.0f;
+  const int64_t slab_a = PK * p.ask, slab_b = PK * p.bsk;
+  const int ni = p.M - i0, nj = p.N - j0, K = p.K;
+  float ra[LA], rb[LB];
+  auto load = [&](int k0) {
+#pragma unroll
+    for (int e = 0; e < LA; ++e) ra[e] = e * ai_step < ni && k0 + ak + e * ak_step < K ? pa[e * sa] : 0.0f;
+#pragma unroll
+    for (int e = 0; e < LB; ++e) rb[e] = e * bj_step < nj && k0 + bk + e * bk_step < K ? pb[e * sb] : 0.0f;
+    pa += slab_a;
+    pb += slab_b;
+  };
+  auto store = [&](int buf) {
+#pragma unroll
+    for (int e = 0; e < LA; ++e) As[(buf * PK + ak + e * ak_step) * LDA + ai + e * ai_step] = fa * ra[e];
+#pragma unroll
+    for (int e = 0; e < LB; ++e) Bs[(buf * PK + bk + e * bk_step) * LDB + bj + e * bj_step] = fb * rb[e];
+  };
+  // Local row of slot r and column of slot c.
+  auto row = [&](int r) { return (r >> 2) * 64 + 4 * tx + (r & 3); };
+  auto col = [&](int c) { return (c / CV) * 64 + CV * ty + c % CV; };
+  float acc[8][CPT];
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+#pragma unroll
+    for (int c = 0; c < CPT; ++c) acc[r][c] = 0.0f;
+  load(0);
+  store(0);
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  const int nk = (K + PK - 1) / PK;
+  for (int kt = 0; kt < nk; ++kt) {
+    const int buf = kt & 1;
+    if (kt + 1 < nk) load((kt + 1) * PK);
+#pragma unroll
+    for (int k = 0; k < PK; ++k) {
+      const float* ar = As + (buf * PK + k) * LDA + 4 * tx;
+      const float* br = Bs + (buf * PK + k) * LDB + CV * ty;
+      float a[8], b[CPT];
+      *reinterpret_cast<float4*>(a) = *reinterpret_cast<const float4*>(ar);
+      *reinterpret_cast<float4*>(a + 4) = *reinterpret_cast<const float4*>(ar + 64);
+#pragma unroll
+      for (int c = 0; c < CPT; c += CV) {
+        if constexpr (CV == 4) *reinterpret_cast<float4*>(b + c) = *reinterpret_cast<const float4*>(br + c / CV * 64);
+        else *reinterpret_cast<float2*>(b) = *reinterpret_cast<const float2*>(br);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < CPT; ++c) acc[r][c] = fmaf(a[r], b[c], acc[r][c]);
     }
-    return s;
+    if (kt + 1 < nk) store(buf ^ 1);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
   }
-  const float* a = p.A + (int64_t)i * p.asi;
-  const float* b = p.B + (int64_t)j * p.bsj;
-  for (int k = 0; k < p.K; ++k) s = fmaf(a[k * p.ask], b[k * p.bsk], s);
-  return s;
+#pragma unroll
+  for (int c = 0; c < CPT; ++c) {
+    const int j = n0 + col(c), mb = mark[BM + col(c)];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+      const int i = m0 + row(r);
+      if (i < p.M && j < p.N && careful(mark[row(r)], mb)) {
+        float* cp = p.C + i + (int64_t)j * p.ldc;
+        *cp = fmaf(p.alpha, acc[r][c], *cp);
+      }
+    }
+  }
 }
 
 template <int TN>
@@ -126,6 +206,8 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(drain + 1);
   __shared__ volatile int s_abort;
   __shared__ int s_mark[2 * BM];  // marks of the tile's rows and columns
+  __shared__ int s_lo[8], s_hi[8];  // their extremes by drain warp (of nonzero marks): rows, then columns
+  __shared__ int s_careful, s_tensor;  // whether the tile has outputs for the plain product, and for the tensor cores
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Output tiles are rasterised in groups of 8 tile rows for L2 reuse.
@@ -139,6 +221,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 
   if (threadIdx.x == 0) {
     s_abort = 0;
+    s_careful = s_tensor = 0;
     for (int s = 0; s < F32_STAGES; ++s) {
       umma::mbar_init(umma::smem_u32(&fullA[s]), 1);
       umma::mbar_init(umma::smem_u32(&fullB[s]), 1);
@@ -222,14 +305,34 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 #pragma unroll 4
       for (int kb = 0; kb < p.num_kb; ++kb) m = max(m, t < BM + TN ? mk[(int64_t)kb * step] : 0);
       s_mark[t] = m;
+      const int lo = __reduce_min_sync(0xffffffffu, m ? m : 1024), hi = __reduce_max_sync(0xffffffffu, m);
+      if (lane == 0) s_lo[t >> 5] = lo, s_hi[t >> 5] = hi;
       asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    // Outputs that are left to the plain product, if any: usually the extremes
+    // exclude them.  When they are all of the tile, nothing else is formed.
+    const int lo_a = min(min(s_lo[0], s_lo[1]), min(s_lo[2], s_lo[3])), lo_b = min(min(s_lo[4], s_lo[5]), min(s_lo[6], s_lo[7]));
+    const int hi_a = max(max(s_hi[0], s_hi[1]), max(s_hi[2], s_hi[3])), hi_b = max(max(s_hi[4], s_hi[5]), max(s_hi[6], s_hi[7]));
+    const bool looked = hi_a >= 256 || hi_b >= 256 || lo_a + lo_b < 166 || hi_a + hi_b > 360;
+    if (looked) {
+      bool some = false, others = false;
+      if (i < p.M)
+        for (int j = 0; j < min(HALF, p.N - c0); ++j) {
+          const bool c = careful(s_mark[q * 32 + lane], s_mark[BM + h * HALF + j]);
+          some |= c;
+          others |= !c;
+        }
+      if (some) s_careful = 1;
+      if (others) s_tensor = 1;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+      if (!s_tensor) s_abort = 1;  // the other warps stop: nothing of what they form is used
     }
     float acc[HALF];
 #pragma unroll
     for (int j = 0; j < HALF; ++j) acc[j] = 0.0f;
-    bool ok = true;
+    bool ok = !looked || s_tensor;
     const int nch = (p.num_kb + F32_CHUNK - 1) / F32_CHUNK;
-    for (int ch = 0; ch < nch; ++ch) {
+    for (int ch = 0; ch < nch && ok; ++ch) {
       const int b = ch & 1;
       ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&cfull[b]), (uint32_t)(ch >> 1) & 1u, &s_abort, p.err, 56));
       if (!ok) break;
@@ -251,7 +354,6 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
       const int ma = s_mark[q * 32 + lane];
       const int* mb = s_mark + BM + h * HALF;
       float* C = p.C + i;
-      bool special = false;
 #pragma unroll
       for (int j0 = 0; j0 < HALF; j0 += CB) {
         // All loads of C before the first store (a store may alias a later load).
@@ -262,17 +364,12 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
           const int col = c0 + j0 + j;
           const bool in = i < p.M && col < p.N;
           cv[j] = in ? C[(int64_t)col * p.ldc] : 0.0f;
-          if (!in || careful(ma, mb[j0 + j])) skip |= 1u << j;
-          special |= in && (skip >> j & 1u);
+          if (!in || (looked && careful(ma, mb[j0 + j]))) skip |= 1u << j;
         }
 #pragma unroll
         for (int j = 0; j < CB; ++j)
           if (!(skip >> j & 1u)) C[(int64_t)(c0 + j0 + j) * p.ldc] = fmaf(p.alpha, acc[j0 + j], cv[j]);
       }
-      if (special)
-        for (int col = c0; col < min(c0 + HALF, p.N); ++col)
-          if (i < p.M && careful(ma, mb[col - c0]))
-            C[(int64_t)col * p.ldc] = fmaf(p.alpha, plain_dot(p, i, col), C[(int64_t)col * p.ldc]);
     }
   }
 
@@ -283,6 +380,8 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
     umma::fence_after_sync();
     umma::tmem_dealloc(tmem, 512);
   }
+  // No load or MMA is in flight any more: the ring is free.
+  if (s_careful && warp >= 3) plain_tile<TN>(p, reinterpret_cast<float*>(smem), s_mark, m0, n0);
 }
 
 // ---------------------------------------------------------------------------
@@ -358,6 +457,8 @@ __global__ void __launch_bounds__(256) stage_f32_kernel(const F32Job a, const F3
     const uint32_t um = max(u0, u1);
     int mk = um ? (int)(um >> 24) + 1 : 0;
     mk = __reduce_max_sync(0xffffffffu, mk);
+    const bool tiny = (u0 && (int)(u0 >> 24) + 1 < MARK_LOW) || (u1 && (int)(u1 >> 24) + 1 < MARK_LOW);
+    if (__any_sync(0xffffffffu, tiny)) mk |= MARK_TINY;
     if (lane == 0) j.mark[(int64_t)blockIdx.y * (j.blocks * 32) + gi] = mk;
   }
 }
