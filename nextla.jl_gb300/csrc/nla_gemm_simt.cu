@@ -12,6 +12,8 @@
 // Tiles are double-buffered in shared memory with a register prefetch of the
 // next K slab.  Operand loads are layout-aware: threads run along whichever
 // index is contiguous in memory for op(A) = A or A^T.
+#include <limits>
+
 #include "nla_common.cuh"
 
 namespace nla {
@@ -157,8 +159,10 @@ int launch_simt(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A, con
 
 // The time of a tiling in units of one output element's share of an SM's
 // FMAs: waves times (tile elements times the tile's cost per element plus a
-// fixed part per tile).
+// fixed part per tile).  Infinite where the columns' tiles exceed a grid's
+// 65535, so that the widest tiling takes the most columns.
 double tiling_cost(int64_t N, int64_t M, int bm, int bn, double per_element, double fixed) {
+  if ((M + bn - 1) / bn > 65535) return std::numeric_limits<double>::infinity();
   const int64_t tiles = ((N + bm - 1) / bm) * ((M + bn - 1) / bn), sms = num_sms();
   return (double)((tiles + sms - 1) / sms) * ((double)bm * bn * per_element + fixed);
 }
@@ -173,7 +177,7 @@ int launch_simt_f64(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A,
   const double c64 = tiling_cost(N, M, 64, 64, 1.0, 64.0), c32 = tiling_cost(N, M, 32, 32, 1.0, 64.0),
                c16 = tiling_cost(N, M, 32, 16, 1.0, 64.0);
   if (c64 <= c32 && c64 <= c16) return launch_simt<T, 2, 4, 16>(N, M, K, alpha, A, B, C, s);
-  if (c32 <= c16 || M > 65535 * 16ll) return launch_simt<T, 1, 2, 32>(N, M, K, alpha, A, B, C, s);
+  if (c32 <= c16) return launch_simt<T, 1, 2, 32>(N, M, K, alpha, A, B, C, s);
   return launch_simt<T, 1, 1, 32>(N, M, K, alpha, A, B, C, s);
 }
 
@@ -186,7 +190,7 @@ int launch_simt_f32(int64_t N, int64_t M, int64_t K, double alpha, const Mat& A,
   const double c128 = tiling_cost(N, M, 128, 128, 1.0, 1024.0), c64 = tiling_cost(N, M, 64, 64, 1.4, 1024.0),
                c32 = tiling_cost(N, M, 32, 32, 3.0, 1024.0);
   if (c128 <= c64 && c128 <= c32) return launch_simt<T, 4, 8, 8>(N, M, K, alpha, A, B, C, s);
-  if (c64 <= c32 || M > 65535 * 32ll) return launch_simt<T, 2, 4, 16>(N, M, K, alpha, A, B, C, s);
+  if (c64 <= c32) return launch_simt<T, 2, 4, 16>(N, M, K, alpha, A, B, C, s);
   return launch_simt<T, 1, 2, 32>(N, M, K, alpha, A, B, C, s);
 }
 
