@@ -581,11 +581,11 @@ __global__ void __launch_bounds__(NT, 2) batched_node_kernel(Args a) {
 // takes a group (longest first, from the same kind of device counter) and
 // solves it block row by block row, left-looking: block rows of at most 64
 // rows, each X[r0 ..] = inv(L) (alpha B[r0 ..] - A[r0 .., 0 .. r0) X[0 .. r0))
-// with the product accumulated in registers over all of K, so that every
-// element of B is read and written once.
+// with the product accumulated in registers (GROUP_SUM values of K at a time),
+// so that every element of B is read and written once.
 // Bound by the products (3.4 of 6.1 ms for 10,000 Float32 systems of 16 to
 // 1024 unknowns, whose FMAs alone would take 1.5), the blocks' loads and the
-// triangles (1.4).  Against the node queue: 10,000 systems 7.00 -> 6.36 ms,
+// triangles (1.4).  Against the node queue: 10,000 systems 7.00 -> 6.50 ms,
 // 3000 2.09 -> 1.88; at 1000 the longest group would exceed a CTA's share.
 // ---------------------------------------------------------------------------
 struct GroupItem {
@@ -607,6 +607,11 @@ struct GroupArgs {
 // Chunk buffers: three chunks of copies in flight (Float32), or one (Float64,
 // whose products take longer than a copy and whose buffers are twice as large).
 __host__ __device__ constexpr int group_stages(int esz) { return esz == 8 ? 2 : 4; }
+
+// Values of K per partial sum: one chain of FMAs over all of K rounds worse
+// than the recursion's separate updates (Float32 error of 10,000 systems
+// 1.20e-7 against 1.12e-7, with partial sums 1.1e-7; 6.36 -> 6.50 ms).
+constexpr int GROUP_SUM = 256;
 
 template <typename Tc, int W>
 __host__ __device__ constexpr size_t group_elems() {
@@ -709,14 +714,16 @@ __device__ void run_group(const GroupArgs& a, const GroupItem& it, void* smem) {
       for (int u = 0; u < B_PER; ++u) Xs[xr * XP + xcb + u * (NT / MAX_ROWS)] = scaled_node<T>(vb[u], a.alpha);
     }
 
-    if (r0 > 0) {
+    int buf = 0;
+#pragma unroll 1
+    for (int s0 = 0; s0 < r0; s0 += GROUP_SUM) {
+      const int s1 = min(s0 + GROUP_SUM, r0);
       Tc acc[RT][CT];
 #pragma unroll
       for (int i = 0; i < RT; ++i)
 #pragma unroll
         for (int c = 0; c < CT; ++c) acc[i][c] = Tc(0);
-      int buf = 0;
-      for (int k0 = 0; k0 < r0; k0 += KC, buf = buf + 1 == ST ? 0 : buf + 1) {
+      for (int k0 = s0; k0 < s1; k0 += KC, buf = buf + 1 == ST ? 0 : buf + 1) {
         const Tc* Ab = As + buf * KC * AP;
         const Tc* Xb = Xk + buf * KC * XP;
         asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
@@ -736,9 +743,17 @@ __device__ void run_group(const GroupArgs& a, const GroupItem& it, void* smem) {
         }
       }
 #pragma unroll
-      for (int i = 0; i < RT; ++i)
+      for (int i = 0; i < RT; ++i) {
+        Tc* x = Xs + (RT * tr + i) * XP + tc * CT;
+        if constexpr (CT == 4) {
+          Tc v[CT];
+          lds_vec<CT>(x, v);
+          sts4(x, v[0] - acc[i][0], v[1] - acc[i][1], v[2] - acc[i][2], v[3] - acc[i][3]);
+        } else {
 #pragma unroll
-        for (int c = 0; c < CT; ++c) Xs[(RT * tr + i) * XP + tc * CT + c] -= acc[i][c];
+          for (int c = 0; c < CT; ++c) x[c] -= acc[i][c];
+        }
+      }
     }
     __syncthreads();
     solve_panels<Tc, W>(Ls, Xs, inv, rows, ncols);
