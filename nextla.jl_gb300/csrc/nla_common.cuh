@@ -258,7 +258,6 @@ CrtStaged crt_layout(void* buf, int64_t rows, int64_t K, int tri, bool row_opera
 int crt_stage(const Mat& X, const CrtStaged& sx, const Mat* Y, const CrtStaged* sy, cudaStream_t s);
 int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C, uint8_t* planes, cudaStream_t s,
              const ResidualTerm* res = nullptr, bool d_col = false);
-int crt_set_wait_limit(uint64_t ns);
 bool crt_enabled();                                           // NLA_EXACT_KERNEL selects the slice kernels instead
 size_t crt_workspace_bytes(int64_t M, int64_t N, int64_t K);  // staged operands and planes of one update
 int workspace_get(cudaStream_t s, size_t bytes, void** out);

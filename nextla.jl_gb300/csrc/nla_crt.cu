@@ -836,11 +836,6 @@ void stage_job(const Mat& X, const CrtStaged& st, Job* j) {
 
 }  // namespace
 
-int crt_set_wait_limit(uint64_t ns) {
-  const cudaError_t e = cudaMemcpyToSymbol(umma::g_wait_limit_ns, &ns, sizeof(ns));
-  return e == cudaSuccess ? NLA_OK : cuda_status(e, "set wait limit");
-}
-
 bool crt_usable(int64_t M, int64_t N, int64_t K) {
   return K <= MAX_K && M <= (1 << 24) && N <= (1 << 24) && L * pad_to(M, BU) < INT32_MAX && L * pad_to(N, BU) < INT32_MAX &&
          pad_to(M, BU) / BU * (pad_to(N, BU) / BU) * L < INT32_MAX && N <= (int64_t)65535 * 8 * FIN_COLS;

@@ -1903,13 +1903,25 @@ int launch_exact_gemm(const Staged& A, const Staged& B, double alpha, const Mat&
 
 namespace {
 std::atomic<uint64_t> g_wait_limit_host{umma::WAIT_LIMIT_NS};
+// The translation units' setters, in a function so that it exists before the
+// first unit registers.
+std::vector<cudaError_t (*)(uint64_t)>& wait_limit_setters() {
+  static std::vector<cudaError_t (*)(uint64_t)> v;
+  return v;
+}
+}  // namespace
+
+bool register_wait_limit(cudaError_t (*set)(uint64_t)) {
+  wait_limit_setters().push_back(set);
+  return true;
 }
 
 int set_wait_limit(uint64_t ns) {
   const uint64_t v = ns == 0 ? umma::WAIT_LIMIT_NS : ns;
-  const cudaError_t e = cudaMemcpyToSymbol(umma::g_wait_limit_ns, &v, sizeof(v));
-  if (e != cudaSuccess) return cuda_status(e, "set wait limit");
-  NLA_TRY(crt_set_wait_limit(v));
+  for (auto set : wait_limit_setters()) {
+    const cudaError_t e = set(v);
+    if (e != cudaSuccess) return cuda_status(e, "set wait limit");
+  }
   g_wait_limit_host.store(v);
   return NLA_OK;
 }

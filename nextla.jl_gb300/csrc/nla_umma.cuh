@@ -7,6 +7,8 @@
 #include <stdint.h>
 
 namespace nla {
+bool register_wait_limit(cudaError_t (*set)(uint64_t));  // nla_umma.cu
+
 namespace umma {
 
 // A bounded wait gives up after this many nanoseconds of %globaltimer.
@@ -55,8 +57,13 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // Limit of the waits that honour aborts (the pipeline waits between the
 // roles of a CTA): WAIT_LIMIT_NS unless nla_set_wait_limit_ns changed it.
 // The waits that drain a CTA's own in-flight work before it exits always use
-// WAIT_LIMIT_NS.
+// WAIT_LIMIT_NS.  Every translation unit has its own copy, which registers
+// itself so that set_wait_limit reaches them all.
 static __device__ uint64_t g_wait_limit_ns = WAIT_LIMIT_NS;
+static cudaError_t set_unit_wait_limit(uint64_t ns) {
+  return cudaMemcpyToSymbol(g_wait_limit_ns, &ns, sizeof(ns));
+}
+static const bool g_wait_limit_registered = register_wait_limit(set_unit_wait_limit);
 
 // Wait for the phase with the given parity to complete.  Returns false (and
 // raises *abort and the device error word) if the wait runs past the limit
