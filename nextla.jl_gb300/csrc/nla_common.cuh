@@ -259,7 +259,18 @@ int crt_stage(const Mat& X, const CrtStaged& sx, const Mat* Y, const CrtStaged* 
 int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C, uint8_t* planes, cudaStream_t s,
              const ResidualTerm* res = nullptr, bool d_col = false);
 bool crt_enabled();                                           // NLA_EXACT_KERNEL selects the slice kernels instead
-size_t crt_workspace_bytes(int64_t M, int64_t N, int64_t K);  // staged operands and planes of one update
+// An update's residues in panels: one operand staged whole, the other (its
+// columns of C with cols, else its rows) `width` at a time, in `bytes` of
+// scratch in all, at most budget unless the narrowest panel takes more.  The
+// results are the same bits for every width.
+struct CrtPanels {
+  bool cols;
+  int64_t width;
+  size_t bytes;
+};
+CrtPanels crt_panels(bool cols, int64_t M, int64_t N, int64_t K, size_t budget);
+size_t crt_budget(size_t slices_bytes, size_t held);
+CrtPanels crt_update_panels(int64_t M, int64_t N, int64_t K, cudaStream_t s);  // in the library's workspace
 int workspace_get(cudaStream_t s, size_t bytes, void** out);
 int device_status(cudaStream_t s);
 int* device_error_word();  // device address of the error word nla_device_status reads (null on failure)

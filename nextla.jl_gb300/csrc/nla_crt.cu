@@ -846,6 +846,32 @@ size_t crt_staged_bytes(int64_t rows, int64_t K) {
 }
 size_t crt_planes_bytes(int64_t M, int64_t N) { return (size_t)L * (size_t)pad_to(M, BU) * (size_t)N; }
 
+// Residues take 32 bytes per element and the planes 16 per element of C,
+// against the slices' 14 and 8, and the workspaces are kept between calls: a
+// whole 16384 x 16384 solve held 8.6 GB instead of 3.9.  So residues are
+// formed in panels within what slices would take (or the stream holds already,
+// or 1 GiB).  That solve takes 72.0 ms whole and 72.4 in panels.
+constexpr int64_t PANEL_MIN = 1024;
+CrtPanels crt_panels(bool cols, int64_t M, int64_t N, int64_t K, size_t budget) {
+  const int64_t dim = cols ? N : M;
+  const size_t fixed = crt_staged_bytes(cols ? M : N, K) + 1024;
+  auto need = [&](int64_t w) {
+    return fixed + crt_staged_bytes(w, K) + (cols ? crt_planes_bytes(M, w) : crt_planes_bytes(w, N));
+  };
+  if (dim <= PANEL_MIN || need(dim) <= budget) return {cols, dim, need(dim)};
+  int64_t w = PANEL_MIN;
+  while (w + PANEL_MIN < dim && need(w + PANEL_MIN) <= budget) w += PANEL_MIN;
+  const int64_t panels = (dim + w - 1) / w;
+  w = pad_to((dim + panels - 1) / panels, 256);  // of about equal width
+  return {cols, w, need(w)};
+}
+
+size_t crt_budget(size_t slices_bytes, size_t held) {
+  constexpr size_t FLOOR = (size_t)1 << 30;
+  const size_t b = slices_bytes > held ? slices_bytes : held;
+  return b > FLOOR ? b : FLOOR;
+}
+
 CrtStaged crt_layout(void* buf, int64_t rows, int64_t K, int tri, bool row_operand) {
   CrtStaged st;
   st.res = buf;

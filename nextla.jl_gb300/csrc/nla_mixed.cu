@@ -1099,28 +1099,26 @@ int leaf_pair_apply(const RecPlan& c, const Mat& A, int64_t n, const Mat& B) {
 // residues (nla_crt.cu) or, where there is no memory for them, as slices.
 struct SplitResidual {
   bool crt = false;
+  CrtPanels panels{};
   uint8_t* base = nullptr;  // op(A), then X, then the planes of the residues
   Staged As{}, Xs{};
   CrtStaged Ac{};
 };
 
-size_t split_residual_bytes(bool crt, char side, int64_t n, int64_t m) {
-  if (!crt) return staged_bytes(n, n, EXACT_SLICES) + staged_bytes(m, n, EXACT_SLICES) + 1024;
-  return crt_staged_bytes(n, n) + crt_staged_bytes(m, n) + (side == 'L' ? crt_planes_bytes(n, m) : crt_planes_bytes(m, n)) +
-         1024;
-}
-
 // The refinement buffers with `extra` bytes before the residual's, which
 // start at the next multiple of 1024.
 int split_residual_buffers(cudaStream_t s, size_t extra, char side, int64_t n, int64_t m, void** buf, SplitResidual* r) {
   extra = (extra + 1023) & ~(size_t)1023;
-  r->crt = crt_enabled() && (side == 'L' ? crt_usable(n, m, n) : crt_usable(m, n, n));
-  int rc = refine_buffers(s, extra + split_residual_bytes(r->crt, side, n, m), buf);
+  const bool L = side == 'L';
+  const size_t slices = staged_bytes(n, n, EXACT_SLICES) + staged_bytes(m, n, EXACT_SLICES) + 1024;
+  r->crt = crt_enabled() && (L ? crt_usable(n, m, n) : crt_usable(m, n, n));
+  r->panels = crt_panels(L, L ? n : m, L ? m : n, n, crt_budget(slices, 0));
+  int rc = refine_buffers(s, extra + (r->crt ? r->panels.bytes : slices), buf);
   if (rc != NLA_OK && r->crt) {
     cudaGetLastError();
     clear_error();
     r->crt = false;
-    rc = refine_buffers(s, extra + split_residual_bytes(false, side, n, m), buf);
+    rc = refine_buffers(s, extra + slices, buf);
   }
   r->base = static_cast<uint8_t*>(*buf) + extra;
   return rc;
@@ -1143,17 +1141,22 @@ int stage_triangle(const Mat& Am, int64_t n, char side, char uplo, SplitResidual
 // rounding (R = alpha*B on entry).
 int split_residual(const Mat& Am, char side, int64_t n, int64_t m, const Mat& Xm, const Mat& Rm, SplitResidual* r,
                    cudaStream_t s) {
-  const ResidualTerm term{static_cast<const double*>(Xm.p), Xm.ld, static_cast<const double*>(Am.p), Am.ld + 1};
+  ResidualTerm term{static_cast<const double*>(Xm.p), Xm.ld, static_cast<const double*>(Am.p), Am.ld + 1};
   // X as rows along K: its columns for side L, its rows for side R.
   const Mat X = side == 'L' ? transposed(Xm) : Xm;
   if (r->crt) {
     uint8_t* xbuf = r->base + crt_staged_bytes(n, n);
-    uint8_t* planes = xbuf + crt_staged_bytes(m, n);
-    const CrtStaged Xc = crt_layout(xbuf, m, n, 0, false);
-    NLA_TRY(crt_stage(X, Xc, nullptr, nullptr, s));
-    // Side R: X op(A) = X (op(A)^T)^T, so the triangle is the column operand.
-    if (side == 'L') return crt_gemm(r->Ac, Xc, -1.0, Rm, planes, s, &term, false);
-    return crt_gemm(Xc, r->Ac, -1.0, Rm, planes, s, &term, true);
+    for (int64_t o = 0; o < m; o += r->panels.width) {
+      const int64_t w = m - o < r->panels.width ? m - o : r->panels.width;
+      uint8_t* planes = xbuf + crt_staged_bytes(w, n);
+      const CrtStaged Xc = crt_layout(xbuf, w, n, 0, false);
+      NLA_TRY(crt_stage(sub(X, o, 0, NLA_F64), Xc, nullptr, nullptr, s));
+      term.x = static_cast<const double*>(Xm.p) + (side == 'L' ? o * Xm.ld : o);
+      // Side R: X op(A) = X (op(A)^T)^T, so the triangle is the column operand.
+      if (side == 'L') NLA_TRY(crt_gemm(r->Ac, Xc, -1.0, sub(Rm, 0, o, NLA_F64), planes, s, &term, false));
+      else NLA_TRY(crt_gemm(Xc, r->Ac, -1.0, sub(Rm, o, 0, NLA_F64), planes, s, &term, true));
+    }
+    return NLA_OK;
   }
   NLA_TRY(stage_operand(X, m, n, NLA_F64, EXACT_SLICES, true, 0, r->base + staged_bytes(n, n, EXACT_SLICES), &r->Xs, s,
                         false));
@@ -1196,7 +1199,7 @@ int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m
   if (n <= c->threshold) return NLA_OK;
   const int64_t rows_c = side == 'L' ? big : m, cols_c = side == 'L' ? m : big;
   if (opts.split_terms == EXACT_SLICES && crt_enabled() && crt_usable(rows_c, cols_c, big) &&
-      workspace_get(s, crt_workspace_bytes(rows_c, cols_c, big), &ws) == NLA_OK)
+      workspace_get(s, crt_update_panels(rows_c, cols_c, big, s).bytes, &ws) == NLA_OK)
     return NLA_OK;
   cudaGetLastError();
   clear_error();

@@ -1488,10 +1488,6 @@ bool crt_enabled() {
   return on;
 }
 
-size_t crt_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  return crt_staged_bytes(M, K) + crt_staged_bytes(N, K) + crt_planes_bytes(M, N) + 1024;
-}
-
 // Scratch of the plain path: stream-ordered allocations from a pool of their
 // own, which keeps up to SCRATCH_KEEP bytes between calls (the default pool
 // would give everything back at each synchronisation).
@@ -1536,10 +1532,22 @@ void scratch_free(cudaStream_t s, void* p) {
   if (p) cudaFreeAsync(p, s);
 }
 
-int workspace_get(cudaStream_t s, size_t bytes, void** out) {
+namespace {
+uint64_t pool_key(cudaStream_t s) {
   int dev = 0;
   cudaGetDevice(&dev);
-  const uint64_t key = ((uint64_t)(uint32_t)dev << 48) ^ (uint64_t)reinterpret_cast<uintptr_t>(s);
+  return ((uint64_t)(uint32_t)dev << 48) ^ (uint64_t)reinterpret_cast<uintptr_t>(s);
+}
+size_t workspace_held(cudaStream_t s) {
+  const uint64_t key = pool_key(s);
+  std::lock_guard<std::mutex> lk(g_pool_mu);
+  const auto it = g_pools.find(key);
+  return it == g_pools.end() ? 0 : it->second.size;
+}
+}  // namespace
+
+int workspace_get(cudaStream_t s, size_t bytes, void** out) {
+  const uint64_t key = pool_key(s);
   std::lock_guard<std::mutex> lk(g_pool_mu);
   Pool& p = g_pools[key];
   if (p.size < bytes) {
@@ -1700,6 +1708,12 @@ size_t sliced_workspace_bytes(int64_t M, int64_t N, int64_t K, int S) {
   return staged_bytes(M, K, S) + staged_bytes(N, K, S) + 1024 + (S == EXACT_SLICES ? fixed_sums_bytes(M, N) : 0);
 }
 
+// The panels of one exact update: along the longer side of C, whose operand
+// is then the one that is staged in parts.
+CrtPanels crt_update_panels(int64_t M, int64_t N, int64_t K, cudaStream_t s) {
+  return crt_panels(N >= M, M, N, K, crt_budget(sliced_workspace_bytes(M, N, K, EXACT_SLICES), workspace_held(s)));
+}
+
 // One tensor-core update.  in_dtype is NLA_F64 (split into S slices of BF16
 // or FP16) or NLA_F16 (S = 1, staged as is).  out_dtype is NLA_F64 or NLA_F16.
 int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat& A, const Mat& B, const Mat& C,
@@ -1714,13 +1728,21 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
     if (out_dtype != NLA_F64) return fail(NLA_ERR_DTYPE, "exact updates produce Float64");
     void* base = ws;
     if (base == nullptr && crt_enabled() && crt_usable(M, N, K)) {
-      if (workspace_get(s, crt_workspace_bytes(M, N, K), &base) == NLA_OK) {
-        const CrtStaged a = crt_layout(base, M, K, 0, true);
-        const CrtStaged b = crt_layout(static_cast<uint8_t*>(base) + crt_staged_bytes(M, K), N, K, 0, false);
-        const Mat Bt = transposed(B);
-        NLA_TRY(crt_stage(A, a, &Bt, &b, s));
-        return crt_gemm(a, b, alpha, C,
-                        static_cast<uint8_t*>(base) + crt_staged_bytes(M, K) + crt_staged_bytes(N, K), s);
+      const CrtPanels pan = crt_update_panels(M, N, K, s);
+      if (workspace_get(s, pan.bytes, &base) == NLA_OK) {
+        const int64_t dim = pan.cols ? N : M;
+        uint8_t* second = static_cast<uint8_t*>(base) + crt_staged_bytes(pan.cols ? M : N, K);
+        for (int64_t o = 0; o < dim; o += pan.width) {
+          const int64_t w = dim - o < pan.width ? dim - o : pan.width, m = pan.cols ? M : w, n = pan.cols ? w : N;
+          const CrtStaged a = crt_layout(pan.cols ? base : second, m, K, 0, true);
+          const CrtStaged b = crt_layout(pan.cols ? second : base, n, K, 0, false);
+          const Mat Ap = pan.cols ? A : sub(A, o, 0, NLA_F64), Bt = transposed(pan.cols ? sub(B, 0, o, NLA_F64) : B);
+          if (o == 0) NLA_TRY(crt_stage(A, a, &Bt, &b, s));
+          else NLA_TRY(pan.cols ? crt_stage(Bt, b, nullptr, nullptr, s) : crt_stage(Ap, a, nullptr, nullptr, s));
+          NLA_TRY(crt_gemm(a, b, alpha, pan.cols ? sub(C, 0, o, NLA_F64) : sub(C, o, 0, NLA_F64),
+                           second + crt_staged_bytes(w, K), s));
+        }
+        return NLA_OK;
       }
       cudaGetLastError();  // too little memory for the residues: the slices take less
       clear_error();
