@@ -6,6 +6,7 @@
 // The canonical-form mapping and the column-per-thread Float64 solve are in
 // nla_leaf.cuh, the strip kernel that runs every other block in
 // nla_leaf_strip.cuh.
+#include <algorithm>
 #include <cstdlib>
 #include <mutex>
 #include <type_traits>
@@ -113,6 +114,145 @@ int launch_strip(const LeafArgs& g, cudaStream_t s) {
   return NLA_OK;
 }
 
+// Blocks of few rows with very many right-hand sides: one right-hand side per
+// thread, its column in shared memory, four rows at a time in registers.  Every
+// FMA is one of the triangle's (a strip's lanes each form a whole panel, which
+// for few rows is mostly wasted), and rows are formed with k increasing.
+constexpr int COL_T = 64;  // right-hand sides and threads per CTA
+constexpr int COL_P = COL_T + 1;
+// The block in packed rows of four: L(i, k), k <= i | 3, at col_at(i, k).
+__host__ __device__ constexpr int col_at(int i, int k) { return 8 * (i >> 2) * ((i >> 2) + 1) + 4 * k + (i & 3); }
+constexpr size_t column_smem_elems(int n) {
+  const int nr = (n + 3) & ~3;
+  return (size_t)col_at(nr, 0) + (size_t)nr * COL_P + 2 * nr;  // the block, X, the diagonal, its reciprocals
+}
+
+template <typename T, bool SOLVE>
+__global__ void __launch_bounds__(COL_T) leaf_column_kernel(const LeafArgs g) {
+  using Tc = typename Elem<T>::compute;
+  using Vec = typename StripTraits<Tc>::Vec;
+  using Mx = StripMath<Tc>;
+  constexpr int VK = StripTraits<Tc>::VK;
+  chain_begin();
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int n = g.n, nr = (n + 3) & ~3, t = threadIdx.x;
+  Tc* L = reinterpret_cast<Tc*>(smem_raw);
+  Tc* X = L + col_at(nr, 0);  // X(i, c) at X[i COL_P + c]
+  Tc* dia = X + nr * COL_P;
+  Tc* inv = dia + nr;
+  const int64_t c0 = (int64_t)blockIdx.x * COL_T;
+  const int ncols = (int)(g.m - c0 < COL_T ? g.m - c0 : COL_T);
+  const int64_t sk = (g.tA ? 1 : g.lda) * (g.rev ? -1 : 1), si = (g.tA ? g.lda : 1) * (g.rev ? -1 : 1);
+  const T* A = static_cast<const T*>(g.A) + (g.rev ? (int64_t)(n - 1) * (g.lda + 1) : 0);
+  const int64_t bi = (g.tB ? g.ldb : 1) * (g.rev ? -1 : 1), bc = g.tB ? 1 : g.ldb;
+  T* B = static_cast<T*>(g.B) + (g.rev ? (int64_t)(n - 1) * (g.tB ? g.ldb : 1) : 0) + c0 * bc;
+
+  for (int idx = t; idx < nr * nr; idx += COL_T) {
+    const int i = g.tA ? idx / nr : idx % nr, k = g.tA ? idx % nr : idx / nr;
+    if (k <= (i | 3)) L[col_at(i, k)] = i < n && k < i ? Mx::conj_if(Elem<T>::load(A + i * si + k * sk), g.cj) : Mx::zero();
+  }
+  for (int i = t; i < nr; i += COL_T) {
+    const Tc d = g.unit || i >= n ? Mx::one() : Mx::conj_if(Elem<T>::load(A + i * (si + sk)), g.cj);
+    dia[i] = d;
+    inv[i] = Mx::inverse(d);
+  }
+  // B along its contiguous index, eight loads in flight per thread.
+  constexpr int BATCH = 8;
+  auto at = [&](int idx, int& i, int& c) { g.tB ? (i = idx / COL_T, c = idx % COL_T) : (c = idx / nr, i = idx % nr); };
+  for (int i0 = t; i0 < nr * COL_T; i0 += COL_T * BATCH) {
+    T v[BATCH];
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) {
+      int i, c;
+      at(i0 + COL_T * u, i, c);
+      v[u] = i < n && c < ncols ? B[i * bi + c * bc] : raw_zero<T>();
+    }
+#pragma unroll
+    for (int u = 0; u < BATCH; ++u) {
+      int i, c;
+      at(i0 + COL_T * u, i, c);
+      if (i0 + COL_T * u < nr * COL_T) X[i * COL_P + c] = Elem<T>::load(&v[u]);
+    }
+  }
+  __syncthreads();
+  Tc* x = X + t;
+  for (int b = 0; b < nr; b += 4) {
+    const int r0 = SOLVE ? b : nr - 4 - b;
+    Tc z[4], y[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      y[i] = x[(r0 + i) * COL_P];
+      z[i] = SOLVE ? y[i] : Mx::zero();
+    }
+#pragma unroll 4
+    for (int k = 0; k < r0; ++k) {
+      Tc l[4];
+#pragma unroll
+      for (int i = 0; i < 4; i += VK) st_unpack(*reinterpret_cast<const Vec*>(L + col_at(r0, k) + i), l + i);
+      const Tc xk = x[k * COL_P];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) z[i] = SOLVE ? Mx::fms_(l[i], xk, z[i]) : Mx::fma_(l[i], xk, z[i]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (SOLVE) y[j] = Mx::divided(z[j], inv[r0 + j], dia[r0 + j]);
+#pragma unroll
+      for (int i = j + 1; i < 4; ++i) {
+        const Tc l = L[col_at(r0 + i, r0 + j)];
+        z[i] = SOLVE ? Mx::fms_(l, y[j], z[i]) : Mx::fma_(l, y[j], z[i]);
+      }
+      x[(r0 + j) * COL_P] = SOLVE ? y[j] : Mx::fma_(dia[r0 + j], y[j], z[j]);
+    }
+  }
+  __syncthreads();
+  for (int idx = t; idx < nr * COL_T; idx += COL_T) {
+    int i, c;
+    at(idx, i, c);
+    if (i < n && c < ncols) Elem<T>::store(B + i * bi + c * bc, X[i * COL_P + c]);
+  }
+}
+
+template <typename T, bool SOLVE>
+int launch_column(const LeafArgs& g, cudaStream_t s) {
+  using Tc = typename Elem<T>::compute;
+  const size_t smem = column_smem_elems(g.n) * sizeof(Tc);
+  const int64_t grid = (g.m + COL_T - 1) / COL_T;
+  if (grid > 2147483647LL) return fail(NLA_ERR_UNSUPPORTED, "leaf: too many right-hand sides");
+  static std::once_flag once;
+  static cudaError_t st = cudaSuccess;
+  std::call_once(once, [] {
+    st = cudaFuncSetAttribute(leaf_column_kernel<T, SOLVE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)STRIP_SMEM_MAX);
+  });
+  if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(leaf_column_kernel)");
+  TraceScope trace(SOLVE ? NLA_K_LEAF_SOLVE : NLA_K_LEAF_MULT, s, (double)g.n * g.n * (double)g.m,
+                   (double)sizeof(T) * ((double)g.n * (g.n + 1) / 2 + 2.0 * (double)g.n * g.m));
+  leaf_column_kernel<T, SOLVE><<<(unsigned)grid, COL_T, smem, s>>>(g);
+  NLA_CHECK_LAUNCH("leaf_column_kernel");
+  return NLA_OK;
+}
+
+// Right-hand sides per SM from which a block of n rows is faster one column
+// per thread: a CTA of columns takes its time whether or not the others are
+// there, until they fill the SMs, while strips' time grows with their number.
+// Blocks of more rows stay on strips, whose products reuse A.  Measured on 152
+// SMs, strips against columns, us (solve): Float64 n = 16 28 / 24 at m = 6000,
+// 137 / 45 at 100000, n = 48 65 / 73 at 8000, 84 / 73 at 12000; Float32 n = 32
+// 22 / 26 at 8000, 33 / 26 at 20000, 71 / 34 at 100000; ComplexF32 n = 32
+// 37 / 41 at 12000, 163 / 73 at 100000; ComplexF64 n = 16 56 / 76 at 4000,
+// 83 / 77 at 6000, 900 / 278 at 100000, n = 64 502 / 483 at 12000, 4114 / 2666
+// at 100000.
+template <typename Tc, bool SOLVE>
+int64_t column_from(int64_t n) {
+  constexpr bool CX = !std::is_floating_point<Tc>::value;
+  constexpr bool F64 = sizeof(Tc) == (CX ? 16 : 8);
+  const int64_t never = INT32_MAX;
+  if (CX && F64) return SOLVE ? (n <= 64 ? 14 + n : never) : n <= 48 ? 40 + n * 5 / 4 : never;
+  if (CX) return n > 48 ? never : SOLVE ? std::min<int64_t>(5 + 3 * n, 105) : std::min<int64_t>(35 + n * 3 / 2, 85);
+  if (F64) return SOLVE ? (n <= 64 ? 22 + n * 15 / 16 : never) : n <= 32 ? 30 + 3 * n : never;
+  return n > 48 ? never : SOLVE ? 45 + n * 3 / 2 : 75 + n * 9 / 8;
+}
+
 // Right-hand sides per CTA: the width with the least ceil(CTAs / SMs) *
 // (width + c), where c is a strip's fixed time (the triangles' chains and
 // the staging of A) in columns' worth of its product: about one column in
@@ -130,6 +270,7 @@ int launch_strips(const LeafArgs& g, cudaStream_t s) {
   constexpr bool F64 = sizeof(Tc) == (CX ? 16 : 8);
   constexpr int WIDEST = F64 ? (CX ? 16 : 32) : (CX ? 32 : 64);
   const int64_t sms = num_sms(), c = F64 ? 1 : CX ? 8 : 32;
+  if (g.m > sms * column_from<Tc, SOLVE>(g.n)) return launch_column<T, SOLVE>(g, s);
   // Warps on 32 and 64 columns.  Float32 products wait for shared memory with
   // two warps per scheduler; a second K group gives it four (and costs one
   // sum through shared memory per panel): solve 256 x 8192 47.9 -> 44.4 us,
@@ -200,16 +341,20 @@ int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m
   if (B.t) return fail(NLA_ERR_UNSUPPORTED, "diag block: transposed B view");
   const LeafArgs g = leaf_args(side, uplo, n, m, A, B, unit);
   if (func == 'S') {
-    // Float64 blocks of up to 128 rows where one wave of wide CTAs fits and
+    // Float64 blocks of 49 to 128 rows where one wave of wide CTAs fits and
     // strips of 32 columns would leave the last wave short: one right-hand
-    // side per thread, or two threads per right-hand side.  Measured at
-    // n = 64 (128) on 152 SMs, strips against columns: m = 8192 58 (174)
-    // against 70 (214) us, 14336 73 (235) against 78 (250), 16384 97 (315)
-    // against 83 (276), 20000 116 (383) against 174 (600).
+    // side per thread, or two threads per right-hand side; from 113 rows also
+    // where several waves are three quarters full.  Measured at n = 64 (128)
+    // on 152 SMs, strips against columns, us: m = 8192 88 (219) against 86
+    // (229), 12000 111 (300) against 92 (265), 16000 144 (391) against 98 (290),
+    // 20000 162 (484) against 187 (617), 30000 235 (675) against 188 (616),
+    // 100000 662 (1961) against 534 (1822); at 64 rows the kernel of one thread
+    // per right-hand side and 64 to a CTA takes the last two (168 and 480).
     // (NLA_LEAF_COLS=0 turns it off, NLA_LEAF_CW pins a width from m = 1024.)
-    const int64_t sms = num_sms();
+    const int64_t sms = num_sms(), wave = 128 * sms, waves = (m + wave - 1) / wave;
     const bool pinned = getenv("NLA_LEAF_CW") != nullptr && m >= 8 * LEAF_THREADS;
-    if (dtype == NLA_F64 && n <= COLS_MAX_N && ((m > 96 * sms && m <= 128 * sms) || pinned) && leaf_cols_mode() != 0)
+    const bool full = waves == 1 ? n > 48 && m > 68 * sms : n > 112 && 4 * m > 3 * wave * waves;
+    if (dtype == NLA_F64 && n <= COLS_MAX_N && (full || pinned) && leaf_cols_mode() != 0)
       return leaf_cols_mode() == 1 ? launch_leaf_cols<1, LEAF_THREADS>(g, s) : launch_leaf_cols2(g, s);
   }
   const bool S = func == 'S';

@@ -78,6 +78,7 @@ template <typename Tc> struct StripMath {
   __device__ static Tc inverse(Tc d) { return Tc(1) / d; }
   // z / d with inv = 1 / d.
   __device__ static Tc quotient(Tc z, Tc inv, Tc) { return z * inv; }
+  __device__ static Tc divided(Tc z, Tc inv, Tc) { return z * inv; }
 };
 template <typename R> struct StripMath<cx::cpx<R>> {
   using Tc = cx::cpx<R>;
@@ -100,7 +101,7 @@ template <typename R> struct StripMath<cx::cpx<R>> {
     return cx::fma_c(cx::fms_c(q, d, z), inv, q);
   }
   __device__ static bool finite(Tc a) { return isfinite(a.re) && isfinite(a.im); }
-  __device__ __noinline__ static Tc divided(Tc z, Tc d) { return cx::div(z, d); }
+  __device__ __noinline__ static Tc divided(Tc z, Tc, Tc d) { return cx::div(z, d); }
 };
 
 template <typename T> __device__ __forceinline__ T raw_zero() { return T(0.0f); }
@@ -183,7 +184,7 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
 
   // Panels in order (SOLVE) with ceil(p0 / KC) chunks each, at least one step.
   // Multiplies take the panel's own columns into the chunks (K < p0 + PB).
-  const int npan = nr / PB;
+  const int npan = (n + PB - 1) / PB;
   auto kend_of = [&](int p) { return SOLVE ? p * PB : min((p + 1) * PB, n); };
   auto chunks_of = [&](int p) { const int ke = kend_of(p); return ke > KC ? (ke + KC - 1) / KC : 1; };
 
@@ -321,9 +322,12 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
                 const Tc xj = Mx::shfl(Mx::quotient(z[q], iv, dr), (lane & ~(PB - 1)) | j);
                 if (row > j) z[q] = Mx::fms_(d[j], xj, z[q]);
               }
+            if constexpr (std::is_floating_point<Tc>::value) {
 #pragma unroll
-            for (int q = 0; q < NC; ++q) z[q] = Mx::quotient(z[q], iv, dr);
-            if constexpr (!std::is_floating_point<Tc>::value) {
+              for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = Mx::quotient(z[q], iv, dr);
+            } else {
+#pragma unroll
+              for (int q = 0; q < NC; ++q) z[q] = Mx::quotient(z[q], iv, dr);
               // The chain's time is in its steps, so the test for results that
               // are not finite (a pivot without a finite reciprocal, a quotient
               // that overflows) comes once per panel; the divisions then give
@@ -339,16 +343,16 @@ __device__ __forceinline__ void strip_block(const LeafArgs& g, unsigned char* sm
                   const Tc dj = Db[row * (PB + 1) + j];
 #pragma unroll
                   for (int q = 0; q < NC; ++q) {
-                    const Tc xj = Mx::shfl(Mx::divided(z[q], dr), (lane & ~(PB - 1)) | j);
+                    const Tc xj = Mx::shfl(Mx::divided(z[q], iv, dr), (lane & ~(PB - 1)) | j);
                     if (row > j) z[q] = Mx::fms_(dj, xj, z[q]);
                   }
                 }
 #pragma unroll
-                for (int q = 0; q < NC; ++q) z[q] = Mx::divided(z[q], dr);
+                for (int q = 0; q < NC; ++q) z[q] = Mx::divided(z[q], iv, dr);
               }
-            }
 #pragma unroll
-            for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = z[q];
+              for (int q = 0; q < NC; ++q) X[(size_t)(col0 + q) * ldx + p0 + row] = z[q];
+            }
             if constexpr (KG == 1) __syncwarp();
           } else {
 #pragma unroll
