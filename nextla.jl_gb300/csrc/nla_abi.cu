@@ -7,6 +7,7 @@
 // (:129-133), with the forward (A11 -> GEMM -> A22) or backward ordering of
 // :153-197.  Each base case is one launch of the diagonal-block kernel and
 // each update one launch of the GEMM kernel, all on the caller's stream.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -181,13 +182,24 @@ static bool umma_enabled() {
 // chain they replace.  Relative error against 64 bits at K = 128, 1024, 8192:
 // normal data 2.0e-7, 5.7e-7, 1.6e-6 before, 7.5e-8, 1.0e-7, 2.2e-7 now;
 // values spread over 2^+-12 1.5e-7, 4.0e-7, 1.1e-6 / 1.2e-7, 1.4e-7, 2.3e-7.
-static bool f32_umma_wanted(int64_t N, int64_t M, int64_t K) {
-  return umma_enabled() && N >= 64 && M >= 64 && K >= 128 && (double)N * (double)M * (double)K >= 3e7;
+// A long operand meets too few products to pay for its staging when the other
+// is narrow and K short: 100000 x K x 64, K = 128, 256, 512: 83 / 127, 151 / 176,
+// 284 / 271 us, 64 x K x 20000 31 / 37, 49 / 50, 85 / 80.
+// Complex (sizes in real rows), whose op(A) is staged as four reals per
+// element: 40000 x 256 x 64 58 / 93, 40000 x 2048 x 64 449 / 473, 200000 x 128 x 128
+// 219 / 268, 200000 x 256 x 128 394 / 389, 2000 x 128 x 256 16 / 22, 512 x 128 x
+// 8000 44 / 40, 4000 x 128 x 2000 71 / 60.
+static bool f32_umma_wanted(int64_t N, int64_t M, int64_t K, bool cplx) {
+  const double work = (double)N * (double)M * (double)K;
+  if (!umma_enabled() || N < 64 || M < 64 || K < 128 || work < 3e7) return false;
+  if (!cplx) return std::min(N, M) >= 96 || std::max(N, M) <= 12288 || K >= 512;
+  return (M >= 96 || N <= 8192) && (K >= 256 || (M >= 256 && work >= 5e8));
 }
 
 size_t update_scratch_bytes(int dtype, int64_t N, int64_t M, int64_t K) {
-  if (dtype == NLA_C32) N *= 2, K *= 2;  // real rows
-  return (dtype == NLA_F32 || dtype == NLA_C32) && f32_umma_wanted(N, M, K) ? f32_update_bytes(N, M, K) : 0;
+  const bool cplx = dtype == NLA_C32;
+  if (cplx) N *= 2, K *= 2;  // real rows
+  return (dtype == NLA_F32 || cplx) && f32_umma_wanted(N, M, K, cplx) ? f32_update_bytes(N, M, K) : 0;
 }
 
 // Float16 updates large enough to fill 128 x 128 tiles run on the tensor
@@ -201,7 +213,10 @@ int launch_gemm(int dtype, int64_t N, int64_t M, int64_t K, double alpha, const 
     const bool cx = dtype == NLA_C32;
     const int64_t rows = cx ? 2 * N : N, k = cx ? 2 * K : K;
     if (ws && ws_bytes >= need) return launch_gemm_f32_umma(rows, M, k, alpha, A, B, C, ws, cx, s);
-    const Scratch own(s, need);
+    // A call of its own also allocates: 256 x 128 x 1000 18 / 22 us, 256 x 256 x 1000
+    // 24 / 22; ComplexF32 128 x 128 x 1000 22 / 25, 256 x 128 x 1000 24 / 23.
+    const bool pays = (double)rows * (double)M * (double)k >= (cx ? 1e8 : 5e7);
+    const Scratch own(s, pays ? need : 0);
     if (own.p) return launch_gemm_f32_umma(rows, M, k, alpha, A, B, C, own.p, cx, s);
   }
   if (is_complex(dtype)) return launch_gemm_complex(dtype, N, M, K, alpha, A, B, C, s);

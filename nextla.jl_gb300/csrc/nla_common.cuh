@@ -252,6 +252,7 @@ struct CrtStaged {
   bool row_operand;
 };
 bool crt_usable(int64_t M, int64_t N, int64_t K);
+bool crt_wanted(int64_t M, int64_t N, int64_t K);  // faster than slices
 size_t crt_staged_bytes(int64_t rows, int64_t K);
 size_t crt_planes_bytes(int64_t M, int64_t N);
 CrtStaged crt_layout(void* buf, int64_t rows, int64_t K, int tri, bool row_operand);

@@ -1199,7 +1199,7 @@ int mixed_plan(char side, char uplo, char trans, char func, int64_t n, int64_t m
   if (n <= c->threshold) return NLA_OK;
   const int64_t rows_c = side == 'L' ? big : m, cols_c = side == 'L' ? m : big;
   if (opts.split_terms == EXACT_SLICES && crt_enabled() && crt_usable(rows_c, cols_c, big) &&
-      workspace_get(s, crt_update_panels(rows_c, cols_c, big, s).bytes, &ws) == NLA_OK)
+      crt_wanted(rows_c, cols_c, big) && workspace_get(s, crt_update_panels(rows_c, cols_c, big, s).bytes, &ws) == NLA_OK)
     return NLA_OK;
   cudaGetLastError();
   clear_error();

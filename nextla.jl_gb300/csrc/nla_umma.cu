@@ -1727,7 +1727,7 @@ int launch_sliced_gemm(int64_t M, int64_t N, int64_t K, double alpha, const Mat&
     if (!bf16) return fail(NLA_ERR_ARG, "exact updates use BF16 slices");
     if (out_dtype != NLA_F64) return fail(NLA_ERR_DTYPE, "exact updates produce Float64");
     void* base = ws;
-    if (base == nullptr && crt_enabled() && crt_usable(M, N, K)) {
+    if (base == nullptr && crt_enabled() && crt_usable(M, N, K) && crt_wanted(M, N, K)) {
       const CrtPanels pan = crt_update_panels(M, N, K, s);
       if (workspace_get(s, pan.bytes, &base) == NLA_OK) {
         const int64_t dim = pan.cols ? N : M;
