@@ -1688,10 +1688,15 @@ int plan_create(nla_batch_plan* out, int dtype, char uplo, char trans, int64_t c
 
   // One CTA per group where the longest group is no longer than the share of
   // all of them that each of the CTAs the GPU holds would have: its nodes need
-  // no queue order then.  Fewer groups than CTAs leave some idle, which the
+  // no queue order then.  In Float64 two CTAs of an SM share its DFMA pipe, the
+  // queue balances that better, and one- and two-block groups gain nothing:
+  // whole groups there only from 1.75 times that share and three block rows on
+  // (queue against whole, us: 1500 systems of up to 1024 x 128 13040 / 17116, 2500
+  // of 700 x 64 7143 / 8574, of 700 x 8 2074 / 1959; 1500 of 64 x 32 203 / 233).
+  // Fewer groups than CTAs (SMs in Float64) leave some idle, which the
   // queue puts to use on a large group's updates; against that stand its nodes'
   // waits, so groups of few block rows go whole all the same, the more the
-  // nearer their number is to the CTAs' (fill).  Measured, whole against the
+  // nearer the number of long ones is to the CTAs' (fill).  Measured, whole against the
   // queue, 2 / 30 / 150 equal systems on 304 CTAs with 16 right-hand sides, us:
   // Float32 n = 400 113 against 122 / 133 / 162, 700 232 against 212 / 258 / 270,
   // 1024 423 against 289 / 400 / 420; Float64 n = 200 258 against 236 / 296 / 365,
@@ -1722,9 +1727,13 @@ int plan_create(nla_batch_plan* out, int dtype, char uplo, char trans, int64_t c
       return rc;
     }
     const int ctas = num_sms() * std::max(per_sm, 1);
-    const double fill = longest > 0 ? total / (ctas * longest) : 1.0;
-    const bool few = (int64_t)groups.size() <= ctas && rows <= (dtype == NLA_F64 ? 3 + 20 * fill : 6 + 50 * fill);
-    p->whole_groups = per_sm > 0 && groups.size() < (size_t)INT32_MAX / 2 && (longest <= total / ctas || few);
+    const bool f64 = dtype == NLA_F64;
+    int64_t near = 0;  // groups at least half as long as the longest
+    for (const double c : cost) near += 2 * c >= longest;
+    const double fill = (double)near / ctas;
+    const bool few = (int64_t)groups.size() <= (f64 ? num_sms() : ctas) && rows <= (f64 ? 1 + 32 * fill : 6 + 30 * fill);
+    const bool many = longest * (f64 ? 1.75 : 1.0) <= total / ctas && (!f64 || rows > 2);
+    p->whole_groups = per_sm > 0 && groups.size() < (size_t)INT32_MAX / 2 && (many || few);
     if (p->whole_groups) {  // longest first
       p->grid = std::max(1, std::min((int)groups.size(), ctas));
       std::vector<int> order(items.size());
