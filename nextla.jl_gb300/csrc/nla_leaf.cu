@@ -247,16 +247,19 @@ int64_t column_from(int64_t n) {
   constexpr bool CX = !std::is_floating_point<Tc>::value;
   constexpr bool F64 = sizeof(Tc) == (CX ? 16 : 8);
   const int64_t never = INT32_MAX;
-  if (CX && F64) return SOLVE ? (n <= 64 ? 14 + n : never) : n <= 48 ? 40 + n * 5 / 4 : never;
-  if (CX) return n > 48 ? never : SOLVE ? std::min<int64_t>(5 + 3 * n, 105) : std::min<int64_t>(35 + n * 3 / 2, 85);
+  if (CX && F64) return SOLVE ? (n <= 64 ? 14 + n : never) : n <= 56 ? 40 + n * 5 / 4 : never;
+  if (CX) return n > 56 ? never : SOLVE ? std::min<int64_t>(5 + 3 * n, 105) : std::min<int64_t>(35 + n * 3 / 2, 85);
   if (F64) return SOLVE ? (n <= 64 ? 22 + n * 15 / 16 : never) : n <= 32 ? 30 + 3 * n : never;
-  return n > 48 ? never : SOLVE ? 45 + n * 3 / 2 : 75 + n * 9 / 8;
+  return n > 56 ? never : SOLVE ? 45 + n * 3 / 2 : 75 + n * 9 / 8;
 }
 
 // Right-hand sides per CTA: the width with the least ceil(CTAs / SMs) *
 // (width + c), where c is a strip's fixed time (the triangles' chains and
 // the staging of A) in columns' worth of its product: about one column in
 // Float64, whose product is bound by the DFMA pipe, and about 32 in Float32.
+// Float64 solves of 4 and 2 columns count as 6 and 5, for their 32-row
+// triangles (n = 128, m = 3000: 4, 8 and 16 columns 139, 117 and 112 us, n = 64
+// in ComplexF64 271, 189 and 209).
 // Float64 takes 16-row panels from 8 columns on (32-row triangles cost the
 // DFMA pipe more than the steps they save), Float32 always 32-row panels.
 // Measured against one warp-group CTA per 16 or 32 columns with 32-row
@@ -284,7 +287,8 @@ int launch_strips(const LeafArgs& g, cudaStream_t s) {
   for (int w : {64, 32, 16, 8, 4, 2}) {
     if (w > WIDEST) continue;
     if (strip_smem_elems<Tc>(g.n, 32, w < 8 ? 1 : w / 8, w < 8 ? w : 8, w < 32 ? 8 : NWW) * sizeof(Tc) > STRIP_SMEM_MAX && w > 2) continue;
-    const int64_t grid = (g.m + w - 1) / w, k = (grid + sms - 1) / sms * (w + c);
+    const int eff = F64 && SOLVE && w < 8 ? w / 2 + 4 : w;
+    const int64_t grid = (g.m + w - 1) / w, k = (grid + sms - 1) / sms * (eff + c);
     if (best == 0 || k < cost) best = w, cost = k;
   }
   switch (best) {
