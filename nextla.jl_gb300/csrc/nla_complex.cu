@@ -139,7 +139,9 @@ int launch_gemm_complex(int dtype, int64_t N, int64_t M, int64_t K, double alpha
   const dim3 grid((unsigned)gx, (unsigned)gy);
   auto run = [&](auto kernel, auto one) {
     using R = decltype(one);
-    kernel<<<grid, 256, 0, s>>>(N, M, K, (R)alpha, static_cast<const cx::cpx<R>*>(A.p), A.ld, A.t, A.c, static_cast<const cx::cpx<R>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<R>*>(C.p), C.ld);
+    kernel<<<grid, 256, 0, s>>>(N, M, K, (R)alpha, static_cast<const cx::cpx<R>*>(A.p), A.ld, A.t, A.c,
+                                static_cast<const cx::cpx<R>*>(B.p), B.ld, B.t, B.c, static_cast<cx::cpx<R>*>(C.p),
+                                C.ld);
   };
   if (dtype == NLA_C64) gt == 64 ? run(cx::cplx_gemm_kernel<double, 64>, 1.0) : run(cx::cplx_gemm_kernel<double, 32>, 1.0);
   else gt == 64 ? run(cx::cplx_gemm_kernel<float, 64>, 1.0f) : run(cx::cplx_gemm_kernel<float, 32>, 1.0f);

@@ -696,9 +696,8 @@ __device__ __forceinline__ void two_sum(double a, double b, double& s, double& e
   e = (a - (s - bp)) + (b - bp);
 }
 
-constexpr int FIN_COLS = 1;      // columns per warp
 constexpr int FIN_PITCH = 36;    // four rows of 32 lanes, staggered over the banks
-// A warp takes 128 rows of one column at a time: each lane reads 4 rows'
+// A warp takes 128 rows of one column: each lane reads 4 rows'
 // bytes of every plane as one word, forms their integers, and the results
 // pass through shared memory so that C is read and written along its rows.
 __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) {
@@ -713,103 +712,99 @@ __global__ void __launch_bounds__(256, 4) crt_finish_kernel(const FinishArgs p) 
     er[r] = ib + r < p.M ? p.ea[ib + r] : 0;
     if (er[r] != NONFINITE_EXP) er[r] = max(er[r], -4000) + p.e_bias;
   }
-#pragma unroll 1
-  for (int cc = 0; cc < FIN_COLS; ++cc) {
-    const int64_t col = ((int64_t)blockIdx.y * 8 + warp) * FIN_COLS + cc;
-    if (col >= p.N) break;
-    uint32_t w[L];
+  const int64_t col = (int64_t)blockIdx.y * 8 + warp;
+  if (col >= p.N) return;
+  uint32_t w[L];
 #pragma unroll
-    for (int l = 0; l < L; ++l)
-      w[l] = *reinterpret_cast<const uint32_t*>(p.planes + l * p.plane + ib + col * p.ldp) ^ 0x80808080u;
-    double cv[4];
+  for (int l = 0; l < L; ++l)
+    w[l] = *reinterpret_cast<const uint32_t*>(p.planes + l * p.plane + ib + col * p.ldp) ^ 0x80808080u;
+  double cv[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int i = i0 + lane + 32 * r;
-      cv[r] = i < p.M ? p.C[i + col * p.ldc] : 0.0;
+  for (int r = 0; r < 4; ++r) {
+    const int i = i0 + lane + 32 * r;
+    cv[r] = i < p.M ? p.C[i + col * p.ldc] : 0.0;
+  }
+  int ejc = p.eb[col];
+  if (ejc != NONFINITE_EXP) ejc = max(ejc, -4000);
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    // x = sum_l y_l (P / p_l) - round(sum_l y_l / p_l) P, |x| < 0.45 P.
+    // The leading limb needs only its value modulo 2^32.
+    unsigned long long a0 = c_t.m0[0], a1 = c_t.m0[1], a2 = c_t.m0[2], qs = c_t.q0;
+    uint32_t a3 = (uint32_t)c_t.m0[3];
+#pragma unroll
+    for (int g = 0; g < GROUPS; ++g) {
+      uint32_t sg = 0;
+#pragma unroll
+      for (int l = 3 * g; l < 3 * g + 3 && l < L; ++l) sg += __byte_perm(w[l], 0, 0x4440 + r) * c_t.in[l];
+      if (g + 1 < GROUPS) qs += (unsigned long long)sg * c_t.q[g];
+      else qs += (unsigned long long)(sg * c_t.q[g]) << 23;
+      a0 += (unsigned long long)sg * c_t.m[g][0];
+      a1 += (unsigned long long)sg * c_t.m[g][1];
+      a2 += (unsigned long long)sg * c_t.m[g][2];
+      a3 += sg * c_t.m[g][3];
     }
-    int ejc = p.eb[col];
-    if (ejc != NONFINITE_EXP) ejc = max(ejc, -4000);
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      // x = sum_l y_l (P / p_l) - round(sum_l y_l / p_l) P, |x| < 0.45 P.
-      // The leading limb needs only its value modulo 2^32.
-      unsigned long long a0 = c_t.m0[0], a1 = c_t.m0[1], a2 = c_t.m0[2], qs = c_t.q0;
-      uint32_t a3 = (uint32_t)c_t.m0[3];
-#pragma unroll
-      for (int g = 0; g < GROUPS; ++g) {
-        uint32_t sg = 0;
-#pragma unroll
-        for (int l = 3 * g; l < 3 * g + 3 && l < L; ++l) sg += __byte_perm(w[l], 0, 0x4440 + r) * c_t.in[l];
-        if (g + 1 < GROUPS) qs += (unsigned long long)sg * c_t.q[g];
-        else qs += (unsigned long long)(sg * c_t.q[g]) << 23;
-        a0 += (unsigned long long)sg * c_t.m[g][0];
-        a1 += (unsigned long long)sg * c_t.m[g][1];
-        a2 += (unsigned long long)sg * c_t.m[g][2];
-        a3 += sg * c_t.m[g][3];
-      }
-      const uint32_t nq = 2 * QB - (uint32_t)(qs >> 54);  // 2 QB - (quotient + QB)
-      a0 += (unsigned long long)nq * c_t.P[0];
-      a1 += (unsigned long long)nq * c_t.P[1] + (a0 >> 32);
-      a2 += (unsigned long long)nq * c_t.P[2] + (a1 >> 32);
-      a3 += nq * c_t.P[3] + (uint32_t)(a2 >> 32);
-      uint32_t u0 = (uint32_t)a0, u1 = (uint32_t)a1, u2 = (uint32_t)a2, u3 = a3;
-      const uint32_t sign = (uint32_t)((int)u3 >> 31);
-      {
-        // |x|
-        const unsigned long long lo = (((unsigned long long)(u1 ^ sign) << 32) | (u0 ^ sign)) + (sign & 1u);
-        const unsigned long long hi =
-            (((unsigned long long)(u3 ^ sign) << 32) | (u2 ^ sign)) + ((sign & 1u) && lo == 0 ? 1ull : 0ull);
-        u0 = (uint32_t)lo;
-        u1 = (uint32_t)(lo >> 32);
-        u2 = (uint32_t)hi;
-        u3 = (uint32_t)(hi >> 32);
-      }
-      const int e = er[r] + ejc;
-      const bool bad = er[r] == NONFINITE_EXP || ejc == NONFINITE_EXP;
-      double v;
-      Wide x{};
-      unsigned long long m = 0;
-      int k = 0;
-      if (p.res_x == nullptr) {
-        v = round_wide(u3, u2, u1, u0, sign, e);
-      } else {
-        x.hi = ((unsigned long long)u3 << 32) | u2;
-        x.lo = ((unsigned long long)u1 << 32) | u0;
-        x.neg = sign != 0;
-        m = leading53(x, k);
-        v = to_f64(m, k + e, x.neg);
-      }
-      if (bad) v = __longlong_as_double(0x7ff8000000000000ll);
-      if (p.res_x != nullptr && ib + r < p.M) {
-        // The rest of the exact product below its leading 53 bits.
-        unsigned __int128 u = ((unsigned __int128)x.hi << 64) | x.lo;
-        const unsigned __int128 head = k >= 0 ? (unsigned __int128)m << k : (unsigned __int128)m >> -k;
-        const __int128 rest = (__int128)(u - head);
-        const unsigned __int128 ra = rest < 0 ? (unsigned __int128)-rest : (unsigned __int128)rest;
-        const Wide rw{(unsigned long long)(ra >> 64), (unsigned long long)ra, (rest < 0) != x.neg};
-        int k2;
-        const unsigned long long m2 = leading53(rw, k2);
-        const double lo = to_f64(m2, k2 + e, rw.neg);
-        const int64_t at = ib + r + col * p.res_ldx;
-        const double dg = p.res_d[(p.d_col ? col : (int64_t)(ib + r)) * p.res_dstride];
-        const double xv = p.res_x[at];
-        const double c = p.C[ib + r + col * p.ldc];
-        const double pr = dg * xv, pe = fma(dg, xv, -pr);
-        double t1, e1, t2, e2;
-        two_sum(c, -v, t1, e1);
-        two_sum(t1, -pr, t2, e2);
-        if (!bad) v = t2 + (((e1 + e2) - pe) - lo);
-      }
-      buf[warp][r * FIN_PITCH + lane] = v;
+    const uint32_t nq = 2 * QB - (uint32_t)(qs >> 54);  // 2 QB - (quotient + QB)
+    a0 += (unsigned long long)nq * c_t.P[0];
+    a1 += (unsigned long long)nq * c_t.P[1] + (a0 >> 32);
+    a2 += (unsigned long long)nq * c_t.P[2] + (a1 >> 32);
+    a3 += nq * c_t.P[3] + (uint32_t)(a2 >> 32);
+    uint32_t u0 = (uint32_t)a0, u1 = (uint32_t)a1, u2 = (uint32_t)a2, u3 = a3;
+    const uint32_t sign = (uint32_t)((int)u3 >> 31);
+    {
+      // |x|
+      const unsigned long long lo = (((unsigned long long)(u1 ^ sign) << 32) | (u0 ^ sign)) + (sign & 1u);
+      const unsigned long long hi =
+          (((unsigned long long)(u3 ^ sign) << 32) | (u2 ^ sign)) + ((sign & 1u) && lo == 0 ? 1ull : 0ull);
+      u0 = (uint32_t)lo;
+      u1 = (uint32_t)(lo >> 32);
+      u2 = (uint32_t)hi;
+      u3 = (uint32_t)(hi >> 32);
     }
-    __syncwarp();
-#pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const int ri = lane + 32 * r;
-      const double v = buf[warp][(ri & 3) * FIN_PITCH + (ri >> 2)];
-      if (i0 + ri < p.M) p.C[i0 + ri + col * p.ldc] = p.res_x != nullptr ? v : fma(p.alpha, v, cv[r]);
+    const int e = er[r] + ejc;
+    const bool bad = er[r] == NONFINITE_EXP || ejc == NONFINITE_EXP;
+    double v;
+    Wide x{};
+    unsigned long long m = 0;
+    int k = 0;
+    if (p.res_x == nullptr) {
+      v = round_wide(u3, u2, u1, u0, sign, e);
+    } else {
+      x.hi = ((unsigned long long)u3 << 32) | u2;
+      x.lo = ((unsigned long long)u1 << 32) | u0;
+      x.neg = sign != 0;
+      m = leading53(x, k);
+      v = to_f64(m, k + e, x.neg);
     }
-    __syncwarp();
+    if (bad) v = __longlong_as_double(0x7ff8000000000000ll);
+    if (p.res_x != nullptr && ib + r < p.M) {
+      // The rest of the exact product below its leading 53 bits.
+      unsigned __int128 u = ((unsigned __int128)x.hi << 64) | x.lo;
+      const unsigned __int128 head = k >= 0 ? (unsigned __int128)m << k : (unsigned __int128)m >> -k;
+      const __int128 rest = (__int128)(u - head);
+      const unsigned __int128 ra = rest < 0 ? (unsigned __int128)-rest : (unsigned __int128)rest;
+      const Wide rw{(unsigned long long)(ra >> 64), (unsigned long long)ra, (rest < 0) != x.neg};
+      int k2;
+      const unsigned long long m2 = leading53(rw, k2);
+      const double lo = to_f64(m2, k2 + e, rw.neg);
+      const int64_t at = ib + r + col * p.res_ldx;
+      const double dg = p.res_d[(p.d_col ? col : (int64_t)(ib + r)) * p.res_dstride];
+      const double xv = p.res_x[at];
+      const double c = p.C[ib + r + col * p.ldc];
+      const double pr = dg * xv, pe = fma(dg, xv, -pr);
+      double t1, e1, t2, e2;
+      two_sum(c, -v, t1, e1);
+      two_sum(t1, -pr, t2, e2);
+      if (!bad) v = t2 + (((e1 + e2) - pe) - lo);
+    }
+    buf[warp][r * FIN_PITCH + lane] = v;
+  }
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const int ri = lane + 32 * r;
+    const double v = buf[warp][(ri & 3) * FIN_PITCH + (ri >> 2)];
+    if (i0 + ri < p.M) p.C[i0 + ri + col * p.ldc] = p.res_x != nullptr ? v : fma(p.alpha, v, cv[r]);
   }
 }
 
@@ -849,7 +844,7 @@ bool crt_wanted(int64_t M, int64_t N, int64_t K) {
 // Sizes that the residues' integers, grids and maps hold.
 bool crt_usable(int64_t M, int64_t N, int64_t K) {
   return K <= MAX_K && M <= (1 << 24) && N <= (1 << 24) && L * pad_to(M, BU) < INT32_MAX && L * pad_to(N, BU) < INT32_MAX &&
-         pad_to(M, BU) / BU * (pad_to(N, BU) / BU) * L < INT32_MAX && N <= (int64_t)65535 * 8 * FIN_COLS;
+         pad_to(M, BU) / BU * (pad_to(N, BU) / BU) * L < INT32_MAX && N <= (int64_t)65535 * 8;
 }
 
 size_t crt_staged_bytes(int64_t rows, int64_t K) {
@@ -984,7 +979,7 @@ int crt_gemm(const CrtStaged& A, const CrtStaged& B, double alpha, const Mat& C,
     f.res_dstride = res->dstride;
     f.d_col = d_col ? 1 : 0;
   }
-  const dim3 grid((unsigned)(A.rows_pad / 128), (unsigned)((g.N + 8 * FIN_COLS - 1) / (8 * FIN_COLS)));
+  const dim3 grid((unsigned)(A.rows_pad / 128), (unsigned)((g.N + 7) / 8));
   launch_chained(crt_finish_kernel, grid, 256, 0, s, f);
   NLA_CHECK_LAUNCH("crt_finish_kernel");
   trace_kernels(1);

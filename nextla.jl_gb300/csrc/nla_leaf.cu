@@ -270,7 +270,7 @@ int64_t column_from(int64_t n) {
 // DFMA pipe more than the steps they save), Float32 always 32-row panels.
 // Measured against one warp-group CTA per 16 or 32 columns with 32-row
 // panels solved by one warp: Float64 96 x 24 97 -> 13 us, 256 x 256 560 ->
-// 42 us; Float32 256 x 8192 110 -> 44 us; Float16 256 x 4096 98 -> 32 us;
+// 54 us; Float32 256 x 8192 110 -> 44 us; Float16 256 x 4096 98 -> 32 us;
 // Float64 multiply 64 x 6144 115 -> 36 us.
 template <typename T, bool SOLVE>
 int launch_strips(const LeafArgs& g, cudaStream_t s) {

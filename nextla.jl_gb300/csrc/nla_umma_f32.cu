@@ -49,7 +49,6 @@ constexpr int BM = 128, BN = 128, BK = 64;
 constexpr int TILE_BYTES = BM * BK * 2;
 constexpr int SL = 3;
 constexpr int F32_THREADS = 352;
-constexpr int F32_CHUNK = 1;  // K blocks of 64 per drained chunk
 // Tiles of 128 rows and TN (128, 64 or 32) columns: two or three stages.
 constexpr int f32_stages(int TN) { return TN == 128 ? 2 : 3; }
 constexpr int f32_stage_bytes(int TN) { return SL * (BM + TN) * BK * 2; }
@@ -264,9 +263,8 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
     if (lane == 0) {
       const uint32_t id1 = umma::idesc_f16(BM, TN, true), id2 = umma::idesc_f16(BM, 2 * TN, true);
       for (int kb = 0; kb < p.num_kb; ++kb) {
-        const int s = kb % F32_STAGES, ch = kb / F32_CHUNK, b = ch & 1;
-        const bool first = kb % F32_CHUNK == 0;
-        if ((first && !umma::mbar_wait(umma::smem_u32(&cempty[b]), ((uint32_t)(ch >> 1) & 1u) ^ 1u, &s_abort, p.err, 53)) ||
+        const int s = kb % F32_STAGES, b = kb & 1;
+        if (!umma::mbar_wait(umma::smem_u32(&cempty[b]), ((uint32_t)(kb >> 1) & 1u) ^ 1u, &s_abort, p.err, 53) ||
             !umma::mbar_wait(umma::smem_u32(&fullA[s]), (uint32_t)(kb / F32_STAGES) & 1u, &s_abort, p.err, 54) ||
             !umma::mbar_wait(umma::smem_u32(&fullB[s]), (uint32_t)(kb / F32_STAGES) & 1u, &s_abort, p.err, 54))
           break;
@@ -278,7 +276,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 #pragma unroll
         for (int kk = 0; kk < BK / 16; ++kk)
           umma::mma_f16(d0, umma::desc_kmajor_sw128(a0 + kk * 32), umma::desc_kmajor_sw128(b0 + kk * 32), id2,
-                        first && kk == 0 ? 0u : 1u);
+                        kk == 0 ? 0u : 1u);
         constexpr int qa[4] = {1, 1, 0, 2}, qb[4] = {0, 1, 2, 0};  // m h, m m, h l, l h
 #pragma unroll
         for (int pr = 0; pr < 4; ++pr)
@@ -287,7 +285,7 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
             umma::mma_f16(d1, umma::desc_kmajor_sw128(a0 + qa[pr] * TILE_BYTES + kk * 32),
                           umma::desc_kmajor_sw128(b0 + qb[pr] * B_BYTES + kk * 32), id1, 1u);
         umma::mma_commit(umma::smem_u32(&empty[s]));
-        if (kb % F32_CHUNK == F32_CHUNK - 1 || kb == p.num_kb - 1) umma::mma_commit(umma::smem_u32(&cfull[b]));
+        umma::mma_commit(umma::smem_u32(&cfull[b]));
       }
       umma::mma_commit(umma::smem_u32(drain));
       umma::mbar_wait(umma::smem_u32(drain), 0, &s_abort, p.err, 55, false);
@@ -331,10 +329,9 @@ __global__ void __launch_bounds__(F32_THREADS, 1)
 #pragma unroll
     for (int j = 0; j < HALF; ++j) acc[j] = 0.0f;
     bool ok = !looked || s_tensor;
-    const int nch = (p.num_kb + F32_CHUNK - 1) / F32_CHUNK;
-    for (int ch = 0; ch < nch && ok; ++ch) {
-      const int b = ch & 1;
-      ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&cfull[b]), (uint32_t)(ch >> 1) & 1u, &s_abort, p.err, 56));
+    for (int kb = 0; kb < p.num_kb && ok; ++kb) {
+      const int b = kb & 1;
+      ok = __all_sync(0xffffffffu, umma::mbar_wait(umma::smem_u32(&cfull[b]), (uint32_t)(kb >> 1) & 1u, &s_abort, p.err, 56));
       if (!ok) break;
       umma::fence_after_sync();
       const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * 2 * TN + h * HALF);
@@ -546,8 +543,8 @@ int launch_gemm_f32_umma(int64_t M, int64_t N, int64_t K, double alpha, const Ma
   if (st != cudaSuccess) return cuda_status(st, "cudaFuncSetAttribute(umma_f32_kernel)");
   TraceScope trace(NLA_K_GEMM_UMMA, s, 6.0 * 2.0 * (double)M * (double)N * (double)K,
                    (double)SL * 2.0 * (double)(Mp + Np) * Kp + 8.0 * (double)M * (double)N);
-  launch_chained(tn == 128 ? umma_f32_kernel<128> : tn == 64 ? umma_f32_kernel<64> : umma_f32_kernel<32>, (unsigned)((int64_t)p.tiles_m * p.tiles_n),
-                 F32_THREADS, f32_smem(tn), s, mA, mB, p);
+  launch_chained(tn == 128 ? umma_f32_kernel<128> : tn == 64 ? umma_f32_kernel<64> : umma_f32_kernel<32>,
+                 (unsigned)((int64_t)p.tiles_m * p.tiles_n), F32_THREADS, f32_smem(tn), s, mA, mB, p);
   NLA_CHECK_LAUNCH("umma_f32_kernel");
   return NLA_OK;
 }
