@@ -362,7 +362,7 @@ int launch_leaf(char func, char side, char uplo, int dtype, int64_t n, int64_t m
     // per right-hand side and 64 to a CTA takes the last two (168 and 480).
     // (NLA_LEAF_COLS=0 turns it off, NLA_LEAF_CW pins a width from m = 1024.)
     const int64_t sms = num_sms(), wave = 128 * sms, waves = (m + wave - 1) / wave;
-    const bool pinned = getenv("NLA_LEAF_CW") != nullptr && m >= 8 * LEAF_THREADS;
+    const bool pinned = m >= 8 * LEAF_THREADS && getenv("NLA_LEAF_CW") != nullptr;
     const bool full = waves == 1 ? n > 48 && m > 68 * sms : n > 112 && 4 * m > 3 * wave * waves;
     if (dtype == NLA_F64 && n <= COLS_MAX_N && (full || pinned) && leaf_cols_mode() != 0)
       return leaf_cols_mode() == 1 ? launch_leaf_cols<1, LEAF_THREADS>(g, s) : launch_leaf_cols2(g, s);
