@@ -246,11 +246,16 @@ __global__ void __launch_bounds__(256) leaf_inverse_kernel(const __grid_constant
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const int i = 4 * u + q;
-      if (rg == q) y[u] *= dinv[i];
+      // Columns of the warp that begin below row i take nothing from it: their
+      // zeros times an infinite reciprocal or a NaN of T would be NaN.
+      const bool in = i >= j;
+      if (rg == q && in) y[u] *= dinv[i];
       const double x = __shfl_sync(0xffffffffu, y[u], base + q);
-      if (rg > q) y[u] -= T[i - q + rg][i] * x;
+      if (in) {
+        if (rg > q) y[u] -= T[i - q + rg][i] * x;
 #pragma unroll
-      for (int v = u + 1; v < LEAF_INV_N / 4; ++v) y[v] -= T[rg + 4 * v][i] * x;
+        for (int v = u + 1; v < LEAF_INV_N / 4; ++v) y[v] -= T[rg + 4 * v][i] * x;
+      }
     }
   }
   double* W = g.W + (int64_t)(g.first_slot + b) * LEAF_INV_N * LEAF_INV_N;
